@@ -266,10 +266,9 @@ uint32_t nvfp4_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uin
 bool gemm_tc_supported(const GemmProblem& p);
 
 // ---- NVFP4 ----------------------------------------------------------------------
-cudaError_t launch_nvfp4_gather_quantize(const __nv_bfloat16* hidden, const int32_t* route_prows,
-                                         uint32_t routes, uint32_t top_k, uint32_t hidden_size,
-                                         float global_scale, uint8_t* packed, uint8_t* scale_tiled,
-                                         cudaStream_t stream);
+// Token rows in token order -> e2m1 codes and scales tiled by token row.
+cudaError_t launch_nvfp4_quantize_rows(const __nv_bfloat16* x, uint32_t rows, uint32_t k, float global_scale,
+                                       uint8_t* packed, uint8_t* scale_tiled, cudaStream_t stream);
 // Gather of already-quantised token rows into the padded permuted layout of sorted routing tables.
 // 128-row tiles: organised by destination tile (coalesced code rows, whole scale tiles; rows past a
 // tile's last row keep stale codes and get zero scales); smaller tiles: launch_nvfp4_gather_packed.

@@ -74,29 +74,30 @@ fp8_gather_quantize_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* _
         scales[static_cast<size_t>(prow) * groups + g] = s;
 }
 
-// One block per (k block, row block, expert): 128 x 128 weights -> codes + one scale.
+// One block per (k block, row block, expert): 128 x 128 weights -> codes + one scale. Sixteen lanes read the
+// 256 bytes of a row together, so a load or store instruction touches whole sectors. Bound by HBM: 2 bytes in,
+// 1 byte out per weight.
 __global__ void __launch_bounds__(256)
 fp8_quantize_weight_kernel(const __nv_bfloat16* __restrict__ w, uint32_t rows, uint32_t k,
                            uint8_t* __restrict__ codes, float* __restrict__ scales)
 {
     __shared__ float s_part[8];
     const uint32_t kb = blockIdx.x, rb = blockIdx.y, e = blockIdx.z;
-    const uint32_t r = rb * 128 + threadIdx.x / 2;
-    const uint32_t c0 = kb * 128 + (threadIdx.x % 2) * 64;
-    const bool live = r < rows;
-    const size_t off = (static_cast<size_t>(e) * rows + r) * k + c0;
+    const uint32_t r0 = rb * 128 + threadIdx.x / 16; // rows r0, r0 + 16, ...
+    const uint32_t c0 = kb * 128 + (threadIdx.x % 16) * 8;
+    const size_t base = (static_cast<size_t>(e) * rows + r0) * k + c0;
     uint4 v[8];
     float amax = 0.0f;
-    if (live) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            v[i] = reinterpret_cast<const uint4*>(w + off)[i];
-            const uint32_t ws[4] = { v[i].x, v[i].y, v[i].z, v[i].w };
+    for (uint32_t i = 0; i < 8; ++i)
+        v[i] = r0 + 16 * i < rows ? *reinterpret_cast<const uint4*>(w + base + static_cast<size_t>(16 * i) * k)
+                                  : make_uint4(0, 0, 0, 0);
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                amax = fmaxf(amax, fmaxf(fabsf(bf16_bits_to_f32(ws[j] & 0xffffu)),
-                                         fabsf(bf16_bits_to_f32(ws[j] >> 16))));
-        }
+    for (uint32_t i = 0; i < 8; ++i) {
+        const uint32_t ws[4] = { v[i].x, v[i].y, v[i].z, v[i].w };
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            amax = fmaxf(amax, fmaxf(fabsf(bf16_bits_to_f32(ws[j] & 0xffffu)), fabsf(bf16_bits_to_f32(ws[j] >> 16))));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
@@ -110,21 +111,15 @@ fp8_quantize_weight_kernel(const __nv_bfloat16* __restrict__ w, uint32_t rows, u
         amax = fmaxf(amax, s_part[i]);
     const float s = fp8_scale_of(amax);
     const float inv = __fdiv_rn(1.0f, s);
-    if (live) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            uint32_t o[4];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint4 q = v[2 * i + h];
-                const float f[8] = { bf16_bits_to_f32(q.x & 0xffffu), bf16_bits_to_f32(q.x >> 16),
-                                     bf16_bits_to_f32(q.y & 0xffffu), bf16_bits_to_f32(q.y >> 16),
-                                     bf16_bits_to_f32(q.z & 0xffffu), bf16_bits_to_f32(q.z >> 16),
-                                     bf16_bits_to_f32(q.w & 0xffffu), bf16_bits_to_f32(q.w >> 16) };
-                o[2 * h] = pack_e4m3x4(f, inv);
-                o[2 * h + 1] = pack_e4m3x4(f + 4, inv);
-            }
-            reinterpret_cast<uint4*>(codes + off)[i] = make_uint4(o[0], o[1], o[2], o[3]);
+    for (uint32_t i = 0; i < 8; ++i) {
+        if (r0 + 16 * i < rows) {
+            const float f[8] = { bf16_bits_to_f32(v[i].x & 0xffffu), bf16_bits_to_f32(v[i].x >> 16),
+                                 bf16_bits_to_f32(v[i].y & 0xffffu), bf16_bits_to_f32(v[i].y >> 16),
+                                 bf16_bits_to_f32(v[i].z & 0xffffu), bf16_bits_to_f32(v[i].z >> 16),
+                                 bf16_bits_to_f32(v[i].w & 0xffffu), bf16_bits_to_f32(v[i].w >> 16) };
+            *reinterpret_cast<uint2*>(codes + base + static_cast<size_t>(16 * i) * k)
+                = make_uint2(pack_e4m3x4(f, inv), pack_e4m3x4(f + 4, inv));
         }
     }
     if (threadIdx.x == 0)

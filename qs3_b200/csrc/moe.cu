@@ -1184,8 +1184,8 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
         if (ferr == cudaSuccess)
             ferr = cudaStreamWaitEvent(side, plan->ev_fork, 0);
         if (ferr == cudaSuccess && !prequant)
-            ferr = launch_nvfp4_gather_quantize(hidden, nullptr, d->num_tokens, 1, p.hidden_size,
-                                                d->act_global_scale, x.sh_xq, x.sh_xq_sf, side);
+            ferr = launch_nvfp4_quantize_rows(hidden, d->num_tokens, p.hidden_size, d->act_global_scale, x.sh_xq,
+                                              x.sh_xq_sf, side);
         if (ferr == cudaSuccess)
             ferr = cudaEventRecord(plan->ev_quant, side);
         if (ferr != cudaSuccess)
@@ -1261,8 +1261,8 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
         if (fork)
             err = cudaStreamWaitEvent(st, plan->ev_quant, 0);
         else if (!prequant)
-            err = launch_nvfp4_gather_quantize(hidden, nullptr, d->num_tokens, 1, p.hidden_size,
-                                               d->act_global_scale, x.sh_xq, x.sh_xq_sf, st);
+            err = launch_nvfp4_quantize_rows(hidden, d->num_tokens, p.hidden_size, d->act_global_scale, x.sh_xq,
+                                             x.sh_xq_sf, st);
         if (err == cudaSuccess)
             err = launch_nvfp4_gather_tiles(x.sh_xq, x.sh_xq_sf, rt, routes, p.top_k, p.hidden_size, wn.xq, wn.xq_sf,
                                             st, 1);
@@ -1688,8 +1688,8 @@ qsfi_status qs3_moe_ep_finish(qsfi_context* ctx, const qsfi_moe_plan* plan, cons
     const __nv_bfloat16* hidden = static_cast<const __nv_bfloat16*>(d->hidden.data);
 
     if ((d->phases & 1u) != 0 && shared) {
-        cudaError_t err = launch_nvfp4_gather_quantize(hidden, nullptr, d->num_tokens, 1, p.hidden_size,
-                                                       d->act_global_scale, x.sh_xq, x.sh_xq_sf, st);
+        cudaError_t err = launch_nvfp4_quantize_rows(hidden, d->num_tokens, p.hidden_size, d->act_global_scale,
+                                                     x.sh_xq, x.sh_xq_sf, st);
         if (err != cudaSuccess)
             return set_cuda_error(ctx, err, "NVFP4 shared expert quantise");
         const float ga = d->act_global_scale == 0.0f ? 1.0f : d->act_global_scale;

@@ -5,6 +5,7 @@
 //   code  = e2m1_rn_sat(x * (1 / (f32(scale) * g)))      (0 when scale == 0)
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
@@ -41,14 +42,10 @@ __device__ __forceinline__ uint32_t pack_e2m1x8(const float* v)
     return r;
 }
 
-// Quantise one block of 16 values held by one thread. Returns the scale code and
-// writes the 16 codes as two 32-bit words.
-__device__ __forceinline__ uint8_t quantize_block16(const float* x, float g, uint32_t* lo, uint32_t* hi)
+// Quantise one block of 16 values with the given largest magnitude, held by one thread. Returns the scale
+// code and writes the 16 codes as two 32-bit words.
+__device__ __forceinline__ uint8_t quantize_block16(const float* x, float amax, float g, uint32_t* lo, uint32_t* hi)
 {
-    float amax = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-        amax = fmaxf(amax, fabsf(x[i]));
     // (x / 1 and 1 / s are spelled so that they cost less; both are the same correctly rounded values)
     const float sixth = __fdiv_rn(amax, 6.0f);
     const uint8_t code = f32_to_e4m3_sat(g == 1.0f ? sixth : __fdiv_rn(sixth, g));
@@ -61,6 +58,29 @@ __device__ __forceinline__ uint8_t quantize_block16(const float* x, float g, uin
     *lo = pack_e2m1x8(q);
     *hi = pack_e2m1x8(q + 8);
     return code;
+}
+
+__device__ __forceinline__ uint8_t quantize_block16(const float* x, float g, uint32_t* lo, uint32_t* hi)
+{
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+        amax = fmaxf(amax, fabsf(x[i]));
+    return quantize_block16(x, amax, g, lo, hi);
+}
+
+// Largest magnitude of bf16 pairs, two elements per instruction (exact: a maximum rounds nothing).
+__device__ __forceinline__ __nv_bfloat162 bf16x2_amax(__nv_bfloat162 m, const uint4& v)
+{
+    const uint32_t w[4] = { v.x, v.y, v.z, v.w };
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w[j])));
+    return m;
+}
+__device__ __forceinline__ float bf16x2_max(__nv_bfloat162 m)
+{
+    return fmaxf(__low2float(m), __high2float(m));
 }
 
 // Byte offset of scale (row, kb) in the tiled layout (see include/qs3_moe.h).

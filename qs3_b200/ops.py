@@ -347,7 +347,7 @@ def nvfp4_quantize_weight(ctx: Context, weight: torch.Tensor, gated: bool, linea
     dev = weight.device
     packed = torch.empty((e, rows, k // 2), dtype=torch.uint8, device=dev)
     sl = torch.empty((e, rows, k // 16), dtype=torch.uint8, device=dev) if linear else None
-    st = torch.zeros(e * nvfp4_tiled_scale_bytes(rows, k), dtype=torch.uint8, device=dev)
+    st = torch.empty(e * nvfp4_tiled_scale_bytes(rows, k), dtype=torch.uint8, device=dev)  # written whole
     g = torch.empty(e, dtype=torch.float32, device=dev)
     d = capi.Nvfp4QuantizeWeightDesc()
     d.weight = _desc(weight, 3)

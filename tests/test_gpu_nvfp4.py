@@ -52,6 +52,20 @@ def test_weight_quantiser_and_scale_tiling_are_bit_exact(ops, ctx, oracle, gated
     assert np.array_equal(to_np(ops.nvfp4_tile_scales(ctx, q.scale_linear, gated)), st_ref)
 
 
+# one block, a k that is no multiple of the 512-element unit, a last row block that is not full, more experts
+# than clusters run at a time
+@pytest.mark.parametrize("e,rows,k,gated", [(1, 128, 64, True), (2, 384, 576, True), (3, 200, 832, False),
+                                            (40, 128, 1024, False)])
+def test_weight_quantiser_edges(ops, ctx, oracle, e, rows, k, gated):
+    rng = np.random.default_rng(rows + k)
+    w = bf16(rng.standard_normal((e, rows, k), dtype=np.float32) * 0.02)
+    w[-1, -1, -1] = 3.0  # the expert's amax sits in its last element
+    q = ops.nvfp4_quantize_weight(ctx, to_dev(w), gated)
+    for got, ref in zip((q.packed, q.scale_linear, q.scale_tiled, q.global_scale),
+                        oracle.nvfp4_quantize_weight(w, gated)):
+        assert np.array_equal(to_np(got), ref)
+
+
 def _check(out, ref):
     assert rel_l2(out, ref) <= 1e-2
     assert max_abs(out, ref) <= 2.0 ** -5 * np.max(np.abs(f32(ref)))
