@@ -133,10 +133,6 @@ cudaError_t launch_gather_bf16(const __nv_bfloat16* hidden, const int32_t* route
                                uint32_t routes, uint32_t top_k, uint32_t hidden_size,
                                __nv_bfloat16* expanded, cudaStream_t stream);
 
-// dst[prow(route), :] = src[route / top_k, :] for rows of row_bytes (a multiple of 4) bytes.
-cudaError_t launch_gather_rows(const void* src, uint32_t row_bytes, const int32_t* route_prows, uint32_t routes,
-                               uint32_t top_k, void* dst, cudaStream_t stream);
-
 struct CombineParams {
     const int32_t* route_prows;   // [T*K]
     const float* topk_weights;    // [T*K]
@@ -288,6 +284,10 @@ uint32_t fp8_tile_rows(uint32_t routes, uint32_t experts);
 cudaError_t launch_fp8_gather_quantize(const __nv_bfloat16* x, const int32_t* route_prows, uint32_t routes,
                                        uint32_t top_k, uint32_t k, uint8_t* codes, float* scales,
                                        cudaStream_t stream);
+// codes[prow] / scales[prow] = those of token route / top_k, already quantised (k a multiple of 128 up to 4096).
+cudaError_t launch_fp8_gather_rows(const uint8_t* codes, const float* scales, const int32_t* route_prows,
+                                   uint32_t routes, uint32_t top_k, uint32_t k, uint8_t* out_codes, float* out_scales,
+                                   cudaStream_t stream);
 cudaError_t launch_fp8_quantize_weight(const __nv_bfloat16* w, uint32_t experts, uint32_t rows, uint32_t k,
                                        uint8_t* codes, float* scales, cudaStream_t stream);
 struct Fp8Gemm {
@@ -304,11 +304,12 @@ struct Fp8Gemm {
     const int32_t* total_tiles;
     uint32_t max_tiles;
     uint32_t est_tiles;      // host-side estimate of *total_tiles, sizes the feature splits
-    uint32_t tile_rows;      // 16 or 32
+    uint32_t tile_rows;      // 16 (decode kernel) or 128 (token rows on the M side, fp8_rows.cu)
     void* out;               // gated: u8 [x_rows, n]; else bf16 [x_rows, n]
     float* out_scale;        // gated: f32 [x_rows, n / 128]
 };
 cudaError_t launch_fp8_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** why_unsupported);
+cudaError_t launch_fp8_rows_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** why_unsupported);
 
 // ---- device helpers ---------------------------------------------------------------
 #ifdef __CUDACC__

@@ -9,8 +9,8 @@
 // The GEMM is written for decode-sized batches, where a handful of tokens meet each
 // expert and the job is to stream the expert weights from HBM once:
 //   * operands are swapped: a 128-feature weight tile is the M operand of the MMA and
-//     the expert's token tile (NT = 16 or 32 rows) the N operand, so no tensor-core rows
-//     are spent on padding tokens;
+//     the expert's token tile (16 rows) the N operand, so no tensor-core rows are spent on
+//     padding tokens (fp8_rows.cu has the kernel for experts with more rows);
 //   * the token panel [NT, K] stays resident in shared memory, only weights stream
 //     through the TMA ring (one 128 x 128-byte tile per stage);
 //   * 128 x 128 block scales are not a tcgen05 block-scale format, so every 128-wide k
@@ -43,35 +43,77 @@ __device__ __forceinline__ uint32_t pack_e4m3x4(const float* f, float inv)
     return r;
 }
 
-// codes[prow, :] / scales[prow, :] = quantise(x[route / top_k, :]); one warp per (route,
-// 128-element group), 4 elements per lane. route_prows == NULL: prow = route.
+// codes[prow, :] / scales[prow, :] = quantise(x[route / top_k, :]); 16 lanes per (route,
+// 128-element group), eight elements (one 16-byte load) per lane. route_prows == NULL: prow = route.
 __global__ void __launch_bounds__(256)
 fp8_gather_quantize_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ route_prows,
                            uint32_t routes, uint32_t top_k, uint32_t k, uint8_t* __restrict__ codes,
                            float* __restrict__ scales)
 {
     const uint32_t groups = k / 128;
-    const uint64_t unit = static_cast<uint64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    const uint32_t lane = threadIdx.x & 31;
-    if (unit >= static_cast<uint64_t>(routes) * groups)
-        return;
-    const uint32_t route = static_cast<uint32_t>(unit / groups), g = static_cast<uint32_t>(unit % groups);
-    const int prow = route_prows != nullptr ? route_prows[route] : static_cast<int>(route);
+    const uint64_t unit = static_cast<uint64_t>(blockIdx.x) * 16 + (threadIdx.x >> 4);
+    const uint32_t sub = threadIdx.x & 15;
+    const bool in_range = unit < static_cast<uint64_t>(routes) * groups;
+    const uint32_t route = in_range ? static_cast<uint32_t>(unit / groups) : 0u;
+    const uint32_t g = static_cast<uint32_t>(unit % groups);
+    const int prow = !in_range ? -1 : route_prows != nullptr ? route_prows[route] : static_cast<int>(route);
+    uint2 v2[2] = { make_uint2(0, 0), make_uint2(0, 0) };
+    if (prow >= 0) { // (the entry points promise 8-byte aligned rows)
+        const uint2* src = reinterpret_cast<const uint2*>(x + static_cast<size_t>(route / top_k) * k + g * 128 + sub * 8);
+        v2[0] = src[0];
+        v2[1] = src[1];
+    }
+    const uint32_t w[4] = { v2[0].x, v2[0].y, v2[1].x, v2[1].y };
+    float f[8];
+    float amax = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        f[2 * j] = bf16_bits_to_f32(w[j] & 0xffffu);
+        f[2 * j + 1] = bf16_bits_to_f32(w[j] >> 16);
+        amax = fmaxf(amax, fmaxf(fabsf(f[2 * j]), fabsf(f[2 * j + 1])));
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     if (prow < 0)
         return;
-    const uint2* src = reinterpret_cast<const uint2*>(x + static_cast<size_t>(route / top_k) * k);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(codes + static_cast<size_t>(prow) * k);
-    const uint2 v = src[g * 32 + lane];
-    const float f[4] = { bf16_bits_to_f32(v.x & 0xffffu), bf16_bits_to_f32(v.x >> 16),
-                         bf16_bits_to_f32(v.y & 0xffffu), bf16_bits_to_f32(v.y >> 16) };
-    float amax = fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3])));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     const float s = fp8_scale_of(amax);
-    dst[g * 32 + lane] = pack_e4m3x4(f, __fdiv_rn(1.0f, s));
-    if (lane == 0)
+    const float inv = __fdiv_rn(1.0f, s);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(codes + static_cast<size_t>(prow) * k + g * 128 + sub * 8);
+    dst[0] = pack_e4m3x4(f, inv);
+    dst[1] = pack_e4m3x4(f + 4, inv);
+    if (sub == 0)
         scales[static_cast<size_t>(prow) * groups + g] = s;
+}
+
+// codes[prow, :] / scales[prow, :] = those of token route / top_k, already quantised. A warp per route, all of a
+// row's loads in flight (k <= 4096: eight 16-byte vectors and one scale word per lane).
+__global__ void __launch_bounds__(256)
+fp8_gather_rows_kernel(const uint4* __restrict__ codes, const uint32_t* __restrict__ scales,
+                       const int32_t* __restrict__ route_prows, uint32_t routes, uint32_t top_k, uint32_t k,
+                       uint4* __restrict__ out_codes, uint32_t* __restrict__ out_scales)
+{
+    const uint32_t route = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (route >= routes)
+        return;
+    const int prow = route_prows[route];
+    if (prow < 0)
+        return;
+    const uint32_t vecs = k / 16, groups = k / 128;
+    const uint4* src = codes + static_cast<size_t>(route / top_k) * vecs;
+    uint4* dst = out_codes + static_cast<size_t>(prow) * vecs;
+    const uint32_t sc = lane < groups ? scales[static_cast<size_t>(route / top_k) * groups + lane] : 0u;
+    uint4 v[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i)
+        if (lane + 32 * i < vecs)
+            v[i] = src[lane + 32 * i];
+#pragma unroll
+    for (uint32_t i = 0; i < 8; ++i)
+        if (lane + 32 * i < vecs)
+            dst[lane + 32 * i] = v[i];
+    if (lane < groups)
+        out_scales[static_cast<size_t>(prow) * groups + lane] = sc;
 }
 
 // One block per (k block, row block, expert): 128 x 128 weights -> codes + one scale. Sixteen lanes read the
@@ -128,11 +170,12 @@ fp8_quantize_weight_kernel(const __nv_bfloat16* __restrict__ w, uint32_t rows, u
 
 // ---- grouped GEMM -------------------------------------------------------------------------
 
+constexpr uint32_t kF8Tokens = 16;           // token rows per tile = MMA N
 constexpr int kF8Threads = 192;   // warps 0-3 epilogue, 4 TMA producer, 5 MMA issuer
 constexpr int kF8Bufs = 4;        // accumulator buffers in tensor memory
 constexpr int kF8MaxStages = 8;
 constexpr int kF8MaxKBlocks = 32; // k <= 4096: one weight-scale register per lane
-constexpr uint32_t kF8MiscBytes = 256 /* barriers */ + 16 + 4 * 32 * 4 /* amax */ + kF8MaxKBlocks * 32 * 4;
+constexpr uint32_t kF8MiscBytes = 256 /* barriers */ + 16 + 4 * 32 * 4 /* amax */ + kF8MaxKBlocks * kF8Tokens * 4;
 
 enum : uint32_t {
     ERR_F8_PANEL_WAIT = 0x54000001u,
@@ -165,16 +208,16 @@ struct Fp8Params {
 // feature blocks [blockIdx.x * fb_per_cta, ...).
 //   TMEM: kF8Bufs buffers of (GATED ? 2 : 1) * NT f32 columns (gate columns, then up columns)
 //   smem: token panel k_blocks x (NT x 128 B) | ring stages x 16 KB | barriers, scales
-template <int NT, bool GATED>
+template <bool GATED>
 __global__ void __launch_bounds__(kF8Threads)
 gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                 const Fp8Params p)
 {
     constexpr uint32_t G = GATED ? 2 : 1;
+    constexpr int NT = kF8Tokens;
     constexpr uint32_t kAccCols = G * NT;
     constexpr uint32_t kTmemCols = kF8Bufs * kAccCols < 32 ? 32 : kF8Bufs * kAccCols;
     constexpr uint32_t kPanelTile = NT * 128;
-    static_assert(NT == 16 || NT == 32, "token tile of 16 or 32 rows");
 
     const uint32_t tile = blockIdx.y;
     if (static_cast<int>(tile) >= *p.total_tiles)
@@ -400,11 +443,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     }
 }
 
-template <int NT, bool GATED>
+template <bool GATED>
 cudaError_t launch_fp8_instance(const CUtensorMap& mw, const CUtensorMap& mx, const Fp8Params& fp, dim3 grid,
                                 size_t smem, cudaStream_t stream)
 {
-    auto kernel = gemm_fp8_kernel<NT, GATED>;
+    auto kernel = gemm_fp8_kernel<GATED>;
     static size_t configured[64] = {}; // largest size set so far, per instantiation and device
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
@@ -426,7 +469,24 @@ cudaError_t launch_fp8_instance(const CUtensorMap& mw, const CUtensorMap& mx, co
 
 uint32_t fp8_tile_rows(uint32_t routes, uint32_t experts)
 {
-    return routes <= 16u * experts ? 16u : 32u;
+    // The 16-row kernel streams an expert's weights once per started 16 rows, so it holds while nearly every
+    // expert fits one tile; beyond that the kernel with token rows on the M side is never slower (128 experts
+    // top-8, layer time: 9 rows per expert 0.159 against 0.199 ms, 16 rows 0.213 against 0.201, 32 rows 0.327
+    // against 0.213).
+    return routes <= 12u * experts ? kF8Tokens : static_cast<uint32_t>(kTileM);
+}
+
+cudaError_t launch_fp8_gather_rows(const uint8_t* codes, const float* scales, const int32_t* route_prows,
+                                   uint32_t routes, uint32_t top_k, uint32_t k, uint8_t* out_codes, float* out_scales,
+                                   cudaStream_t stream)
+{
+    if (routes == 0)
+        return cudaSuccess;
+    fp8_gather_rows_kernel<<<(routes + 7) / 8, 256, 0, stream>>>(
+        reinterpret_cast<const uint4*>(codes), reinterpret_cast<const uint32_t*>(scales), route_prows, routes, top_k, k,
+        reinterpret_cast<uint4*>(out_codes), reinterpret_cast<uint32_t*>(out_scales));
+    note_launch();
+    return cudaGetLastError();
 }
 
 cudaError_t launch_fp8_gather_quantize(const __nv_bfloat16* x, const int32_t* route_prows, uint32_t routes,
@@ -436,7 +496,7 @@ cudaError_t launch_fp8_gather_quantize(const __nv_bfloat16* x, const int32_t* ro
     if (routes == 0)
         return cudaSuccess;
     const uint64_t units = static_cast<uint64_t>(routes) * (k / 128);
-    fp8_gather_quantize_kernel<<<static_cast<uint32_t>((units + 7) / 8), 256, 0, stream>>>(
+    fp8_gather_quantize_kernel<<<static_cast<uint32_t>((units + 15) / 16), 256, 0, stream>>>(
         x, route_prows, routes, top_k, k, codes, scales);
     note_launch();
     return cudaGetLastError();
@@ -462,10 +522,14 @@ cudaError_t launch_fp8_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** 
         return fail("FP8 GEMM needs n and k divisible by 128");
     if (g.k / 128 > kF8MaxKBlocks)
         return fail("FP8 GEMM supports k <= 4096");
-    if (g.tile_rows != 16 && g.tile_rows != 32)
-        return fail("FP8 GEMM token tiles are 16 or 32 rows");
+    if (g.tile_rows != kF8Tokens && g.tile_rows != kTileM)
+        return fail("FP8 GEMM token tiles are 16 or 128 rows");
     if ((reinterpret_cast<uintptr_t>(g.x) & 15u) != 0 || (reinterpret_cast<uintptr_t>(g.w) & 15u) != 0)
         return fail("FP8 GEMM operands must be 16-byte aligned");
+    if (g.max_tiles == 0 || g.max_tiles > 65535)
+        return fail("FP8 GEMM launch grid is too large");
+    if (g.tile_rows == kTileM)
+        return launch_fp8_rows_gemm(g, stream, why);
     Fp8Params fp {};
     fp.n = g.n;
     fp.k_blocks = g.k / 128;
@@ -496,8 +560,6 @@ cudaError_t launch_fp8_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** 
     const uint32_t want = std::max(1u, (slots + g.est_tiles - 1) / std::max(1u, g.est_tiles));
     fp.fb_per_cta = std::max(1u, (fp.num_fb + want - 1) / want);
     const uint32_t splits = (fp.num_fb + fp.fb_per_cta - 1) / fp.fb_per_cta;
-    if (g.max_tiles == 0 || g.max_tiles > 65535)
-        return fail("FP8 GEMM launch grid is too large");
 
     CUtensorMap mw, mx;
     if (!make_operand_map(&mw, true, g.w, g.k, static_cast<uint64_t>(g.groups) * fp.b_rows, g.k, 128)
@@ -507,11 +569,8 @@ cudaError_t launch_fp8_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** 
         return cudaErrorInvalidValue;
     }
     const dim3 grid(splits, g.max_tiles, 1);
-    if (g.tile_rows == 16)
-        return g.gated ? launch_fp8_instance<16, true>(mw, mx, fp, grid, smem, stream)
-                       : launch_fp8_instance<16, false>(mw, mx, fp, grid, smem, stream);
-    return g.gated ? launch_fp8_instance<32, true>(mw, mx, fp, grid, smem, stream)
-                   : launch_fp8_instance<32, false>(mw, mx, fp, grid, smem, stream);
+    return g.gated ? launch_fp8_instance<true>(mw, mx, fp, grid, smem, stream)
+                   : launch_fp8_instance<false>(mw, mx, fp, grid, smem, stream);
 }
 
 } // namespace qs3

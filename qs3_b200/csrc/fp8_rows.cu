@@ -1,0 +1,383 @@
+// FP8 block-scaled grouped GEMM for experts with more rows than a decode batch gives them (fp8.cu has the kernel
+// for those): token rows are the M side of the MMA again.
+//
+// A 128 x 256 output tile per unit: 128 token rows of one expert x 256 weight rows (gated: 128 gate rows and the
+// 128 up rows of the same features). The block scales are promoted outside the tensor core as in the decode
+// kernel, but with tokens in the tensor-memory lanes a lane needs ONE factor per k block and 128-feature block
+// (x_scale[token] * w_scale[block]), so promoting an element is a single FMA without any shared-memory operand:
+// 128 x 256 partials cost eight warps about 300 cycles against the ~690 cycles of their four MMAs.
+//
+//   persistent  one CTA per SM; the (token tile, feature block) units are cut into equal contiguous ranges, so
+//               the last round is never nearly empty and neighbouring CTAs share an expert's weights in L2
+//   smem        ring of stages: A 128 x 128 B, B 256 x 128 B; plain: + four 16-KB boxes staging the bf16 tile for
+//               TMA stores
+//   TMEM        two 256-column buffers: k block i + 1 is multiplied while k block i is promoted
+//   warps       0-7 promotion and epilogue (lane quadrant warp % 4, column half warp / 4), 8 producer, 9 MMA
+//
+// Bound by operand delivery: a k block moves 48 KB into the SM for 128 x 256 x 128 products, and the weights, of
+// which every byte is wanted by two or three CTAs, arrive at 45 GB/s per SM (1.09 us per k block; 0.63 us without
+// the loads, 0.76 with promotion but without loads). 4096 tokens x 128 experts top-8 (hidden 2048, intermediate
+// 768): gate_up 0.800 -> 0.231 ms, down 0.238 -> 0.106 ms against the decode kernel on 32-row tiles, which
+// streamed every weight through shared memory once per 32 rows.
+#include "tcgen05.cuh"
+
+#include <algorithm>
+
+namespace qs3 {
+namespace {
+
+using namespace tc;
+
+constexpr int kFrThreads = 320;
+constexpr uint32_t kFrN = 256;                        // weight rows per unit = MMA N
+constexpr uint32_t kFrStageBytes = 3 * kTileBytes;    // A tile + two B tiles
+constexpr uint32_t kFrMaxStages = 4;
+constexpr uint32_t kFrTmemCols = 512;
+
+enum : uint32_t {
+    ERR_FR_FULL_WAIT = 0x58000001u,
+    ERR_FR_EMPTY_WAIT = 0x58000002u,
+    ERR_FR_ACC_FULL_WAIT = 0x58000003u,
+    ERR_FR_ACC_EMPTY_WAIT = 0x58000004u,
+};
+
+struct Fp8RowsParams {
+    uint32_t n;            // output features per group (gated: intermediate size); multiple of 128
+    uint32_t k_blocks;     // k / 128
+    uint32_t b_rows;       // weight rows per group (gated: 2 n)
+    uint32_t units_per_tile; // gated: n / 128; plain: ceil(n / 256)
+    uint32_t num_fb;       // n / 128
+    const float* x_scale;  // [rows, k_blocks]
+    const float* w_scale;  // [groups, b_rows / 128, k_blocks]
+    const int32_t* tile_expert;
+    const int32_t* tile_row0;
+    const int32_t* tile_nrows;
+    const int32_t* total_tiles;
+    void* out;             // gated: e4m3 codes [rows, n]; plain: written through map_o
+    float* out_scale;      // gated: f32 [rows, n / 128]
+    uint32_t* err;
+};
+
+__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t* r)
+{
+    tc_ld16(taddr, r);
+    tc_ld16(taddr + 16, r + 16);
+}
+
+template <bool GATED>
+__global__ void __launch_bounds__(kFrThreads, 1)
+gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
+                     const __grid_constant__ CUtensorMap map_o, const Fp8RowsParams p)
+{
+    constexpr uint32_t kStages = GATED ? kFrMaxStages : kFrMaxStages - 1;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t* staging = smem + kStages * kFrStageBytes; // plain: four 16-KB boxes
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(staging + (GATED ? 0 : 4 * kTileBytes));
+    uint64_t* empty_bar = full_bar + kFrMaxStages;
+    uint64_t* acc_full = empty_bar + kFrMaxStages;
+    uint64_t* acc_empty = acc_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+    float* s_amax = reinterpret_cast<float*>(tmem_slot + 4); // [2][128]
+
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < kStages; ++s) {
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 8); // one arrival per promotion warp
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 9) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(kFrTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    const uint64_t total = static_cast<uint64_t>(*p.total_tiles) * p.units_per_tile;
+    const uint32_t u0 = static_cast<uint32_t>(total * blockIdx.x / gridDim.x);
+    const uint32_t u1 = static_cast<uint32_t>(total * (blockIdx.x + 1) / gridDim.x);
+
+    if (warp == 8) {
+        // ------------------------------------------------------------ producer --
+        if (lane == 0) {
+            uint32_t s = 0, ph = 0;
+            bool ok = true;
+            for (uint32_t u = u0; u < u1 && ok; ++u) {
+                const uint32_t tile = u / p.units_per_tile, nb = u % p.units_per_tile;
+                const int row0 = p.tile_row0[tile];
+                const int b_row = p.tile_expert[tile] * static_cast<int>(p.b_rows)
+                    + static_cast<int>(nb * (GATED ? 128 : kFrN));
+                // the second B tile: the up rows of the features, or the next 128 features (the last unit of an odd
+                // count has none: it loads its own tile again and drops the result)
+                const bool second = GATED || (nb * kFrN + 128 < p.n);
+                const int b_row2 = b_row + (GATED ? static_cast<int>(p.n) : second ? 128 : 0);
+                for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
+                    if (!mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_FR_EMPTY_WAIT)) {
+                        ok = false;
+                        break;
+                    }
+                    uint8_t* sa = smem + s * kFrStageBytes;
+                    mbar_expect_tx(&full_bar[s], kFrStageBytes);
+                    const int c0 = static_cast<int>(kb * 128);
+                    tma_load_2d(sa + kTileBytes, &map_w, &full_bar[s], c0, b_row);
+                    tma_load_2d(sa + 2 * kTileBytes, &map_w, &full_bar[s], c0, b_row2);
+                    tma_load_2d(sa, &map_x, &full_bar[s], c0, row0);
+                    if (++s == kStages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp == 9) {
+        // ---------------------------------------------------------- MMA issuer --
+        if (lane == 0) {
+            // M = 128 tokens, N = 256 weight rows, e4m3 x e4m3 -> f32, both operands K-major
+            constexpr uint32_t kIdesc = (1u << 4) | ((kFrN >> 3) << 17) | ((kBM >> 4) << 24);
+            uint32_t s = 0, ph = 0, b = 0, bph = 0;
+            bool ok = true;
+            for (uint32_t u = u0; u < u1 && ok; ++u) {
+                for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
+                    if (!mbar_wait<true>(&acc_empty[b], bph ^ 1, abort_flag, p.err, ERR_FR_ACC_EMPTY_WAIT)
+                        || !mbar_wait<true>(&full_bar[s], ph, abort_flag, p.err, ERR_FR_FULL_WAIT)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t sa = smem_u32(smem + s * kFrStageBytes);
+                    const uint64_t da = operand_desc(sa);
+                    const uint64_t db = operand_desc(sa + kTileBytes); // 256 rows: two tiles back to back
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j)
+                        tc_mma_f8(tmem_base + b * kFrN, da + 2 * j, db + 2 * j, kIdesc, j > 0 ? 1u : 0u);
+                    tc_commit(&empty_bar[s]);
+                    tc_commit(&acc_full[b]);
+                    if (++s == kStages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                    b ^= 1;
+                    bph ^= b == 0;
+                }
+            }
+        }
+    } else {
+        // ------------------------------------------------- promotion, epilogue --
+        const uint32_t quad = warp & 3, half = warp >> 2;
+        const uint32_t r = quad * 32 + lane; // token row of the tile = TMEM lane
+        // columns of this warp: gated 64 gate columns and the 64 up columns of the same features; plain 128 columns
+        const uint32_t col0 = (quad * 32) << 16 | (GATED ? half * 64 : half * 128);
+        constexpr uint32_t kSecond = GATED ? 128 : 64; // distance of the second 64 columns
+        uint32_t b = 0, bph = 0;
+        bool ok = true;
+        for (uint32_t u = u0; u < u1; ++u) {
+            const uint32_t tile = u / p.units_per_tile, nb = u % p.units_per_tile;
+            const int expert = p.tile_expert[tile];
+            const uint32_t row0 = static_cast<uint32_t>(p.tile_row0[tile]);
+            const int nrows = p.tile_nrows[tile];
+            const bool live = static_cast<int>(quad * 32) < nrows; // whole warps without a valid row only count along
+            const uint32_t w_blocks = p.b_rows / 128;
+            const uint32_t fb = GATED ? nb : min(2 * nb + half, p.num_fb - 1);
+            const float* xs = p.x_scale + static_cast<size_t>(row0 + r) * p.k_blocks;
+            const float* ws = p.w_scale + (static_cast<size_t>(expert) * w_blocks + fb) * p.k_blocks;
+            const float* wu = ws + static_cast<size_t>(GATED ? p.num_fb : 0) * p.k_blocks;
+            float acc[2][64];
+#pragma unroll
+            for (int i = 0; i < 64; ++i)
+                acc[0][i] = acc[1][i] = 0.0f;
+            float xs_next = live ? xs[0] : 0.0f, ws_next = ws[0], wu_next = GATED ? wu[0] : 0.0f;
+            for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
+                const float s0 = ws_next * xs_next;
+                const float s1 = GATED ? wu_next * xs_next : s0;
+                if (kb + 1 < p.k_blocks) { // the factors of the next k block travel while this one is waited for
+                    xs_next = live ? xs[kb + 1] : 0.0f;
+                    ws_next = ws[kb + 1];
+                    if (GATED)
+                        wu_next = wu[kb + 1];
+                }
+                ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], bph, abort_flag, p.err, ERR_FR_ACC_FULL_WAIT));
+                if (!ok)
+                    break;
+                tc_fence_after();
+                if (live) {
+                    const uint32_t src = tmem_base + b * kFrN + col0;
+#pragma unroll
+                    for (uint32_t c = 0; c < 4; ++c) {
+                        uint32_t v[32];
+                        tc_ld32(src + (c >> 1) * kSecond + (c & 1) * 32, v);
+                        tc_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            acc[c >> 1][(c & 1) * 32 + i]
+                                = fmaf(__uint_as_float(v[i]), (c >> 1) ? s1 : s0, acc[c >> 1][(c & 1) * 32 + i]);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(&acc_empty[b]);
+                b ^= 1;
+                bph ^= b == 0;
+            }
+            if constexpr (GATED) {
+                // SwiGLU, then one e4m3 scale per token and 128 features: the two halves of a row are in the two
+                // warps of a lane quadrant, which exchange their maxima
+                float amax = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 64; ++i) {
+                    const float g = acc[0][i];
+                    acc[0][i] = __fdividef(g, 1.0f + __expf(-g)) * acc[1][i];
+                    amax = fmaxf(amax, fabsf(acc[0][i]));
+                }
+                s_amax[half * 128 + r] = amax;
+                ok = group_all(1 + quad, 64, ok); // the two warps stop together
+                if (!ok)
+                    break;
+                amax = fmaxf(amax, s_amax[(half ^ 1) * 128 + r]);
+                asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory"); // both have read: the next unit may write
+                if (static_cast<int>(r) < nrows) {
+                    const float sc = fmaxf(__fdiv_rn(amax, 448.0f), 1.0e-30f);
+                    const float inv = __fdiv_rn(1.0f, sc);
+                    uint8_t* out = static_cast<uint8_t*>(p.out) + static_cast<size_t>(row0 + r) * p.n + fb * 128 + half * 64;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            w[j] = 0;
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                w[j] |= static_cast<uint32_t>(f32_to_e4m3_sat(__fmul_rn(acc[0][16 * i + 4 * j + q], inv)))
+                                    << (8 * q);
+                        }
+                        reinterpret_cast<uint4*>(out)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                    if (half == 0)
+                        p.out_scale[static_cast<size_t>(row0 + r) * p.num_fb + fb] = sc;
+                }
+            } else {
+                // bf16 rows through shared memory and TMA stores (64-column boxes). Every row of the tile is written:
+                // rows past the segment end are padding rows of the same expert.
+                ok = group_all(1 + half, 128, ok);
+                if (!ok)
+                    break;
+                const bool issuer = quad == 0 && lane == 0;
+                if (issuer) // the half's previous boxes have left the staging
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+#pragma unroll
+                for (uint32_t c = 0; c < 2; ++c) {
+                    uint8_t* row_smem = staging + (half * 2 + c) * kTileBytes + r * 128;
+#pragma unroll
+                    for (uint32_t q = 0; q < 8; ++q) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            w[i] = pack_bf16x2(acc[c][8 * q + 2 * i], acc[c][8 * q + 2 * i + 1]);
+                        *reinterpret_cast<uint4*>(row_smem + ((q ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+                if (issuer) {
+                    const uint32_t n0 = nb * kFrN + half * 128;
+                    for (uint32_t c = 0; c < 2 && n0 < p.n; ++c)
+                        asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                                         reinterpret_cast<uint64_t>(&map_o)),
+                                     "r"(smem_u32(staging + (half * 2 + c) * kTileBytes)),
+                                     "r"(static_cast<int>(n0 + c * 64)), "r"(static_cast<int>(row0))
+                                     : "memory");
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                }
+            }
+        }
+        if (!GATED && quad == 0 && lane == 0)
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); // stores done before smem goes away
+    }
+
+    // ---- teardown ----
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 9) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kFrTmemCols)
+                     : "memory");
+    }
+}
+
+template <bool GATED>
+cudaError_t launch_rows_instance(const CUtensorMap& mx, const CUtensorMap& mw, const CUtensorMap& mo,
+                                 const Fp8RowsParams& fp, uint32_t grid, cudaStream_t stream)
+{
+    auto kernel = gemm_fp8_rows_kernel<GATED>;
+    constexpr size_t smem = 1024 + (GATED ? kFrMaxStages * kFrStageBytes
+                                          : (kFrMaxStages - 1) * kFrStageBytes + 4 * kTileBytes) + 2048;
+    static bool configured[64] = {}; // per instantiation and device
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess)
+        return err;
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (err != cudaSuccess)
+            return err;
+        if (dev >= 0 && dev < 64)
+            configured[dev] = true;
+    }
+    kernel<<<grid, kFrThreads, smem, stream>>>(mx, mw, mo, fp);
+    note_launch();
+    return cudaGetLastError();
+}
+
+} // namespace
+
+cudaError_t launch_fp8_rows_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** why)
+{
+    Fp8RowsParams fp {};
+    fp.n = g.n;
+    fp.k_blocks = g.k / 128;
+    fp.b_rows = g.gated ? 2 * g.n : g.n;
+    fp.num_fb = g.n / 128;
+    fp.units_per_tile = g.gated ? g.n / 128 : (g.n + kFrN - 1) / kFrN;
+    fp.x_scale = g.x_scale;
+    fp.w_scale = g.w_scale;
+    fp.tile_expert = g.tile_expert;
+    fp.tile_row0 = g.tile_row0;
+    fp.tile_nrows = g.tile_nrows;
+    fp.total_tiles = g.total_tiles;
+    fp.out = g.out;
+    fp.out_scale = g.out_scale;
+    fp.err = device_error_word();
+    CUtensorMap mx, mw, mo;
+    bool ok = make_operand_map(&mx, true, g.x, g.k, g.x_rows, g.k, 128)
+        && make_operand_map(&mw, true, g.w, g.k, static_cast<uint64_t>(g.groups) * fp.b_rows, g.k, 128);
+    mo = mx;
+    if (ok && !g.gated)
+        ok = make_operand_map(&mo, false, g.out, g.n, g.x_rows, static_cast<uint64_t>(g.n) * 2, 128);
+    if (!ok) {
+        if (why != nullptr)
+            *why = "cuTensorMapEncodeTiled failed";
+        return cudaErrorInvalidValue;
+    }
+    const uint32_t grid = static_cast<uint32_t>(
+        std::min<uint64_t>(static_cast<uint64_t>(g.max_tiles) * fp.units_per_tile, device_sm_count()));
+    return g.gated ? launch_rows_instance<true>(mx, mw, mo, fp, grid, stream)
+                   : launch_rows_instance<false>(mx, mw, mo, fp, grid, stream);
+}
+
+} // namespace qs3

@@ -165,6 +165,8 @@ struct LayerExtra {
     uint8_t* sh_xq_sf;
     uint8_t* sh_actq;       // [T128, Is/2]
     uint8_t* sh_actq_sf;
+    uint8_t* f8_x;          // FP8 plans with 128-row token tiles: hidden quantised in token order [T, H]
+    float* f8_s;            // [T, H/128]
     size_t bytes;
 };
 
@@ -183,6 +185,11 @@ LayerExtra carve_layer(char* base, size_t start, const qsfi_moe_plan_desc& d, ui
         const size_t t128 = align_up(t, kTileM);
         x.sh_xq = carve<uint8_t>(base, off, t128 * h / 2);
         x.sh_xq_sf = carve<uint8_t>(base, off, qs3_nvfp4_tiled_scale_bytes(t128, h));
+    }
+    if (is_fp8_plan(d) && fp8_tile_rows(num_tokens * d.top_k, d.local_num_experts) == kTileM) {
+        // a token meets top_k experts: quantised once here, its codes are gathered
+        x.f8_x = carve<uint8_t>(base, off, t * h);
+        x.f8_s = carve<float>(base, off, t * (h / 128));
     }
     if (shared_inter != 0) {
         x.sh_out = carve<__nv_bfloat16>(base, off, t * h);
@@ -1241,10 +1248,18 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
 
     const __nv_bfloat16* y2 = nullptr;
     if (fp8) {
-        // 4. quantise the routed rows straight from the bf16 tokens; 5./6. grouped GEMMs
+        // 4. quantise the routed rows: straight from the bf16 tokens in a decode batch (one launch), otherwise every
+        //    token once and then a gather of the codes; 5./6. grouped GEMMs
         stage_mark(st, STAGE_GATHER);
-        err = launch_fp8_gather_quantize(hidden, rt.route_prows, routes, p.top_k, p.hidden_size, wf.xq, wf.xq_s,
-                                         st);
+        if (x.f8_x == nullptr) {
+            err = launch_fp8_gather_quantize(hidden, rt.route_prows, routes, p.top_k, p.hidden_size, wf.xq, wf.xq_s,
+                                             st);
+        } else {
+            err = launch_fp8_gather_quantize(hidden, nullptr, d->num_tokens, 1, p.hidden_size, x.f8_x, x.f8_s, st);
+            if (err == cudaSuccess)
+                err = launch_fp8_gather_rows(x.f8_x, x.f8_s, rt.route_prows, routes, p.top_k, p.hidden_size, wf.xq,
+                                             wf.xq_s, st);
+        }
         if (err != cudaSuccess)
             return set_cuda_error(ctx, err, "FP8 MoE gather");
         status = run_routed_fp8(ctx, p, wf, d->num_tokens, static_cast<const uint8_t*>(d->gate_up_weight.data),
@@ -2032,11 +2047,9 @@ qsfi_status qs3_moe_execute_fp8(qsfi_context* ctx, const qsfi_moe_plan* plan, co
                                         p.local_expert_offset, p.local_num_experts, w.rt, st);
     // gather the quantised token rows (codes and their scales) into expert order
     if (err == cudaSuccess)
-        err = launch_gather_rows(desc->hidden.data, static_cast<uint32_t>(h), w.rt.route_prows, routes, p.top_k,
-                                 w.xq, st);
-    if (err == cudaSuccess)
-        err = launch_gather_rows(desc->hidden_scale.data, static_cast<uint32_t>(h / 128 * 4), w.rt.route_prows,
-                                 routes, p.top_k, w.xq_s, st);
+        err = launch_fp8_gather_rows(static_cast<const uint8_t*>(desc->hidden.data),
+                                     static_cast<const float*>(desc->hidden_scale.data), w.rt.route_prows, routes,
+                                     p.top_k, p.hidden_size, w.xq, w.xq_s, st);
     if (err != cudaSuccess)
         return set_cuda_error(ctx, err, "FP8 MoE routing");
     status = run_routed_fp8(ctx, p, w, desc->num_tokens, static_cast<const uint8_t*>(desc->gate_up_weight.data),

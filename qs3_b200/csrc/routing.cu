@@ -294,23 +294,6 @@ gather_bf16_kernel(const uint4* __restrict__ hidden, const int32_t* __restrict__
         dst[i] = src[i];
 }
 
-// Same gather for rows whose length is only a multiple of 4 bytes.
-__global__ void __launch_bounds__(256)
-gather_words_kernel(const uint32_t* __restrict__ src, const int32_t* __restrict__ route_prows,
-                    uint32_t routes, uint32_t top_k, uint32_t words_per_row, uint32_t* __restrict__ dst)
-{
-    const uint32_t route = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (route >= routes)
-        return;
-    const int prow = route_prows[route];
-    if (prow < 0)
-        return;
-    const uint32_t* s = src + static_cast<size_t>(route / top_k) * words_per_row;
-    uint32_t* d = dst + static_cast<size_t>(prow) * words_per_row;
-    for (uint32_t i = threadIdx.x & 31; i < words_per_row; i += 32)
-        d[i] = s[i];
-}
-
 // out[t, :] = bf16(sum_k w[t,k] * f32(Y2[prow(t,k), :])) (+ shared-expert term).
 // Four tokens per block, 64 threads per token; a thread owns two 8-element chunks of the row
 // per step and issues the loads of up to four routes for both chunks together (eight 16-byte
@@ -1077,23 +1060,6 @@ cudaError_t launch_route_sort(const int32_t* topk_ids, const float* topk_weights
     route_place_kernel<<<rt.route_blocks, kSortWarps * 32, smem, stream>>>(
         topk_ids, topk_weights, routes, top_k, local_offset, experts, rt);
     note_launch(3);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_gather_rows(const void* src, uint32_t row_bytes, const int32_t* route_prows, uint32_t routes,
-                               uint32_t top_k, void* dst, cudaStream_t stream)
-{
-    if (row_bytes % 4 != 0)
-        return cudaErrorInvalidValue;
-    const bool vec16 = row_bytes % 16 == 0 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0;
-    if (vec16)
-        gather_bf16_kernel<<<(routes + 7) / 8, 256, 0, stream>>>(static_cast<const uint4*>(src), route_prows, routes,
-                                                                top_k, row_bytes / 16, static_cast<uint4*>(dst));
-    else
-        gather_words_kernel<<<(routes + 7) / 8, 256, 0, stream>>>(static_cast<const uint32_t*>(src), route_prows,
-                                                                 routes, top_k, row_bytes / 4,
-                                                                 static_cast<uint32_t*>(dst));
-    note_launch();
     return cudaGetLastError();
 }
 

@@ -62,7 +62,9 @@ def _plan(ops, ctx, t, h, i, e, k, off=0, le=None):
 @pytest.mark.parametrize("cfg", [
     dict(t=16, h=256, e=8, k=2, i=128),                       # a few rows per expert, 16-row token tiles
     dict(t=40, h=512, e=4, k=2, i=256),                       # 20 rows per expert: two 16-row tiles each
-    dict(t=200, h=512, e=4, k=2, i=256),                      # 100 rows per expert: 32-row token tiles
+    dict(t=200, h=512, e=4, k=2, i=256),                      # 100 rows per expert: 128-row token tiles
+    dict(t=700, h=384, e=4, k=2, i=384),                      # several tiles per expert, half-filled last column unit
+    dict(t=65, h=128, e=4, k=2, i=128, local=(1, 2)),         # one k block, one column unit, partial expert range
     dict(t=96, h=384, e=16, k=4, i=128, local=(4, 8)),        # partial local expert range
     dict(t=64, h=2048, e=128, k=8, i=768),                    # decode configuration (Qwen3-30B-A3B shape)
 ])
@@ -112,6 +114,7 @@ def test_execute_fp8_is_deterministic_and_linear_in_routing_weight(ops, ctx, ora
 @pytest.mark.parametrize("cfg", [
     dict(t=32, h=256, e=8, k=2, i=128),
     dict(t=64, h=2048, e=128, k=8, i=768),   # decode configuration
+    dict(t=301, h=256, e=8, k=2, i=384),     # 128-row token tiles: tokens quantised once, codes gathered
 ])
 def test_whole_layer_fp8_matches_oracle(ops, ctx, oracle, cfg):
     t, h, e, k, i = cfg["t"], cfg["h"], cfg["e"], cfg["k"], cfg["i"]
