@@ -208,6 +208,12 @@ struct GemmProblem {
     uint64_t a_rows;
     uint64_t a_pitch_bytes;
     const uint8_t* a_scale_tiled; // NVFP4 only
+    // decode kernel only: A rows still in token order (a_scale_linear: with row-major scales), found through the
+    // routing tables; NULL: A rows are the padded rows
+    const int32_t* row_tokens;
+    const int32_t* indptr;
+    const int32_t* pad_indptr;
+    int a_scale_linear;
     // B operand: [groups, b_rows, k]; b_rows = 2*n for gated problems
     const void* b;
     uint64_t b_pitch_bytes;
@@ -224,8 +230,7 @@ struct GemmProblem {
     const int32_t* tile_nrows;
     const int32_t* total_tiles;
     uint32_t max_tiles;
-    uint32_t tile_rows;  // rows per tile of the tables: 128, or 32 (NVFP4 decode kernel, operands swapped)
-    uint32_t est_tiles;  // expected number of tiles (sizes the splits of the decode kernel), 0: unknown
+    uint32_t tile_rows;  // rows per tile of the tables: 128, or 32 / 64 (NVFP4 decode kernel, operands swapped)
     // pair tiles of the route sort (RouteTables::pair_*), NULL: no CTA-pair kernel for this problem
     const int32_t* pair_expert;
     const int32_t* pair_row0;
@@ -255,9 +260,9 @@ cudaError_t launch_gemm_dense_bf16(const GemmProblem& p, cudaStream_t stream, co
 // NVFP4 GEMM on CTA pairs (256 x 256 instructions, weights cross L2 -> SM once per 256 rows; gemm_pair.cu).
 bool nvfp4_pair_gemm_supported(const GemmProblem& p);
 cudaError_t launch_nvfp4_pair_gemm(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);
-// NVFP4 grouped GEMM for 32-row token tiles (decode batches): weights are the M side of the MMA.
+// NVFP4 grouped GEMM for 32- and 64-row token tiles (few rows per expert): weights are the M side of the MMA.
 cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);
-// Rows per token tile of an NVFP4 plan: 32 (decode kernel) when experts get few rows each, else 128.
+// Rows per token tile of an NVFP4 plan: 32 or 64 (decode kernel) when experts get few rows each, else 128.
 uint32_t nvfp4_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter);
 bool gemm_tc_supported(const GemmProblem& p);
 
@@ -265,17 +270,13 @@ bool gemm_tc_supported(const GemmProblem& p);
 // Token rows in token order -> e2m1 codes and scales tiled by token row.
 cudaError_t launch_nvfp4_quantize_rows(const __nv_bfloat16* x, uint32_t rows, uint32_t k, float global_scale,
                                        uint8_t* packed, uint8_t* scale_tiled, cudaStream_t stream);
-// Gather of already-quantised token rows into the padded permuted layout of sorted routing tables.
-// 128-row tiles: organised by destination tile (coalesced code rows, whole scale tiles; rows past a
-// tile's last row keep stale codes and get zero scales); smaller tiles: launch_nvfp4_gather_packed.
+// Gather of already-quantised token rows into the padded permuted layout of sorted routing tables with
+// 128-row tiles, organised by destination tile (coalesced code rows, whole scale tiles; rows past a tile's last
+// row keep stale codes and get zero scales). `src_scale_tiled`: the source scales are tiled by token row
+// instead of row-major.
 cudaError_t launch_nvfp4_gather_tiles(const uint8_t* hidden_packed, const uint8_t* hidden_scale, const RouteTables& rt,
-                                      uint32_t routes, uint32_t top_k, uint32_t hidden_size, uint8_t* packed,
-                                      uint8_t* scale_tiled, cudaStream_t stream, int src_scale_tiled = 0);
-// `src_scale_tiled`: the source scales are tiled by token row instead of row-major.
-cudaError_t launch_nvfp4_gather_packed(const uint8_t* hidden_packed, const uint8_t* hidden_scale,
-                                       const int32_t* route_prows, uint32_t routes, uint32_t top_k,
-                                       uint32_t hidden_size, uint8_t* packed, uint8_t* scale_tiled,
-                                       cudaStream_t stream, int src_scale_tiled = 0);
+                                      uint32_t hidden_size, uint8_t* packed, uint8_t* scale_tiled, cudaStream_t stream,
+                                      int src_scale_tiled = 0);
 
 // ---- FP8 (e4m3, 128 x 128 weight blocks, per-token 128-element activation groups) ----
 // Rows of one token tile of the FP8 grouped GEMM for this many routes over this many experts.

@@ -91,8 +91,8 @@ Bf16Workspace carve_bf16(char* base, const qsfi_moe_plan_desc& d, uint32_t num_t
 
 struct Nvfp4Workspace {
     RouteTables rt;
-    uint8_t* xq;       // [pad_rows, H/2]
-    uint8_t* xq_sf;    // tiled(pad_rows, H)
+    uint8_t* xq;       // [pad_rows, H/2], 128-row tiles only
+    uint8_t* xq_sf;    // tiled(pad_rows, H), 128-row tiles only
     uint8_t* act;      // [pad_rows, I/2]
     uint8_t* act_sf;   // tiled(pad_rows, I)
     __nv_bfloat16* y2; // [pad_rows, H]
@@ -109,8 +109,10 @@ Nvfp4Workspace carve_nvfp4(char* base, const qsfi_moe_plan_desc& d, uint32_t num
                                     nvfp4_tile_rows(routes, d.local_num_experts, d.hidden_size, d.intermediate_size));
     const size_t rows = w.rt.max_pad_rows;
     const size_t h = d.hidden_size, i = d.intermediate_size, e = d.local_num_experts;
-    w.xq = carve<uint8_t>(base, off, rows * h / 2);
-    w.xq_sf = carve<uint8_t>(base, off, qs3_nvfp4_tiled_scale_bytes(rows, h));
+    if (w.rt.tile_rows == static_cast<uint32_t>(kTileM)) { // smaller tiles read the token rows in place
+        w.xq = carve<uint8_t>(base, off, rows * h / 2);
+        w.xq_sf = carve<uint8_t>(base, off, qs3_nvfp4_tiled_scale_bytes(rows, h));
+    }
     w.act = carve<uint8_t>(base, off, rows * i / 2);
     w.act_sf = carve<uint8_t>(base, off, qs3_nvfp4_tiled_scale_bytes(rows, i));
     w.y2 = carve<__nv_bfloat16>(base, off, rows * h);
@@ -419,22 +421,35 @@ struct Nvfp4Weights {
     const float* d_global;  // optional
 };
 
-// Routed experts on NVFP4 operands; activation rows are already in w.xq / w.xq_sf.
+// Routed experts on NVFP4 operands. `tokens` / `token_sf` are the quantised rows in token order (scales tiled by
+// token row, or row-major with `sf_linear`): gathered into w.xq / w.xq_sf for 128-row tiles, read in place by the
+// kernel for smaller ones.
 qsfi_status run_routed_nvfp4(qsfi_context* ctx, const qsfi_moe_plan_desc& p, const Nvfp4Workspace& w,
+                             const uint8_t* tokens, const uint8_t* token_sf, bool sf_linear, uint32_t num_tokens,
                              const Nvfp4Weights& wt, float act_global, float act2_global)
 {
     const float ga = act_global == 0.0f ? 1.0f : act_global;
     const float ga2 = act2_global == 0.0f ? 1.0f : act2_global;
+    const bool in_place = w.rt.tile_rows != static_cast<uint32_t>(kTileM);
+    if (!in_place) {
+        const cudaError_t err = launch_nvfp4_gather_tiles(tokens, token_sf, w.rt, p.hidden_size, w.xq, w.xq_sf,
+                                                          ctx->stream, sf_linear ? 0 : 1);
+        if (err != cudaSuccess)
+            return set_cuda_error(ctx, err, "NVFP4 MoE gather");
+    }
     stage_mark(ctx->stream, STAGE_GATE_UP_GEMM);
-    const uint32_t routes_hint = static_cast<uint32_t>(w.rt.max_pad_rows); // upper bound of the padded rows
-    const uint32_t est_tiles = std::min<uint32_t>(w.rt.max_tiles,
-                                                  p.local_num_experts + routes_hint / w.rt.tile_rows);
     GemmProblem g1 = grouped_problem(w.rt, p.local_num_experts);
-    g1.est_tiles = est_tiles;
     g1.nvfp4 = 1;
-    g1.a = w.xq;
+    g1.a = in_place ? tokens : w.xq;
     g1.a_pitch_bytes = p.hidden_size / 2;
-    g1.a_scale_tiled = w.xq_sf;
+    g1.a_scale_tiled = in_place ? token_sf : w.xq_sf;
+    if (in_place) {
+        g1.a_rows = num_tokens;
+        g1.row_tokens = w.rt.row_tokens;
+        g1.indptr = w.rt.indptr;
+        g1.pad_indptr = w.rt.pad_indptr;
+        g1.a_scale_linear = sf_linear;
+    }
     g1.b = wt.gu_packed;
     g1.b_pitch_bytes = p.hidden_size / 2;
     g1.b_scale_tiled = wt.gu_sf_tiled;
@@ -454,7 +469,6 @@ qsfi_status run_routed_nvfp4(qsfi_context* ctx, const qsfi_moe_plan_desc& p, con
         return status;
     stage_mark(ctx->stream, STAGE_DOWN_GEMM);
     GemmProblem g2 = grouped_problem(w.rt, p.local_num_experts);
-    g2.est_tiles = est_tiles;
     g2.nvfp4 = 1;
     g2.a = w.act;
     g2.a_pitch_bytes = p.intermediate_size / 2;
@@ -892,10 +906,6 @@ qsfi_status qsfi_moe_execute_nvfp4(qsfi_context* ctx, const qsfi_moe_plan* plan,
         err = launch_route_sort(static_cast<const int32_t*>(desc->topk_ids.data),
                                 static_cast<const float*>(desc->topk_weights.data), routes, p.top_k,
                                 p.local_expert_offset, p.local_num_experts, w.rt, st);
-    if (err == cudaSuccess)
-        err = launch_nvfp4_gather_tiles(static_cast<const uint8_t*>(desc->hidden_packed.data),
-                                        static_cast<const uint8_t*>(desc->hidden_scale.data), w.rt, routes,
-                                        p.top_k, p.hidden_size, w.xq, w.xq_sf, st);
     if (err != cudaSuccess)
         return set_cuda_error(ctx, err, "NVFP4 MoE routing");
     Nvfp4Weights wt {};
@@ -904,7 +914,9 @@ qsfi_status qsfi_moe_execute_nvfp4(qsfi_context* ctx, const qsfi_moe_plan* plan,
     wt.d_packed = static_cast<const uint8_t*>(desc->down_weight_packed.data);
     wt.d_sf_tiled = w.d_sf;
     wt.d_global = static_cast<const float*>(desc->expert_output_scale.data);
-    status = run_routed_nvfp4(ctx, p, w, wt, 1.0f, 1.0f);
+    status = run_routed_nvfp4(ctx, p, w, static_cast<const uint8_t*>(desc->hidden_packed.data),
+                              static_cast<const uint8_t*>(desc->hidden_scale.data), true, desc->num_tokens, wt, 1.0f,
+                              1.0f);
     if (status != QSFI_STATUS_OK)
         return status;
     CombineParams cp {};
@@ -1270,17 +1282,14 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
             return status;
         y2 = wf.y2;
     } else if (nvfp4) {
-        // 4. quantise every token once (token order), then gather the codes by expert;
-        //    5./6. grouped GEMMs
+        // 4. quantise every token once (token order); 5./6. grouped GEMMs, after a gather of the codes by expert
+        //    or with the routed rows read in place
         stage_mark(st, STAGE_GATHER);
         if (fork)
             err = cudaStreamWaitEvent(st, plan->ev_quant, 0);
         else if (!prequant)
             err = launch_nvfp4_quantize_rows(hidden, d->num_tokens, p.hidden_size, d->act_global_scale, x.sh_xq,
                                              x.sh_xq_sf, st);
-        if (err == cudaSuccess)
-            err = launch_nvfp4_gather_tiles(x.sh_xq, x.sh_xq_sf, rt, routes, p.top_k, p.hidden_size, wn.xq, wn.xq_sf,
-                                            st, 1);
         if (err != cudaSuccess)
             return set_cuda_error(ctx, err, "NVFP4 MoE gather");
         Nvfp4Weights wt {};
@@ -1291,7 +1300,8 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
         wt.d_packed = static_cast<const uint8_t*>(d->down_weight.data);
         wt.d_sf_tiled = static_cast<const uint8_t*>(d->down_scale_tiled.data);
         wt.d_global = static_cast<const float*>(d->down_global_scale.data);
-        status = run_routed_nvfp4(ctx, p, wn, wt, d->act_global_scale, d->act2_global_scale);
+        status = run_routed_nvfp4(ctx, p, wn, x.sh_xq, x.sh_xq_sf, false, d->num_tokens, wt, d->act_global_scale,
+                                  d->act2_global_scale);
         if (status != QSFI_STATUS_OK)
             return status;
         y2 = wn.y2;
@@ -1583,10 +1593,6 @@ qsfi_status qs3_moe_execute_nvfp4_prepared(qsfi_context* ctx, const qsfi_moe_pla
                                         static_cast<const float*>(d->topk_weights.data), routes, p.top_k,
                                         p.local_expert_offset, p.local_num_experts, w.rt, st);
     stage_mark(st, STAGE_GATHER);
-    if (err == cudaSuccess)
-        err = launch_nvfp4_gather_tiles(static_cast<const uint8_t*>(d->hidden_packed.data),
-                                        static_cast<const uint8_t*>(d->hidden_scale.data), w.rt, routes,
-                                        p.top_k, p.hidden_size, w.xq, w.xq_sf, st);
     if (err != cudaSuccess)
         return set_cuda_error(ctx, err, "NVFP4 MoE routing");
     Nvfp4Weights wt {};
@@ -1597,7 +1603,9 @@ qsfi_status qs3_moe_execute_nvfp4_prepared(qsfi_context* ctx, const qsfi_moe_pla
     wt.d_packed = static_cast<const uint8_t*>(d->down_weight.data);
     wt.d_sf_tiled = static_cast<const uint8_t*>(d->down_scale_tiled.data);
     wt.d_global = static_cast<const float*>(d->down_global_scale.data);
-    status = run_routed_nvfp4(ctx, p, w, wt, d->act_global_scale, d->act2_global_scale);
+    status = run_routed_nvfp4(ctx, p, w, static_cast<const uint8_t*>(d->hidden_packed.data),
+                              static_cast<const uint8_t*>(d->hidden_scale.data), true, d->num_tokens, wt,
+                              d->act_global_scale, d->act2_global_scale);
     if (status != QSFI_STATUS_OK)
         return status;
     CombineParams cp {};

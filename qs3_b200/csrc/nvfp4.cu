@@ -193,37 +193,8 @@ quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, uint32_t rows, uint32_
         *reinterpret_cast<uint32_t*>(scale_tiled + tiled_scale_offset(row, kb, k / 64)) = sf;
 }
 
-// Gather of already-quantised rows (declared layout) into the padded permuted
-// layout; scales move from linear [T, H/16] to tiled. One thread per (route, k group).
-__global__ void __launch_bounds__(256)
-gather_packed_kernel(const uint8_t* __restrict__ hidden_packed, const uint8_t* __restrict__ hidden_scale,
-                     const int32_t* __restrict__ route_prows, uint64_t total, uint32_t top_k,
-                     uint32_t hidden_size, uint8_t* __restrict__ packed, uint8_t* __restrict__ scale_tiled,
-                     int src_scale_tiled)
-{
-    const uint64_t idx = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx >= total)
-        return;
-    const uint32_t kgroups = hidden_size / 64;
-    const uint32_t kg = static_cast<uint32_t>(idx % kgroups);
-    const uint32_t route = static_cast<uint32_t>(idx / kgroups);
-    const int prow = route_prows[route];
-    if (prow < 0)
-        return;
-    const uint64_t token = route / top_k;
-    const uint4* src = reinterpret_cast<const uint4*>(hidden_packed + token * (hidden_size / 2) + kg * 32);
-    uint4* dst = reinterpret_cast<uint4*>(packed + static_cast<uint64_t>(prow) * (hidden_size / 2) + kg * 32);
-    dst[0] = src[0];
-    dst[1] = src[1];
-    // source scales: row-major [T, H/16], or already tiled by token row
-    const uint64_t src_off = src_scale_tiled ? tiled_scale_offset(token, 4ull * kg, kgroups)
-                                             : token * (hidden_size / 16) + kg * 4;
-    const uint32_t sf = *reinterpret_cast<const uint32_t*>(hidden_scale + src_off);
-    *reinterpret_cast<uint32_t*>(scale_tiled + tiled_scale_offset(prow, 4ull * kg, kgroups)) = sf;
-}
-
-// The same gather organised by destination tile, for 128-row token tiles: block (k chunk, tile)
-// moves the rows of one token tile of one expert for 512 elements of k. The codes of a row chunk are 256 contiguous
+// Gather of already-quantised rows into the padded permuted layout, organised by destination tile (128-row token
+// tiles; the kernel for smaller tiles fetches its rows itself): block (k chunk, tile) moves the rows of one token tile of one expert for 512 elements of k. The codes of a row chunk are 256 contiguous
 // bytes (16 threads x 16 bytes), and a scale tile of the destination (512 bytes: 32 lanes x
 // four 32-row groups) is written with one 16-byte store per lane instead of 128 scattered
 // 4-byte stores. Rows are found through the
@@ -317,29 +288,12 @@ cudaError_t launch_nvfp4_quantize_rows(const __nv_bfloat16* x, uint32_t rows, ui
     return cudaGetLastError();
 }
 
-cudaError_t launch_nvfp4_gather_packed(const uint8_t* hidden_packed, const uint8_t* hidden_scale,
-                                       const int32_t* route_prows, uint32_t routes, uint32_t top_k,
-                                       uint32_t hidden_size, uint8_t* packed, uint8_t* scale_tiled,
-                                       cudaStream_t stream, int src_scale_tiled)
-{
-    const uint64_t total = static_cast<uint64_t>(routes) * (hidden_size / 64);
-    gather_packed_kernel<<<blocks_for(total, 256), 256, 0, stream>>>(
-        hidden_packed, hidden_scale, route_prows, total, top_k, hidden_size, packed, scale_tiled,
-        src_scale_tiled);
-    note_launch();
-    return cudaGetLastError();
-}
-
 cudaError_t launch_nvfp4_gather_tiles(const uint8_t* hidden_packed, const uint8_t* hidden_scale, const RouteTables& rt,
-                                      uint32_t routes, uint32_t top_k, uint32_t hidden_size, uint8_t* packed,
-                                      uint8_t* scale_tiled, cudaStream_t stream, int src_scale_tiled)
+                                      uint32_t hidden_size, uint8_t* packed, uint8_t* scale_tiled, cudaStream_t stream,
+                                      int src_scale_tiled)
 {
     if (rt.max_tiles == 0)
         return cudaSuccess;
-    // 32-row tiles (decode batches) hold a few rows each: a thread per (route, k group) does better there
-    if (rt.tile_rows != 128)
-        return launch_nvfp4_gather_packed(hidden_packed, hidden_scale, rt.route_prows, routes, top_k, hidden_size,
-                                          packed, scale_tiled, stream, src_scale_tiled);
     const dim3 grid((hidden_size + kGatherChunk - 1) / kGatherChunk, rt.max_tiles, 1);
     gather_packed_tiles_kernel<<<grid, 256, 0, stream>>>(hidden_packed, hidden_scale, rt, hidden_size, packed,
                                                         scale_tiled, src_scale_tiled);

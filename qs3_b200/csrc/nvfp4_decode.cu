@@ -1,28 +1,33 @@
-// NVFP4 grouped GEMMs for decode-sized batches, where an expert gets a handful of rows.
+// NVFP4 grouped GEMMs for experts with few rows (decode batches, chunks of a prefill): weight streaming.
 //
-// The prefill kernel (gemm.cu) makes the expert's token rows the M = 128 side of the MMA:
-// with three rows per expert 97 % of every instruction multiplies padding, and the tensor
-// pipe, not the weight stream, bounds the layer. Here the operands are swapped, as in the FP8
-// decode kernel: the 128 WEIGHT rows of a feature block are M, the expert's token tile of 32
-// padded rows is N, so one instruction is a quarter of the work and the kernel runs at the
-// speed the weights arrive from HBM.
+// With token rows as the M = 128 side of the MMA most of every instruction multiplies padding. Here the operands are
+// swapped: the 128 WEIGHT rows of a feature block are M, the expert's token tile of NT (32 or 64) padded rows is N,
+// and the kernel runs at the speed the weights arrive from HBM.
 //
-//   grid   (feature splits, token tiles); one CTA = one 32-row token tile of one expert and a
-//          range of 128-row feature blocks of that expert's weight
-//   smem   token panel (all of k: k/256 tiles of 32 x 128 B) resident, its scale tiles (later the
-//          gate / up exchange buffer);
-//          weight ring: stages x (128 x 128 B codes + 4 scale tiles)
-//   TMEM   2 accumulators of 32 columns (lane = feature, column = token) | 2 x 16 columns of
-//          weight scales (alternating per k block) | token scales of all of k
-//   warps  0-3 epilogue, 4 producer (TMA), 5 MMA issuer
+//   grid   persistent, one CTA per SM; the (token tile, feature block) units are cut into equal contiguous ranges
+//          (the CTA-per-tile grid of an earlier version lost a load latency per CTA and its last wave)
+//   smem   token panel (all of k: k/256 tiles of NT x 128 B), its scale tiles, weight ring: stages x (128 x 128 B
+//          codes + 4 scale tiles); gated: f32 exchange buffer of 32 tokens x (64 gate + 64 up) values
+//   TMEM   2 or 4 accumulators of NT columns (lane = weight row, column = token) | 16 columns of weight scales per ring
+//          stage | 2 x token scales of all of k (alternating per tile)
+//   warps  0-3 epilogue, 4 weight producer (TMA), 5 and 11 MMA issuers, 6 scale copier, 7-10 panel loaders
 //
-// Scale tiles are the library's tiled layout (include/qs3_moe.h): 512 bytes per (128-row
-// block, 64-element k group), byte = (row % 32) * 16 + (row / 32 % 4) * 4 + k / 16 % 4, which
-// tcgen05.cp.32x128b.warpx4 turns into four TMEM columns, one per group of 32 rows. A token
-// tile of 32 rows is one such group. Its scale words are picked out of the tiles in global
-// memory by the epilogue warps (idle until the first accumulator is ready) and laid down in
-// shared memory as tiles whose group 0 is this token tile, so that the MMA reads them from the
-// first column of a 4-column aligned tensor-memory address like any other scale operand.
+// The panel loaders fetch the token rows themselves, through the routing tables when the rows are still in token
+// order (no gather pass), and hold the next tile's rows in registers while the current tile is multiplied, so that a
+// change of tile costs the MMA thread only their shared-memory stores; the ring covers those. The scale copies
+// (tcgen05.cp) come from a warp of their own: from the MMA thread each costs ~50 cycles.
+//
+// Gated epilogue: gate rows are lanes 0-63, up rows lanes 64-127. The values go through shared memory so that one
+// thread holds one 16-feature block of one token: SwiGLU, block maximum and quantisation without shuffles, and the
+// time does not grow with the rows of the tile.
+//
+// Scale tiles are the library's tiled layout (include/qs3_moe.h): 512 bytes per (128-row block, 64-element k group),
+// byte = (row % 32) * 16 + (row / 32 % 4) * 4 + k / 16 % 4, which tcgen05.cp.32x128b.warpx4 turns into four TMEM
+// columns, one per group of 32 rows. The loaders lay the token tile's scale words down as groups 0 (and 1) of such
+// tiles, so that the MMA reads them from a 4-column aligned tensor-memory address like any other scale operand.
+//
+// Bound by HBM: hit experts * weight bytes. 128 tokens, 512 experts top-10 (471 hit): gate_up 0.112 -> 0.092 ms
+// (6.0 TB/s), down 0.055 -> 0.050; 1021 tokens: gate_up 0.150 -> 0.110, down 0.110 -> 0.058 ms against 128-row tiles.
 #include "common.cuh"
 #include "nvfp4.cuh"
 #include "tcgen05.cuh"
@@ -34,15 +39,16 @@ namespace {
 
 using namespace tc;
 
-constexpr int kSwThreads = 192;
-constexpr uint32_t kSwTokens = 32;                // token rows per tile = MMA N
-constexpr uint32_t kSwPanelTile = kSwTokens * 128; // one k block of the token panel
+constexpr int kSwThreads = 384;
+constexpr uint32_t kSwLoaders = 128;               // threads of the panel loaders
 constexpr uint32_t kSwStageBytes = kTileBytes + kSfBytes;
-constexpr uint32_t kSwMaxStages = 8;
-constexpr uint32_t kSwMaxKBlocks = 8;             // k <= 2048
-constexpr uint32_t kSwMiscBytes = 1024;
-constexpr uint32_t kSwUpBytes = 64 * kSwTokens * 4; // gated: up values handed to the gate warps
-constexpr uint32_t kSwTmemCols = 256;             // 64 acc + 32 weight scales + <= 128 token scales
+constexpr uint32_t kSwMaxStages = 9;
+constexpr uint32_t kSwMaxAcc = 4;
+constexpr uint32_t kSwMaxKBlocks = 8;              // k <= 2048
+constexpr uint32_t kSwMiscBytes = 512;
+constexpr uint32_t kSwExPitch = 68;                // floats per token row of the exchange buffer (no bank conflicts)
+constexpr uint32_t kSwExBytes = 2 * 32 * kSwExPitch * 4;
+constexpr uint32_t kSwBatch = 16;                  // 16-byte vectors a loader thread keeps in registers
 
 enum : uint32_t {
     ERR_SW_PANEL_WAIT = 0x54000001u,
@@ -50,6 +56,8 @@ enum : uint32_t {
     ERR_SW_EMPTY_WAIT = 0x54000003u,
     ERR_SW_ACC_FULL_WAIT = 0x54000004u,
     ERR_SW_ACC_EMPTY_WAIT = 0x54000005u,
+    ERR_SW_PANEL_FREE_WAIT = 0x54000006u,
+    ERR_SW_SF_WAIT = 0x54000007u,
 };
 
 struct SwapParams {
@@ -58,9 +66,14 @@ struct SwapParams {
     uint32_t kgroups;    // k / 64
     uint32_t b_rows;     // weight rows per group (gated: 2 n)
     uint32_t num_fb;     // feature blocks: n / 128 (gated: n / 64)
-    uint32_t fb_per_cta;
     uint32_t stages;
-    const uint8_t* x_sf; // token scales, tiled by padded row
+    uint32_t acc_mask;   // accumulators - 1 (2 or 4 of them)
+    const uint8_t* x;    // token codes [rows, k / 2]
+    const uint8_t* x_sf; // their scales, tiled by row (x_sf_linear: row-major)
+    int x_sf_linear;
+    const int32_t* row_tokens; // NULL: x rows are the padded rows; else dense row -> x row
+    const int32_t* indptr;     // with row_tokens: segment starts, dense and padded
+    const int32_t* pad_indptr;
     const uint8_t* w_sf; // weight scales, tiled per group
     uint64_t w_sf_group_stride;
     const int32_t* tile_expert;
@@ -76,40 +89,31 @@ struct SwapParams {
     uint32_t* err;
 };
 
-template <bool GATED>
-__global__ void __launch_bounds__(kSwThreads, 2)
-gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-                       const SwapParams p)
+template <int NT, bool GATED>
+__global__ void __launch_bounds__(kSwThreads, 1)
+gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const SwapParams p)
 {
-    const uint32_t tile = blockIdx.y;
-    if (static_cast<int>(tile) >= *p.total_tiles)
-        return;
-    const uint32_t fb0 = blockIdx.x * p.fb_per_cta;
-    const uint32_t fb1 = min(p.num_fb, fb0 + p.fb_per_cta);
-    if (fb0 >= fb1)
-        return;
-    const int expert = p.tile_expert[tile];
-    const int row0 = p.tile_row0[tile];
-    const int nrows = p.tile_nrows[tile];
     constexpr uint32_t kFeat = GATED ? 64 : 128; // output features per feature block
+    constexpr uint32_t kPanelTile = NT * 128;    // one k block of the token panel
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    uint8_t* panel = smem;                                   // k_blocks x 4 KB
-    uint8_t* panel_sf = panel + p.k_blocks * kSwPanelTile;   // kgroups x 512 B
-    uint8_t* ring = panel_sf + max((p.kgroups * 512u + 1023u) & ~1023u, GATED ? kSwUpBytes : 0u);
-    uint8_t* misc = ring + p.stages * kSwStageBytes;
+    uint8_t* panel = smem;                                        // k_blocks x NT x 128 B
+    uint8_t* ring = panel + p.k_blocks * kPanelTile;
+    uint8_t* panel_sf = ring + p.stages * kSwStageBytes;          // kgroups x 512 B
+    float* s_ex = reinterpret_cast<float*>(panel_sf + p.kgroups * 512); // gated: [2][32][kSwExPitch]
+    uint8_t* misc = panel_sf + p.kgroups * 512 + (GATED ? kSwExBytes : 0);
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(misc);
     uint64_t* empty_bar = full_bar + kSwMaxStages;
-    uint64_t* acc_full = empty_bar + kSwMaxStages;
-    uint64_t* acc_empty = acc_full + 2;
-    uint64_t* panel_bar = acc_empty + 2;
-    uint64_t* sf_bar = panel_bar + 1;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(misc + 256);
+    uint64_t* sf_ready = empty_bar + kSwMaxStages;
+    uint64_t* acc_full = sf_ready + kSwMaxStages;
+    uint64_t* acc_empty = acc_full + kSwMaxAcc;
+    uint64_t* panel_full = acc_empty + kSwMaxAcc;  // loaders -> MMA: the tile's codes are in the panel
+    uint64_t* panel_free = panel_full + 1; // MMA -> loaders: the tile's MMAs are done
+    uint64_t* psf_full = panel_free + 1;   // loaders -> copier: the tile's scale words are in panel_sf
+    uint64_t* psf_free = psf_full + 1;     // copier -> loaders: they are in tensor memory
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(psf_free + 1);
     volatile uint32_t* abort_flag = tmem_slot + 1;
-    // [token][64 features], gated only; reuses the token scale tiles, which are dead once copied to
-    // tensor memory (the first accumulator is complete only after those copies)
-    float* s_up = reinterpret_cast<float*>(panel_sf);
 
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31;
@@ -118,20 +122,23 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         for (uint32_t s = 0; s < p.stages; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
+            mbar_init(&sf_ready[s], 1);
         }
-        for (int b = 0; b < 2; ++b) {
+        for (uint32_t b = 0; b < kSwMaxAcc; ++b) {
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 4); // one arrival per epilogue warp
         }
-        mbar_init(panel_bar, 1);
-        mbar_init(sf_bar, 1);
+        mbar_init(panel_full, 1);
+        mbar_init(panel_free, 2); // one arrival per MMA issuer
+        mbar_init(psf_full, 1);
+        mbar_init(psf_free, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 5) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(kSwTmemCols)
+                     "r"(512u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -139,18 +146,25 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t tmem_wsf = tmem_base + 64;  // 2 x 16 columns
-    const uint32_t tmem_xsf = tmem_base + 96;  // kgroups x 4 columns
+    const uint32_t tmem_wsf = tmem_base + (p.acc_mask + 1) * NT; // 16 columns per ring stage
+    const uint32_t tmem_xsf = tmem_wsf + 16 * p.stages;          // 2 x 4 columns per k group
+    const uint32_t xsf_cols = 4 * p.kgroups;
+
+    // this CTA's units: feature blocks [u0, u1) of the tiles in order
+    const uint64_t total = static_cast<uint64_t>(*p.total_tiles) * p.num_fb;
+    const uint32_t u0 = static_cast<uint32_t>(total * blockIdx.x / gridDim.x);
+    const uint32_t u1 = static_cast<uint32_t>(total * (blockIdx.x + 1) / gridDim.x);
+    const uint32_t tile_first = u0 / p.num_fb, fb_first = u0 % p.num_fb;
+    const uint32_t acc_shift = p.acc_mask == 3 ? 2 : 1;
 
     if (warp == 4) {
         // ------------------------------------------------------------ producer --
         if (lane == 0) {
-            mbar_expect_tx(panel_bar, p.k_blocks * kSwPanelTile);
-            for (uint32_t kb = 0; kb < p.k_blocks; ++kb)
-                tma_load_2d(panel + kb * kSwPanelTile, &map_x, panel_bar, static_cast<int>(kb * 128), row0);
             uint32_t s = 0, ph = 0;
             bool ok = true;
-            for (uint32_t fb = fb0; fb < fb1 && ok; ++fb) {
+            uint32_t tile = tile_first, fb = fb_first;
+            for (uint32_t u = u0; u < u1 && ok; ++u) {
+                const int expert = p.tile_expert[tile];
                 const int w_row = expert * static_cast<int>(p.b_rows) + static_cast<int>(fb * kFeat);
                 const uint8_t* sf_src = p.w_sf + static_cast<uint64_t>(expert) * p.w_sf_group_stride
                     + (static_cast<uint64_t>(fb) * p.kgroups) * 512;
@@ -174,147 +188,285 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                         ph ^= 1;
                     }
                 }
+                if (++fb == p.num_fb) {
+                    fb = 0;
+                    ++tile;
+                }
             }
         }
-    } else if (warp == 5) {
-        // ---------------------------------------------------------- MMA issuer --
+    } else if (warp == 5 || warp == 11) {
+        // --------------------------------------------------------- MMA issuers --
+        // Alternate feature blocks: one thread's instructions, waits and commits take longer than the weights of a
+        // feature block with a short k (down of a 128-token batch: one issuer 0.056 ms, two 0.050).
         if (lane == 0) {
-            // M = 128 weight rows, N = 32 tokens, e2m1 x e2m1 with e4m3 block scales, f32 accumulate
-            constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((kSwTokens >> 3) << 17) | ((kBM >> 4) << 24);
-            bool ok = mbar_wait<true>(panel_bar, 0, abort_flag, p.err, ERR_SW_PANEL_WAIT)
-                && mbar_wait<true>(sf_bar, 0, abort_flag, p.err, ERR_SW_PANEL_WAIT);
-            if (ok) {
-                tc_fence_after();
-                for (uint32_t g = 0; g < p.kgroups; ++g)
-                    tc_cp_scales(tmem_xsf + 4 * g, scale_desc(smem_u32(panel_sf) + g * 512));
-            }
-            uint32_t s = 0, ph = 0, sf_flip = 0, u = 0;
-            for (uint32_t fb = fb0; fb < fb1 && ok; ++fb, ++u) {
-                const uint32_t buf = u & 1;
-                if (!mbar_wait<true>(&acc_empty[buf], ((u >> 1) & 1) ^ 1, abort_flag, p.err, ERR_SW_ACC_EMPTY_WAIT)) {
+            // M = 128 weight rows, N = NT tokens, e2m1 x e2m1 with e4m3 block scales, f32 accumulate
+            constexpr uint32_t kIdesc
+                = (1u << 7) | (1u << 10) | ((static_cast<uint32_t>(NT) >> 3) << 17) | ((kBM >> 4) << 24);
+            const uint32_t mine = warp == 5 ? 0 : 1; // parity of this issuer's feature blocks
+            uint32_t s = 0, ph = 0, fb = fb_first, i = 0; // i: tiles this CTA has started
+            bool ok = true;
+            for (uint32_t u = u0; u < u1 && ok; ++u) {
+                const bool first = u == u0 || fb == 0;
+                if (++fb == p.num_fb)
+                    fb = 0;
+                const bool last = u + 1 == u1 || fb == 0;
+                const uint32_t buf = (u - u0) & p.acc_mask;
+                if (first) {
+                    ok = mbar_wait<true>(panel_full, i & 1, abort_flag, p.err, ERR_SW_PANEL_WAIT);
+                    ++i;
+                }
+                if (ok && ((u - u0) & 1) != mine) {
+                    // the other issuer's: its stages are waited for all the same, because a parity tells two
+                    // successive uses of a stage apart and no more
+                    for (uint32_t kb = 0; kb < p.k_blocks && ok; ++kb) {
+                        ok = mbar_wait<true>(&sf_ready[s], ph, abort_flag, p.err, ERR_SW_SF_WAIT);
+                        if (++s == p.stages) {
+                            s = 0;
+                            ph ^= 1;
+                        }
+                    }
+                    if (ok && last)
+                        tc_commit(panel_free);
+                    continue;
+                }
+                if (!ok
+                    || !mbar_wait<true>(&acc_empty[buf], (((u - u0) >> acc_shift) & 1) ^ 1, abort_flag, p.err,
+                                        ERR_SW_ACC_EMPTY_WAIT)) {
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t d = tmem_base + buf * kSwTokens;
+                const uint32_t d = tmem_base + buf * NT;
+                const uint32_t xsf = tmem_xsf + xsf_cols * ((i - 1) & 1);
                 for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
-                    if (!mbar_wait<true>(&full_bar[s], ph, abort_flag, p.err, ERR_SW_FULL_WAIT)) {
+                    // the stage's scales are in tensor memory (the copier waited for the stage's loads)
+                    if (!mbar_wait<true>(&sf_ready[s], ph, abort_flag, p.err, ERR_SW_SF_WAIT)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sb = smem_u32(ring + s * kSwStageBytes);
-                    const uint32_t wsf = tmem_wsf + 16 * sf_flip;
-                    sf_flip ^= 1;
+                    const uint64_t da = operand_desc(smem_u32(ring + s * kSwStageBytes));
+                    const uint64_t db = operand_desc(smem_u32(panel + kb * kPanelTile));
 #pragma unroll
                     for (uint32_t j = 0; j < 4; ++j)
-                        tc_cp_scales(wsf + 4 * j, scale_desc(sb + kTileBytes + j * 512));
-                    const uint64_t da = operand_desc(sb);
-                    const uint64_t db = operand_desc(smem_u32(panel + kb * kSwPanelTile));
-#pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j)
-                        tc_mma_nvfp4(d, da + 2 * j, db + 2 * j, kIdesc, (kb > 0 || j > 0) ? 1u : 0u, wsf + 4 * j,
-                                     tmem_xsf + 16 * kb + 4 * j);
+                        tc_mma_nvfp4(d, da + 2 * j, db + 2 * j, kIdesc, (kb > 0 || j > 0) ? 1u : 0u,
+                                     tmem_wsf + 16 * s + 4 * j, xsf + 16 * kb + 4 * j);
                     tc_commit(&empty_bar[s]);
                     if (++s == p.stages) {
                         s = 0;
                         ph ^= 1;
                     }
                 }
-                if (ok)
+                if (ok) {
                     tc_commit(&acc_full[buf]);
+                    if (last)
+                        tc_commit(panel_free);
+                }
             }
+        }
+    } else if (warp == 6) {
+        // -------------------------------------------------------- scale copier --
+        if (lane == 0) {
+            uint32_t s = 0, ph = 0, fb = fb_first, i = 0;
+            bool ok = true;
+            for (uint32_t u = u0; u < u1 && ok; ++u) {
+                if (u == u0 || fb == 0) {
+                    // the tile's token scales, into the columns of the tile before last: its MMAs are done, because
+                    // the loaders waited for that before they filled the panel of the tile in between
+                    ok = mbar_wait<true>(psf_full, i & 1, abort_flag, p.err, ERR_SW_PANEL_WAIT);
+                    if (!ok)
+                        break;
+                    tc_fence_after();
+                    for (uint32_t g = 0; g < p.kgroups; ++g)
+                        tc_cp_scales(tmem_xsf + xsf_cols * (i & 1) + 4 * g, scale_desc(smem_u32(panel_sf) + g * 512));
+                    tc_commit(psf_free);
+                    ++i;
+                }
+                if (++fb == p.num_fb)
+                    fb = 0;
+                for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
+                    // the stage was refilled, so the MMAs that read its scale columns last time round are done
+                    if (!mbar_wait<true>(&full_bar[s], ph, abort_flag, p.err, ERR_SW_FULL_WAIT)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t sf = smem_u32(ring + s * kSwStageBytes) + kTileBytes;
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j)
+                        tc_cp_scales(tmem_wsf + 16 * s + 4 * j, scale_desc(sf + j * 512));
+                    tc_commit(&sf_ready[s]);
+                    if (++s == p.stages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp >= 7 && warp <= 10) {
+        // ------------------------------------------------------- panel loaders --
+        const uint32_t t = threadIdx.x - 7 * 32;
+        const uint32_t vecs = p.k_blocks * 8;      // 16-byte vectors per row
+        uint32_t i = 0;
+        bool ok = true;
+        for (uint32_t u = u0; u < u1 && ok; u = (u / p.num_fb + 1) * p.num_fb, ++i) {
+            const uint32_t tile = u / p.num_fb;
+            const uint32_t row0 = static_cast<uint32_t>(p.tile_row0[tile]);
+            const uint32_t nrows = static_cast<uint32_t>(p.tile_nrows[tile]);
+            const int32_t* rows = nullptr;
+            if (p.row_tokens != nullptr) {
+                const int expert = p.tile_expert[tile];
+                rows = p.row_tokens + p.indptr[expert] + (row0 - static_cast<uint32_t>(p.pad_indptr[expert]));
+            }
+            const auto src_row = [&](uint32_t j) -> uint64_t {
+                return rows != nullptr ? static_cast<uint64_t>(rows[j]) : static_cast<uint64_t>(row0) + j;
+            };
+            // the tile's codes (the first kSwBatch vectors a thread) and scale words travel together
+            const uint32_t items = nrows * vecs, words = p.kgroups * NT;
+            uint4 v[kSwBatch];
+            const auto load_codes = [&](uint32_t c0) {
+#pragma unroll
+                for (uint32_t q = 0; q < kSwBatch; ++q) {
+                    const uint32_t c = c0 + q * kSwLoaders + t;
+                    if (c < items)
+                        v[q] = *reinterpret_cast<const uint4*>(p.x + src_row(c / vecs) * (vecs * 16) + (c % vecs) * 16);
+                }
+            };
+            const auto store_codes = [&](uint32_t c0) {
+#pragma unroll
+                for (uint32_t q = 0; q < kSwBatch; ++q) {
+                    const uint32_t c = c0 + q * kSwLoaders + t;
+                    if (c < items) {
+                        const uint32_t j = c / vecs, col = c % vecs;
+                        *reinterpret_cast<uint4*>(panel + (col >> 3) * kPanelTile + j * 128 + (((col & 7) ^ (j & 7)) << 4)) = v[q];
+                    }
+                }
+            };
+            load_codes(0);
+            // scale words: (row, k group), a warp takes the rows of one k group
+            for (uint32_t c0 = t; c0 < words; c0 += 8 * kSwLoaders) {
+                uint32_t w[8];
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q) {
+                    const uint32_t c = c0 + q * kSwLoaders, j = c % NT, kg = c / NT;
+                    w[q] = 0;
+                    if (c < words && j < nrows) {
+                        const uint64_t r = src_row(j);
+                        w[q] = *reinterpret_cast<const uint32_t*>(
+                            p.x_sf + (p.x_sf_linear ? r * (p.kgroups * 4) + kg * 4 : tiled_scale_offset(r, 4ull * kg, p.kgroups)));
+                    }
+                }
+                if (c0 == t && i >= 1)
+                    ok = mbar_wait(psf_free, (i - 1) & 1, abort_flag, p.err, ERR_SW_PANEL_FREE_WAIT);
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q) {
+                    const uint32_t c = c0 + q * kSwLoaders, j = c % NT, kg = c / NT;
+                    if (c < words && ok)
+                        *reinterpret_cast<uint32_t*>(panel_sf + kg * 512 + (j & 31) * 16 + (j >> 5) * 4) = w[q];
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // tcgen05.cp reads through the async proxy
+            ok = group_all(2, kSwLoaders, ok);
+            if (!ok)
+                break;
+            if (t == 0)
+                mbar_arrive(psf_full);
+            if (i >= 1)
+                ok = mbar_wait(panel_free, (i - 1) & 1, abort_flag, p.err, ERR_SW_PANEL_FREE_WAIT);
+            for (uint32_t c0 = 0; c0 < items && ok; c0 += kSwBatch * kSwLoaders) {
+                if (c0 != 0)
+                    load_codes(c0);
+                store_codes(c0);
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            ok = group_all(2, kSwLoaders, ok);
+            if (ok && t == 0)
+                mbar_arrive(panel_full);
         }
     } else {
         // ------------------------------------------------------------ epilogue --
-        {
-            // token scales of this tile: word (row, k group) of the tiled layout -> group 0 of a
-            // tile of the same layout in shared memory
-            const uint8_t* src = p.x_sf + (static_cast<uint64_t>(row0 >> 7) * p.kgroups) * 512
-                + ((static_cast<uint32_t>(row0) >> 5) & 3u) * 4;
-            for (uint32_t i = threadIdx.x; i < p.kgroups * 32; i += 128) {
-                const uint32_t kg = i >> 5, r = i & 31;
-                const uint32_t word = *reinterpret_cast<const uint32_t*>(src + kg * 512 + r * 16);
-                *reinterpret_cast<uint4*>(panel_sf + kg * 512 + r * 16) = make_uint4(word, 0u, 0u, 0u);
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // tcgen05.cp reads through the async proxy
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (threadIdx.x == 0)
-                mbar_arrive(sf_bar);
-        }
         const uint32_t lane_base = (warp * 32) << 16;
-        float scale = p.alpha == 0.0f ? 1.0f : p.alpha;
-        float scale_up = scale;
-        if (p.group_scale != nullptr)
-            scale *= p.group_scale[expert];
-        scale_up *= p.group_scale_up != nullptr ? p.group_scale_up[expert]
-                                                : (p.group_scale != nullptr ? p.group_scale[expert] : 1.0f);
-        uint32_t u = 0;
-        for (uint32_t fb = fb0; fb < fb1; ++fb, ++u) {
-            const uint32_t buf = u & 1;
-            bool ready = __all_sync(
-                0xffffffffu, mbar_wait(&acc_full[buf], (u >> 1) & 1, abort_flag, p.err, ERR_SW_ACC_FULL_WAIT));
+        uint32_t tile = tile_first, fb_next = fb_first, row0 = 0, nrows = 0;
+        float scale = 1.0f, scale_up = 1.0f;
+        for (uint32_t u = u0; u < u1; ++u) {
+            const uint32_t buf = (u - u0) & p.acc_mask;
+            const uint32_t fb = fb_next;
+            if (u == u0 || fb == 0) { // another tile
+                const int expert = p.tile_expert[tile];
+                row0 = static_cast<uint32_t>(p.tile_row0[tile]);
+                nrows = static_cast<uint32_t>(p.tile_nrows[tile]);
+                scale = p.alpha == 0.0f ? 1.0f : p.alpha;
+                scale_up = scale;
+                if (p.group_scale != nullptr)
+                    scale *= p.group_scale[expert];
+                scale_up *= p.group_scale_up != nullptr ? p.group_scale_up[expert]
+                                                        : (p.group_scale != nullptr ? p.group_scale[expert] : 1.0f);
+            }
+            if (++fb_next == p.num_fb) {
+                fb_next = 0;
+                ++tile;
+            }
+            bool ready = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], ((u - u0) >> acc_shift) & 1, abort_flag, p.err,
+                                                           ERR_SW_ACC_FULL_WAIT));
             if constexpr (GATED)
                 ready = group_all(1, 128, ready); // the four warps meet at barrier 1 below: stop together
             if (!ready)
                 break;
             tc_fence_after();
-            uint32_t v[kSwTokens];
-            tc_ld16(tmem_base + lane_base + buf * kSwTokens, v);
-            tc_ld16(tmem_base + lane_base + buf * kSwTokens + 16, v + 16);
-            tc_ld_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0)
-                mbar_arrive(&acc_empty[buf]);
-            if constexpr (GATED) {
-                // lanes 0-63 of the tile are gate features, lanes 64-127 the up values of the same
-                // features: warps 2 and 3 hand theirs to warps 0 and 1 through shared memory
-                if (warp >= 2) {
 #pragma unroll
-                    for (uint32_t t = 0; t < kSwTokens; ++t)
-                        s_up[t * 64 + (warp - 2) * 32 + lane] = __uint_as_float(v[t]) * scale_up;
+            for (uint32_t hh = 0; hh < NT / 32; ++hh) {
+                const bool any = hh * 32 < nrows; // uniform over the block
+                uint32_t v[32];
+                if (any) {
+                    tc_ld16(tmem_base + lane_base + buf * NT + hh * 32, v);
+                    tc_ld16(tmem_base + lane_base + buf * NT + hh * 32 + 16, v + 16);
+                    tc_ld_wait();
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (warp < 2) {
-                    const uint32_t f = fb * 64 + warp * 32 + lane; // feature of this lane
-                    uint8_t* out = static_cast<uint8_t*>(p.out);
-                    const uint32_t out_kgroups = p.n / 64;
+                if (hh + 1 == NT / 32) { // the accumulator has been read
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0)
+                        mbar_arrive(&acc_empty[buf]);
+                }
+                if (!any)
+                    continue;
+                if constexpr (GATED) {
+                    float* dst = s_ex + (warp >> 1) * 32 * kSwExPitch + (warp & 1) * 32 + lane;
+                    const float sc = warp >= 2 ? scale_up : scale;
 #pragma unroll
-                    for (uint32_t t = 0; t < kSwTokens; ++t) {
-                        if (static_cast<int>(t) < nrows) { // uniform across the warp
-                            const float g = __uint_as_float(v[t]) * scale;
-                            const float a = __fdividef(g, 1.0f + __expf(-g)) * s_up[t * 64 + warp * 32 + lane];
-                            // one scale per 16 features = per half warp (same arithmetic as quantize_block16)
-                            float amax = fabsf(a);
+                    for (uint32_t t = 0; t < 32; ++t)
+                        dst[t * kSwExPitch] = __uint_as_float(v[t]) * sc;
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    // thread = (16-feature block `warp`, token `lane`)
+                    const uint32_t j = hh * 32 + lane;
+                    if (j < nrows) {
+                        const float4* g4 = reinterpret_cast<const float4*>(s_ex + lane * kSwExPitch + warp * 16);
+                        const float4* u4 = reinterpret_cast<const float4*>(s_ex + (32 + lane) * kSwExPitch + warp * 16);
+                        float a[16];
 #pragma unroll
-                            for (int m = 1; m < 16; m <<= 1)
-                                amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
-                            const uint8_t code = f32_to_e4m3_sat(__fdiv_rn(__fdiv_rn(amax, 6.0f), p.out_global));
-                            const float sc = __fmul_rn(e4m3_to_f32(code), p.out_global);
-                            const float q = __fmul_rn(a, sc > 0.0f ? __fdiv_rn(1.0f, sc) : 0.0f);
-                            const float q_next = __shfl_down_sync(0xffffffffu, q, 1);
-                            const uint64_t prow = static_cast<uint64_t>(row0) + t;
-                            if ((lane & 1) == 0) {
-                                uint16_t two; // the code pair in both bytes; the first source is the upper nibble
-                                asm("{\n\t.reg .b8 b;\n\tcvt.rn.satfinite.e2m1x2.f32 b, %2, %1;\n\tmov.b16 %0, {b, b};\n\t}"
-                                    : "=h"(two)
-                                    : "f"(q), "f"(q_next));
-                                out[prow * (p.n / 2) + f / 2] = static_cast<uint8_t>(two & 0xffu);
-                            }
-                            if ((lane & 15) == 0)
-                                p.out_sf[tiled_scale_offset(prow, f / 16, out_kgroups)] = code;
+                        for (int q = 0; q < 4; ++q) {
+                            const float4 g = g4[q], up = u4[q];
+                            a[4 * q] = __fdividef(g.x, 1.0f + __expf(-g.x)) * up.x;
+                            a[4 * q + 1] = __fdividef(g.y, 1.0f + __expf(-g.y)) * up.y;
+                            a[4 * q + 2] = __fdividef(g.z, 1.0f + __expf(-g.z)) * up.z;
+                            a[4 * q + 3] = __fdividef(g.w, 1.0f + __expf(-g.w)) * up.w;
                         }
+                        uint32_t lo, hi;
+                        const uint8_t code = quantize_block16(a, p.out_global, &lo, &hi);
+                        const uint64_t prow = static_cast<uint64_t>(row0) + j;
+                        *reinterpret_cast<uint2*>(static_cast<uint8_t*>(p.out) + prow * (p.n / 2) + fb * 32 + warp * 8)
+                            = make_uint2(lo, hi);
+                        p.out_sf[tiled_scale_offset(prow, fb * 4 + warp, p.n / 64)] = code;
                     }
-                }
-                asm volatile("bar.sync 1, 128;" ::: "memory"); // s_up is reused by the next block
-            } else {
-                const uint32_t f = fb * 128 + warp * 32 + lane;
-                __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
+                    asm volatile("bar.sync 1, 128;" ::: "memory"); // the exchange buffer is reused
+                } else {
+                    const uint32_t f = fb * 128 + warp * 32 + lane;
+                    __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out) + (static_cast<uint64_t>(row0) + hh * 32) * p.n + f;
 #pragma unroll
-                for (uint32_t t = 0; t < kSwTokens; ++t)
-                    if (static_cast<int>(t) < nrows)
-                        out[(static_cast<uint64_t>(row0) + t) * p.n + f] = __float2bfloat16(__uint_as_float(v[t]) * scale);
+                    for (uint32_t t = 0; t < 32; ++t)
+                        if (hh * 32 + t < nrows)
+                            out[static_cast<uint64_t>(t) * p.n] = __float2bfloat16(__uint_as_float(v[t]) * scale);
+                }
             }
         }
     }
@@ -324,29 +476,28 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     __syncthreads();
     if (warp == 5) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kSwTmemCols)
-                     : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
 }
 
-template <bool GATED>
-cudaError_t launch_swap_instance(const CUtensorMap& mw, const CUtensorMap& mx, const SwapParams& sp, dim3 grid,
-                                 size_t smem, cudaStream_t stream)
+template <int NT, bool GATED>
+cudaError_t launch_swap_instance(const CUtensorMap& mw, const SwapParams& sp, uint32_t grid, size_t smem,
+                                 cudaStream_t stream)
 {
-    auto kernel = gemm_nvfp4_swap_kernel<GATED>;
-    static size_t configured[64] = {}; // largest size set so far, per instantiation and device
+    auto kernel = gemm_nvfp4_swap_kernel<NT, GATED>;
+    static bool configured[64] = {}; // per instantiation and device
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess)
         return err;
-    if (dev < 0 || dev >= 64 || configured[dev] < smem) {
-        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (err != cudaSuccess)
             return err;
         if (dev >= 0 && dev < 64)
-            configured[dev] = smem;
+            configured[dev] = true;
     }
-    kernel<<<grid, kSwThreads, smem, stream>>>(mw, mx, sp);
+    kernel<<<grid, kSwThreads, smem, stream>>>(mw, sp);
     note_launch();
     return cudaGetLastError();
 }
@@ -357,7 +508,13 @@ uint32_t nvfp4_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uin
 {
     const bool fits = hidden % 256 == 0 && inter % 256 == 0 && hidden / 256 <= kSwMaxKBlocks
         && inter / 256 <= kSwMaxKBlocks;
-    return fits && routes <= 16u * experts ? kSwTokens : static_cast<uint32_t>(kTileM);
+    if (!fits)
+        return static_cast<uint32_t>(kTileM);
+    // 32-row tiles while nearly every expert fits one; 64-row tiles up to where 128-row tiles of CTA pairs win. The
+    // second line depends on the skew, which the host does not know: with even routing (512 experts top-10) 64-row
+    // tiles win up to ~70 routes per expert (2200 tokens: 0.284 against 0.361 ms), with a Zipf-skewed router only up
+    // to ~22 (1021 tokens: 0.180 against 0.188 ms, 2048: 0.247 against 0.216), so the line lies where neither loses.
+    return routes <= 8 * experts ? 32u : routes <= 22 * experts ? 64u : static_cast<uint32_t>(kTileM);
 }
 
 cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& g, cudaStream_t stream, const char** why)
@@ -368,8 +525,8 @@ cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& g, cudaStream_t stream, co
         return cudaErrorNotSupported;
     };
     const bool gated = g.gated != 0;
-    if (g.tile_expert == nullptr || g.tile_rows != kSwTokens)
-        return fail("the decode NVFP4 GEMM takes grouped problems with 32-row token tiles");
+    if (g.tile_expert == nullptr || (g.tile_rows != 32 && g.tile_rows != 64))
+        return fail("the decode NVFP4 GEMM takes grouped problems with 32- or 64-row token tiles");
     if (g.k % 256 != 0 || g.k / 256 > kSwMaxKBlocks || g.n % 128 != 0 || g.n == 0)
         return fail("the decode NVFP4 GEMM needs k divisible by 256 (<= 2048) and n divisible by 128");
     if (gated ? g.epilogue != EPI_SWIGLU_NVFP4 : g.epilogue != EPI_STORE_BF16)
@@ -388,7 +545,12 @@ cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& g, cudaStream_t stream, co
     sp.kgroups = g.k / 64;
     sp.b_rows = gated ? 2 * g.n : g.n;
     sp.num_fb = gated ? g.n / 64 : g.n / 128;
+    sp.x = static_cast<const uint8_t*>(g.a);
     sp.x_sf = g.a_scale_tiled;
+    sp.x_sf_linear = g.a_scale_linear;
+    sp.row_tokens = g.row_tokens;
+    sp.indptr = g.indptr;
+    sp.pad_indptr = g.pad_indptr;
     sp.w_sf = g.b_scale_tiled;
     sp.w_sf_group_stride = qs3_nvfp4_tiled_scale_bytes(sp.b_rows, g.k);
     sp.tile_expert = g.tile_expert;
@@ -403,32 +565,30 @@ cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& g, cudaStream_t stream, co
     sp.out_global = g.out_global_scale == 0.0f ? 1.0f : g.out_global_scale;
     sp.err = device_error_word();
 
-    const size_t fixed = 1024 + static_cast<size_t>(sp.k_blocks) * kSwPanelTile
-        + std::max((static_cast<size_t>(sp.kgroups) * 512 + 1023) & ~static_cast<size_t>(1023),
-                   static_cast<size_t>(gated ? kSwUpBytes : 0))
-        + kSwMiscBytes;
-    // two CTAs per SM: one CTA's start-up (token panel, scale tiles) hides behind the other's weight stream
-    const size_t budget = 112 * 1024;
-    sp.stages = static_cast<uint32_t>(std::min<size_t>(kSwMaxStages, (budget - fixed) / kSwStageBytes));
+    const size_t fixed = 1024 + static_cast<size_t>(sp.k_blocks) * g.tile_rows * 128 + static_cast<size_t>(sp.kgroups) * 512
+        + (gated ? kSwExBytes : 0) + kSwMiscBytes;
+    // tensor memory: accumulators, 16 scale columns per stage, 2 x 4 token-scale columns per k group. Four accumulators
+    // where they fit: handing one over takes longer than the MMAs of a feature block with a short k (down of a
+    // 128-token batch 0.061 ms with two, 0.056 with four).
+    sp.stages = static_cast<uint32_t>(std::min<size_t>(kSwMaxStages, (227 * 1024 - fixed) / kSwStageBytes));
+    sp.acc_mask = 4 * g.tile_rows + 16 * sp.stages + 8 * sp.kgroups <= 512 ? 3 : 1;
+    sp.stages = std::min(sp.stages, (512 - (sp.acc_mask + 1) * g.tile_rows - 8 * sp.kgroups) / 16);
     const size_t smem = fixed + static_cast<size_t>(sp.stages) * kSwStageBytes;
+    const uint32_t grid = static_cast<uint32_t>(
+        std::min<uint64_t>(static_cast<uint64_t>(g.max_tiles) * sp.num_fb, device_sm_count()));
 
-    // feature splits: about eight CTAs per SM over the launch, so that the tail is short
-    const uint32_t tiles = std::max(1u, std::min(g.max_tiles, g.est_tiles != 0 ? g.est_tiles : g.max_tiles));
-    const uint32_t want = std::max(1u, (8u * device_sm_count() + tiles - 1) / tiles);
-    sp.fb_per_cta = std::max(1u, (sp.num_fb + want - 1) / want);
-    const uint32_t splits = (sp.num_fb + sp.fb_per_cta - 1) / sp.fb_per_cta;
-
-    CUtensorMap mw, mx;
+    CUtensorMap mw;
     if (!make_operand_map(&mw, true, g.b, g.k / 2, static_cast<uint64_t>(g.groups) * sp.b_rows, g.k / 2,
-                          gated ? 64 : 128)
-        || !make_operand_map(&mx, true, g.a, g.k / 2, g.a_rows, g.k / 2, kSwTokens)) {
+                          gated ? 64 : 128)) {
         if (why != nullptr)
             *why = "cuTensorMapEncodeTiled failed";
         return cudaErrorInvalidValue;
     }
-    const dim3 grid(splits, g.max_tiles, 1);
-    return gated ? launch_swap_instance<true>(mw, mx, sp, grid, smem, stream)
-                 : launch_swap_instance<false>(mw, mx, sp, grid, smem, stream);
+    if (g.tile_rows == 32)
+        return gated ? launch_swap_instance<32, true>(mw, sp, grid, smem, stream)
+                     : launch_swap_instance<32, false>(mw, sp, grid, smem, stream);
+    return gated ? launch_swap_instance<64, true>(mw, sp, grid, smem, stream)
+                 : launch_swap_instance<64, false>(mw, sp, grid, smem, stream);
 }
 
 } // namespace qs3

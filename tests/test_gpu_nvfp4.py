@@ -261,3 +261,44 @@ def test_decode_batches_take_the_swapped_operand_kernel(ops, ctx, oracle, cfg):
     ref = oracle.moe_nvfp4(hp, hs, to_np(ids_t), to_np(w_t), _triple(gu), _triple(dn), act_global=0.5,
                            act2_global=0.25, shared=shared_ref, hidden_bf16=d["hidden"])
     _check(to_np(out), ref)
+
+
+@pytest.mark.parametrize("cfg", [
+    dict(t=200, h=512, e=8, k=2, i=256, linear=False),   # 50 rows per expert: 64-row token tiles
+    dict(t=61, h=2048, e=2, k=2, i=512, linear=True),    # 61 rows: a full k panel, a row group that is not full
+    dict(t=33, h=2048, e=2, k=2, i=256, linear=True),    # one row in the second 32-row half
+    dict(t=90, h=256, e=8, k=2, i=256, linear=True, local=(3, 4)),
+])
+def test_64_row_token_tiles(ops, ctx, oracle, cfg):
+    """More than a decode batch's rows per expert, still too few for 128-row tiles: token rows read in place
+    from tiled (layer call) and row-major (declared call) scales."""
+    t, h, e, k, i = (cfg[n] for n in ("t", "h", "e", "k", "i"))
+    off, le = cfg.get("local", (0, e))
+    d = make_moe_inputs(43, t, h, e, i)
+    d["gate_up"], d["down"] = d["gate_up"][off:off + le], d["down"][off:off + le]
+    gu, dn, _ = _quantise_all(ops, ctx, d, False)
+    plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=t, hidden_size=h, intermediate_size=i, num_experts=e,
+                                              top_k=k, local_expert_offset=off, local_num_experts=le,
+                                              backend=ops.capi.MOE_BACKEND_NVFP4))
+    ids, w = oracle.router_topk(oracle.gemm_bf16(d["hidden"], d["router"], "f32"), k, 0, True, 1.0)
+    out = torch.empty((t, h), dtype=torch.bfloat16, device="cuda")
+    hp, hs = oracle.nvfp4_quantize_act(d["hidden"], 1.0)
+    gu_ref, dn_ref = _triple(gu), _triple(dn)
+    if cfg["linear"]:  # this call has no gate_up global scale: quantised against 1, weights scaled up
+        def quantise(x):
+            q = oracle.nvfp4_quantize_act(bf16(f32(x) * 8.0).reshape(-1, x.shape[2]), 1.0)
+            return tuple(v.reshape(le, x.shape[1], -1) for v in q) + (np.ones(le, np.float32),)
+        gu_ref, dn_ref = quantise(d["gate_up"]), quantise(d["down"])
+        ws = torch.zeros(plan.workspace_size(t), dtype=torch.uint8, device="cuda")
+        ops.moe_execute_nvfp4(plan, to_dev(hp), to_dev(hs), to_dev(ids), to_dev(w), *map(to_dev, gu_ref[:2]),
+                              *map(to_dev, dn_ref[:2]), out, ws)
+    else:
+        ws = torch.zeros(plan.layer_workspace_size(t, 0), dtype=torch.uint8, device="cuda")
+        ids_t = torch.empty((t, k), dtype=torch.int32, device="cuda")
+        w_t = torch.empty((t, k), dtype=torch.float32, device="cuda")
+        ops.moe_layer_execute(plan, to_dev(d["hidden"]), to_dev(d["router"]), gu, dn, out, ws, topk_ids=ids_t,
+                              topk_weights=w_t)
+        ids, w = to_np(ids_t), to_np(w_t)
+    torch.cuda.synchronize()
+    assert ctx.read_device_error() == 0
+    _check(to_np(out), oracle.moe_nvfp4(hp, hs, ids, w, gu_ref, dn_ref, local_offset=off))
