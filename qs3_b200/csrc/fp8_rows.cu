@@ -7,18 +7,18 @@
 // (x_scale[token] * w_scale[block]), so promoting an element is a single FMA without any shared-memory operand:
 // 128 x 256 partials cost eight warps about 300 cycles against the ~690 cycles of their four MMAs.
 //
-//   persistent  one CTA per SM; the (token tile, feature block) units are cut into equal contiguous ranges, so
-//               the last round is never nearly empty and neighbouring CTAs share an expert's weights in L2
+//   persistent  one CTA per SM, every gridDim.x-th (token tile, feature block) unit: the CTAs of a round hold
+//               neighbouring units, so a token tile and the weights of an expert with several tiles are read by
+//               several SMs at about the same time (contiguous ranges: gate_up 0.231, down 0.106 ms of the case below)
 //   smem        ring of stages: A 128 x 128 B, B 256 x 128 B; plain: + four 16-KB boxes staging the bf16 tile for
 //               TMA stores
 //   TMEM        two 256-column buffers: k block i + 1 is multiplied while k block i is promoted
 //   warps       0-7 promotion and epilogue (lane quadrant warp % 4, column half warp / 4), 8 producer, 9 MMA
 //
-// Bound by operand delivery: a k block moves 48 KB into the SM for 128 x 256 x 128 products, and the weights, of
-// which every byte is wanted by two or three CTAs, arrive at 45 GB/s per SM (1.09 us per k block; 0.63 us without
-// the loads, 0.76 with promotion but without loads). 4096 tokens x 128 experts top-8 (hidden 2048, intermediate
-// 768): gate_up 0.800 -> 0.231 ms, down 0.238 -> 0.106 ms against the decode kernel on 32-row tiles, which
-// streamed every weight through shared memory once per 32 rows.
+// Bound by operand delivery (48 KB per k block for 128 x 256 x 128 products) and the hand-over of the two buffers:
+// 0.76 us per k block, 0.63 without the loads. 4096 tokens x 128 experts top-8 (hidden 2048, intermediate 768):
+// gate_up 0.800 -> 0.159 ms, down 0.238 -> 0.088 ms against the decode kernel on 32-row tiles, which streamed every
+// weight through shared memory once per 32 rows.
 #include "tcgen05.cuh"
 
 #include <algorithm>
@@ -108,16 +108,16 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    const uint64_t total = static_cast<uint64_t>(*p.total_tiles) * p.units_per_tile;
-    const uint32_t u0 = static_cast<uint32_t>(total * blockIdx.x / gridDim.x);
-    const uint32_t u1 = static_cast<uint32_t>(total * (blockIdx.x + 1) / gridDim.x);
+    // units of this CTA: every gridDim.x-th one. The CTAs of a round hold neighbouring units, so that a token tile
+    // and the weights of an expert with several tiles are read by several SMs at about the same time
+    const uint32_t total = static_cast<uint32_t>(*p.total_tiles) * p.units_per_tile;
 
     if (warp == 8) {
         // ------------------------------------------------------------ producer --
         if (lane == 0) {
             uint32_t s = 0, ph = 0;
             bool ok = true;
-            for (uint32_t u = u0; u < u1 && ok; ++u) {
+            for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x) {
                 const uint32_t tile = u / p.units_per_tile, nb = u % p.units_per_tile;
                 const int row0 = p.tile_row0[tile];
                 const int b_row = p.tile_expert[tile] * static_cast<int>(p.b_rows)
@@ -151,7 +151,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
             constexpr uint32_t kIdesc = (1u << 4) | ((kFrN >> 3) << 17) | ((kBM >> 4) << 24);
             uint32_t s = 0, ph = 0, b = 0, bph = 0;
             bool ok = true;
-            for (uint32_t u = u0; u < u1 && ok; ++u) {
+            for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x) {
                 for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
                     if (!mbar_wait<true>(&acc_empty[b], bph ^ 1, abort_flag, p.err, ERR_FR_ACC_EMPTY_WAIT)
                         || !mbar_wait<true>(&full_bar[s], ph, abort_flag, p.err, ERR_FR_FULL_WAIT)) {
@@ -185,7 +185,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         constexpr uint32_t kSecond = GATED ? 128 : 64; // distance of the second 64 columns
         uint32_t b = 0, bph = 0;
         bool ok = true;
-        for (uint32_t u = u0; u < u1; ++u) {
+        for (uint32_t u = blockIdx.x; u < total; u += gridDim.x) {
             const uint32_t tile = u / p.units_per_tile, nb = u % p.units_per_tile;
             const int expert = p.tile_expert[tile];
             const uint32_t row0 = static_cast<uint32_t>(p.tile_row0[tile]);
