@@ -1,0 +1,311 @@
+// Grouped bf16 GEMM of the routed experts: weight streaming with the operands swapped (weight rows are the M side of
+// the MMA, the expert's token tile of NT padded rows the N side).
+//
+//   unit   one token tile x 256 weight rows of its expert: gated: 128 gate rows and the 128 up rows of the same
+//          features (two accumulators with the same lanes, so SwiGLU needs no exchange); plain: 256 features
+//   grid   persistent, one CTA per SM, every gridDim.x-th unit: the CTAs of a round hold neighbouring units, so a
+//          token tile and the weights of an expert with several tiles are read by several SMs at about the same
+//          time (contiguous ranges of units instead: gate_up of the 2048-token case below 0.425 ms)
+//   smem   ring of stages: two weight tiles 128 x 64 (32 KB) + token tile NT x 64
+//   TMEM   two buffers of two NT-column accumulators (lane = weight row, column = token)
+//   warps  0-3 epilogue, 4 producer (TMA), 5 MMA issuer
+//
+// Bound by HBM while experts have few rows: hit experts * weight bytes. A 128 x 128 tile per CTA moved as many token
+// (mostly padding) as weight bytes into shared memory and multiplied the padding; here a stage moves NT / 256 as
+// many. 33 tokens x 128 experts top-8 (hidden 2048, intermediate 768): gate_up 0.148 -> 0.114 (6.2 TB/s), down
+// 0.072 -> 0.059 ms; 2048 tokens x 512 experts top-10 (intermediate 512): gate_up 0.443 -> 0.370 (5.8 TB/s), down
+// 0.222 -> 0.182 ms.
+#include "tcgen05.cuh"
+
+#include <algorithm>
+
+namespace qs3 {
+namespace {
+
+using namespace tc;
+
+constexpr int kBsThreads = 192;
+constexpr uint32_t kBsMaxStages = 6;
+
+enum : uint32_t {
+    ERR_BS_FULL_WAIT = 0x59000001u,
+    ERR_BS_EMPTY_WAIT = 0x59000002u,
+    ERR_BS_ACC_FULL_WAIT = 0x59000003u,
+    ERR_BS_ACC_EMPTY_WAIT = 0x59000004u,
+};
+
+struct Bf16StreamParams {
+    uint32_t n;            // output features per group (gated: intermediate size)
+    uint32_t k_blocks;     // ceil(k / 64)
+    uint32_t b_rows;       // weight rows per group (gated: 2 n)
+    uint32_t units_per_tile; // gated: ceil(n / 128); plain: ceil(n / 256)
+    const int32_t* tile_expert;
+    const int32_t* tile_row0;
+    const int32_t* tile_nrows;
+    const int32_t* total_tiles;
+    __nv_bfloat16* out;    // [rows, n]
+    uint32_t* err;
+};
+
+template <int NT> struct BsRing {
+    static constexpr uint32_t kStageBytes = 2 * kTileBytes + NT * 128;
+    static constexpr uint32_t kStages = NT == 32 ? kBsMaxStages : NT == 64 ? 5 : 4;
+};
+
+template <int NT, bool GATED>
+__global__ void __launch_bounds__(kBsThreads, 1)
+gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                        const Bf16StreamParams p)
+{
+    constexpr uint32_t kStageBytes = BsRing<NT>::kStageBytes;
+    constexpr uint32_t kNumStages = BsRing<NT>::kStages;
+    constexpr uint32_t kTmemCols = 4 * NT;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kNumStages * kStageBytes);
+    uint64_t* empty_bar = full_bar + kBsMaxStages;
+    uint64_t* acc_full = empty_bar + kBsMaxStages;
+    uint64_t* acc_empty = acc_full + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < kNumStages; ++s) {
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 4); // one arrival per epilogue warp
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 5) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    // unit i of this CTA: the CTAs of a round hold neighbouring units, so that a token tile (and the weights of an
+    // expert with several tiles) is read by several SMs at about the same time
+    const uint32_t total = static_cast<uint32_t>(*p.total_tiles) * p.units_per_tile;
+    const uint32_t my_units = blockIdx.x < total ? (total - blockIdx.x - 1) / gridDim.x + 1 : 0;
+
+    if (warp == 4) {
+        // ------------------------------------------------------------ producer --
+        if (lane == 0) {
+            uint32_t s = 0, ph = 0;
+            bool ok = true;
+            for (uint32_t i = 0; i < my_units && ok; ++i) {
+                const uint32_t u = blockIdx.x + i * gridDim.x, tile = u / p.units_per_tile, nb = u % p.units_per_tile;
+                const int row0 = p.tile_row0[tile];
+                // rows of a tile past the last feature belong to something else and are dropped by the epilogue
+                const int w_row = p.tile_expert[tile] * static_cast<int>(p.b_rows) + static_cast<int>(nb * (GATED ? 128 : 256));
+                const int w_row2 = w_row + (GATED ? static_cast<int>(p.n) : 128);
+                for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
+                    if (!mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_BS_EMPTY_WAIT)) {
+                        ok = false;
+                        break;
+                    }
+                    uint8_t* sw = smem + s * kStageBytes;
+                    mbar_expect_tx(&full_bar[s], kStageBytes);
+                    const int c0 = static_cast<int>(kb) * 64;
+                    tma_load_2d(sw, &map_w, &full_bar[s], c0, w_row);
+                    tma_load_2d(sw + kTileBytes, &map_w, &full_bar[s], c0, w_row2);
+                    tma_load_2d(sw + 2 * kTileBytes, &map_x, &full_bar[s], c0, row0);
+                    if (++s == kNumStages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+            }
+        }
+    } else if (warp == 5) {
+        // ---------------------------------------------------------- MMA issuer --
+        if (lane == 0) {
+            // M = 128 weight rows, N = NT tokens, bf16 x bf16 -> f32, both operands K-major
+            constexpr uint32_t kIdesc
+                = (1u << 4) | (1u << 7) | (1u << 10) | ((static_cast<uint32_t>(NT) >> 3) << 17) | ((kBM >> 4) << 24);
+            uint32_t s = 0, ph = 0;
+            bool ok = true;
+            for (uint32_t i = 0; i < my_units && ok; ++i) {
+                const uint32_t buf = i & 1;
+                if (!mbar_wait<true>(&acc_empty[buf], ((i >> 1) & 1) ^ 1, abort_flag, p.err, ERR_BS_ACC_EMPTY_WAIT))
+                    break;
+                tc_fence_after();
+                const uint32_t d = tmem_base + buf * 2 * NT;
+                for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
+                    if (!mbar_wait<true>(&full_bar[s], ph, abort_flag, p.err, ERR_BS_FULL_WAIT)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t sw = smem_u32(smem + s * kStageBytes);
+                    const uint64_t dw = operand_desc(sw), dw2 = operand_desc(sw + kTileBytes);
+                    const uint64_t dx = operand_desc(sw + 2 * kTileBytes);
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; ++j) {
+                        const uint32_t acc = (kb > 0 || j > 0) ? 1u : 0u;
+                        tc_mma_bf16(d, dw + 2 * j, dx + 2 * j, kIdesc, acc);
+                        tc_mma_bf16(d + NT, dw2 + 2 * j, dx + 2 * j, kIdesc, acc);
+                    }
+                    tc_commit(&empty_bar[s]);
+                    if (++s == kNumStages) {
+                        s = 0;
+                        ph ^= 1;
+                    }
+                }
+                if (ok)
+                    tc_commit(&acc_full[buf]);
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ epilogue --
+        const uint32_t lane_base = (warp * 32) << 16;
+        for (uint32_t i = 0; i < my_units; ++i) {
+            const uint32_t u = blockIdx.x + i * gridDim.x, tile = u / p.units_per_tile, nb = u % p.units_per_tile;
+            const uint32_t buf = i & 1;
+            const uint32_t nrows = static_cast<uint32_t>(p.tile_nrows[tile]);
+            const uint64_t row0 = static_cast<uint64_t>(p.tile_row0[tile]);
+            const uint32_t f = nb * (GATED ? 128 : 256) + warp * 32 + lane; // plain: and f + 128
+            const bool ready = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (i >> 1) & 1, abort_flag, p.err,
+                                                                 ERR_BS_ACC_FULL_WAIT));
+            if (!ready)
+                break;
+            tc_fence_after();
+            const uint32_t src = tmem_base + lane_base + buf * 2 * NT;
+            __nv_bfloat16* out = p.out + row0 * p.n + f;
+#pragma unroll
+            for (uint32_t c = 0; c < NT / 16; ++c) {
+                if (c * 16 >= nrows)
+                    break;
+                uint32_t va[16], vb[16];
+                tc_ld16(src + c * 16, va);
+                tc_ld16(src + NT + c * 16, vb);
+                tc_ld_wait();
+#pragma unroll
+                for (uint32_t t = 0; t < 16; ++t) {
+                    if (c * 16 + t < nrows) { // uniform
+                        const float a = __uint_as_float(va[t]), b = __uint_as_float(vb[t]);
+                        __nv_bfloat16* o = out + static_cast<uint64_t>(c * 16 + t) * p.n;
+                        if constexpr (GATED) {
+                            // upstream stores the gate_up product as bf16 before SwiGLU (qsfi_moe.cu:638-651,445-463)
+                            const float g = round_bf16(a), up = round_bf16(b);
+                            if (f < p.n)
+                                *o = __float2bfloat16(g * sigmoid_fast(g) * up);
+                        } else {
+                            if (f < p.n)
+                                *o = __float2bfloat16(a);
+                            if (f + 128 < p.n)
+                                o[128] = __float2bfloat16(b);
+                        }
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(&acc_empty[buf]);
+        }
+    }
+
+    // ---- teardown ----
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 5) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols)
+                     : "memory");
+    }
+}
+
+template <int NT, bool GATED>
+cudaError_t launch_stream_instance(const CUtensorMap& mw, const CUtensorMap& mx, const Bf16StreamParams& sp,
+                                   uint32_t grid, cudaStream_t stream)
+{
+    auto kernel = gemm_bf16_stream_kernel<NT, GATED>;
+    constexpr size_t smem = 1024 + BsRing<NT>::kStages * BsRing<NT>::kStageBytes + 256;
+    static bool configured[64] = {}; // per instantiation and device
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess)
+        return err;
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (err != cudaSuccess)
+            return err;
+        if (dev >= 0 && dev < 64)
+            configured[dev] = true;
+    }
+    kernel<<<grid, kBsThreads, smem, stream>>>(mw, mx, sp);
+    note_launch();
+    return cudaGetLastError();
+}
+
+} // namespace
+
+uint32_t bf16_tile_rows(uint32_t routes, uint32_t experts)
+{
+    // Token bytes per weight byte grow with the tile, weight passes with the tiles of an expert. Layer times, 128
+    // experts top-8: 8 routes per expert 0.239 ms with 32-row against 0.243 with 64-row tiles, 32 routes of a skewed
+    // router 0.229 against 0.203; 64 routes 0.287 with 64-row against 0.291 with 128-row tiles, 128 routes 0.380
+    // against 0.367.
+    return routes <= 12u * experts ? 32u : routes <= 96u * experts ? 64u : static_cast<uint32_t>(kTileM);
+}
+
+bool bf16_stream_gemm_supported(const GemmProblem& g)
+{
+    return !g.nvfp4 && g.tile_expert != nullptr && (g.tile_rows == 32 || g.tile_rows == 64 || g.tile_rows == 128)
+        && (g.gated ? g.epilogue == EPI_SWIGLU_BF16 : g.epilogue == EPI_STORE_BF16) && g.k % 8 == 0
+        && (g.alpha == 0.0f || g.alpha == 1.0f) && g.beta == 0.0f && g.group_scale == nullptr
+        && g.group_scale_up == nullptr && g.bias == nullptr && g.out_pitch_elems == g.n
+        && (reinterpret_cast<uintptr_t>(g.a) & 15u) == 0 && (reinterpret_cast<uintptr_t>(g.b) & 15u) == 0
+        && g.a_pitch_bytes % 16 == 0 && g.b_pitch_bytes % 16 == 0;
+}
+
+cudaError_t launch_bf16_stream_gemm(const GemmProblem& g, cudaStream_t stream, const char** why)
+{
+    Bf16StreamParams sp {};
+    sp.n = g.n;
+    sp.k_blocks = (g.k + 63) / 64;
+    sp.b_rows = g.gated ? 2 * g.n : g.n;
+    sp.units_per_tile = g.gated ? (g.n + 127) / 128 : (g.n + 255) / 256;
+    sp.tile_expert = g.tile_expert;
+    sp.tile_row0 = g.tile_row0;
+    sp.tile_nrows = g.tile_nrows;
+    sp.total_tiles = g.total_tiles;
+    sp.out = static_cast<__nv_bfloat16*>(g.out);
+    sp.err = device_error_word();
+    CUtensorMap mw, mx;
+    if (!make_operand_map(&mw, false, g.b, g.k, static_cast<uint64_t>(g.groups) * sp.b_rows, g.b_pitch_bytes, 128)
+        || !make_operand_map(&mx, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, g.tile_rows)) {
+        if (why != nullptr)
+            *why = "cuTensorMapEncodeTiled failed";
+        return cudaErrorInvalidValue;
+    }
+    const uint32_t grid = static_cast<uint32_t>(
+        std::min<uint64_t>(static_cast<uint64_t>(g.max_tiles) * sp.units_per_tile, device_sm_count()));
+    switch (g.tile_rows) {
+    case 32:
+        return g.gated ? launch_stream_instance<32, true>(mw, mx, sp, grid, stream)
+                       : launch_stream_instance<32, false>(mw, mx, sp, grid, stream);
+    case 64:
+        return g.gated ? launch_stream_instance<64, true>(mw, mx, sp, grid, stream)
+                       : launch_stream_instance<64, false>(mw, mx, sp, grid, stream);
+    default:
+        return g.gated ? launch_stream_instance<128, true>(mw, mx, sp, grid, stream)
+                       : launch_stream_instance<128, false>(mw, mx, sp, grid, stream);
+    }
+}
+
+} // namespace qs3

@@ -265,6 +265,11 @@ cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& p, cudaStream_t stream, co
 // Rows per token tile of an NVFP4 plan: 32 or 64 (decode kernel) when experts get few rows each, else 128.
 uint32_t nvfp4_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter);
 bool gemm_tc_supported(const GemmProblem& p);
+// bf16 grouped GEMM of the routed experts, weights streamed as the M side (bf16_stream.cu), and the rows per token
+// tile of a bf16 plan.
+bool bf16_stream_gemm_supported(const GemmProblem& p);
+cudaError_t launch_bf16_stream_gemm(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);
+uint32_t bf16_tile_rows(uint32_t routes, uint32_t experts);
 
 // ---- NVFP4 ----------------------------------------------------------------------
 // Token rows in token order -> e2m1 codes and scales tiled by token row.

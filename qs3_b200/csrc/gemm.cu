@@ -1,11 +1,11 @@
 // Grouped / dense GEMM  D[m, n] = sum_k A[m, k] * B[g][n, k]. Kernels in this file:
-//   gemm_tc_kernel        tcgen05, one 128 x 128 tile per CTA: grouped bf16 problems, NVFP4 with k > 2048
-//                         (dense bf16 problems with more than 64 rows go to gemm_dense.cu)
+//   gemm_tc_kernel        tcgen05, one 128 x 128 tile per CTA: dense bf16 problems with few tiles, NVFP4 with
+//                         k > 2048 (grouped bf16 problems go to bf16_stream.cu, larger dense ones to gemm_dense.cu)
 //   gemm_tc_astat_kernel  tcgen05, NVFP4 with the A panel resident in shared memory (k <= 2048)
 //   gemm_skinny_kernel    CUDA cores, bf16 with at most 64 rows (router logits of a decode batch)
 //   gemm_simt_kernel      CUDA cores, shapes the tensor-core tiles cannot address
-// launch_gemm() at the end picks one of these, the dense kernel of gemm_dense.cu or the decode
-// kernel of nvfp4_decode.cu.
+// launch_gemm() at the end picks one of these, a kernel of gemm_dense.cu, gemm_pair.cu or bf16_stream.cu, or the
+// decode kernel of nvfp4_decode.cu.
 //
 // gemm_tc_kernel: one 128 x 128 output tile per CTA on the 5th-generation tensor cores:
 //
@@ -967,6 +967,8 @@ cudaError_t launch_gemm(const GemmProblem& g, cudaStream_t stream, const char** 
         *why = nullptr;
     if (g.nvfp4 && g.tile_expert != nullptr && g.tile_rows != 0 && g.tile_rows != static_cast<uint32_t>(kBM))
         return launch_nvfp4_swap_gemm(g, stream, why);
+    if (bf16_stream_gemm_supported(g))
+        return g.max_tiles == 0 || g.n == 0 ? cudaSuccess : launch_bf16_stream_gemm(g, stream, why);
     TcParams tp = make_params(g);
     const uint32_t m_tiles = g.tile_expert != nullptr
         ? g.max_tiles

@@ -80,7 +80,8 @@ Bf16Workspace carve_bf16(char* base, const qsfi_moe_plan_desc& d, uint32_t num_t
 {
     Bf16Workspace w {};
     const uint32_t routes = num_tokens * d.top_k;
-    size_t off = route_tables_carve(base, routes, d.local_num_experts, &w.rt);
+    size_t off = route_tables_carve(base, routes, d.local_num_experts, &w.rt,
+                                    bf16_tile_rows(routes, d.local_num_experts));
     const size_t rows = w.rt.max_pad_rows;
     w.expanded = carve<__nv_bfloat16>(base, off, rows * d.hidden_size);
     w.act = carve<__nv_bfloat16>(base, off, rows * d.intermediate_size);

@@ -59,6 +59,8 @@ def _check(out, ref):
     dict(t=77, h=72, e=5, k=3, i=40),        # ragged k and n tails on the tensor-core kernel
     dict(t=300, h=512, e=16, k=4, i=192),    # several row tiles per expert
     dict(t=64, h=1024, e=64, k=8, i=256, hot=True),
+    dict(t=97, h=264, e=6, k=2, i=136),      # 64-row token tiles; features one block past the weight tiles
+    dict(t=400, h=128, e=4, k=2, i=264),     # 128-row token tiles, several per expert; plain n of half a unit
 ])
 def test_matches_oracle(ops, oracle, cfg):
     t, h, e, k, i = cfg["t"], cfg["h"], cfg["e"], cfg["k"], cfg["i"]
