@@ -2,7 +2,8 @@
 
 ``python -m qs3_b200._build`` compiles every translation unit under
 ``qs3_b200/csrc`` with nvcc for ``sm_100a`` and links them into
-``qs3_b200/libqs3moe.so``. nvcc cross-compiles without a GPU, so this also runs
+``qs3_b200/libqs3moe.so``, and the descriptor-marshalling extension ``qs3_b200/_marshal.so``
+with g++. nvcc cross-compiles without a GPU, so this also runs
 on a CPU-only machine; the shared object is what a GPU machine loads.
 """
 from __future__ import annotations
@@ -17,6 +18,7 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 SRC_DIR = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(SRC_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libqs3moe.so")
+MARSHAL_PATH = os.path.join(PKG_DIR, "_marshal.so")
 CHECKED_LIB_PATH = os.path.join(PKG_DIR, "libqs3moe_checked.so")
 
 SOURCES = ["context.cu", "router.cu", "routing.cu", "gemm.cu", "gemm_api.cu", "nvfp4.cu", "moe.cu",
@@ -44,6 +46,26 @@ def _stale(target: str, deps: list[str]) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_marshal(force: bool = False) -> str:
+    """Compile the Python extension that fills descriptors from torch tensors (``csrc/marshal.cpp``)."""
+    src = os.path.join(SRC_DIR, "marshal.cpp")
+    if force or _stale(MARSHAL_PATH, [src, os.path.join(SRC_DIR, HEADERS[-1])]):
+        import sysconfig
+
+        import torch
+        base = os.path.dirname(torch.__file__)
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", src, "-o", MARSHAL_PATH,
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               *(f"-I{d}" for d in (os.path.join(base, "include"),
+                                    os.path.join(base, "include", "torch", "csrc", "api", "include"),
+                                    sysconfig.get_paths()["include"])),
+               f"-L{os.path.join(base, 'lib')}", "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed on {src}:\n{r.stdout}\n{r.stderr}")
+    return MARSHAL_PATH
+
+
 def build(force: bool = False, verbose: bool = False, checked: bool = False) -> str:
     """Compile the library in-tree. ``checked`` builds the variant with device-side input
     validation (``-DQSFI_ENABLE_CHECKED_VALIDATION=1``, as upstream's checked test binary):
@@ -69,12 +91,14 @@ def build(force: bool = False, verbose: bool = False, checked: bool = False) -> 
         r = subprocess.run(cmd, capture_output=True, text=True)
         return s, r
 
-    with cf.ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as pool:
+    with cf.ThreadPoolExecutor(max_workers=min(8, len(jobs) + 1)) as pool:
+        marshal = pool.submit(build_marshal, force)
         for s, r in pool.map(compile_one, jobs):
             if verbose and r.stderr:
                 sys.stderr.write(r.stderr)
             if r.returncode != 0:
                 raise RuntimeError(f"nvcc failed on {s}:\n{r.stdout}\n{r.stderr}")
+        marshal.result()
     objs = [os.path.join(obj_dir, s.replace(".cu", ".o")) for s in SOURCES]
     if force or jobs or _stale(lib_path, objs):
         cmd = [nvcc, "-shared", "-o", lib_path, *objs, "-Xcompiler", "-fPIC"]

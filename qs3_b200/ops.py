@@ -11,11 +11,17 @@ error classes: a failing call raises :class:`Qs3Error` carrying the
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from dataclasses import dataclass
 
 import torch
 
 from . import capi
+
+try:
+    from . import _marshal
+except ImportError as exc:
+    raise RuntimeError("qs3_b200/_marshal.so is missing: build it with `python -m qs3_b200._build`") from exc
 
 _STATUS_NAMES = {0: "Ok", 1: "InvalidArgument", 2: "Unsupported", 3: "OutOfMemory",
                  4: "CudaError", 5: "BackendError", 6: "InternalError"}
@@ -28,27 +34,72 @@ class Qs3Error(RuntimeError):
         super().__init__(f"{_STATUS_NAMES.get(status, status)}: {message}")
 
 
-_TORCH_DTYPES = {
-    torch.float32: capi.DTYPE_F32, torch.float16: capi.DTYPE_F16, torch.bfloat16: capi.DTYPE_BF16,
-    torch.int32: capi.DTYPE_I32, torch.int8: capi.DTYPE_I8, torch.uint8: capi.DTYPE_U8,
-    torch.float8_e4m3fn: capi.DTYPE_FP8_E4M3,
-}
+def _layout(cls, *fields):
+    """Precomputed marshalling plan of the tensor fields of a descriptor class: (packed offsets, ranks and
+    dtype overrides, ranks). A field is a name, (name, dtype code), or (name, dtype code or None, 0) for a
+    rank-1 field filled with all elements of a contiguous tensor."""
+    types = {n: t for n, t, *_ in cls._fields_}
+    packed, ranks = [], []
+    for f in fields:
+        name, dtype, rank = (f, None, None) if isinstance(f, str) else f if len(f) == 3 else (*f, None)
+        full = types[name].shape.size // C.sizeof(C.c_int64)
+        packed.append(struct.pack("3i", getattr(cls, name).offset, full if rank is None else rank,
+                                  -1 if dtype is None else dtype))
+        ranks.append(full)
+    return b"".join(packed), ranks
+
+
+def _fill(d, layout, *tensors):
+    """Fill the tensor fields of descriptor ``d`` (None -> absent optional tensor)."""
+    bad = _marshal.fill(C.addressof(d), layout[0], tensors)
+    if bad >= 0:
+        raise Qs3Error(capi.STATUS_INVALID_ARGUMENT,
+                       f"expected a rank-{layout[1][bad]} tensor, got {tensors[bad].dim()}")
 
 
 def _desc(t, rank, dtype=None):
     """qsfi_tensorN view of a torch tensor (None -> absent optional tensor)."""
-    cls = {1: capi.Tensor1, 2: capi.Tensor2, 3: capi.Tensor3}[rank]
-    d = cls()
-    if t is None:
-        return d
-    if t.dim() != rank:
+    d = (capi.Tensor1, capi.Tensor2, capi.Tensor3)[rank - 1]()
+    if t is not None and _marshal.fill(C.addressof(d), struct.pack("3i", 0, rank, -1 if dtype is None else dtype),
+                                       (t,)) >= 0:
         raise Qs3Error(capi.STATUS_INVALID_ARGUMENT, f"expected a rank-{rank} tensor, got {t.dim()}")
-    d.data = t.data_ptr()
-    d.dtype = dtype if dtype is not None else _TORCH_DTYPES.get(t.dtype, capi.DTYPE_INVALID)
-    for i in range(rank):
-        d.shape[i] = t.shape[i]
-        d.stride[i] = t.stride(i)
     return d
+
+
+_ROUTER_TOPK_DESC = _layout(capi.RouterTopkDesc, "logits", "topk_ids", "topk_weights")
+_SILU_AND_MUL_DESC = _layout(capi.SiluAndMulDesc, "gate", "up", "out")
+_SHARED_EXPERT_GATE_ADD_DESC = _layout(capi.SharedExpertGateAddDesc, "gate_logits", "shared", "out")
+_MOE_BF16_EXECUTE_DESC = _layout(capi.MoeBf16ExecuteDesc, "hidden", "topk_ids", "topk_weights", "gate_up_weight",
+    "down_weight", "out", "workspace")
+_MOE_NVFP4_EXECUTE_DESC = _layout(capi.MoeNvfp4ExecuteDesc, "hidden_packed", ("hidden_scale", capi.DTYPE_FP8_E4M3),
+    "topk_ids", "topk_weights", "gate_up_weight_packed", ("gate_up_weight_scale", capi.DTYPE_FP8_E4M3),
+    "down_weight_packed", ("down_weight_scale", capi.DTYPE_FP8_E4M3), "expert_output_scale", "out", "workspace")
+_NVFP4_QUANTIZE_WEIGHT_DESC = _layout(capi.Nvfp4QuantizeWeightDesc, "weight", "packed",
+    ("scale_linear", capi.DTYPE_FP8_E4M3), "scale_tiled", "global_scale")
+_NVFP4_QUANTIZE_ACT_DESC = _layout(capi.Nvfp4QuantizeActDesc, "x", "packed", ("scale_linear", capi.DTYPE_FP8_E4M3))
+_NVFP4_TILE_SCALES_DESC = _layout(capi.Nvfp4TileScalesDesc, ("scale_linear", capi.DTYPE_FP8_E4M3), "scale_tiled")
+_FP8_QUANTIZE_WEIGHT_DESC = _layout(capi.Fp8QuantizeWeightDesc, "weight", ("codes", capi.DTYPE_FP8_E4M3), "scale")
+_FP8_QUANTIZE_ACT_DESC = _layout(capi.Fp8QuantizeActDesc, "x", ("codes", capi.DTYPE_FP8_E4M3), "scale")
+_MOE_FP8_EXECUTE_DESC = _layout(capi.MoeFp8ExecuteDesc, ("hidden", capi.DTYPE_FP8_E4M3), "hidden_scale", "topk_ids",
+    "topk_weights", ("gate_up_weight", capi.DTYPE_FP8_E4M3), "gate_up_weight_scale",
+    ("down_weight", capi.DTYPE_FP8_E4M3), "down_weight_scale", "out", "workspace")
+
+
+def _layer_layout(gate_up_fp8, down_fp8):
+    weight = lambda n, fp8: ((f"{n}_weight", capi.DTYPE_FP8_E4M3 if fp8 else None),
+                             (f"{n}_scale_tiled", None, 0) if fp8 else f"{n}_scale_tiled", f"{n}_global_scale")
+    return _layout(capi.MoeLayerDesc, "hidden", "router_weight", "router_bias", *weight("gate_up", gate_up_fp8),
+                   *weight("down", down_fp8), *weight("shared_gate_up", False), *weight("shared_down", False),
+                   "shared_gate_weight", "out", "topk_ids", "topk_weights", "router_logits", "workspace",
+                   "hidden_packed", "hidden_scale_tiled", "residual_inout", "next_norm_weight")
+
+
+_MOE_LAYER_DESC = {(g, d): _layer_layout(g, d) for g in (False, True) for d in (False, True)}
+_QSCB_GEMM_DESC = _layout(capi.QscbGemmDesc, "x", "weight", "out")
+_RMSNORM_DESC = _layout(capi.RmsnormDesc, "x", "weight", "out")
+_FUSED_ADD_RMSNORM_DESC = _layout(capi.FusedAddRmsnormDesc, "x", "residual_inout", "weight", "out")
+_FUSED_ADD_RMSNORM_NVFP4_DESC = _layout(capi.FusedAddRmsnormNvfp4Desc, "packed", "scale_tiled")
+_ROUTE_SORT_STATIC_DESC = _layout(capi.RouteSortStaticDesc, "topk_ids", "topk_weights")
 
 
 def _stream_ptr(device=None) -> int:
@@ -205,9 +256,7 @@ def router_topk(logits, topk_ids, topk_weights, *, score=capi.ROUTER_SCORE_SOFTM
     """``qscu_router_topk`` (upstream qscu.h:278; builder src/runtime/kernels.rs:692-741)."""
     lib = capi.load() if lib is None else lib
     d = capi.RouterTopkDesc()
-    d.logits = _desc(logits, 2)
-    d.topk_ids = _desc(topk_ids, 2)
-    d.topk_weights = _desc(topk_weights, 2)
+    _fill(d, _ROUTER_TOPK_DESC, logits, topk_ids, topk_weights)
     d.num_tokens = logits.shape[0] if num_tokens is None else num_tokens
     d.num_experts = logits.shape[1] if num_experts is None else num_experts
     d.top_k = topk_ids.shape[1] if top_k is None else top_k
@@ -223,9 +272,7 @@ def silu_and_mul_bf16(gate, up, out, stream=None):
     """``qscu_silu_and_mul_bf16`` (upstream qscu.h:35)."""
     lib = capi.load()
     d = capi.SiluAndMulDesc()
-    d.gate = _desc(gate, 2)
-    d.up = _desc(up, 2)
-    d.out = _desc(out, 2)
+    _fill(d, _SILU_AND_MUL_DESC, gate, up, out)
     d.num_tokens = out.shape[0]
     d.intermediate_size = out.shape[1]
     status = lib.qscu_silu_and_mul_bf16(C.byref(d), C.c_void_p(_stream_ptr() if stream is None else stream))
@@ -237,9 +284,7 @@ def shared_expert_gate_add_bf16(gate_logits, shared, out, stream=None):
     """``qscu_qwen36_shared_expert_gate_add_bf16`` (upstream qscu.h:50-52)."""
     lib = capi.load()
     d = capi.SharedExpertGateAddDesc()
-    d.gate_logits = _desc(gate_logits, 2)
-    d.shared = _desc(shared, 2)
-    d.out = _desc(out, 2)
+    _fill(d, _SHARED_EXPERT_GATE_ADD_DESC, gate_logits, shared, out)
     d.num_tokens = out.shape[0]
     d.hidden_size = out.shape[1]
     status = lib.qscu_qwen36_shared_expert_gate_add_bf16(
@@ -274,9 +319,7 @@ class GemmContext:
     def gemm_bf16(self, x, weight, out, alpha=0.0, beta=0.0):
         """out = alpha * x @ weight.T + beta * out (``qscb_gemm_bf16``)."""
         d = capi.QscbGemmDesc()
-        d.x = _desc(x, 2)
-        d.weight = _desc(weight, 2)
-        d.out = _desc(out, 2)
+        _fill(d, _QSCB_GEMM_DESC, x, weight, out)
         d.rows = x.shape[0]
         d.in_features = x.shape[1]
         d.out_features = weight.shape[0]
@@ -296,13 +339,7 @@ def moe_execute_bf16(plan: MoePlan, hidden, topk_ids, topk_weights, gate_up_weig
     """``qsfi_moe_execute_bf16`` (upstream qsfi.h:339-341)."""
     ctx = plan.ctx
     d = capi.MoeBf16ExecuteDesc()
-    d.hidden = _desc(hidden, 2)
-    d.topk_ids = _desc(topk_ids, 2)
-    d.topk_weights = _desc(topk_weights, 2)
-    d.gate_up_weight = _desc(gate_up_weight, 3)
-    d.down_weight = _desc(down_weight, 3)
-    d.out = _desc(out, 2)
-    d.workspace = _desc(workspace, 1)
+    _fill(d, _MOE_BF16_EXECUTE_DESC, hidden, topk_ids, topk_weights, gate_up_weight, down_weight, out, workspace)
     d.num_tokens = hidden.shape[0] if num_tokens is None else num_tokens
     ctx.check(ctx._lib.qsfi_moe_execute_bf16(ctx.handle, plan.handle, C.byref(d)))
 
@@ -313,17 +350,8 @@ def moe_execute_nvfp4(plan: MoePlan, hidden_packed, hidden_scale, topk_ids, topk
     """``qsfi_moe_execute_nvfp4`` (upstream qsfi.h:342-344; declared layout qsfi.h:249-266)."""
     ctx = plan.ctx
     d = capi.MoeNvfp4ExecuteDesc()
-    d.hidden_packed = _desc(hidden_packed, 2)
-    d.hidden_scale = _desc(hidden_scale, 2, capi.DTYPE_FP8_E4M3)
-    d.topk_ids = _desc(topk_ids, 2)
-    d.topk_weights = _desc(topk_weights, 2)
-    d.gate_up_weight_packed = _desc(gate_up_weight_packed, 3)
-    d.gate_up_weight_scale = _desc(gate_up_weight_scale, 3, capi.DTYPE_FP8_E4M3)
-    d.down_weight_packed = _desc(down_weight_packed, 3)
-    d.down_weight_scale = _desc(down_weight_scale, 3, capi.DTYPE_FP8_E4M3)
-    d.expert_output_scale = _desc(expert_output_scale, 1)
-    d.out = _desc(out, 2)
-    d.workspace = _desc(workspace, 1)
+    _fill(d, _MOE_NVFP4_EXECUTE_DESC, hidden_packed, hidden_scale, topk_ids, topk_weights, gate_up_weight_packed,
+          gate_up_weight_scale, down_weight_packed, down_weight_scale, expert_output_scale, out, workspace)
     d.num_tokens = hidden_packed.shape[0] if num_tokens is None else num_tokens
     ctx.check(ctx._lib.qsfi_moe_execute_nvfp4(ctx.handle, plan.handle, C.byref(d)))
 
@@ -350,11 +378,7 @@ def nvfp4_quantize_weight(ctx: Context, weight: torch.Tensor, gated: bool, linea
     st = torch.empty(e * nvfp4_tiled_scale_bytes(rows, k), dtype=torch.uint8, device=dev)  # written whole
     g = torch.empty(e, dtype=torch.float32, device=dev)
     d = capi.Nvfp4QuantizeWeightDesc()
-    d.weight = _desc(weight, 3)
-    d.packed = _desc(packed, 3)
-    d.scale_linear = _desc(sl, 3, capi.DTYPE_FP8_E4M3)
-    d.scale_tiled = _desc(st, 1)
-    d.global_scale = _desc(g, 1)
+    _fill(d, _NVFP4_QUANTIZE_WEIGHT_DESC, weight, packed, sl, st, g)
     d.gated_rows = 1 if gated else 0
     ctx.check(ctx._lib.qs3_nvfp4_quantize_weight(ctx.handle, C.byref(d)))
     return Nvfp4Weight(packed, sl, st, g)
@@ -366,9 +390,7 @@ def nvfp4_quantize_act(ctx: Context, x: torch.Tensor, global_scale: float = 1.0)
     packed = torch.empty((rows, k // 2), dtype=torch.uint8, device=x.device)
     scale = torch.empty((rows, k // 16), dtype=torch.uint8, device=x.device)
     d = capi.Nvfp4QuantizeActDesc()
-    d.x = _desc(x, 2)
-    d.packed = _desc(packed, 2)
-    d.scale_linear = _desc(scale, 2, capi.DTYPE_FP8_E4M3)
+    _fill(d, _NVFP4_QUANTIZE_ACT_DESC, x, packed, scale)
     d.global_scale = global_scale
     d.rows = rows
     ctx.check(ctx._lib.qs3_nvfp4_quantize_act(ctx.handle, C.byref(d)))
@@ -380,8 +402,7 @@ def nvfp4_tile_scales(ctx: Context, scale_linear: torch.Tensor, gated: bool) -> 
     e, rows, kb = scale_linear.shape
     st = torch.zeros(e * nvfp4_tiled_scale_bytes(rows, kb * 16), dtype=torch.uint8, device=scale_linear.device)
     d = capi.Nvfp4TileScalesDesc()
-    d.scale_linear = _desc(scale_linear, 3, capi.DTYPE_FP8_E4M3)
-    d.scale_tiled = _desc(st, 1)
+    _fill(d, _NVFP4_TILE_SCALES_DESC, scale_linear, st)
     d.gated_rows = 1 if gated else 0
     ctx.check(ctx._lib.qs3_nvfp4_tile_scales(ctx.handle, C.byref(d)))
     return st
@@ -400,9 +421,7 @@ def fp8_quantize_weight(ctx: Context, weight: torch.Tensor) -> Fp8Weight:
     codes = torch.empty((e, rows, k), dtype=torch.uint8, device=weight.device)
     scale = torch.empty((e, (rows + 127) // 128, k // 128), dtype=torch.float32, device=weight.device)
     d = capi.Fp8QuantizeWeightDesc()
-    d.weight = _desc(weight, 3)
-    d.codes = _desc(codes, 3, capi.DTYPE_FP8_E4M3)
-    d.scale = _desc(scale, 3)
+    _fill(d, _FP8_QUANTIZE_WEIGHT_DESC, weight, codes, scale)
     ctx.check(ctx._lib.qs3_fp8_quantize_weight(ctx.handle, C.byref(d)))
     return Fp8Weight(codes, scale)
 
@@ -413,9 +432,7 @@ def fp8_quantize_act(ctx: Context, x: torch.Tensor):
     codes = torch.empty((rows, k), dtype=torch.uint8, device=x.device)
     scale = torch.empty((rows, k // 128), dtype=torch.float32, device=x.device)
     d = capi.Fp8QuantizeActDesc()
-    d.x = _desc(x, 2)
-    d.codes = _desc(codes, 2, capi.DTYPE_FP8_E4M3)
-    d.scale = _desc(scale, 2)
+    _fill(d, _FP8_QUANTIZE_ACT_DESC, x, codes, scale)
     d.rows = rows
     ctx.check(ctx._lib.qs3_fp8_quantize_act(ctx.handle, C.byref(d)))
     return codes, scale
@@ -426,16 +443,8 @@ def moe_execute_fp8(plan: MoePlan, hidden_codes, hidden_scale, topk_ids, topk_we
     """``qs3_moe_execute_fp8``: routed experts on FP8 block-scaled operands."""
     ctx = plan.ctx
     d = capi.MoeFp8ExecuteDesc()
-    d.hidden = _desc(hidden_codes, 2, capi.DTYPE_FP8_E4M3)
-    d.hidden_scale = _desc(hidden_scale, 2)
-    d.topk_ids = _desc(topk_ids, 2)
-    d.topk_weights = _desc(topk_weights, 2)
-    d.gate_up_weight = _desc(gate_up.codes, 3, capi.DTYPE_FP8_E4M3)
-    d.gate_up_weight_scale = _desc(gate_up.scale, 3)
-    d.down_weight = _desc(down.codes, 3, capi.DTYPE_FP8_E4M3)
-    d.down_weight_scale = _desc(down.scale, 3)
-    d.out = _desc(out, 2)
-    d.workspace = _desc(workspace, 1)
+    _fill(d, _MOE_FP8_EXECUTE_DESC, hidden_codes, hidden_scale, topk_ids, topk_weights, gate_up.codes,
+          gate_up.scale, down.codes, down.scale, out, workspace)
     d.num_tokens = hidden_codes.shape[0] if num_tokens is None else num_tokens
     ctx.check(ctx._lib.qs3_moe_execute_fp8(ctx.handle, plan.handle, C.byref(d)))
 
@@ -447,6 +456,15 @@ class SharedExpert:
     down: object             # bf16 [1, H, Is] tensor or Nvfp4Weight
     gate_weight: torch.Tensor  # bf16 [1, H]
     intermediate_size: int
+
+
+def _weight_tensors(w):
+    """(weight, block scales, global scale) tensors of an expert weight as the layer descriptor takes them."""
+    if isinstance(w, Nvfp4Weight):
+        return w.packed, w.scale_tiled, w.global_scale
+    if isinstance(w, Fp8Weight):
+        return w.codes, w.scale if w.scale.is_contiguous() else w.scale.reshape(-1), None
+    return w, None, None
 
 
 def moe_layer_execute(plan: MoePlan, hidden, router_weight, gate_up, down, out, workspace, *,
@@ -461,43 +479,20 @@ def moe_layer_execute(plan: MoePlan, hidden, router_weight, gate_up, down, out, 
     block-scaled plan."""
     ctx = plan.ctx
     d = capi.MoeLayerDesc()
-    d.hidden = _desc(hidden, 2)
-    d.router_weight = _desc(router_weight, 2)
-    d.router_bias = _desc(router_bias, 1)
-
-    def put(prefix, w):
-        if isinstance(w, Nvfp4Weight):
-            setattr(d, f"{prefix}_weight", _desc(w.packed, 3))
-            setattr(d, f"{prefix}_scale_tiled", _desc(w.scale_tiled, 1))
-            setattr(d, f"{prefix}_global_scale", _desc(w.global_scale, 1))
-        elif isinstance(w, Fp8Weight):
-            setattr(d, f"{prefix}_weight", _desc(w.codes, 3, capi.DTYPE_FP8_E4M3))
-            setattr(d, f"{prefix}_scale_tiled", _desc(w.scale.reshape(-1), 1))
-        else:
-            setattr(d, f"{prefix}_weight", _desc(w, 3))
-
-    put("gate_up", gate_up)
-    put("down", down)
+    sgu = sdn = (None, None, None)
+    shared_gate = None
     if shared is not None:
-        put("shared_gate_up", shared.gate_up)
-        put("shared_down", shared.down)
-        d.shared_gate_weight = _desc(shared.gate_weight, 2)
+        sgu, sdn, shared_gate = _weight_tensors(shared.gate_up), _weight_tensors(shared.down), shared.gate_weight
         d.shared_intermediate_size = shared.intermediate_size
+    _fill(d, _MOE_LAYER_DESC[isinstance(gate_up, Fp8Weight), isinstance(down, Fp8Weight)], hidden, router_weight,
+          router_bias, *_weight_tensors(gate_up), *_weight_tensors(down), *sgu, *sdn, shared_gate, out, topk_ids,
+          topk_weights, router_logits, workspace, hidden_packed, hidden_scale_tiled, residual_inout, next_norm_weight)
     d.score = score
     d.renormalize = 1 if renormalize else 0
     d.routed_scaling_factor = routed_scaling_factor
     d.act_global_scale = act_global_scale
     d.act2_global_scale = act2_global_scale
-    d.out = _desc(out, 2)
-    d.topk_ids = _desc(topk_ids, 2)
-    d.topk_weights = _desc(topk_weights, 2)
-    d.router_logits = _desc(router_logits, 2)
-    d.workspace = _desc(workspace, 1)
     d.num_tokens = hidden.shape[0] if num_tokens is None else num_tokens
-    d.hidden_packed = _desc(hidden_packed, 2)
-    d.hidden_scale_tiled = _desc(hidden_scale_tiled, 1)
-    d.residual_inout = _desc(residual_inout, 2)
-    d.next_norm_weight = _desc(next_norm_weight, 1)
     d.next_norm_eps = next_norm_eps
     ctx.check(ctx._lib.qs3_moe_layer_execute(ctx.handle, plan.handle, C.byref(d)))
 
@@ -525,8 +520,7 @@ def route_sort_static(ctx: Context, topk_ids, topk_weights, local_expert_offset:
                torch.empty(t * k, dtype=torch.int32, device=dev),
                torch.empty(t * k, dtype=torch.float32, device=dev))
     d = capi.RouteSortStaticDesc()
-    d.topk_ids = _desc(topk_ids, 2)
-    d.topk_weights = _desc(topk_weights, 2)
+    _fill(d, _ROUTE_SORT_STATIC_DESC, topk_ids, topk_weights)
     d.counts, d.indptr, d.route_rows, d.row_tokens, d.row_scales = (_desc(x, 1) for x in out)
     d.num_tokens, d.top_k = t, k
     d.local_expert_offset, d.local_num_experts = local_expert_offset, local_num_experts
@@ -608,21 +602,20 @@ def operand_stream_probe(ctx: Context, buffer, tile_bytes: int = 16384, stages: 
 def rmsnorm(ctx: Context, x, weight, out, eps: float = 1e-6, weight_bias: float = 0.0):
     """``qsfi_rmsnorm`` (upstream qsfi.h:160-167, 330)."""
     d = capi.RmsnormDesc()
-    d.x, d.weight, d.out = _desc(x, 2), _desc(weight, 1), _desc(out, 2)
+    _fill(d, _RMSNORM_DESC, x, weight, out)
     d.hidden_size, d.weight_bias, d.eps = x.shape[1], weight_bias, eps
     ctx.check(ctx._lib.qsfi_rmsnorm(ctx.handle, C.byref(d)))
 
 
-def _fused_desc(x, residual, weight, eps):
-    d = capi.FusedAddRmsnormDesc()
-    d.x, d.residual_inout, d.weight, d.out = _desc(x, 2), _desc(residual, 2), _desc(weight, 1), _desc(x, 2)
+def _fill_fused(d, x, residual, weight, eps):
+    _fill(d, _FUSED_ADD_RMSNORM_DESC, x, residual, weight, x)
     d.hidden_size, d.eps = x.shape[1], eps
-    return d
 
 
 def fused_add_rmsnorm(ctx: Context, x, residual, weight, eps: float = 1e-6):
     """``qsfi_fused_add_rmsnorm`` (upstream qsfi.h:169-176, 331): residual += x; x = norm(residual)."""
-    d = _fused_desc(x, residual, weight, eps)
+    d = capi.FusedAddRmsnormDesc()
+    _fill_fused(d, x, residual, weight, eps)
     ctx.check(ctx._lib.qsfi_fused_add_rmsnorm(ctx.handle, C.byref(d)))
 
 
@@ -637,7 +630,8 @@ def fused_add_rmsnorm_nvfp4(ctx: Context, x, residual, weight, eps: float = 1e-6
     if tiled is None:
         tiled = torch.zeros(nvfp4_tiled_scale_bytes(rows, hidden), dtype=torch.uint8, device=x.device)
     d = capi.FusedAddRmsnormNvfp4Desc()
-    d.norm = _fused_desc(x, residual, weight, eps)
-    d.packed, d.scale_tiled, d.global_scale = _desc(packed, 2), _desc(tiled, 1), global_scale
+    _fill_fused(d.norm, x, residual, weight, eps)
+    _fill(d, _FUSED_ADD_RMSNORM_NVFP4_DESC, packed, tiled)
+    d.global_scale = global_scale
     ctx.check(ctx._lib.qs3_fused_add_rmsnorm_nvfp4(ctx.handle, C.byref(d)))
     return packed, tiled
