@@ -246,14 +246,13 @@ struct GemmProblem {
     const float* group_scale_up; // gated: optional multiplier of the up rows (NULL: group_scale)
     const float* bias;          // optional f32 [n] (EPI_STORE_F32)
     float out_global_scale;     // EPI_SWIGLU_NVFP4: global scale of the quantised output
-    // optional scratch for split-k (dense bf16 problems with f32 output, few output tiles and a long k:
-    // router logits of a decode batch); NULL: never split
-    float* splitk_scratch;
-    size_t splitk_scratch_bytes;
 };
 // Chooses the tcgen05 kernel when the shape allows it and the plain CUDA-core
 // kernel otherwise (tiny or unaligned shapes; bf16 only).
 cudaError_t launch_gemm(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);
+// Dense bf16 problems with few output tiles: k split over the CTAs of a cluster (gemm_splitk.cu).
+bool gemm_splitk_supported(const GemmProblem& p);
+cudaError_t launch_gemm_splitk(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);
 // Persistent 128 x 256 kernel for dense bf16 problems with more than 64 rows (gemm_dense.cu).
 bool gemm_dense_bf16_supported(const GemmProblem& p);
 cudaError_t launch_gemm_dense_bf16(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);

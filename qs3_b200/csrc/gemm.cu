@@ -1,10 +1,9 @@
 // Grouped / dense GEMM  D[m, n] = sum_k A[m, k] * B[g][n, k]. Kernels in this file:
-//   gemm_tc_kernel        tcgen05, one 128 x 128 tile per CTA: dense bf16 problems with few tiles, NVFP4 with
+//   gemm_tc_kernel        tcgen05, one 128 x 128 tile per CTA: gated dense bf16 problems and ragged k, NVFP4 with
 //                         k > 2048 (grouped bf16 problems go to bf16_stream.cu, larger dense ones to gemm_dense.cu)
 //   gemm_tc_astat_kernel  tcgen05, NVFP4 with the A panel resident in shared memory (k <= 2048)
-//   gemm_skinny_kernel    CUDA cores, bf16 with at most 64 rows (router logits of a decode batch)
 //   gemm_simt_kernel      CUDA cores, shapes the tensor-core tiles cannot address
-// launch_gemm() at the end picks one of these, a kernel of gemm_dense.cu, gemm_pair.cu or bf16_stream.cu, or the
+// launch_gemm() at the end picks one of these, a kernel of gemm_splitk.cu, gemm_dense.cu, gemm_pair.cu or bf16_stream.cu, or the
 // decode kernel of nvfp4_decode.cu.
 //
 // gemm_tc_kernel: one 128 x 128 output tile per CTA on the 5th-generation tensor cores:
@@ -60,9 +59,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const uint32_t nt = blockIdx.x;
     constexpr uint32_t kFeat = GATED ? kBN / 2 : kBN; // output features per tile
     const uint32_t n0 = nt * kFeat;
-    // the k blocks this CTA reduces (all of them unless the launch is split over grid.z)
-    const uint32_t kb_base = p.split_kb != 0 ? blockIdx.z * p.split_kb : 0u;
-    const uint32_t kb_count = p.split_kb != 0 ? min(p.split_kb, p.k_blocks - kb_base) : p.k_blocks;
+    const uint32_t kb_count = p.k_blocks;
 
     // ---- shared memory carve-up ----
     extern __shared__ uint8_t smem_raw[];
@@ -121,7 +118,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 uint8_t* sb = sa + kTileBytes;
                 mbar_expect_tx(&full_bar[s], kStageBytes);
                 // inner coordinate in elements of the map's type (bf16 elements / bytes)
-                const int c0 = static_cast<int>(kb_base + kb) * (NVFP4 ? 128 : 64);
+                const int c0 = static_cast<int>(kb) * (NVFP4 ? 128 : 64);
                 tma_load_2d(sa, &map_a, &full_bar[s], c0, row0);
                 if (GATED) {
                     tma_load_2d(sb, &map_b, &full_bar[s], c0, b_row);
@@ -131,10 +128,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                     tma_load_2d(sb, &map_b, &full_bar[s], c0, b_row);
                 }
                 if (NVFP4) {
-                    bulk_load(sb + kTileBytes, sfa_src + static_cast<uint64_t>(kb_base + kb) * kSfBytes, kSfBytes,
+                    bulk_load(sb + kTileBytes, sfa_src + static_cast<uint64_t>(kb) * kSfBytes, kSfBytes, &full_bar[s]);
+                    bulk_load(sb + kTileBytes + kSfBytes, sfb_src + static_cast<uint64_t>(kb) * kSfBytes, kSfBytes,
                               &full_bar[s]);
-                    bulk_load(sb + kTileBytes + kSfBytes, sfb_src + static_cast<uint64_t>(kb_base + kb) * kSfBytes,
-                              kSfBytes, &full_bar[s]);
                 }
             }
         }
@@ -186,8 +182,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const bool ready = __all_sync(0xffffffffu, mbar_wait(acc_bar, 0, abort_flag, p.err, ERR_ACC_WAIT));
         tc_fence_after();
         if (ready) {
-            epilogue_tile<GATED, EPI>(p, tmem_base, warp, lane, expert,
-                                      row0 + static_cast<int>(blockIdx.z * p.split_row_stride), nrows, nt);
+            epilogue_tile<GATED, EPI>(p, tmem_base, warp, lane, expert, row0, nrows, nt);
         }
     }
 
@@ -740,114 +735,6 @@ bool pair_down_enabled()
     return enabled;
 }
 
-// ---- skinny bf16 GEMM for decode-sized batches ------------------------------------------------
-//
-// out[t, n] = sum_k A[t, k] * B[n, k] for a handful of rows (router logits of a decode batch):
-// one 128 x 128 tensor-core tile would stream all of k through a single SM, so instead every
-// output feature gets a block; a warp keeps its slice of the weight row in registers and
-// walks two rows of A (L2-resident), lanes split k, one shuffle reduction per output.
-constexpr uint32_t kSkinnyWarps = 8;
-constexpr uint32_t kSkinnyRowsPerWarp = 2;
-constexpr uint32_t kSkinnyMaxChunks = 16; // k <= 4096, in 256-element chunks (8 per lane)
-
-__global__ void __launch_bounds__(kSkinnyWarps * 32)
-gemm_skinny_kernel(const __nv_bfloat16* __restrict__ a, uint64_t a_pitch, const __nv_bfloat16* __restrict__ b,
-                   uint64_t b_pitch, uint32_t rows, uint32_t k, float* __restrict__ out, uint64_t out_pitch,
-                   float alpha, float beta, const float* __restrict__ bias)
-{
-    const uint32_t n = blockIdx.x;
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t chunks = k / 256;
-    const uint4* wrow = reinterpret_cast<const uint4*>(b + static_cast<uint64_t>(n) * b_pitch);
-    uint4 wv[kSkinnyMaxChunks];
-#pragma unroll
-    for (uint32_t c = 0; c < kSkinnyMaxChunks; ++c)
-        wv[c] = c < chunks ? wrow[c * 32 + lane] : make_uint4(0, 0, 0, 0);
-    const uint32_t row0 = (blockIdx.y * kSkinnyWarps + warp) * kSkinnyRowsPerWarp;
-    for (uint32_t r = row0; r < min(rows, row0 + kSkinnyRowsPerWarp); ++r) {
-        const uint4* xrow = reinterpret_cast<const uint4*>(a + static_cast<uint64_t>(r) * a_pitch);
-        float acc = 0.0f;
-#pragma unroll
-        for (uint32_t c = 0; c < kSkinnyMaxChunks; ++c) {
-            if (c < chunks) {
-                const uint4 xv = xrow[c * 32 + lane];
-                const uint32_t xs[4] = { xv.x, xv.y, xv.z, xv.w };
-                const uint32_t ws[4] = { wv[c].x, wv[c].y, wv[c].z, wv[c].w };
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    acc = fmaf(bf16_bits_to_f32(xs[j] & 0xffffu), bf16_bits_to_f32(ws[j] & 0xffffu), acc);
-                    acc = fmaf(bf16_bits_to_f32(xs[j] >> 16), bf16_bits_to_f32(ws[j] >> 16), acc);
-                }
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) {
-            float* o = out + static_cast<uint64_t>(r) * out_pitch + n;
-            float v = acc * (alpha == 0.0f ? 1.0f : alpha);
-            if (beta != 0.0f)
-                v += beta * *o;
-            if (bias != nullptr)
-                v += bias[n];
-            *o = v;
-        }
-    }
-}
-
-// out[r, n] = alpha * sum over slices (in slice order) of partial[slice][r, n] + beta * out[r, n] + bias[n];
-// four features per thread. `partial` is [slices][rows_pad, n] f32, slice_stride elements apart.
-__global__ void __launch_bounds__(256)
-splitk_reduce_kernel(const float* __restrict__ partial, uint32_t slices, uint64_t slice_stride, uint64_t rows,
-                     uint32_t n, float* __restrict__ out, uint64_t out_pitch, float alpha, float beta,
-                     const float* __restrict__ bias)
-{
-    const uint64_t q = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const uint32_t per_row = n / 4;
-    if (q >= rows * per_row)
-        return;
-    const uint64_t r = q / per_row;
-    const uint32_t c = static_cast<uint32_t>(q % per_row) * 4;
-    float4 acc = *reinterpret_cast<const float4*>(partial + r * n + c);
-    for (uint32_t s = 1; s < slices; ++s) {
-        const float4 v = *reinterpret_cast<const float4*>(partial + s * slice_stride + r * n + c);
-        acc.x += v.x;
-        acc.y += v.y;
-        acc.z += v.z;
-        acc.w += v.w;
-    }
-    float* o = out + r * out_pitch + c;
-    float f[4] = { acc.x * alpha, acc.y * alpha, acc.z * alpha, acc.w * alpha };
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if (beta != 0.0f)
-            f[i] += beta * o[i];
-        if (bias != nullptr)
-            f[i] += bias[c + i];
-        o[i] = f[i];
-    }
-}
-
-// Dense bf16 problem with f32 output whose rows would not fill one tensor-core tile.
-bool skinny_supported(const GemmProblem& g)
-{
-    return !g.nvfp4 && !g.gated && g.epilogue == EPI_STORE_F32 && g.tile_expert == nullptr && g.groups == 1
-        && g.group_scale == nullptr && g.a_rows <= 64 && g.k % 256 == 0 && g.k / 256 <= kSkinnyMaxChunks
-        && aligned16(g.a) && aligned16(g.b) && g.a_pitch_bytes % 16 == 0 && g.b_pitch_bytes % 16 == 0
-        && g.n <= 65535;
-}
-
-cudaError_t launch_skinny(const GemmProblem& g, cudaStream_t stream)
-{
-    const uint32_t rows = static_cast<uint32_t>(g.a_rows);
-    const dim3 grid(g.n, (rows + kSkinnyWarps * kSkinnyRowsPerWarp - 1) / (kSkinnyWarps * kSkinnyRowsPerWarp));
-    gemm_skinny_kernel<<<grid, kSkinnyWarps * 32, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(g.a), g.a_pitch_bytes / 2, static_cast<const __nv_bfloat16*>(g.b),
-        g.b_pitch_bytes / 2, rows, g.k, static_cast<float*>(g.out), g.out_pitch_elems, g.alpha, g.beta, g.bias);
-    note_launch();
-    return cudaGetLastError();
-}
-
 TcParams make_params(const GemmProblem& g)
 {
     TcParams tp {};
@@ -980,8 +867,8 @@ cudaError_t launch_gemm(const GemmProblem& g, cudaStream_t stream, const char** 
             *why = "more than 65535 row tiles";
         return cudaErrorNotSupported;
     }
-    if (skinny_supported(g))
-        return launch_skinny(g, stream);
+    if (gemm_splitk_supported(g))
+        return launch_gemm_splitk(g, stream, why);
     if (gemm_dense_bf16_supported(g))
         return launch_gemm_dense_bf16(g, stream, why);
     if (pair_kernel_wanted(g))
@@ -1032,43 +919,8 @@ cudaError_t launch_gemm(const GemmProblem& g, cudaStream_t stream, const char** 
                 return launch_tc<false, true, EPI_SWIGLU_BF16>(ma, mb, tp, grid, stream);
             if (!g.gated && g.epilogue == EPI_STORE_BF16)
                 return launch_tc<false, false, EPI_STORE_BF16>(ma, mb, tp, grid, stream);
-            if (!g.gated && g.epilogue == EPI_STORE_F32) {
-                // A handful of output tiles with a long k (router logits of a decode batch: 128 x 512 x 2048
-                // = four tiles) would stream all of k through four SMs: split k over grid.z, partial tiles
-                // into the caller's scratch, then one pass that sums the slices in slice order (so the
-                // result does not depend on timing) and applies alpha, beta and the bias.
-                const uint32_t tiles = grid.x * grid.y;
-                uint32_t splits = 1;
-                if (g.splitk_scratch != nullptr && g.tile_expert == nullptr && 8 * tiles <= sm_count()
-                    && tp.k_blocks >= 8) {
-                    splits = std::min<uint32_t>({ 8u, tp.k_blocks / 4, sm_count() / tiles });
-                    const size_t need = static_cast<size_t>(splits) * grid.y * kBM * g.n * sizeof(float);
-                    if (splits < 2 || need > g.splitk_scratch_bytes || !aligned16(g.splitk_scratch) || g.n % 4 != 0)
-                        splits = 1;
-                }
-                if (splits > 1) {
-                    TcParams ts = tp;
-                    ts.split_kb = (tp.k_blocks + splits - 1) / splits;
-                    splits = (tp.k_blocks + ts.split_kb - 1) / ts.split_kb;
-                    ts.split_row_stride = grid.y * kBM;
-                    ts.out = g.splitk_scratch;
-                    ts.out_pitch = g.n;
-                    ts.alpha = 1.0f;
-                    ts.beta = 0.0f;
-                    ts.bias = nullptr;
-                    grid.z = splits;
-                    cudaError_t err = launch_tc<false, false, EPI_STORE_F32>(ma, mb, ts, grid, stream);
-                    if (err != cudaSuccess)
-                        return err;
-                    const uint64_t quads = g.a_rows * (g.n / 4);
-                    splitk_reduce_kernel<<<static_cast<unsigned>((quads + 255) / 256), 256, 0, stream>>>(
-                        g.splitk_scratch, splits, static_cast<uint64_t>(ts.split_row_stride) * g.n, g.a_rows, g.n,
-                        static_cast<float*>(g.out), g.out_pitch_elems, g.alpha == 0.0f ? 1.0f : g.alpha, g.beta, g.bias);
-                    note_launch();
-                    return cudaGetLastError();
-                }
+            if (!g.gated && g.epilogue == EPI_STORE_F32)
                 return launch_tc<false, false, EPI_STORE_F32>(ma, mb, tp, grid, stream);
-            }
         }
         if (why != nullptr)
             *why = "no tensor-core kernel for this operand/epilogue combination";

@@ -1,0 +1,313 @@
+// Dense bf16 GEMM with few output tiles  D[m, n] = alpha * sum_k A[m, k] * B[n, k] (+ beta * D) (+ bias[n]):
+// router logits, and projections of a decode batch. One CTA per output tile would stream all of k through a handful
+// of SMs (128 x 512 x 2048: four), so k is split over the CTAs of a cluster, whose partial tiles are summed through
+// distributed shared memory in rank order (the result does not depend on timing) without a scratch buffer or a
+// second launch.
+//
+//   grid    (splits, ceil(n / 128), ceil(m / NT)), clusters of `splits` CTAs
+//   tile    128 weight rows (M side) x NT rows of A (N side, 16..128): accumulator lane = feature, column = row
+//   smem    ring of stages: B 128 x 64 + A NT x 64; then the f32 partial tile [NT][128] (the ring is idle by then)
+//   warps   0-3 accumulator -> shared memory, 4 producer (TMA), 5 MMA issuer; all six sum and store
+//
+// Bound by latency: launch, one trip to HBM for the weights (and, at decode sizes, the code), two cluster barriers.
+// Router logits, hidden 2048: 512 experts, 1 token 0.0065 -> 0.0056 ms (a block per expert on CUDA cores), 128 tokens
+// 0.0153 -> 0.0098 (split over grid.z with a reduction pass), 1021 tokens 0.0194 -> 0.0112; 128 experts, 64 tokens
+// 0.0120 -> 0.0072, 4096 tokens 0.0204 -> 0.0128.
+#include "tcgen05.cuh"
+
+#include <cooperative_groups.h>
+
+#include <algorithm>
+
+namespace qs3 {
+namespace {
+
+using namespace tc;
+
+constexpr int kSkThreads = 192;
+constexpr uint32_t kSkStages = 4;
+constexpr uint32_t kSkMaxSplits = 8; // the largest portable cluster
+constexpr uint32_t kSkPitch = 132; // floats per row of the partial tile
+
+enum : uint32_t {
+    ERR_SK_FULL_WAIT = 0x5a000001u,
+    ERR_SK_EMPTY_WAIT = 0x5a000002u,
+    ERR_SK_ACC_WAIT = 0x5a000003u,
+};
+
+struct SplitkParams {
+    uint32_t m, n;
+    uint32_t k_blocks, kb_per_split;
+    void* out;
+    uint64_t out_pitch;
+    float alpha, beta;
+    const float* bias;
+    uint32_t* err;
+};
+
+template <int NT> struct SkSmem {
+    static constexpr uint32_t kStageBytes = kTileBytes + NT * 128;
+    static constexpr uint32_t kRing = kSkStages * kStageBytes;
+    static constexpr uint32_t kPartial = NT * kSkPitch * 4;
+    static constexpr uint32_t kBytes = kRing > kPartial ? kRing : kPartial;
+};
+
+template <int NT, bool F32>
+__global__ void __launch_bounds__(kSkThreads)
+gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_a,
+                   const SplitkParams p)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t rank = cluster.block_rank(), splits = cluster.num_blocks();
+    constexpr uint32_t kStageBytes = SkSmem<NT>::kStageBytes;
+    constexpr uint32_t kTmemCols = NT < 32 ? 32 : NT;
+
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    float* part = reinterpret_cast<float*>(smem); // [NT][kSkPitch], after the ring
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + SkSmem<NT>::kBytes);
+    uint64_t* empty_bar = full_bar + kSkStages;
+    uint64_t* acc_bar = empty_bar + kSkStages;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
+    volatile uint32_t* abort_flag = tmem_slot + 1;
+
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t n0 = blockIdx.y * 128, m0 = blockIdx.z * NT;
+    const uint32_t kb0 = min(rank * p.kb_per_split, p.k_blocks), kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
+
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < kSkStages; ++s) {
+            mbar_init(&full_bar[s], 1);
+            mbar_init(&empty_bar[s], 1);
+        }
+        mbar_init(acc_bar, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 5) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    bool ready = true;
+    if (warp == 4) {
+        // ------------------------------------------------------------ producer --
+        if (lane == 0) {
+            for (uint32_t i = 0; i < kb1 - kb0; ++i) {
+                const uint32_t s = i % kSkStages, ph = (i / kSkStages) & 1;
+                if (!mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_SK_EMPTY_WAIT))
+                    break;
+                uint8_t* sb = smem + s * kStageBytes;
+                mbar_expect_tx(&full_bar[s], kStageBytes);
+                const int c0 = static_cast<int>(kb0 + i) * 64;
+                tma_load_2d(sb, &map_b, &full_bar[s], c0, static_cast<int>(n0));
+                tma_load_2d(sb + kTileBytes, &map_a, &full_bar[s], c0, static_cast<int>(m0));
+            }
+        }
+    } else if (warp == 5) {
+        // ---------------------------------------------------------- MMA issuer --
+        if (lane == 0) {
+            // M = 128 weight rows, N = NT rows of A, bf16 x bf16 -> f32, both operands K-major
+            constexpr uint32_t kIdesc
+                = (1u << 4) | (1u << 7) | (1u << 10) | ((static_cast<uint32_t>(NT) >> 3) << 17) | ((kBM >> 4) << 24);
+            bool ok = true;
+            for (uint32_t i = 0; i < kb1 - kb0; ++i) {
+                const uint32_t s = i % kSkStages, ph = (i / kSkStages) & 1;
+                if (!mbar_wait<true>(&full_bar[s], ph, abort_flag, p.err, ERR_SK_FULL_WAIT)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t sb = smem_u32(smem + s * kStageBytes);
+                const uint64_t db = operand_desc(sb), da = operand_desc(sb + kTileBytes);
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j)
+                    tc_mma_bf16(tmem_base, db + 2 * j, da + 2 * j, kIdesc, (i > 0 || j > 0) ? 1u : 0u);
+                tc_commit(&empty_bar[s]);
+            }
+            if (ok)
+                tc_commit(acc_bar);
+        }
+    } else {
+        // ------------------------------------- accumulator -> partial tile in smem --
+        ready = __all_sync(0xffffffffu, mbar_wait(acc_bar, 0, abort_flag, p.err, ERR_SK_ACC_WAIT));
+        tc_fence_after();
+        if (ready) { // every load has been consumed: the ring is free
+            const bool some = kb1 > kb0; // a rank past the end of k adds zeros
+#pragma unroll
+            for (uint32_t c = 0; c < NT / 16; ++c) {
+                if (m0 + c * 16 >= p.m)
+                    break;
+                uint32_t v[16];
+                tc_ld16(tmem_base + ((warp * 32) << 16) + c * 16, v);
+                tc_ld_wait();
+#pragma unroll
+                for (uint32_t t = 0; t < 16; ++t)
+                    part[(c * 16 + t) * kSkPitch + warp * 32 + lane] = some ? __uint_as_float(v[t]) : 0.0f;
+            }
+        }
+        tc_fence_before();
+    }
+    cluster.sync(); // every partial tile is complete
+    // rows of the tile are dealt out over the cluster's warps; a lane sums four features over the ranks, in order
+    // (kept short: at decode sizes the code itself comes from HBM, and unrolling this over rows took longer)
+    const float alpha = p.alpha == 0.0f ? 1.0f : p.alpha;
+    const uint32_t rows = min(static_cast<uint32_t>(NT), p.m - m0);
+    const uint32_t f = n0 + lane * 4;
+    for (uint32_t t = rank * (kSkThreads / 32) + warp; t < rows && *abort_flag == 0; t += splits * (kSkThreads / 32)) {
+        float4 v[kSkMaxSplits];
+#pragma unroll
+        for (uint32_t s = 0; s < kSkMaxSplits; ++s)
+            v[s] = s < splits ? *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, s) + t * kSkPitch + lane * 4)
+                              : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float a[4] = { v[0].x, v[0].y, v[0].z, v[0].w };
+#pragma unroll
+        for (uint32_t s = 1; s < kSkMaxSplits; ++s) {
+            a[0] += v[s].x;
+            a[1] += v[s].y;
+            a[2] += v[s].z;
+            a[3] += v[s].w;
+        }
+        const uint64_t at = static_cast<uint64_t>(m0 + t) * p.out_pitch + f;
+        const uint32_t left = f < p.n ? min(4u, p.n - f) : 0u;
+        if (p.beta != 0.0f || p.bias != nullptr || alpha != 1.0f) {
+            for (uint32_t q = 0; q < left; ++q) {
+                a[q] *= alpha;
+                if (p.beta != 0.0f)
+                    a[q] += p.beta * (F32 ? static_cast<const float*>(p.out)[at + q]
+                                          : __bfloat162float(static_cast<const __nv_bfloat16*>(p.out)[at + q]));
+                if (p.bias != nullptr)
+                    a[q] += p.bias[f + q];
+            }
+        }
+        if constexpr (F32) {
+            float* o = static_cast<float*>(p.out) + at;
+            if (left == 4 && (reinterpret_cast<uintptr_t>(o) & 15u) == 0)
+                *reinterpret_cast<float4*>(o) = make_float4(a[0], a[1], a[2], a[3]);
+            else
+                for (uint32_t q = 0; q < left; ++q)
+                    o[q] = a[q];
+        } else {
+            __nv_bfloat16* o = static_cast<__nv_bfloat16*>(p.out) + at;
+            if (left == 4 && (reinterpret_cast<uintptr_t>(o) & 7u) == 0)
+                *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16x2(a[0], a[1]), pack_bf16x2(a[2], a[3]));
+            else
+                for (uint32_t q = 0; q < left; ++q)
+                    o[q] = __float2bfloat16(a[q]);
+        }
+    }
+    cluster.sync(); // no CTA leaves while a peer still reads its partial tile
+    if (warp == 5) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols)
+                     : "memory");
+    }
+}
+
+template <int NT, bool F32>
+cudaError_t launch_splitk_instance(const CUtensorMap& mb, const CUtensorMap& ma, const SplitkParams& sp, dim3 grid,
+                                   cudaStream_t stream)
+{
+    auto kernel = gemm_splitk_kernel<NT, F32>;
+    constexpr size_t smem = 1024 + SkSmem<NT>::kBytes + 128;
+    static bool configured[64] = {}; // per instantiation and device
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess)
+        return err;
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (err != cudaSuccess)
+            return err;
+        if (dev >= 0 && dev < 64)
+            configured[dev] = true;
+    }
+    cudaLaunchConfig_t cfg {};
+    cudaLaunchAttribute attr {};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim = { grid.x, 1, 1 };
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(kSkThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    err = cudaLaunchKernelEx(&cfg, kernel, mb, ma, sp);
+    note_launch();
+    return err;
+}
+
+// Rows of A per tile: the fewest MMA columns that hold them, 64 above that (128 x 4096 x 2048: 0.0125 ms against
+// 0.0145 with 128) as long as every tile can still be split.
+uint32_t splitk_tile_rows(uint64_t m) { return m <= 16 ? 16u : m <= 32 ? 32u : 64u; }
+
+uint64_t splitk_tiles(const GemmProblem& g, uint32_t nt) { return (g.n + 127ull) / 128 * ((g.a_rows + nt - 1) / nt); }
+
+// Tile rows of a problem that this kernel takes, 0: it does not. At least two CTAs per tile without exceeding one CTA
+// per SM, since more tiles fill the device as they are; a long k is split with 128-row tiles too (2048 x 4096 x 512:
+// 0.0207 against 0.0269 ms for the 128 x 256 kernel, but 512 x 2048 x 2048: 0.0163 against 0.0145).
+uint32_t splitk_choice(const GemmProblem& g)
+{
+    const uint32_t nt = splitk_tile_rows(g.a_rows);
+    if (2 * splitk_tiles(g, nt) <= device_sm_count())
+        return nt;
+    return nt == 64 && g.k >= 3072 && 2 * splitk_tiles(g, 128) <= device_sm_count() ? 128u : 0u;
+}
+
+} // namespace
+
+bool gemm_splitk_supported(const GemmProblem& g)
+{
+    return !g.nvfp4 && !g.gated && g.tile_expert == nullptr && g.groups == 1 && g.group_scale == nullptr && g.k % 8 == 0
+        && (g.epilogue == EPI_STORE_BF16 || g.epilogue == EPI_STORE_F32)
+        && (reinterpret_cast<uintptr_t>(g.a) & 15u) == 0 && (reinterpret_cast<uintptr_t>(g.b) & 15u) == 0
+        && g.a_pitch_bytes % 16 == 0 && g.b_pitch_bytes % 16 == 0
+        && splitk_choice(g) != 0;
+}
+
+cudaError_t launch_gemm_splitk(const GemmProblem& g, cudaStream_t stream, const char** why)
+{
+    SplitkParams sp {};
+    sp.m = static_cast<uint32_t>(g.a_rows);
+    sp.n = g.n;
+    sp.k_blocks = (g.k + 63) / 64;
+    sp.out = g.out;
+    sp.out_pitch = g.out_pitch_elems;
+    sp.alpha = g.alpha;
+    sp.beta = g.beta;
+    sp.bias = g.bias;
+    sp.err = device_error_word();
+    const uint32_t nt = splitk_choice(g);
+    const uint64_t tiles = splitk_tiles(g, nt);
+    // as many splits as fit one CTA per SM, two k blocks each at least
+    uint32_t splits = 1;
+    while (splits < kSkMaxSplits && 2 * splits * tiles <= device_sm_count() && 2 * (2 * splits) <= sp.k_blocks)
+        splits *= 2;
+    sp.kb_per_split = (sp.k_blocks + splits - 1) / splits;
+    CUtensorMap mb, ma;
+    if (!make_operand_map(&mb, false, g.b, g.k, g.n, g.b_pitch_bytes, 128)
+        || !make_operand_map(&ma, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, nt)) {
+        if (why != nullptr)
+            *why = "cuTensorMapEncodeTiled failed";
+        return cudaErrorInvalidValue;
+    }
+    const dim3 grid(splits, (g.n + 127) / 128, static_cast<uint32_t>((g.a_rows + nt - 1) / nt));
+    const bool f32 = g.epilogue == EPI_STORE_F32;
+    switch (nt) {
+    case 16: return f32 ? launch_splitk_instance<16, true>(mb, ma, sp, grid, stream) : launch_splitk_instance<16, false>(mb, ma, sp, grid, stream);
+    case 32: return f32 ? launch_splitk_instance<32, true>(mb, ma, sp, grid, stream) : launch_splitk_instance<32, false>(mb, ma, sp, grid, stream);
+    case 64: return f32 ? launch_splitk_instance<64, true>(mb, ma, sp, grid, stream) : launch_splitk_instance<64, false>(mb, ma, sp, grid, stream);
+    default: return f32 ? launch_splitk_instance<128, true>(mb, ma, sp, grid, stream) : launch_splitk_instance<128, false>(mb, ma, sp, grid, stream);
+    }
+}
+
+} // namespace qs3

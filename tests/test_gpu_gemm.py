@@ -105,6 +105,31 @@ def test_tensor_peak_probe_runs(kind):
     assert ctx.read_device_error() == 0
 
 
+# split k: one row, every tile height and its neighbours, n and k tails, splits past the end of k (k = 576: nine
+# blocks over eight ranks of two), several row tiles
+@pytest.mark.parametrize("shape", [(1, 2048, 512), (17, 576, 130), (33, 2056, 100), (64, 128, 2048), (65, 2048, 131),
+                                   (257, 512, 512)])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+def test_splitk_kernel(gemm, shape, beta):
+    rows, k, n = shape
+    rng = np.random.default_rng(rows + k + n)
+    x = bf16(rng.standard_normal((rows, k), dtype=np.float32))
+    w = bf16(rng.standard_normal((n, k), dtype=np.float32) * 0.05)
+    c = rng.standard_normal((rows, n), dtype=np.float32)
+    full = torch.full((rows, n + 3), 7.0, dtype=torch.float32, device="cuda")
+    out = full[:, :n]
+    out.copy_(torch.from_numpy(c))
+    gemm.gemm_bf16(to_dev(x), to_dev(w), out, alpha=0.25, beta=beta)
+    want = 0.25 * _ref(x, w) + beta * c.astype(np.float64)
+    got = to_np(out).astype(np.float64)
+    assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
+    assert torch.all(full[:, n:] == 7.0)
+    again = out.clone()
+    out.copy_(torch.from_numpy(c))
+    gemm.gemm_bf16(to_dev(x), to_dev(w), out, alpha=0.25, beta=beta)
+    assert torch.equal(again, out)
+
+
 @pytest.mark.parametrize("shape", [(65, 64, 128), (129, 64, 257), (257, 192, 300), (700, 1024, 2304), (128, 2048, 5000),
                                    (2100, 256, 2400), (2305, 128, 2048)])   # the last two: CTA-pair kernel
 @pytest.mark.parametrize("out_dtype", ["f32", "bf16"])
