@@ -1,5 +1,6 @@
 // Grouped bf16 GEMM of the routed experts: weight streaming with the operands swapped (weight rows are the M side of
-// the MMA, the expert's token tile of NT padded rows the N side).
+// the MMA, the expert's token tile of NT padded rows the N side). The plain variant also takes dense problems of at
+// most 128 rows with many features (the LM head of a decode batch): one row tile, no tables.
 //
 //   unit   one token tile x 256 weight rows of its expert: gated: 128 gate rows and the 128 up rows of the same
 //          features (two accumulators with the same lanes, so SwiGLU needs no exchange); plain: 256 features
@@ -14,7 +15,8 @@
 // (mostly padding) as weight bytes into shared memory and multiplied the padding; here a stage moves NT / 256 as
 // many. 33 tokens x 128 experts top-8 (hidden 2048, intermediate 768): gate_up 0.148 -> 0.114 (6.2 TB/s), down
 // 0.072 -> 0.059 ms; 2048 tokens x 512 experts top-10 (intermediate 512): gate_up 0.443 -> 0.370 (5.8 TB/s), down
-// 0.222 -> 0.182 ms.
+// 0.222 -> 0.182 ms. LM head, 2048 -> 151936: 1 row 0.151 -> 0.097 ms, 64 rows 0.116 -> 0.102, 128 rows 0.118 -> 0.113
+// (0.131 -> 0.123 in a loop of seconds, where the board's 1000 W hold the clocks at 1.55 GHz).
 #include "tcgen05.cuh"
 
 #include <algorithm>
@@ -43,7 +45,10 @@ struct Bf16StreamParams {
     const int32_t* tile_row0;
     const int32_t* tile_nrows;
     const int32_t* total_tiles;
+    uint32_t dense_rows;   // no tile tables: one group, row tiles in order
+    uint32_t half;         // weight rows of each of a unit's two tiles, 128 (dense: a multiple of 8 up to 128)
     __nv_bfloat16* out;    // [rows, n]
+    uint64_t out_pitch;
     uint32_t* err;
 };
 
@@ -98,7 +103,8 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
 
     // unit i of this CTA: the CTAs of a round hold neighbouring units, so that a token tile (and the weights of an
     // expert with several tiles) is read by several SMs at about the same time
-    const uint32_t total = static_cast<uint32_t>(*p.total_tiles) * p.units_per_tile;
+    const bool grouped = p.tile_expert != nullptr;
+    const uint32_t total = (grouped ? static_cast<uint32_t>(*p.total_tiles) : (p.dense_rows + NT - 1) / NT) * p.units_per_tile;
     const uint32_t my_units = blockIdx.x < total ? (total - blockIdx.x - 1) / gridDim.x + 1 : 0;
 
     if (warp == 4) {
@@ -108,17 +114,18 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             bool ok = true;
             for (uint32_t i = 0; i < my_units && ok; ++i) {
                 const uint32_t u = blockIdx.x + i * gridDim.x, tile = u / p.units_per_tile, nb = u % p.units_per_tile;
-                const int row0 = p.tile_row0[tile];
+                const int row0 = grouped ? p.tile_row0[tile] : static_cast<int>(tile * NT);
                 // rows of a tile past the last feature belong to something else and are dropped by the epilogue
-                const int w_row = p.tile_expert[tile] * static_cast<int>(p.b_rows) + static_cast<int>(nb * (GATED ? 128 : 256));
-                const int w_row2 = w_row + (GATED ? static_cast<int>(p.n) : 128);
+                const int w_row = (grouped ? p.tile_expert[tile] * static_cast<int>(p.b_rows) : 0)
+                    + static_cast<int>(nb * (GATED ? 1 : 2) * p.half);
+                const int w_row2 = w_row + static_cast<int>(GATED ? p.n : p.half);
                 for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
                     if (!mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_BS_EMPTY_WAIT)) {
                         ok = false;
                         break;
                     }
                     uint8_t* sw = smem + s * kStageBytes;
-                    mbar_expect_tx(&full_bar[s], kStageBytes);
+                    mbar_expect_tx(&full_bar[s], 2 * p.half * 128 + NT * 128);
                     const int c0 = static_cast<int>(kb) * 64;
                     tma_load_2d(sw, &map_w, &full_bar[s], c0, w_row);
                     tma_load_2d(sw + kTileBytes, &map_w, &full_bar[s], c0, w_row2);
@@ -175,16 +182,18 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         for (uint32_t i = 0; i < my_units; ++i) {
             const uint32_t u = blockIdx.x + i * gridDim.x, tile = u / p.units_per_tile, nb = u % p.units_per_tile;
             const uint32_t buf = i & 1;
-            const uint32_t nrows = static_cast<uint32_t>(p.tile_nrows[tile]);
-            const uint64_t row0 = static_cast<uint64_t>(p.tile_row0[tile]);
-            const uint32_t f = nb * (GATED ? 128 : 256) + warp * 32 + lane; // plain: and f + 128
+            const uint32_t row0 = grouped ? static_cast<uint32_t>(p.tile_row0[tile]) : tile * NT;
+            const uint32_t nrows = grouped ? static_cast<uint32_t>(p.tile_nrows[tile]) : min(static_cast<uint32_t>(NT), p.dense_rows - row0);
+            const uint32_t r = warp * 32 + lane; // weight row of each tile; rows past `half` hold nothing
+            const uint32_t f = nb * (GATED ? 1 : 2) * p.half + r; // plain: and f + half
+            const bool live = r < p.half && f < p.n, live2 = r < p.half && f + p.half < p.n;
             const bool ready = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (i >> 1) & 1, abort_flag, p.err,
                                                                  ERR_BS_ACC_FULL_WAIT));
             if (!ready)
                 break;
             tc_fence_after();
             const uint32_t src = tmem_base + lane_base + buf * 2 * NT;
-            __nv_bfloat16* out = p.out + row0 * p.n + f;
+            __nv_bfloat16* out = p.out + row0 * p.out_pitch + f;
 #pragma unroll
             for (uint32_t c = 0; c < NT / 16; ++c) {
                 if (c * 16 >= nrows)
@@ -197,17 +206,17 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                 for (uint32_t t = 0; t < 16; ++t) {
                     if (c * 16 + t < nrows) { // uniform
                         const float a = __uint_as_float(va[t]), b = __uint_as_float(vb[t]);
-                        __nv_bfloat16* o = out + static_cast<uint64_t>(c * 16 + t) * p.n;
+                        __nv_bfloat16* o = out + (c * 16 + t) * p.out_pitch;
                         if constexpr (GATED) {
                             // upstream stores the gate_up product as bf16 before SwiGLU (qsfi_moe.cu:638-651,445-463)
                             const float g = round_bf16(a), up = round_bf16(b);
-                            if (f < p.n)
+                            if (live)
                                 *o = __float2bfloat16(g * sigmoid_fast(g) * up);
                         } else {
-                            if (f < p.n)
+                            if (live)
                                 *o = __float2bfloat16(a);
-                            if (f + 128 < p.n)
-                                o[128] = __float2bfloat16(b);
+                            if (live2)
+                                o[p.half] = __float2bfloat16(b);
                         }
                     }
                 }
@@ -265,12 +274,16 @@ uint32_t bf16_tile_rows(uint32_t routes, uint32_t experts)
 
 bool bf16_stream_gemm_supported(const GemmProblem& g)
 {
-    return !g.nvfp4 && g.tile_expert != nullptr && (g.tile_rows == 32 || g.tile_rows == 64 || g.tile_rows == 128)
-        && (g.gated ? g.epilogue == EPI_SWIGLU_BF16 : g.epilogue == EPI_STORE_BF16) && g.k % 8 == 0
-        && (g.alpha == 0.0f || g.alpha == 1.0f) && g.beta == 0.0f && g.group_scale == nullptr
-        && g.group_scale_up == nullptr && g.bias == nullptr && g.out_pitch_elems == g.n
+    const bool plain = !g.nvfp4 && g.k % 8 == 0 && (g.alpha == 0.0f || g.alpha == 1.0f) && g.beta == 0.0f
+        && g.group_scale == nullptr && g.group_scale_up == nullptr && g.bias == nullptr
         && (reinterpret_cast<uintptr_t>(g.a) & 15u) == 0 && (reinterpret_cast<uintptr_t>(g.b) & 15u) == 0
         && g.a_pitch_bytes % 16 == 0 && g.b_pitch_bytes % 16 == 0;
+    if (g.tile_expert == nullptr) {
+        return plain && !g.gated && g.groups == 1 && g.epilogue == EPI_STORE_BF16 && g.a_rows <= 128
+            && (g.n + 255) / 256 >= device_sm_count();
+    }
+    return plain && (g.tile_rows == 32 || g.tile_rows == 64 || g.tile_rows == 128)
+        && (g.gated ? g.epilogue == EPI_SWIGLU_BF16 : g.epilogue == EPI_STORE_BF16);
 }
 
 cudaError_t launch_bf16_stream_gemm(const GemmProblem& g, cudaStream_t stream, const char** why)
@@ -279,23 +292,40 @@ cudaError_t launch_bf16_stream_gemm(const GemmProblem& g, cudaStream_t stream, c
     sp.n = g.n;
     sp.k_blocks = (g.k + 63) / 64;
     sp.b_rows = g.gated ? 2 * g.n : g.n;
-    sp.units_per_tile = g.gated ? (g.n + 127) / 128 : (g.n + 255) / 256;
+    sp.half = 128;
+    if (g.tile_expert == nullptr) {
+        // One row tile: the rounds of the CTAs are few, so the weight rows of a unit are chosen for a full last round
+        // (151936 features: 594 units of 256 on 148 SMs leave two units to a fifth round; 208 fill five).
+        uint32_t best = ~0u;
+        for (uint32_t half = 128; half >= 64; half -= 8) {
+            const uint32_t units = (g.n + 2 * half - 1) / (2 * half);
+            const uint32_t cost = (units + device_sm_count() - 1) / device_sm_count() * (2 * half + 8);
+            if (cost < best) {
+                best = cost;
+                sp.half = half;
+            }
+        }
+    }
+    sp.units_per_tile = (g.n + (g.gated ? 1 : 2) * sp.half - 1) / ((g.gated ? 1 : 2) * sp.half);
     sp.tile_expert = g.tile_expert;
     sp.tile_row0 = g.tile_row0;
     sp.tile_nrows = g.tile_nrows;
     sp.total_tiles = g.total_tiles;
+    sp.dense_rows = static_cast<uint32_t>(g.a_rows);
     sp.out = static_cast<__nv_bfloat16*>(g.out);
+    sp.out_pitch = g.out_pitch_elems;
     sp.err = device_error_word();
+    const uint32_t nt = g.tile_expert != nullptr ? g.tile_rows : g.a_rows <= 32 ? 32u : g.a_rows <= 64 ? 64u : 128u;
     CUtensorMap mw, mx;
-    if (!make_operand_map(&mw, false, g.b, g.k, static_cast<uint64_t>(g.groups) * sp.b_rows, g.b_pitch_bytes, 128)
-        || !make_operand_map(&mx, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, g.tile_rows)) {
+    if (!make_operand_map(&mw, false, g.b, g.k, static_cast<uint64_t>(g.groups) * sp.b_rows, g.b_pitch_bytes, sp.half)
+        || !make_operand_map(&mx, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, nt)) {
         if (why != nullptr)
             *why = "cuTensorMapEncodeTiled failed";
         return cudaErrorInvalidValue;
     }
     const uint32_t grid = static_cast<uint32_t>(
-        std::min<uint64_t>(static_cast<uint64_t>(g.max_tiles) * sp.units_per_tile, device_sm_count()));
-    switch (g.tile_rows) {
+        std::min<uint64_t>((g.tile_expert != nullptr ? g.max_tiles : (g.a_rows + nt - 1) / nt) * static_cast<uint64_t>(sp.units_per_tile), device_sm_count()));
+    switch (nt) {
     case 32:
         return g.gated ? launch_stream_instance<32, true>(mw, mx, sp, grid, stream)
                        : launch_stream_instance<32, false>(mw, mx, sp, grid, stream);

@@ -855,7 +855,7 @@ cudaError_t launch_gemm(const GemmProblem& g, cudaStream_t stream, const char** 
     if (g.nvfp4 && g.tile_expert != nullptr && g.tile_rows != 0 && g.tile_rows != static_cast<uint32_t>(kBM))
         return launch_nvfp4_swap_gemm(g, stream, why);
     if (bf16_stream_gemm_supported(g))
-        return g.max_tiles == 0 || g.n == 0 ? cudaSuccess : launch_bf16_stream_gemm(g, stream, why);
+        return (g.tile_expert != nullptr && g.max_tiles == 0) || g.n == 0 ? cudaSuccess : launch_bf16_stream_gemm(g, stream, why);
     TcParams tp = make_params(g);
     const uint32_t m_tiles = g.tile_expert != nullptr
         ? g.max_tiles

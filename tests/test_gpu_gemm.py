@@ -130,6 +130,21 @@ def test_splitk_kernel(gemm, shape, beta):
     assert torch.equal(again, out)
 
 
+# at most 128 rows and more than 148 units of features: weights streamed as the M side, unit height chosen for full
+# rounds (37889 = 148 * 256 + 1 features: the last unit holds one), every row tile height
+@pytest.mark.parametrize("rows,k,n", [(1, 64, 37889), (33, 200, 40000), (128, 128, 50007)])
+def test_feature_streaming_kernel(gemm, rows, k, n):
+    rng = np.random.default_rng(rows + k)
+    x = bf16(rng.standard_normal((rows, k), dtype=np.float32))
+    w = bf16(rng.standard_normal((n, k), dtype=np.float32) * 0.05)
+    full = torch.full((rows, n + 1), 7.0, dtype=torch.bfloat16, device="cuda")
+    gemm.gemm_bf16(to_dev(x), to_dev(w), full[:, :n])
+    want = torch.from_numpy(_ref(x, w)).to(torch.bfloat16).float().numpy()
+    got = full[:, :n].float().cpu().numpy()
+    assert np.max(np.abs(got - want)) <= 2.0 ** -7 * np.max(np.abs(want))
+    assert torch.all(full[:, n] == 7.0)
+
+
 @pytest.mark.parametrize("shape", [(65, 64, 128), (129, 64, 257), (257, 192, 300), (700, 1024, 2304), (128, 2048, 5000),
                                    (2100, 256, 2400), (2305, 128, 2048)])   # the last two: CTA-pair kernel
 @pytest.mark.parametrize("out_dtype", ["f32", "bf16"])
