@@ -279,7 +279,7 @@ bool bf16_stream_gemm_supported(const GemmProblem& g)
         && (reinterpret_cast<uintptr_t>(g.a) & 15u) == 0 && (reinterpret_cast<uintptr_t>(g.b) & 15u) == 0
         && g.a_pitch_bytes % 16 == 0 && g.b_pitch_bytes % 16 == 0;
     if (g.tile_expert == nullptr) {
-        return plain && !g.gated && g.groups == 1 && g.epilogue == EPI_STORE_BF16 && g.a_rows <= 128
+        return plain && !g.gated && g.groups == 1 && g.epilogue == EPI_STORE_BF16 && g.a_rows <= 64
             && (g.n + 255) / 256 >= device_sm_count();
     }
     return plain && (g.tile_rows == 32 || g.tile_rows == 64 || g.tile_rows == 128)

@@ -6,7 +6,9 @@
 //
 //   persistent   one CTA per SM walks the output tiles (row tile fastest, so the CTAs of a wave
 //                share one or two B panels through L2)
-//   128 x 256    tcgen05.mma kind::f16 with N = 256: the widest single-CTA instruction
+//   128 x 256    tcgen05.mma kind::f16 with N = 256: the widest single-CTA instruction; or fewer columns where
+//                that fills the last round of the SMs (151936 features: 594 tiles of 256 columns leave two tiles to a
+//                fifth round, 208 columns fill five)
 //   TMEM         two 256-column f32 accumulators: the epilogue of tile i (eight warps, two per
 //                lane quadrant) overlaps the main loop of tile i + 1
 //   smem         ring of four stages, each A 128 x 64 bf16 (16 KB) + B 256 x 64 bf16 (32 KB),
@@ -42,7 +44,7 @@ enum : uint32_t {
 template <int EPI>
 __global__ void __launch_bounds__(kDnThreads, 1)
 gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                       const TcParams p, const uint32_t tiles_m, const uint32_t tiles_n)
+                       const TcParams p, const uint32_t tiles_m, const uint32_t tiles_n, const uint32_t bn)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -88,18 +90,18 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             bool ok = true;
             for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
                 const int row0 = static_cast<int>((t % tiles_m) * kBM);
-                const int col0 = static_cast<int>((t / tiles_m) * kDnBN);
+                const int col0 = static_cast<int>((t / tiles_m) * bn);
                 for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
                     if (!mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_DN_EMPTY_WAIT)) {
                         ok = false;
                         break;
                     }
                     uint8_t* sa = smem + s * kDnStageBytes;
-                    mbar_expect_tx(&full_bar[s], kDnStageBytes);
+                    mbar_expect_tx(&full_bar[s], kTileBytes + bn * 128);
                     const int c0 = static_cast<int>(kb) * 64;
                     tma_load_2d(sa, &map_a, &full_bar[s], c0, row0);
                     tma_load_2d(sa + kTileBytes, &map_b, &full_bar[s], c0, col0);
-                    tma_load_2d(sa + 2 * kTileBytes, &map_b, &full_bar[s], c0, col0 + 128);
+                    tma_load_2d(sa + kTileBytes + bn * 64, &map_b, &full_bar[s], c0, col0 + static_cast<int>(bn / 2));
                     if (++s == kDnStages) {
                         s = 0;
                         ph ^= 1;
@@ -110,8 +112,8 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     } else if (warp == 9) {
         // ---------------------------------------------------------- MMA issuer --
         if (lane == 0) {
-            // M = 128, N = 256, bf16 x bf16 -> f32, both operands K-major
-            constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((kDnBN >> 3) << 17) | ((kBM >> 4) << 24);
+            // M = 128, N = bn, bf16 x bf16 -> f32, both operands K-major
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((bn >> 3) << 17) | ((kBM >> 4) << 24);
             uint32_t s = 0, ph = 0, u = 0;
             bool ok = true;
             for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x, ++u) {
@@ -128,10 +130,10 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                     tc_fence_after();
                     const uint32_t sa = smem_u32(smem + s * kDnStageBytes);
                     const uint64_t da = operand_desc(sa);
-                    const uint64_t db = operand_desc(sa + kTileBytes); // 256 rows: two tiles back to back
+                    const uint64_t db = operand_desc(sa + kTileBytes); // bn rows: two tiles back to back
 #pragma unroll
                     for (uint32_t j = 0; j < 4; ++j)
-                        tc_mma_bf16(d, da + 2 * j, db + 2 * j, kIdesc, (kb > 0 || j > 0) ? 1u : 0u);
+                        tc_mma_bf16(d, da + 2 * j, db + 2 * j, idesc, (kb > 0 || j > 0) ? 1u : 0u);
                     tc_commit(&empty_bar[s]);
                     if (++s == kDnStages) {
                         s = 0;
@@ -154,11 +156,17 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             tc_fence_after();
             const int row0 = static_cast<int>((t % tiles_m) * kBM);
             const int nrows = min(kBM, static_cast<int>(p.dense_rows) - row0);
-            const uint32_t nt = (t / tiles_m) * 2; // in units of the 128-column epilogue tile
+            // the tile's columns as a problem of their own: the epilogue works in units of 128 of them
+            const uint32_t col0 = (t / tiles_m) * bn;
+            TcParams q = p;
+            q.n = min(bn, p.n - col0);
+            q.out = static_cast<uint8_t*>(p.out) + static_cast<uint64_t>(col0) * (EPI == EPI_STORE_F32 ? 4 : 2);
+            if (p.bias != nullptr)
+                q.bias = p.bias + col0;
 #pragma unroll
             for (uint32_t h = 0; h < 2; ++h)
-                epilogue_tile<false, EPI, 2>(p, tmem_base + buf * kDnBN + h * kBN, warp & 3, lane, 0, row0, nrows,
-                                             nt + h, warp >> 2);
+                epilogue_tile<false, EPI, 2>(q, tmem_base + buf * kDnBN + h * kBN, warp & 3, lane, 0, row0, nrows, h,
+                                             warp >> 2);
             tc_fence_before();
             __syncwarp();
             if (lane == 0)
@@ -405,7 +413,7 @@ cudaError_t launch_pair_instance(const CUtensorMap& ma, const CUtensorMap& mb, c
 
 template <int EPI>
 cudaError_t launch_dense_instance(const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& tp, uint32_t tiles_m,
-                                  uint32_t tiles_n, cudaStream_t stream)
+                                  uint32_t tiles_n, uint32_t bn, cudaStream_t stream)
 {
     auto kernel = gemm_dense_bf16_kernel<EPI>;
     constexpr size_t smem = 1024 + kDnStages * kDnStageBytes + 256;
@@ -422,7 +430,7 @@ cudaError_t launch_dense_instance(const CUtensorMap& ma, const CUtensorMap& mb, 
             configured[dev] = true;
     }
     const uint32_t grid = std::min(tiles_m * tiles_n, device_sm_count());
-    kernel<<<grid, kDnThreads, smem, stream>>>(ma, mb, tp, tiles_m, tiles_n);
+    kernel<<<grid, kDnThreads, smem, stream>>>(ma, mb, tp, tiles_m, tiles_n, bn);
     note_launch();
     return cudaGetLastError();
 }
@@ -454,21 +462,35 @@ cudaError_t launch_gemm_dense_bf16(const GemmProblem& g, cudaStream_t stream, co
     tp.bias = g.bias;
     tp.err = device_error_word();
     const uint32_t tiles_m = static_cast<uint32_t>((g.a_rows + kBM - 1) / kBM);
-    const uint32_t tiles_n = (g.n + kDnBN - 1) / kDnBN;
+    // enough 256 x 256 tiles to give every CTA pair work: two SMs per tile, B shared between them
+    const uint32_t pair_m = static_cast<uint32_t>((g.a_rows + 255) / 256), pair_n = (g.n + 255) / 256;
+    const bool pair = static_cast<uint64_t>(pair_m) * pair_n >= kPrMinTiles && g.a_rows >= 1024;
+    // columns per tile: rounds of the SMs x columns, the narrower tiles charged for moving A more often
+    uint32_t bn = kDnBN;
+    if (!pair) {
+        uint64_t best = ~0ull;
+        for (uint32_t c = kDnBN; c >= 160; c -= 16) {
+            const uint64_t tiles = static_cast<uint64_t>(tiles_m) * ((g.n + c - 1) / c);
+            const uint64_t cost = (tiles + device_sm_count() - 1) / device_sm_count() * (c + 128);
+            if (cost < best) {
+                best = cost;
+                bn = c;
+            }
+        }
+    }
+    const uint32_t tiles_n = (g.n + bn - 1) / bn;
     CUtensorMap ma, mb;
     if (!make_operand_map(&ma, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, kBM)
-        || !make_operand_map(&mb, false, g.b, g.k, g.n, g.b_pitch_bytes, 128)) {
+        || !make_operand_map(&mb, false, g.b, g.k, g.n, g.b_pitch_bytes, pair ? 128 : bn / 2)) {
         if (why != nullptr)
             *why = "cuTensorMapEncodeTiled failed";
         return cudaErrorInvalidValue;
     }
-    // enough 256 x 256 tiles to give every CTA pair work: two SMs per tile, B shared between them
-    const uint32_t pair_m = static_cast<uint32_t>((g.a_rows + 255) / 256), pair_n = (g.n + 255) / 256;
-    if (static_cast<uint64_t>(pair_m) * pair_n >= kPrMinTiles && g.a_rows >= 1024)
+    if (pair)
         return g.epilogue == EPI_STORE_F32 ? launch_pair_instance<EPI_STORE_F32>(ma, mb, tp, pair_m, pair_n, stream)
                                            : launch_pair_instance<EPI_STORE_BF16>(ma, mb, tp, pair_m, pair_n, stream);
-    return g.epilogue == EPI_STORE_F32 ? launch_dense_instance<EPI_STORE_F32>(ma, mb, tp, tiles_m, tiles_n, stream)
-                                       : launch_dense_instance<EPI_STORE_BF16>(ma, mb, tp, tiles_m, tiles_n, stream);
+    return g.epilogue == EPI_STORE_F32 ? launch_dense_instance<EPI_STORE_F32>(ma, mb, tp, tiles_m, tiles_n, bn, stream)
+                                       : launch_dense_instance<EPI_STORE_BF16>(ma, mb, tp, tiles_m, tiles_n, bn, stream);
 }
 
 } // namespace qs3
