@@ -109,16 +109,27 @@ struct RouteTables {
     uint32_t max_pad_rows;
     uint32_t route_blocks;
     uint32_t tile_rows;    // rows of one tile: expert segments are padded to a multiple of it
+    // > 0: a shared expert joins the grouped GEMMs as group number E. The sort appends tiles of these rows (all tokens,
+    // in token order) after the experts' tiles; their padded rows start at pad_indptr[E].
+    uint32_t shared_rows;
 };
 
 size_t route_tables_bytes(uint32_t routes, uint32_t experts);
 // Carves the tables out of `base` (may be NULL for sizing); returns bytes used.
 size_t route_tables_carve(char* base, uint32_t routes, uint32_t experts, RouteTables* out,
-                          uint32_t tile_rows = kTileM);
+                          uint32_t tile_rows = kTileM, uint32_t shared_rows = 0);
+// Tokens to quantise (NVFP4) beside the sort.
+struct TokenQuant {
+    const __nv_bfloat16* x; // [rows, k]
+    uint32_t rows, k;
+    float global_scale;
+    uint8_t* packed;
+    uint8_t* scale_tiled;
+};
 // Counting sort of the routes by local expert, stable in route index.
 cudaError_t launch_route_sort(const int32_t* topk_ids, const float* topk_weights, uint32_t routes,
                               uint32_t top_k, uint32_t local_offset, uint32_t experts,
-                              const RouteTables& rt, cudaStream_t stream);
+                              const RouteTables& rt, cudaStream_t stream, const TokenQuant* quant = nullptr);
 
 // ---- router -----------------------------------------------------------------------
 // `bias` (optional f32 [num_experts]) is added to the logits before scoring.
@@ -141,6 +152,7 @@ struct CombineParams {
     uint32_t num_tokens, top_k, hidden_size;
     // optional shared expert term: out += sigmoid(x . gate_w) * shared_out
     const __nv_bfloat16* shared_out; // [T, H] or NULL
+    const int32_t* shared_row0;      // optional: row of token 0 in shared_out (NULL: 0)
     const __nv_bfloat16* hidden;     // [T, H] for the gate logit
     const __nv_bfloat16* gate_w;     // [H]
     int round_before_shared;         // 1: round the routed sum to bf16 first (upstream chain)
@@ -214,6 +226,11 @@ struct GemmProblem {
     const int32_t* indptr;
     const int32_t* pad_indptr;
     int a_scale_linear;
+    // decode kernel only: weights of a shared expert that is group number `groups` of the tile tables (NULL: none)
+    const void* shared_b;
+    const uint8_t* shared_b_scale_tiled;
+    const float* shared_scale;    // optional f32 [1] multiplier, and that of the up rows
+    const float* shared_scale_up;
     // B operand: [groups, b_rows, k]; b_rows = 2*n for gated problems
     const void* b;
     uint64_t b_pitch_bytes;

@@ -102,12 +102,17 @@ struct Nvfp4Workspace {
     size_t bytes;
 };
 
-Nvfp4Workspace carve_nvfp4(char* base, const qsfi_moe_plan_desc& d, uint32_t num_tokens, bool retile)
+// `shared_inter`: intermediate size of a shared expert of the layer call, 0: none. One of the experts' size joins the
+// grouped GEMMs of a decode batch (RouteTables::shared_rows).
+Nvfp4Workspace carve_nvfp4(char* base, const qsfi_moe_plan_desc& d, uint32_t num_tokens, bool retile,
+                           uint32_t shared_inter = 0)
 {
     Nvfp4Workspace w {};
     const uint32_t routes = num_tokens * d.top_k;
-    size_t off = route_tables_carve(base, routes, d.local_num_experts, &w.rt,
-                                    nvfp4_tile_rows(routes, d.local_num_experts, d.hidden_size, d.intermediate_size));
+    const uint32_t tile_rows = nvfp4_tile_rows(routes, d.local_num_experts, d.hidden_size, d.intermediate_size);
+    // (64-row tiles of all tokens at the end of the CTAs' ranges made a long last round: 1021 tokens 0.283 against 0.232 ms)
+    const bool merge = shared_inter == d.intermediate_size && tile_rows == 32;
+    size_t off = route_tables_carve(base, routes, d.local_num_experts, &w.rt, tile_rows, merge ? num_tokens : 0);
     const size_t rows = w.rt.max_pad_rows;
     const size_t h = d.hidden_size, i = d.intermediate_size, e = d.local_num_experts;
     if (w.rt.tile_rows == static_cast<uint32_t>(kTileM)) { // smaller tiles read the token rows in place
@@ -420,6 +425,9 @@ struct Nvfp4Weights {
     const uint8_t* d_packed;
     const uint8_t* d_sf_tiled;
     const float* d_global;  // optional
+    // shared expert that joins the grouped GEMMs (NULL: none), same meaning
+    const uint8_t *sh_gu_packed, *sh_gu_sf_tiled, *sh_d_packed, *sh_d_sf_tiled;
+    const float *sh_gu_global, *sh_gu_global_up, *sh_d_global;
 };
 
 // Routed experts on NVFP4 operands. `tokens` / `token_sf` are the quantised rows in token order (scales tiled by
@@ -464,6 +472,10 @@ qsfi_status run_routed_nvfp4(qsfi_context* ctx, const qsfi_moe_plan_desc& p, con
     g1.alpha = ga;
     g1.group_scale = wt.gu_global;
     g1.group_scale_up = wt.gu_global_up;
+    g1.shared_b = wt.sh_gu_packed;
+    g1.shared_b_scale_tiled = wt.sh_gu_sf_tiled;
+    g1.shared_scale = wt.sh_gu_global;
+    g1.shared_scale_up = wt.sh_gu_global_up;
     g1.out_global_scale = ga2;
     qsfi_status status = gemm_or_error(ctx, g1, "NVFP4 MoE gate_up GEMM");
     if (status != QSFI_STATUS_OK)
@@ -484,6 +496,9 @@ qsfi_status run_routed_nvfp4(qsfi_context* ctx, const qsfi_moe_plan_desc& p, con
     g2.out_pitch_elems = p.hidden_size;
     g2.alpha = ga2;
     g2.group_scale = wt.d_global;
+    g2.shared_b = wt.sh_d_packed;
+    g2.shared_b_scale_tiled = wt.sh_d_sf_tiled;
+    g2.shared_scale = wt.sh_d_global;
     return gemm_or_error(ctx, g2, "NVFP4 MoE down GEMM");
 }
 
@@ -966,7 +981,7 @@ qsfi_status qs3_moe_layer_workspace_size(qsfi_context* ctx, const qsfi_moe_plan*
         return set_invalid_arg(ctx, "MoE expanded route count overflows size_t");
     const bool nvfp4 = p.backend == QSFI_MOE_BACKEND_FLASHINFER_NVFP4;
     const size_t base = is_fp8_plan(p) ? carve_fp8(nullptr, p, num_tokens).bytes
-        : nvfp4                        ? carve_nvfp4(nullptr, p, num_tokens, false).bytes
+        : nvfp4                        ? carve_nvfp4(nullptr, p, num_tokens, false, shared_intermediate_size).bytes
                                        : carve_bf16(nullptr, p, num_tokens).bytes;
     *device_bytes = carve_layer(nullptr, base, p, num_tokens, shared_intermediate_size, nvfp4).bytes;
     return QSFI_STATUS_OK;
@@ -1131,7 +1146,7 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
         wf = carve_fp8(base, p, d->num_tokens);
         routed_bytes = wf.bytes;
     } else if (nvfp4) {
-        wn = carve_nvfp4(base, p, d->num_tokens, false);
+        wn = carve_nvfp4(base, p, d->num_tokens, false, shared ? is : 0);
         routed_bytes = wn.bytes;
     } else {
         wb = carve_bf16(base, p, d->num_tokens);
@@ -1197,7 +1212,9 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
     // the tokens only: they run on the plan's side stream beside the router chain (logits
     // GEMM, top-k, sort) and join the main stream where their results are consumed. The
     // per-stage recorder needs one timeline, so a profiled call stays on the main stream.
-    const bool fork = nvfp4 && shared && !stage_recording() && plan_side_stream(plan);
+    // (In a decode batch it joins the grouped GEMMs instead and the quantiser runs beside the sort: no fork.)
+    const bool merged = rt.shared_rows != 0;
+    const bool fork = nvfp4 && shared && !merged && !stage_recording() && plan_side_stream(plan);
     if (fork) {
         cudaStream_t side = plan->side_stream;
         cudaError_t ferr = cudaEventRecord(plan->ev_fork, st);
@@ -1247,8 +1264,12 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
                                          d->routed_scaling_factor, st);
     // 3. permutation
     stage_mark(st, STAGE_ROUTE_SORT);
+    const bool small_tiles = nvfp4 && rt.tile_rows != static_cast<uint32_t>(kTileM);
+    TokenQuant tq { hidden, d->num_tokens, p.hidden_size, d->act_global_scale == 0.0f ? 1.0f : d->act_global_scale,
+                    x.sh_xq, x.sh_xq_sf };
     if (err == cudaSuccess)
-        err = launch_route_sort(ids, wts, routes, p.top_k, p.local_expert_offset, p.local_num_experts, rt, st);
+        err = launch_route_sort(ids, wts, routes, p.top_k, p.local_expert_offset, p.local_num_experts, rt, st,
+                                small_tiles && !fork && !prequant ? &tq : nullptr);
     if (err != cudaSuccess)
         return set_cuda_error(ctx, err, "MoE routing");
 
@@ -1281,7 +1302,7 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
         stage_mark(st, STAGE_GATHER);
         if (fork)
             err = cudaStreamWaitEvent(st, plan->ev_quant, 0);
-        else if (!prequant)
+        else if (!prequant && !small_tiles)
             err = launch_nvfp4_quantize_rows(hidden, d->num_tokens, p.hidden_size, d->act_global_scale, x.sh_xq,
                                              x.sh_xq_sf, st);
         if (err != cudaSuccess)
@@ -1294,12 +1315,21 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
         wt.d_packed = static_cast<const uint8_t*>(d->down_weight.data);
         wt.d_sf_tiled = static_cast<const uint8_t*>(d->down_scale_tiled.data);
         wt.d_global = static_cast<const float*>(d->down_global_scale.data);
+        if (merged) {
+            wt.sh_gu_packed = static_cast<const uint8_t*>(d->shared_gate_up_weight.data);
+            wt.sh_gu_sf_tiled = static_cast<const uint8_t*>(d->shared_gate_up_scale_tiled.data);
+            wt.sh_gu_global = static_cast<const float*>(d->shared_gate_up_global_scale.data);
+            wt.sh_gu_global_up = gate_up_global_up(d->shared_gate_up_global_scale, 1);
+            wt.sh_d_packed = static_cast<const uint8_t*>(d->shared_down_weight.data);
+            wt.sh_d_sf_tiled = static_cast<const uint8_t*>(d->shared_down_scale_tiled.data);
+            wt.sh_d_global = static_cast<const float*>(d->shared_down_global_scale.data);
+        }
         status = run_routed_nvfp4(ctx, p, wn, x.sh_xq, x.sh_xq_sf, false, d->num_tokens, wt, d->act_global_scale,
                                   d->act2_global_scale);
         if (status != QSFI_STATUS_OK)
             return status;
         y2 = wn.y2;
-        if (shared) {
+        if (shared && !merged) {
             // 7. shared expert
             stage_mark(st, STAGE_SHARED);
             if (fork) {
@@ -1368,7 +1398,8 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
     cp.top_k = p.top_k;
     cp.hidden_size = p.hidden_size;
     if (shared) {
-        cp.shared_out = x.sh_out;
+        cp.shared_out = merged ? y2 : x.sh_out;
+        cp.shared_row0 = merged ? rt.pad_indptr + p.local_num_experts : nullptr;
         cp.hidden = hidden;
         cp.gate_w = static_cast<const __nv_bfloat16*>(d->shared_gate_weight.data);
         cp.round_before_shared = nvfp4 ? 0 : 1;

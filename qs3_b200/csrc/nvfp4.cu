@@ -10,21 +10,6 @@ namespace qs3 {
 
 namespace {
 
-__device__ __forceinline__ void unpack16_bf16(const uint4& a, const uint4& b, float* x)
-{
-    const uint32_t w[8] = { a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w };
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        x[2 * i] = bf16_bits_to_f32(w[i] & 0xffffu);
-        x[2 * i + 1] = bf16_bits_to_f32(w[i] >> 16);
-    }
-}
-
-__device__ __forceinline__ void load16_bf16(const __nv_bfloat16* src, float* x)
-{
-    unpack16_bf16(reinterpret_cast<const uint4*>(src)[0], reinterpret_cast<const uint4*>(src)[1], x);
-}
-
 // Weight quantisation in ONE launch: a cluster of kQwCluster blocks per expert finds the expert's amax
 // (pass 1, exchanged through distributed shared memory) and then quantises it (pass 2, whose reads come
 // from L2: about seventeen experts are in flight, 70 MB for 4-MB gate_up experts, against 126 MB of L2).
@@ -163,7 +148,7 @@ __global__ void quantize_act_linear_kernel(const __nv_bfloat16* __restrict__ x, 
     scale_linear[idx] = code;
 }
 
-// Token rows, in token order, to codes and tiled scales. A warp takes 512 elements of one row, a lane one
+// Token rows, in token order, to codes and tiled scales (quantize_row_chunk). A warp takes 512 elements of one row, a lane one
 // 16-element block: a load instruction covers contiguous sectors and four neighbouring lanes share the 32-bit
 // scale word of a 64-element group (a thread per group read with a 128-byte stride between lanes). Bound by
 // HBM (2 bytes in, 0.56 out): 8192 x 2048 beside the router GEMM 0.027 -> 0.023 ms.
@@ -171,26 +156,7 @@ __global__ void __launch_bounds__(256)
 quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, uint32_t rows, uint32_t k, float g,
                      uint8_t* __restrict__ packed, uint8_t* __restrict__ scale_tiled)
 {
-    const uint32_t chunks = (k + 511) / 512;
-    const uint64_t unit = static_cast<uint64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t row = unit / chunks;
-    const uint32_t kb = static_cast<uint32_t>(unit % chunks) * 32 + lane;
-    if (row >= rows)
-        return;
-    const bool live = kb < k / 16; // k is a multiple of 64: four lanes of a group are live together
-    uint32_t sf = 0;
-    if (live) {
-        float v[16];
-        load16_bf16(x + row * k + static_cast<uint64_t>(kb) * 16, v);
-        uint32_t lo, hi;
-        sf = static_cast<uint32_t>(quantize_block16(v, g, &lo, &hi)) << (8 * (lane & 3));
-        *reinterpret_cast<uint2*>(packed + row * (k / 2) + static_cast<uint64_t>(kb) * 8) = make_uint2(lo, hi);
-    }
-    sf |= __shfl_xor_sync(0xffffffffu, sf, 1);
-    sf |= __shfl_xor_sync(0xffffffffu, sf, 2);
-    if (live && (lane & 3) == 0)
-        *reinterpret_cast<uint32_t*>(scale_tiled + tiled_scale_offset(row, kb, k / 64)) = sf;
+    quantize_row_chunk(x, rows, k, g, packed, scale_tiled, static_cast<uint64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5));
 }
 
 // Gather of already-quantised rows into the padded permuted layout, organised by destination tile (128-row token

@@ -98,4 +98,45 @@ __host__ __device__ __forceinline__ uint64_t gated_tiled_row(uint64_t n, uint64_
     return (i >> 6) * 128 + (up ? 64 : 0) + (i & 63);
 }
 
+__device__ __forceinline__ void unpack16_bf16(const uint4& a, const uint4& b, float* x)
+{
+    const uint32_t w[8] = { a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w };
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        x[2 * i] = __uint_as_float(w[i] << 16);
+        x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+}
+
+__device__ __forceinline__ void load16_bf16(const __nv_bfloat16* src, float* x)
+{
+    unpack16_bf16(reinterpret_cast<const uint4*>(src)[0], reinterpret_cast<const uint4*>(src)[1], x);
+}
+
+// One warp quantises 512 elements (unit = row * ceil(k / 512) + chunk) of a [rows, k] bf16 matrix: a 16-element block
+// per lane; four neighbouring lanes share the 32-bit scale word of a 64-element group. k is a multiple of 64.
+__device__ __forceinline__ void quantize_row_chunk(const __nv_bfloat16* __restrict__ x, uint32_t rows, uint32_t k,
+                                                   float g, uint8_t* __restrict__ packed,
+                                                   uint8_t* __restrict__ scale_tiled, uint64_t unit)
+{
+    const uint32_t chunks = (k + 511) / 512, lane = threadIdx.x & 31;
+    const uint64_t row = unit / chunks;
+    const uint32_t kb = static_cast<uint32_t>(unit % chunks) * 32 + lane;
+    if (row >= rows)
+        return;
+    const bool live = kb < k / 16; // four lanes of a group are live together
+    uint32_t sf = 0;
+    if (live) {
+        float v[16];
+        load16_bf16(x + row * k + static_cast<uint64_t>(kb) * 16, v);
+        uint32_t lo, hi;
+        sf = static_cast<uint32_t>(quantize_block16(v, g, &lo, &hi)) << (8 * (lane & 3));
+        *reinterpret_cast<uint2*>(packed + row * (k / 2) + static_cast<uint64_t>(kb) * 8) = make_uint2(lo, hi);
+    }
+    sf |= __shfl_xor_sync(0xffffffffu, sf, 1);
+    sf |= __shfl_xor_sync(0xffffffffu, sf, 2);
+    if (live && (lane & 3) == 0)
+        *reinterpret_cast<uint32_t*>(scale_tiled + tiled_scale_offset(row, kb, k / 64)) = sf;
+}
+
 } // namespace qs3

@@ -17,6 +17,10 @@
 // change of tile costs the MMA thread only their shared-memory stores; the ring covers those. The scale copies
 // (tcgen05.cp) come from a warp of their own: from the MMA thread each costs ~50 cycles.
 //
+// A shared expert of the same intermediate size is one more group whose rows are all tokens in order, with weights of
+// its own: as GEMMs of their own on a side stream its two launches and the fork and join cost a single-token layer
+// more host time than the GPU work they overlapped.
+//
 // Gated epilogue: gate rows are lanes 0-63, up rows lanes 64-127. The values go through shared memory so that one
 // thread holds one 16-feature block of one token: SwiGLU, block maximum and quantisation without shuffles, and the
 // time does not grow with the rows of the tile.
@@ -86,12 +90,17 @@ struct SwapParams {
     const float* group_scale;
     const float* group_scale_up;
     float out_global;
+    int shared_group;        // group number of a shared expert with weights of its own (map_ws, ...), -1: none
+    const uint8_t* shared_w_sf;
+    const float* shared_scale;
+    const float* shared_scale_up;
     uint32_t* err;
 };
 
 template <int NT, bool GATED>
 __global__ void __launch_bounds__(kSwThreads, 1)
-gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const SwapParams p)
+gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_ws,
+                       const SwapParams p)
 {
     constexpr uint32_t kFeat = GATED ? 64 : 128; // output features per feature block
     constexpr uint32_t kPanelTile = NT * 128;    // one k block of the token panel
@@ -165,8 +174,10 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const SwapPara
             uint32_t tile = tile_first, fb = fb_first;
             for (uint32_t u = u0; u < u1 && ok; ++u) {
                 const int expert = p.tile_expert[tile];
-                const int w_row = expert * static_cast<int>(p.b_rows) + static_cast<int>(fb * kFeat);
-                const uint8_t* sf_src = p.w_sf + static_cast<uint64_t>(expert) * p.w_sf_group_stride
+                const bool shared = expert == p.shared_group;
+                const CUtensorMap* map = shared ? &map_ws : &map_w;
+                const int w_row = (shared ? 0 : expert * static_cast<int>(p.b_rows)) + static_cast<int>(fb * kFeat);
+                const uint8_t* sf_src = (shared ? p.shared_w_sf : p.w_sf + static_cast<uint64_t>(expert) * p.w_sf_group_stride)
                     + (static_cast<uint64_t>(fb) * p.kgroups) * 512;
                 for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
                     if (!mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_SW_EMPTY_WAIT)) {
@@ -176,11 +187,11 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const SwapPara
                     uint8_t* sb = ring + s * kSwStageBytes;
                     mbar_expect_tx(&full_bar[s], kSwStageBytes);
                     if (GATED) { // 64 gate rows, then the 64 up rows of the same features
-                        tma_load_2d(sb, &map_w, &full_bar[s], static_cast<int>(kb * 128), w_row);
-                        tma_load_2d(sb + kTileBytes / 2, &map_w, &full_bar[s], static_cast<int>(kb * 128),
+                        tma_load_2d(sb, map, &full_bar[s], static_cast<int>(kb * 128), w_row);
+                        tma_load_2d(sb + kTileBytes / 2, map, &full_bar[s], static_cast<int>(kb * 128),
                                     w_row + static_cast<int>(p.n));
                     } else {
-                        tma_load_2d(sb, &map_w, &full_bar[s], static_cast<int>(kb * 128), w_row);
+                        tma_load_2d(sb, map, &full_bar[s], static_cast<int>(kb * 128), w_row);
                     }
                     bulk_load(sb + kTileBytes, sf_src + static_cast<uint64_t>(kb) * kSfBytes, kSfBytes, &full_bar[s]);
                     if (++s == p.stages) {
@@ -314,12 +325,15 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const SwapPara
             const uint32_t row0 = static_cast<uint32_t>(p.tile_row0[tile]);
             const uint32_t nrows = static_cast<uint32_t>(p.tile_nrows[tile]);
             const int32_t* rows = nullptr;
+            uint32_t first = row0; // source row of the tile's first row when they are consecutive
             if (p.row_tokens != nullptr) {
                 const int expert = p.tile_expert[tile];
-                rows = p.row_tokens + p.indptr[expert] + (row0 - static_cast<uint32_t>(p.pad_indptr[expert]));
+                first = row0 - static_cast<uint32_t>(p.pad_indptr[expert]); // a shared expert takes the tokens in order
+                if (expert != p.shared_group)
+                    rows = p.row_tokens + p.indptr[expert] + first;
             }
             const auto src_row = [&](uint32_t j) -> uint64_t {
-                return rows != nullptr ? static_cast<uint64_t>(rows[j]) : static_cast<uint64_t>(row0) + j;
+                return rows != nullptr ? static_cast<uint64_t>(rows[j]) : static_cast<uint64_t>(first) + j;
             };
             // the tile's codes (the first kSwBatch vectors a thread) and scale words travel together
             const uint32_t items = nrows * vecs, words = p.kgroups * NT;
@@ -397,10 +411,12 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const SwapPara
                 nrows = static_cast<uint32_t>(p.tile_nrows[tile]);
                 scale = p.alpha == 0.0f ? 1.0f : p.alpha;
                 scale_up = scale;
-                if (p.group_scale != nullptr)
-                    scale *= p.group_scale[expert];
-                scale_up *= p.group_scale_up != nullptr ? p.group_scale_up[expert]
-                                                        : (p.group_scale != nullptr ? p.group_scale[expert] : 1.0f);
+                const bool shared = expert == p.shared_group;
+                const float* gs = shared ? p.shared_scale : p.group_scale != nullptr ? p.group_scale + expert : nullptr;
+                const float* gs_up = shared ? p.shared_scale_up : p.group_scale_up != nullptr ? p.group_scale_up + expert : nullptr;
+                if (gs != nullptr)
+                    scale *= *gs;
+                scale_up *= gs_up != nullptr ? *gs_up : (gs != nullptr ? *gs : 1.0f);
             }
             if (++fb_next == p.num_fb) {
                 fb_next = 0;
@@ -481,7 +497,7 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const SwapPara
 }
 
 template <int NT, bool GATED>
-cudaError_t launch_swap_instance(const CUtensorMap& mw, const SwapParams& sp, uint32_t grid, size_t smem,
+cudaError_t launch_swap_instance(const CUtensorMap& mw, const CUtensorMap& mws, const SwapParams& sp, uint32_t grid, size_t smem,
                                  cudaStream_t stream)
 {
     auto kernel = gemm_nvfp4_swap_kernel<NT, GATED>;
@@ -497,7 +513,7 @@ cudaError_t launch_swap_instance(const CUtensorMap& mw, const SwapParams& sp, ui
         if (dev >= 0 && dev < 64)
             configured[dev] = true;
     }
-    kernel<<<grid, kSwThreads, smem, stream>>>(mw, sp);
+    kernel<<<grid, kSwThreads, smem, stream>>>(mw, mws, sp);
     note_launch();
     return cudaGetLastError();
 }
@@ -563,6 +579,10 @@ cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& g, cudaStream_t stream, co
     sp.group_scale = g.group_scale;
     sp.group_scale_up = g.group_scale_up;
     sp.out_global = g.out_global_scale == 0.0f ? 1.0f : g.out_global_scale;
+    sp.shared_group = g.shared_b != nullptr ? static_cast<int>(g.groups) : -1;
+    sp.shared_w_sf = g.shared_b_scale_tiled;
+    sp.shared_scale = g.shared_scale;
+    sp.shared_scale_up = g.shared_scale_up;
     sp.err = device_error_word();
 
     const size_t fixed = 1024 + static_cast<size_t>(sp.k_blocks) * g.tile_rows * 128 + static_cast<size_t>(sp.kgroups) * 512
@@ -577,18 +597,22 @@ cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& g, cudaStream_t stream, co
     const uint32_t grid = static_cast<uint32_t>(
         std::min<uint64_t>(static_cast<uint64_t>(g.max_tiles) * sp.num_fb, device_sm_count()));
 
-    CUtensorMap mw;
-    if (!make_operand_map(&mw, true, g.b, g.k / 2, static_cast<uint64_t>(g.groups) * sp.b_rows, g.k / 2,
-                          gated ? 64 : 128)) {
+    CUtensorMap mw, mws;
+    bool mapped = make_operand_map(&mw, true, g.b, g.k / 2, static_cast<uint64_t>(g.groups) * sp.b_rows, g.k / 2,
+                                   gated ? 64 : 128);
+    mws = mw;
+    if (mapped && g.shared_b != nullptr)
+        mapped = make_operand_map(&mws, true, g.shared_b, g.k / 2, sp.b_rows, g.k / 2, gated ? 64 : 128);
+    if (!mapped) {
         if (why != nullptr)
             *why = "cuTensorMapEncodeTiled failed";
         return cudaErrorInvalidValue;
     }
     if (g.tile_rows == 32)
-        return gated ? launch_swap_instance<32, true>(mw, sp, grid, smem, stream)
-                     : launch_swap_instance<32, false>(mw, sp, grid, smem, stream);
-    return gated ? launch_swap_instance<64, true>(mw, sp, grid, smem, stream)
-                 : launch_swap_instance<64, false>(mw, sp, grid, smem, stream);
+        return gated ? launch_swap_instance<32, true>(mw, mws, sp, grid, smem, stream)
+                     : launch_swap_instance<32, false>(mw, mws, sp, grid, smem, stream);
+    return gated ? launch_swap_instance<64, true>(mw, mws, sp, grid, smem, stream)
+                 : launch_swap_instance<64, false>(mw, mws, sp, grid, smem, stream);
 }
 
 } // namespace qs3

@@ -2,6 +2,7 @@
 // weighted combine. Replaces upstream count_routes / prefix_sum / fill_route_rows /
 // scatter_hidden / finalize (qsfi_moe.cu:327-409,465-492).
 #include "common.cuh"
+#include "nvfp4.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -69,6 +70,16 @@ route_hist_kernel(const int32_t* __restrict__ ids, uint32_t routes, uint32_t loc
 {
     extern __shared__ uint16_t s_hist[];
     route_hist_body(ids, routes, local_offset, experts, block_hist, s_hist, blockIdx.x);
+}
+
+// Tiles of the shared expert (all tokens in order), after the experts' `tiles` tiles; called by a whole block.
+__device__ __forceinline__ void append_shared_tiles(const RouteTables& rt, uint32_t experts, uint32_t tiles)
+{
+    for (uint32_t m = threadIdx.x; m * rt.tile_rows < rt.shared_rows; m += blockDim.x) {
+        rt.tile_expert[tiles + m] = static_cast<int32_t>(experts);
+        rt.tile_row0[tiles + m] = static_cast<int32_t>((tiles + m) * rt.tile_rows);
+        rt.tile_nrows[tiles + m] = static_cast<int32_t>(min(rt.tile_rows, rt.shared_rows - m * rt.tile_rows));
+    }
 }
 
 // Single block: per expert, exclusive scan of the block histograms (column scan),
@@ -175,10 +186,11 @@ __device__ __forceinline__ void route_scan_body(int32_t* __restrict__ block_hist
         }
         __syncthreads();
     }
+    append_shared_tiles(rt, experts, static_cast<uint32_t>(s_carry[2]));
     if (threadIdx.x == 0) {
         rt.indptr[experts] = s_carry[0];
         rt.pad_indptr[experts] = s_carry[1];
-        *rt.total_tiles = s_carry[2];
+        *rt.total_tiles = s_carry[2] + static_cast<int>((rt.shared_rows + rt.tile_rows - 1) / rt.tile_rows);
         if (rt.pair_counts != nullptr) {
             rt.pair_counts[0] = s_carry[3];
             rt.pair_counts[1] = s_carry[4];
@@ -385,10 +397,11 @@ __device__ __forceinline__ void block_sort(const BlockSortSmem& s, const float* 
         }
         ex0 += tiles << 16 | n;
     }
+    append_shared_tiles(rt, experts, all0 >> 16);
     if (threadIdx.x == 0) {
         rt.indptr[experts] = static_cast<int32_t>(all0 & 0xffffu);
         rt.pad_indptr[experts] = static_cast<int32_t>((all0 >> 16) * tile_rows);
-        *rt.total_tiles = static_cast<int32_t>(all0 >> 16);
+        *rt.total_tiles = static_cast<int32_t>((all0 >> 16) + (rt.shared_rows + tile_rows - 1) / tile_rows);
         if (rt.pair_counts != nullptr) {
             rt.pair_counts[0] = static_cast<int32_t>(all1 >> 16);
             rt.pair_counts[1] = static_cast<int32_t>(all1 & 0xffffu);
@@ -425,8 +438,13 @@ __device__ __forceinline__ void block_sort(const BlockSortSmem& s, const float* 
 // 0.0078 ms, 10 routes 0.0058 -> 0.0042 against 256 threads with global histograms.
 __global__ void __launch_bounds__(kBlockSortThreads)
 route_sort_block_kernel(const int32_t* __restrict__ ids, const float* __restrict__ weights, uint32_t routes,
-                        uint32_t top_k, uint32_t local_offset, uint32_t experts, RouteTables rt)
+                        uint32_t top_k, uint32_t local_offset, uint32_t experts, RouteTables rt, TokenQuant quant)
 {
+    if (blockIdx.x > 0) { // the other blocks quantise the tokens meanwhile
+        quantize_row_chunk(quant.x, quant.rows, quant.k, quant.global_scale, quant.packed, quant.scale_tiled,
+                           static_cast<uint64_t>(blockIdx.x - 1) * kBlockSortWarps + (threadIdx.x >> 5));
+        return;
+    }
     extern __shared__ __align__(16) uint8_t s_dyn[];
     const BlockSortSmem s = block_sort_carve(s_dyn, experts);
     for (uint32_t i = threadIdx.x; i < routes; i += kBlockSortThreads)
@@ -514,7 +532,8 @@ __device__ __forceinline__ void sum_routes(const CombineParams& p, const int* ro
 __device__ __forceinline__ void add_shared(const CombineParams& p, uint32_t token, uint32_t vec_per_row, uint32_t i,
                                            float gate, float* acc)
 {
-    const uint4 sv = reinterpret_cast<const uint4*>(p.shared_out)[static_cast<size_t>(token) * vec_per_row + i];
+    const size_t row = (p.shared_row0 != nullptr ? static_cast<size_t>(*p.shared_row0) : 0) + token;
+    const uint4 sv = reinterpret_cast<const uint4*>(p.shared_out)[row * vec_per_row + i];
     const uint32_t ss[4] = { sv.x, sv.y, sv.z, sv.w };
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -1119,13 +1138,15 @@ cudaError_t launch_ep_rank_routes(int32_t* rows, float* weights, uint32_t tokens
     return cudaGetLastError();
 }
 
-size_t route_tables_carve(char* base, uint32_t routes, uint32_t experts, RouteTables* out, uint32_t tile_rows)
+size_t route_tables_carve(char* base, uint32_t routes, uint32_t experts, RouteTables* out, uint32_t tile_rows,
+                          uint32_t shared_rows)
 {
     RouteTables rt {};
     size_t off = 0;
     const uint64_t seg = routes < experts ? routes : experts; // experts that can hold a row
-    const uint64_t max_pad_rows = align_up(routes, tile_rows) + seg * tile_rows;
+    const uint64_t max_pad_rows = align_up(routes, tile_rows) + seg * tile_rows + align_up(shared_rows, tile_rows);
     rt.tile_rows = tile_rows;
+    rt.shared_rows = shared_rows;
     rt.max_pad_rows = static_cast<uint32_t>(max_pad_rows);
     rt.max_tiles = static_cast<uint32_t>(max_pad_rows / tile_rows);
     rt.route_blocks = (routes + kSortChunk - 1) / kSortChunk;
@@ -1159,13 +1180,26 @@ size_t route_tables_bytes(uint32_t routes, uint32_t experts)
 
 cudaError_t launch_route_sort(const int32_t* topk_ids, const float* topk_weights, uint32_t routes,
                               uint32_t top_k, uint32_t local_offset, uint32_t experts,
-                              const RouteTables& rt, cudaStream_t stream)
+                              const RouteTables& rt, cudaStream_t stream, const TokenQuant* quant)
 {
     if (routes <= kBlockSortRoutes && experts <= kBlockSortExperts) {
-        route_sort_block_kernel<<<1, kBlockSortThreads, block_sort_smem(experts), stream>>>(
-            topk_ids, topk_weights, routes, top_k, local_offset, experts, rt);
+        TokenQuant tq {};
+        uint32_t blocks = 1;
+        if (quant != nullptr) {
+            tq = *quant;
+            const uint64_t units = static_cast<uint64_t>(tq.rows) * ((tq.k + 511) / 512);
+            blocks += static_cast<uint32_t>((units + kBlockSortWarps - 1) / kBlockSortWarps);
+        }
+        route_sort_block_kernel<<<blocks, kBlockSortThreads, block_sort_smem(experts), stream>>>(
+            topk_ids, topk_weights, routes, top_k, local_offset, experts, rt, tq);
         note_launch();
         return cudaGetLastError();
+    }
+    if (quant != nullptr) {
+        const cudaError_t err = launch_nvfp4_quantize_rows(quant->x, quant->rows, quant->k, quant->global_scale,
+                                                           quant->packed, quant->scale_tiled, stream);
+        if (err != cudaSuccess)
+            return err;
     }
     const size_t smem = static_cast<size_t>(kSortWarps) * experts * sizeof(uint16_t);
     if (smem > 200 * 1024)
