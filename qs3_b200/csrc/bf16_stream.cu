@@ -100,6 +100,7 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    chain_begin();
 
     // unit i of this CTA: the CTAs of a round hold neighbouring units, so that a token tile (and the weights of an
     // expert with several tiles) is read by several SMs at about the same time
@@ -256,9 +257,7 @@ cudaError_t launch_stream_instance(const CUtensorMap& mw, const CUtensorMap& mx,
         if (dev >= 0 && dev < 64)
             configured[dev] = true;
     }
-    kernel<<<grid, kBsThreads, smem, stream>>>(mw, mx, sp);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(kernel, dim3(grid), kBsThreads, smem, stream, mw, mx, sp);
 }
 
 } // namespace

@@ -226,6 +226,7 @@ struct GemmProblem {
     const int32_t* indptr;
     const int32_t* pad_indptr;
     int a_scale_linear;
+    int tables_ready; // decode kernel only: the tile tables were complete before the predecessor in the stream started
     // decode kernel only: weights of a shared expert that is group number `groups` of the tile tables (NULL: none)
     const void* shared_b;
     const uint8_t* shared_b_scale_tiled;
@@ -335,6 +336,46 @@ cudaError_t launch_fp8_rows_gemm(const Fp8Gemm& g, cudaStream_t stream, const ch
 
 // ---- device helpers ---------------------------------------------------------------
 #ifdef __CUDACC__
+// Chained launches (programmatic dependent launch): a kernel launched by launch_chained may start while its
+// predecessor in the stream still runs, so that launch latency, set-up and the fetch of its code overlap the
+// predecessor's tail. The rules: every thread of such a kernel executes chain_begin() before it touches global memory that
+// a predecessor reads or writes (and before it exits); chain_begin() first waits for the predecessor to complete, which has
+// itself waited for its own, so at most two neighbouring kernels overlap and everything older is complete.
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_begin()
+{
+    chain_wait();
+    chain_release();
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_chained_cluster(void (*kernel)(KArgs...), uint32_t cluster, dim3 grid, uint32_t block, size_t smem,
+                                   cudaStream_t stream, Args&&... args)
+{
+    cudaLaunchConfig_t cfg {};
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim = { cluster, 1, 1 };
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    note_launch();
+    return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, uint32_t block, size_t smem, cudaStream_t stream,
+                           Args&&... args)
+{
+    return launch_chained_cluster(kernel, 1, grid, block, smem, stream, args...);
+}
+
 __device__ __forceinline__ float bf16_bits_to_f32(uint32_t bits16)
 {
     return __uint_as_float(bits16 << 16);

@@ -50,6 +50,7 @@ fp8_gather_quantize_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* _
                            uint32_t routes, uint32_t top_k, uint32_t k, uint8_t* __restrict__ codes,
                            float* __restrict__ scales)
 {
+    chain_begin();
     const uint32_t groups = k / 128;
     const uint64_t unit = static_cast<uint64_t>(blockIdx.x) * 16 + (threadIdx.x >> 4);
     const uint32_t sub = threadIdx.x & 15;
@@ -93,6 +94,7 @@ fp8_gather_rows_kernel(const uint4* __restrict__ codes, const uint32_t* __restri
                        const int32_t* __restrict__ route_prows, uint32_t routes, uint32_t top_k, uint32_t k,
                        uint4* __restrict__ out_codes, uint32_t* __restrict__ out_scales)
 {
+    chain_begin();
     const uint32_t route = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (route >= routes)
         return;
@@ -219,6 +221,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant
     constexpr uint32_t kTmemCols = kF8Bufs * kAccCols < 32 ? 32 : kF8Bufs * kAccCols;
     constexpr uint32_t kPanelTile = NT * 128;
 
+    chain_begin();
     const uint32_t tile = blockIdx.y;
     if (static_cast<int>(tile) >= *p.total_tiles)
         return;
@@ -460,9 +463,7 @@ cudaError_t launch_fp8_instance(const CUtensorMap& mw, const CUtensorMap& mx, co
         if (dev >= 0 && dev < 64)
             configured[dev] = smem;
     }
-    kernel<<<grid, kF8Threads, smem, stream>>>(mw, mx, fp);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(kernel, grid, kF8Threads, smem, stream, mw, mx, fp);
 }
 
 } // namespace
@@ -482,11 +483,9 @@ cudaError_t launch_fp8_gather_rows(const uint8_t* codes, const float* scales, co
 {
     if (routes == 0)
         return cudaSuccess;
-    fp8_gather_rows_kernel<<<(routes + 7) / 8, 256, 0, stream>>>(
-        reinterpret_cast<const uint4*>(codes), reinterpret_cast<const uint32_t*>(scales), route_prows, routes, top_k, k,
-        reinterpret_cast<uint4*>(out_codes), reinterpret_cast<uint32_t*>(out_scales));
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(fp8_gather_rows_kernel, dim3((routes + 7) / 8), 256, 0, stream,
+                          reinterpret_cast<const uint4*>(codes), reinterpret_cast<const uint32_t*>(scales), route_prows,
+                          routes, top_k, k, reinterpret_cast<uint4*>(out_codes), reinterpret_cast<uint32_t*>(out_scales));
 }
 
 cudaError_t launch_fp8_gather_quantize(const __nv_bfloat16* x, const int32_t* route_prows, uint32_t routes,
@@ -496,10 +495,8 @@ cudaError_t launch_fp8_gather_quantize(const __nv_bfloat16* x, const int32_t* ro
     if (routes == 0)
         return cudaSuccess;
     const uint64_t units = static_cast<uint64_t>(routes) * (k / 128);
-    fp8_gather_quantize_kernel<<<static_cast<uint32_t>((units + 15) / 16), 256, 0, stream>>>(
-        x, route_prows, routes, top_k, k, codes, scales);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(fp8_gather_quantize_kernel, dim3(static_cast<uint32_t>((units + 15) / 16)), 256, 0, stream, x,
+                          route_prows, routes, top_k, k, codes, scales);
 }
 
 cudaError_t launch_fp8_quantize_weight(const __nv_bfloat16* w, uint32_t experts, uint32_t rows, uint32_t k,

@@ -107,6 +107,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    chain_begin();
 
     // units of this CTA: every gridDim.x-th one. The CTAs of a round hold neighbouring units, so that a token tile
     // and the weights of an expert with several tiles are read by several SMs at about the same time
@@ -339,9 +340,7 @@ cudaError_t launch_rows_instance(const CUtensorMap& mx, const CUtensorMap& mw, c
         if (dev >= 0 && dev < 64)
             configured[dev] = true;
     }
-    kernel<<<grid, kFrThreads, smem, stream>>>(mx, mw, mo, fp);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(kernel, dim3(grid), kFrThreads, smem, stream, mx, mw, mo, fp);
 }
 
 } // namespace

@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(kThreads)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const TcParams p)
 {
+    chain_begin();
     // ---- which tile ----
     const uint32_t tile = blockIdx.y;
     int expert = 0, row0 = 0, nrows = 0;
@@ -244,6 +245,7 @@ gemm_tc_astat_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                      const __grid_constant__ CUtensorMap map_o, const TcParams p, const uint32_t stages,
                      const uint32_t nt_per_split, const uint32_t kbs)
 {
+    chain_begin();
     const uint32_t tile = blockIdx.y;
     int expert = 0, row0 = 0, nrows = 0;
     if (p.tile_expert != nullptr) {
@@ -673,9 +675,7 @@ cudaError_t launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const TcPara
         if (dev >= 0 && dev < 64)
             configured[dev] = true;
     }
-    kernel<<<grid, kThreads, smem, stream>>>(ma, mb, tp);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(kernel, grid, kThreads, smem, stream, ma, mb, tp);
 }
 
 template <bool GATED, int EPI>
@@ -704,9 +704,7 @@ cudaError_t launch_astat(const CUtensorMap& ma, const CUtensorMap& mb, const CUt
         if (dev >= 0 && dev < 64)
             configured[dev] = true;
     }
-    kernel<<<grid, kAsThreads, smem, stream>>>(ma, mb, mo, tp, stages, nt_per_split, kbs);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(kernel, grid, kAsThreads, smem, stream, ma, mb, mo, tp, stages, nt_per_split, kbs);
 }
 
 uint32_t sm_count()

@@ -82,6 +82,7 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    chain_begin();
 
     if (warp == 8) {
         // ------------------------------------------------------------ producer --
@@ -277,6 +278,7 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     cluster.sync();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    chain_begin();
 
     if (warp == 8) {
         // ------------------------------------------------------------ producer --
@@ -406,9 +408,7 @@ cudaError_t launch_pair_instance(const CUtensorMap& ma, const CUtensorMap& mb, c
             configured[dev] = true;
     }
     const uint32_t pairs = std::min(tiles_m * tiles_n, device_sm_count() / 2);
-    kernel<<<2 * pairs, kDnThreads, smem, stream>>>(ma, mb, tp, tiles_m, tiles_n);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(kernel, dim3(2 * pairs), kDnThreads, smem, stream, ma, mb, tp, tiles_m, tiles_n);
 }
 
 template <int EPI>
@@ -430,9 +430,7 @@ cudaError_t launch_dense_instance(const CUtensorMap& ma, const CUtensorMap& mb, 
             configured[dev] = true;
     }
     const uint32_t grid = std::min(tiles_m * tiles_n, device_sm_count());
-    kernel<<<grid, kDnThreads, smem, stream>>>(ma, mb, tp, tiles_m, tiles_n, bn);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(kernel, dim3(grid), kDnThreads, smem, stream, ma, mb, tp, tiles_m, tiles_n, bn);
 }
 
 } // namespace

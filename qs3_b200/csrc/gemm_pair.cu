@@ -449,6 +449,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     cluster.sync();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    chain_begin();
     const uint32_t tmem_sfa = tmem_base + 256;
     const uint32_t tmem_sfb = tmem_base + 384;
 
@@ -950,9 +951,7 @@ cudaError_t launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUte
             configured[dev] = true;
     }
     const uint32_t clusters = std::max(1u, std::min(max_units, device_sm_count() / 2));
-    kernel<<<2 * clusters, kPgThreads, smem, stream>>>(ma, mb, msa, msb, mo, pp);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(kernel, dim3(2 * clusters), kPgThreads, smem, stream, ma, mb, msa, msb, mo, pp);
 }
 
 } // namespace

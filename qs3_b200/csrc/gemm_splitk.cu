@@ -97,6 +97,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    chain_begin();
 
     bool ready = true;
     if (warp == 4) {
@@ -231,19 +232,7 @@ cudaError_t launch_splitk_instance(const CUtensorMap& mb, const CUtensorMap& ma,
         if (dev >= 0 && dev < 64)
             configured[dev] = true;
     }
-    cudaLaunchConfig_t cfg {};
-    cudaLaunchAttribute attr {};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim = { grid.x, 1, 1 };
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(kSkThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    err = cudaLaunchKernelEx(&cfg, kernel, mb, ma, sp);
-    note_launch();
-    return err;
+    return launch_chained_cluster(kernel, grid.x, grid, kSkThreads, smem, stream, mb, ma, sp);
 }
 
 // Rows of A per tile: the fewest MMA columns that hold them, 64 above that (128 x 4096 x 2048: 0.0125 ms against

@@ -495,6 +495,7 @@ qsfi_status run_routed_nvfp4(qsfi_context* ctx, const qsfi_moe_plan_desc& p, con
     g2.out = w.y2;
     g2.out_pitch_elems = p.hidden_size;
     g2.alpha = ga2;
+    g2.tables_ready = 1;
     g2.group_scale = wt.d_global;
     g2.shared_b = wt.sh_d_packed;
     g2.shared_b_scale_tiled = wt.sh_d_sf_tiled;

@@ -100,6 +100,7 @@ template <typename T, bool FUSED, bool VEC, bool QUANT>
 __global__ void __launch_bounds__(kNormThreads) rmsnorm_kernel(NormParams p)
 {
     __shared__ float s_part[kNormThreads / 32];
+    chain_begin();
     constexpr int E = Vec<T>::kElems;
     const uint32_t row = blockIdx.x;
     const T* x = static_cast<const T*>(p.x) + static_cast<uint64_t>(row) * p.x_stride;
@@ -223,17 +224,13 @@ template <typename T, bool FUSED> cudaError_t launch_norm(const NormParams& p, b
         if constexpr (sizeof(T) == 2 && FUSED) {
             if (!vec)
                 return cudaErrorInvalidValue;
-            rmsnorm_kernel<T, true, true, true><<<p.rows, kNormThreads, 0, stream>>>(p);
+            return launch_chained(rmsnorm_kernel<T, true, true, true>, dim3(p.rows), kNormThreads, 0, stream, p);
         } else {
             return cudaErrorInvalidValue;
         }
-    } else if (vec) {
-        rmsnorm_kernel<T, FUSED, true, false><<<p.rows, kNormThreads, 0, stream>>>(p);
-    } else {
-        rmsnorm_kernel<T, FUSED, false, false><<<p.rows, kNormThreads, 0, stream>>>(p);
     }
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(vec ? rmsnorm_kernel<T, FUSED, true, false> : rmsnorm_kernel<T, FUSED, false, false>,
+                          dim3(p.rows), kNormThreads, 0, stream, p);
 }
 
 // ---- validation, same checks and messages as upstream qsfi_norm_rope.cu:72-146, 208-238 ----

@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(256)
 quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, uint32_t rows, uint32_t k, float g,
                      uint8_t* __restrict__ packed, uint8_t* __restrict__ scale_tiled)
 {
+    chain_begin();
     quantize_row_chunk(x, rows, k, g, packed, scale_tiled, static_cast<uint64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5));
 }
 
@@ -172,6 +173,7 @@ gather_packed_tiles_kernel(const uint8_t* __restrict__ hidden_packed, const uint
                            const RouteTables rt, uint32_t hidden_size, uint8_t* __restrict__ packed,
                            uint8_t* __restrict__ scale_tiled, int src_scale_tiled)
 {
+    chain_begin();
     const uint32_t tile = blockIdx.y;
     if (static_cast<int>(tile) >= *rt.total_tiles)
         return;
@@ -248,10 +250,8 @@ cudaError_t launch_nvfp4_quantize_rows(const __nv_bfloat16* x, uint32_t rows, ui
                                        uint8_t* packed, uint8_t* scale_tiled, cudaStream_t stream)
 {
     const uint64_t units = static_cast<uint64_t>(rows) * ((k + 511) / 512);
-    quantize_rows_kernel<<<blocks_for(units, 8), 256, 0, stream>>>(x, rows, k, global_scale == 0.0f ? 1.0f : global_scale,
-                                                                   packed, scale_tiled);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(quantize_rows_kernel, dim3(blocks_for(units, 8)), 256, 0, stream, x, rows, k,
+                          global_scale == 0.0f ? 1.0f : global_scale, packed, scale_tiled);
 }
 
 cudaError_t launch_nvfp4_gather_tiles(const uint8_t* hidden_packed, const uint8_t* hidden_scale, const RouteTables& rt,
@@ -261,10 +261,8 @@ cudaError_t launch_nvfp4_gather_tiles(const uint8_t* hidden_packed, const uint8_
     if (rt.max_tiles == 0)
         return cudaSuccess;
     const dim3 grid((hidden_size + kGatherChunk - 1) / kGatherChunk, rt.max_tiles, 1);
-    gather_packed_tiles_kernel<<<grid, 256, 0, stream>>>(hidden_packed, hidden_scale, rt, hidden_size, packed,
-                                                        scale_tiled, src_scale_tiled);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(gather_packed_tiles_kernel, grid, 256, 0, stream, hidden_packed, hidden_scale, rt, hidden_size,
+                          packed, scale_tiled, src_scale_tiled);
 }
 
 cudaError_t launch_tile_scales(const uint8_t* linear, uint32_t experts, uint32_t rows, uint32_t k,

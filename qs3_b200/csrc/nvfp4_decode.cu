@@ -90,6 +90,7 @@ struct SwapParams {
     const float* group_scale;
     const float* group_scale_up;
     float out_global;
+    int tables_ready;        // the tile tables were complete before the predecessor in the stream started
     int shared_group;        // group number of a shared expert with weights of its own (map_ws, ...), -1: none
     const uint8_t* shared_w_sf;
     const float* shared_scale;
@@ -159,8 +160,14 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     const uint32_t tmem_xsf = tmem_wsf + 16 * p.stages;          // 2 x 4 columns per k group
     const uint32_t xsf_cols = 4 * p.kgroups;
 
+    // The tables of the down projection are older than its predecessor (the gate_up GEMM, whose start means that the
+    // sort is complete), and weights are older still: its producer fills the ring before it waits. Every other role
+    // touches what the predecessor wrote.
+    if (!p.tables_ready || warp != 4)
+        chain_begin();
+
     // this CTA's units: feature blocks [u0, u1) of the tiles in order
-    const uint64_t total = static_cast<uint64_t>(*p.total_tiles) * p.num_fb;
+    const uint64_t total = static_cast<uint64_t>(__ldcg(p.total_tiles)) * p.num_fb;
     const uint32_t u0 = static_cast<uint32_t>(total * blockIdx.x / gridDim.x);
     const uint32_t u1 = static_cast<uint32_t>(total * (blockIdx.x + 1) / gridDim.x);
     const uint32_t tile_first = u0 / p.num_fb, fb_first = u0 % p.num_fb;
@@ -173,7 +180,7 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             bool ok = true;
             uint32_t tile = tile_first, fb = fb_first;
             for (uint32_t u = u0; u < u1 && ok; ++u) {
-                const int expert = p.tile_expert[tile];
+                const int expert = __ldcg(p.tile_expert + tile);
                 const bool shared = expert == p.shared_group;
                 const CUtensorMap* map = shared ? &map_ws : &map_w;
                 const int w_row = (shared ? 0 : expert * static_cast<int>(p.b_rows)) + static_cast<int>(fb * kFeat);
@@ -488,6 +495,8 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     }
 
     // ---- teardown ----
+    if (p.tables_ready && warp == 4)
+        chain_begin();
     tc_fence_before();
     __syncthreads();
     if (warp == 5) {
@@ -513,9 +522,7 @@ cudaError_t launch_swap_instance(const CUtensorMap& mw, const CUtensorMap& mws, 
         if (dev >= 0 && dev < 64)
             configured[dev] = true;
     }
-    kernel<<<grid, kSwThreads, smem, stream>>>(mw, mws, sp);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(kernel, dim3(grid), kSwThreads, smem, stream, mw, mws, sp);
 }
 
 } // namespace
@@ -579,6 +586,7 @@ cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& g, cudaStream_t stream, co
     sp.group_scale = g.group_scale;
     sp.group_scale_up = g.group_scale_up;
     sp.out_global = g.out_global_scale == 0.0f ? 1.0f : g.out_global_scale;
+    sp.tables_ready = g.tables_ready;
     sp.shared_group = g.shared_b != nullptr ? static_cast<int>(g.groups) : -1;
     sp.shared_w_sf = g.shared_b_scale_tiled;
     sp.shared_scale = g.shared_scale;

@@ -323,6 +323,7 @@ router_topk_reg_kernel(const LogitT* __restrict__ logits, const float* __restric
                        int renormalize, float scaling)
 {
     __shared__ uint32_t s_cand[kRouterWarps][64];
+    chain_begin();
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t token = blockIdx.x * kRouterWarps + warp;
     if (token >= num_tokens)
@@ -422,9 +423,9 @@ cudaError_t launch_router_topk(const void* logits, int logits_bf16, const float*
         // register-resident variant: ITEMS = experts per lane, rounded up to a power of two
         const uint32_t per_lane = (num_experts + 31) / 32;
 #define QS3_ROUTER_REG(T, N)                                                                        \
-    router_topk_reg_kernel<T, N><<<blocks, kRouterWarps * 32, 0, stream>>>(                         \
-        static_cast<const T*>(logits), bias, ids, weights, num_tokens, num_experts, top_k,          \
-        sigmoid_score, renormalize, scaling)
+    return launch_chained(router_topk_reg_kernel<T, N>, dim3(blocks), kRouterWarps * 32, 0, stream,  \
+                          static_cast<const T*>(logits), bias, ids, weights, num_tokens,             \
+                          num_experts, top_k, sigmoid_score, renormalize, scaling)
 #define QS3_ROUTER_REG_PICK(T)                                                                      \
     do {                                                                                            \
         if (per_lane <= 1)                                                                          \
@@ -444,8 +445,6 @@ cudaError_t launch_router_topk(const void* logits, int logits_bf16, const float*
             QS3_ROUTER_REG_PICK(float);
 #undef QS3_ROUTER_REG_PICK
 #undef QS3_ROUTER_REG
-        note_launch();
-        return cudaGetLastError();
     }
     if (logits_bf16) {
         auto kernel = router_topk_kernel<__nv_bfloat16>;

@@ -69,6 +69,7 @@ route_hist_kernel(const int32_t* __restrict__ ids, uint32_t routes, uint32_t loc
                   uint32_t experts, int32_t* __restrict__ block_hist)
 {
     extern __shared__ uint16_t s_hist[];
+    chain_begin();
     route_hist_body(ids, routes, local_offset, experts, block_hist, s_hist, blockIdx.x);
 }
 
@@ -202,6 +203,7 @@ __global__ void __launch_bounds__(1024)
 route_scan_kernel(int32_t* __restrict__ block_hist, uint32_t num_blocks, uint32_t experts,
                   RouteTables rt)
 {
+    chain_begin();
     route_scan_body(block_hist, num_blocks, experts, rt);
 }
 
@@ -264,6 +266,7 @@ route_place_kernel(const int32_t* __restrict__ ids, const float* __restrict__ we
                    RouteTables rt)
 {
     extern __shared__ uint16_t s_hist[];
+    chain_begin();
     warp_histogram(ids, routes, local_offset, experts, s_hist, blockIdx.x);
     route_place_body(ids, weights, routes, top_k, local_offset, experts, rt, s_hist, blockIdx.x);
 }
@@ -440,6 +443,7 @@ __global__ void __launch_bounds__(kBlockSortThreads)
 route_sort_block_kernel(const int32_t* __restrict__ ids, const float* __restrict__ weights, uint32_t routes,
                         uint32_t top_k, uint32_t local_offset, uint32_t experts, RouteTables rt, TokenQuant quant)
 {
+    chain_begin();
     if (blockIdx.x > 0) { // the other blocks quantise the tokens meanwhile
         quantize_row_chunk(quant.x, quant.rows, quant.k, quant.global_scale, quant.packed, quant.scale_tiled,
                            static_cast<uint64_t>(blockIdx.x - 1) * kBlockSortWarps + (threadIdx.x >> 5));
@@ -458,6 +462,7 @@ gather_bf16_kernel(const uint4* __restrict__ hidden, const int32_t* __restrict__
                    uint32_t routes, uint32_t top_k, uint32_t vec_per_row,
                    uint4* __restrict__ expanded)
 {
+    chain_begin();
     const uint32_t route = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (route >= routes)
         return;
@@ -555,6 +560,7 @@ __global__ void __launch_bounds__(kCombineThreads, TOKENS == 1 ? 2 : 4) combine_
     __shared__ float s_w[TOKENS][32];
     __shared__ float s_dot[TOKENS][kGroup / 32];
     __shared__ int s_any[TOKENS];
+    chain_begin();
     const uint32_t group = threadIdx.x / kGroup, gl = threadIdx.x % kGroup;
     const uint32_t token = blockIdx.x * TOKENS + group;
     const bool live = token < p.num_tokens;
@@ -654,6 +660,7 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_norm_kernel(Combin
     __shared__ float s_dot[TOKENS][kGroup / 32];
     __shared__ float s_sq[TOKENS][kGroup / 32];
     __shared__ int s_any[TOKENS];
+    chain_begin();
     const uint32_t group = threadIdx.x / kGroup, gl = threadIdx.x % kGroup;
     const uint32_t token = blockIdx.x * TOKENS + group;
     const bool live = token < p.num_tokens;
@@ -1190,10 +1197,8 @@ cudaError_t launch_route_sort(const int32_t* topk_ids, const float* topk_weights
             const uint64_t units = static_cast<uint64_t>(tq.rows) * ((tq.k + 511) / 512);
             blocks += static_cast<uint32_t>((units + kBlockSortWarps - 1) / kBlockSortWarps);
         }
-        route_sort_block_kernel<<<blocks, kBlockSortThreads, block_sort_smem(experts), stream>>>(
-            topk_ids, topk_weights, routes, top_k, local_offset, experts, rt, tq);
-        note_launch();
-        return cudaGetLastError();
+        return launch_chained(route_sort_block_kernel, dim3(blocks), kBlockSortThreads, block_sort_smem(experts), stream,
+                              topk_ids, topk_weights, routes, top_k, local_offset, experts, rt, tq);
     }
     if (quant != nullptr) {
         const cudaError_t err = launch_nvfp4_quantize_rows(quant->x, quant->rows, quant->k, quant->global_scale,
@@ -1215,30 +1220,23 @@ cudaError_t launch_route_sort(const int32_t* topk_ids, const float* topk_weights
         if (err != cudaSuccess)
             return err;
     }
-    route_hist_kernel<<<rt.route_blocks, kSortWarps * 32, smem, stream>>>(
-        topk_ids, routes, local_offset, experts, rt.block_hist);
-    cudaError_t err = cudaGetLastError();
-    if (err != cudaSuccess)
-        return err;
-    route_scan_kernel<<<1, 1024, 0, stream>>>(rt.block_hist, rt.route_blocks, experts, rt);
-    err = cudaGetLastError();
-    if (err != cudaSuccess)
-        return err;
-    route_place_kernel<<<rt.route_blocks, kSortWarps * 32, smem, stream>>>(
-        topk_ids, topk_weights, routes, top_k, local_offset, experts, rt);
-    note_launch(3);
-    return cudaGetLastError();
+    cudaError_t err = launch_chained(route_hist_kernel, dim3(rt.route_blocks), kSortWarps * 32, smem, stream, topk_ids,
+                                     routes, local_offset, experts, rt.block_hist);
+    if (err == cudaSuccess)
+        err = launch_chained(route_scan_kernel, dim3(1), 1024, 0, stream, rt.block_hist, rt.route_blocks, experts, rt);
+    if (err == cudaSuccess)
+        err = launch_chained(route_place_kernel, dim3(rt.route_blocks), kSortWarps * 32, smem, stream, topk_ids,
+                             topk_weights, routes, top_k, local_offset, experts, rt);
+    return err;
 }
 
 cudaError_t launch_gather_bf16(const __nv_bfloat16* hidden, const int32_t* route_prows,
                                uint32_t routes, uint32_t top_k, uint32_t hidden_size,
                                __nv_bfloat16* expanded, cudaStream_t stream)
 {
-    gather_bf16_kernel<<<(routes + 7) / 8, 256, 0, stream>>>(
-        reinterpret_cast<const uint4*>(hidden), route_prows, routes, top_k, hidden_size / 8,
-        reinterpret_cast<uint4*>(expanded));
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(gather_bf16_kernel, dim3((routes + 7) / 8), 256, 0, stream,
+                          reinterpret_cast<const uint4*>(hidden), route_prows, routes, top_k, hidden_size / 8,
+                          reinterpret_cast<uint4*>(expanded));
 }
 
 cudaError_t launch_combine(const CombineParams& p, cudaStream_t stream)
@@ -1252,17 +1250,11 @@ cudaError_t launch_combine(const CombineParams& p, cudaStream_t stream)
     if (p.residual != nullptr) {
         if (p.hidden_size > kCombineThreads * 8 || p.skip_empty)
             return cudaErrorNotSupported;
-        if (spread)
-            combine_norm_kernel<1, 16><<<blocks, kCombineThreads, 0, stream>>>(p);
-        else
-            combine_norm_kernel<4, 4><<<blocks, kCombineThreads, 0, stream>>>(p);
-    } else if (spread) {
-        combine_kernel<1, 1, 16><<<blocks, kCombineThreads, 0, stream>>>(p);
-    } else {
-        combine_kernel<4, 2, 4><<<blocks, kCombineThreads, 0, stream>>>(p);
+        return launch_chained(spread ? combine_norm_kernel<1, 16> : combine_norm_kernel<4, 4>, dim3(blocks),
+                              kCombineThreads, 0, stream, p);
     }
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(spread ? combine_kernel<1, 1, 16> : combine_kernel<4, 2, 4>, dim3(blocks), kCombineThreads, 0,
+                          stream, p);
 }
 
 } // namespace qs3
