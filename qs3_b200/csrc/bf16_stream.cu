@@ -9,13 +9,15 @@
 //          time (contiguous ranges of units instead: gate_up of the 2048-token case below 0.425 ms)
 //   smem   ring of stages: two weight tiles 128 x 64 (32 KB) + token tile NT x 64
 //   TMEM   two buffers of two NT-column accumulators (lane = weight row, column = token)
-//   warps  0-3 epilogue, 4 producer (TMA), 5 MMA issuer
+//   warps  0-3 epilogue, 4 producer (TMA; token rows by gather4), 5 MMA issuer
 //
 // Bound by HBM while experts have few rows: hit experts * weight bytes. A 128 x 128 tile per CTA moved as many token
 // (mostly padding) as weight bytes into shared memory and multiplied the padding; here a stage moves NT / 256 as
 // many. 33 tokens x 128 experts top-8 (hidden 2048, intermediate 768): gate_up 0.148 -> 0.114 (6.2 TB/s), down
 // 0.072 -> 0.059 ms; 2048 tokens x 512 experts top-10 (intermediate 512): gate_up 0.443 -> 0.370 (5.8 TB/s), down
-// 0.222 -> 0.182 ms. LM head, 2048 -> 151936: 1 row 0.151 -> 0.097 ms, 64 rows 0.116 -> 0.102, 128 rows 0.118 -> 0.113
+// 0.222 -> 0.174 ms. The token rows come by gather4 straight from the caller's tensor: a pass that copied each route's
+// row first, and the loads of rows that only pad a tile, cost 7 us of the 33-token layer (0.187 -> 0.180 ms) and 56 us of
+// the 2048-token one (0.680 -> 0.624). LM head, 2048 -> 151936: 1 row 0.151 -> 0.097 ms, 64 rows 0.116 -> 0.102, 128 rows 0.118 -> 0.113
 // (0.131 -> 0.123 in a loop of seconds, where the board's 1000 W hold the clocks at 1.55 GHz).
 #include "tcgen05.cuh"
 
@@ -45,6 +47,9 @@ struct Bf16StreamParams {
     const int32_t* tile_row0;
     const int32_t* tile_nrows;
     const int32_t* total_tiles;
+    const int32_t* row_tokens; // NULL: A rows are the padded rows; else dense row -> A row
+    const int32_t* indptr;     // with row_tokens: segment starts, dense and padded
+    const int32_t* pad_indptr;
     uint32_t dense_rows;   // no tile tables: one group, row tiles in order
     uint32_t half;         // weight rows of each of a unit's two tiles, 128 (dense: a multiple of 8 up to 128)
     __nv_bfloat16* out;    // [rows, n]
@@ -110,31 +115,43 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
 
     if (warp == 4) {
         // ------------------------------------------------------------ producer --
-        if (lane == 0) {
-            uint32_t s = 0, ph = 0;
-            bool ok = true;
-            for (uint32_t i = 0; i < my_units && ok; ++i) {
-                const uint32_t u = blockIdx.x + i * gridDim.x, tile = u / p.units_per_tile, nb = u % p.units_per_tile;
-                const int row0 = grouped ? p.tile_row0[tile] : static_cast<int>(tile * NT);
-                // rows of a tile past the last feature belong to something else and are dropped by the epilogue
-                const int w_row = (grouped ? p.tile_expert[tile] * static_cast<int>(p.b_rows) : 0)
-                    + static_cast<int>(nb * (GATED ? 1 : 2) * p.half);
-                const int w_row2 = w_row + static_cast<int>(GATED ? p.n : p.half);
-                for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
-                    if (!mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_BS_EMPTY_WAIT)) {
-                        ok = false;
-                        break;
-                    }
-                    uint8_t* sw = smem + s * kStageBytes;
-                    mbar_expect_tx(&full_bar[s], 2 * p.half * 128 + NT * 128);
-                    const int c0 = static_cast<int>(kb) * 64;
+        // Lane 0 loads the weight tiles, lane j rows 4 j .. 4 j + 3 of the token tile (gather4: the rows are found
+        // through the routing tables, so no gather pass is needed, and rows past the tile's last are not moved).
+        uint32_t s = 0, ph = 0;
+        bool ok = true;
+        for (uint32_t i = 0; i < my_units && ok; ++i) {
+            const uint32_t u = blockIdx.x + i * gridDim.x, tile = u / p.units_per_tile, nb = u % p.units_per_tile;
+            const int row0 = grouped ? p.tile_row0[tile] : static_cast<int>(tile * NT);
+            const int nrows = grouped ? p.tile_nrows[tile] : static_cast<int>(min(static_cast<uint32_t>(NT), p.dense_rows - row0));
+            const int expert = grouped ? p.tile_expert[tile] : 0;
+            // rows of a tile past the last feature belong to something else and are dropped by the epilogue
+            const int w_row = expert * static_cast<int>(p.b_rows) + static_cast<int>(nb * (GATED ? 1 : 2) * p.half);
+            const int w_row2 = w_row + static_cast<int>(GATED ? p.n : p.half);
+            const int quads = (nrows + 3) / 4;
+            const int dense0 = p.row_tokens != nullptr ? p.indptr[expert] + row0 - p.pad_indptr[expert] : 0;
+            int row[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int j = min(static_cast<int>(lane) * 4 + q, nrows - 1);
+                row[q] = p.row_tokens != nullptr ? p.row_tokens[dense0 + j] : row0 + j;
+            }
+            for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
+                ok = __all_sync(0xffffffffu, mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_BS_EMPTY_WAIT));
+                if (!ok)
+                    break;
+                uint8_t* sw = smem + s * kStageBytes;
+                const int c0 = static_cast<int>(kb) * 64;
+                if (lane == 0) {
+                    mbar_expect_tx(&full_bar[s], 2 * p.half * 128 + static_cast<uint32_t>(quads) * 512);
                     tma_load_2d(sw, &map_w, &full_bar[s], c0, w_row);
                     tma_load_2d(sw + kTileBytes, &map_w, &full_bar[s], c0, w_row2);
-                    tma_load_2d(sw + 2 * kTileBytes, &map_x, &full_bar[s], c0, row0);
-                    if (++s == kNumStages) {
-                        s = 0;
-                        ph ^= 1;
-                    }
+                }
+                __syncwarp();
+                if (static_cast<int>(lane) < quads)
+                    tma_gather4(sw + 2 * kTileBytes + lane * 512, &map_x, &full_bar[s], c0, row);
+                if (++s == kNumStages) {
+                    s = 0;
+                    ph ^= 1;
                 }
             }
         }
@@ -311,13 +328,16 @@ cudaError_t launch_bf16_stream_gemm(const GemmProblem& g, cudaStream_t stream, c
     sp.tile_nrows = g.tile_nrows;
     sp.total_tiles = g.total_tiles;
     sp.dense_rows = static_cast<uint32_t>(g.a_rows);
+    sp.row_tokens = g.row_tokens;
+    sp.indptr = g.indptr;
+    sp.pad_indptr = g.pad_indptr;
     sp.out = static_cast<__nv_bfloat16*>(g.out);
     sp.out_pitch = g.out_pitch_elems;
     sp.err = device_error_word();
     const uint32_t nt = g.tile_expert != nullptr ? g.tile_rows : g.a_rows <= 32 ? 32u : g.a_rows <= 64 ? 64u : 128u;
     CUtensorMap mw, mx;
     if (!make_operand_map(&mw, false, g.b, g.k, static_cast<uint64_t>(g.groups) * sp.b_rows, g.b_pitch_bytes, sp.half)
-        || !make_operand_map(&mx, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, nt)) {
+        || !make_operand_map(&mx, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, 1)) {
         if (why != nullptr)
             *why = "cuTensorMapEncodeTiled failed";
         return cudaErrorInvalidValue;

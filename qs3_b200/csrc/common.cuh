@@ -140,10 +140,6 @@ cudaError_t launch_router_topk(const void* logits, int logits_bf16, const float*
 qsfi_status validate_router_desc(const qscu_router_topk_desc* d);
 
 // ---- permute / combine ----------------------------------------------------------
-cudaError_t launch_gather_bf16(const __nv_bfloat16* hidden, const int32_t* route_prows,
-                               uint32_t routes, uint32_t top_k, uint32_t hidden_size,
-                               __nv_bfloat16* expanded, cudaStream_t stream);
-
 struct CombineParams {
     const int32_t* route_prows;   // [T*K]
     const float* topk_weights;    // [T*K]
@@ -220,8 +216,8 @@ struct GemmProblem {
     uint64_t a_rows;
     uint64_t a_pitch_bytes;
     const uint8_t* a_scale_tiled; // NVFP4 only
-    // decode kernel only: A rows still in token order (a_scale_linear: with row-major scales), found through the
-    // routing tables; NULL: A rows are the padded rows
+    // NVFP4 decode and bf16 streaming kernels: A rows still in token order (a_scale_linear: with row-major scales), found
+    // through the routing tables; NULL: A rows are the padded rows
     const int32_t* row_tokens;
     const int32_t* indptr;
     const int32_t* pad_indptr;

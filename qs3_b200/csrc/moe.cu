@@ -70,7 +70,6 @@ bool upstream_bf16_workspace_bytes(const qsfi_moe_plan_desc& d, uint32_t num_tok
 
 struct Bf16Workspace {
     RouteTables rt;
-    __nv_bfloat16* expanded; // [pad_rows, H]
     __nv_bfloat16* act;      // [pad_rows, I]
     __nv_bfloat16* y2;       // [pad_rows, H]
     size_t bytes;
@@ -83,7 +82,6 @@ Bf16Workspace carve_bf16(char* base, const qsfi_moe_plan_desc& d, uint32_t num_t
     size_t off = route_tables_carve(base, routes, d.local_num_experts, &w.rt,
                                     bf16_tile_rows(routes, d.local_num_experts));
     const size_t rows = w.rt.max_pad_rows;
-    w.expanded = carve<__nv_bfloat16>(base, off, rows * d.hidden_size);
     w.act = carve<__nv_bfloat16>(base, off, rows * d.intermediate_size);
     w.y2 = carve<__nv_bfloat16>(base, off, rows * d.hidden_size);
     w.bytes = align_up(off, kWorkspaceAlign);
@@ -365,19 +363,18 @@ bool plan_side_stream(const qsfi_moe_plan* plan)
 }
 
 // Routed experts in bf16 on rows already described by `rt`:
-// gather -> gate_up GEMM + SwiGLU -> down GEMM. Leaves Y2 in w.y2.
+// gate_up GEMM + SwiGLU -> down GEMM. Leaves Y2 in w.y2.
 qsfi_status run_routed_bf16(qsfi_context* ctx, const qsfi_moe_plan_desc& p, const Bf16Workspace& w,
                             const __nv_bfloat16* hidden, uint32_t num_tokens,
                             const __nv_bfloat16* gate_up, const __nv_bfloat16* down)
 {
-    const uint32_t routes = num_tokens * p.top_k;
-    cudaError_t err = launch_gather_bf16(hidden, w.rt.route_prows, routes, p.top_k, p.hidden_size,
-                                         w.expanded, ctx->stream);
-    if (err != cudaSuccess)
-        return set_cuda_error(ctx, err, "MoE gather");
     stage_mark(ctx->stream, STAGE_GATE_UP_GEMM);
     GemmProblem g1 = grouped_problem(w.rt, p.local_num_experts);
-    g1.a = w.expanded;
+    g1.a = hidden; // token rows are read in place, through the routing tables
+    g1.a_rows = num_tokens;
+    g1.row_tokens = w.rt.row_tokens;
+    g1.indptr = w.rt.indptr;
+    g1.pad_indptr = w.rt.pad_indptr;
     g1.a_pitch_bytes = static_cast<uint64_t>(p.hidden_size) * 2;
     g1.b = gate_up;
     g1.b_pitch_bytes = static_cast<uint64_t>(p.hidden_size) * 2;

@@ -456,25 +456,6 @@ route_sort_block_kernel(const int32_t* __restrict__ ids, const float* __restrict
     block_sort(s, weights, routes, top_k, experts, rt); // (starts with a barrier)
 }
 
-// expanded[prow, :] = hidden[route / top_k, :]; one warp per route, 16-byte copies.
-__global__ void __launch_bounds__(256)
-gather_bf16_kernel(const uint4* __restrict__ hidden, const int32_t* __restrict__ route_prows,
-                   uint32_t routes, uint32_t top_k, uint32_t vec_per_row,
-                   uint4* __restrict__ expanded)
-{
-    chain_begin();
-    const uint32_t route = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (route >= routes)
-        return;
-    const int prow = route_prows[route];
-    if (prow < 0)
-        return;
-    const uint4* src = hidden + static_cast<size_t>(route / top_k) * vec_per_row;
-    uint4* dst = expanded + static_cast<size_t>(prow) * vec_per_row;
-    for (uint32_t i = threadIdx.x & 31; i < vec_per_row; i += 32)
-        dst[i] = src[i];
-}
-
 // out[t, :] = bf16(sum_k w[t,k] * f32(Y2[prow(t,k), :])) (+ shared-expert term).
 // TOKENS tokens per block, GROUP threads per token; a thread owns CHUNKS 8-element chunks of the row per step and
 // issues the loads of up to BATCH routes for all of them together. k ascending and f32 accumulation as upstream
@@ -1228,15 +1209,6 @@ cudaError_t launch_route_sort(const int32_t* topk_ids, const float* topk_weights
         err = launch_chained(route_place_kernel, dim3(rt.route_blocks), kSortWarps * 32, smem, stream, topk_ids,
                              topk_weights, routes, top_k, local_offset, experts, rt);
     return err;
-}
-
-cudaError_t launch_gather_bf16(const __nv_bfloat16* hidden, const int32_t* route_prows,
-                               uint32_t routes, uint32_t top_k, uint32_t hidden_size,
-                               __nv_bfloat16* expanded, cudaStream_t stream)
-{
-    return launch_chained(gather_bf16_kernel, dim3((routes + 7) / 8), 256, 0, stream,
-                          reinterpret_cast<const uint4*>(hidden), route_prows, routes, top_k, hidden_size / 8,
-                          reinterpret_cast<uint4*>(expanded));
 }
 
 cudaError_t launch_combine(const CombineParams& p, cudaStream_t stream)
