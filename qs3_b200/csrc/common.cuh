@@ -299,10 +299,11 @@ cudaError_t launch_nvfp4_gather_tiles(const uint8_t* hidden_packed, const uint8_
 // ---- FP8 (e4m3, 128 x 128 weight blocks, per-token 128-element activation groups) ----
 // Rows of one token tile of the FP8 grouped GEMM for this many routes over this many experts.
 uint32_t fp8_tile_rows(uint32_t routes, uint32_t experts);
-// codes[prow] / scales[prow] = quantise(x[route / top_k]); route_prows NULL: dense, prow = route.
-cudaError_t launch_fp8_gather_quantize(const __nv_bfloat16* x, const int32_t* route_prows, uint32_t routes,
-                                       uint32_t top_k, uint32_t k, uint8_t* codes, float* scales,
-                                       cudaStream_t stream);
+// Whether the token rows are gathered by expert before the gate_up GEMM (otherwise it finds them itself).
+bool fp8_gather_first(uint32_t routes, uint32_t experts);
+// codes / scales = quantise(x) row by row (k a multiple of 128).
+cudaError_t launch_fp8_quantize_rows(const __nv_bfloat16* x, uint32_t rows, uint32_t k, uint8_t* codes, float* scales,
+                                     cudaStream_t stream);
 // codes[prow] / scales[prow] = those of token route / top_k, already quantised (k a multiple of 128 up to 4096).
 cudaError_t launch_fp8_gather_rows(const uint8_t* codes, const float* scales, const int32_t* route_prows,
                                    uint32_t routes, uint32_t top_k, uint32_t k, uint8_t* out_codes, float* out_scales,
@@ -310,9 +311,12 @@ cudaError_t launch_fp8_gather_rows(const uint8_t* codes, const float* scales, co
 cudaError_t launch_fp8_quantize_weight(const __nv_bfloat16* w, uint32_t experts, uint32_t rows, uint32_t k,
                                        uint8_t* codes, float* scales, cudaStream_t stream);
 struct Fp8Gemm {
-    const uint8_t* x;        // e4m3 [x_rows, k], rows in the padded (tile_rows) layout
+    const uint8_t* x;        // e4m3 [x_rows, k]: rows in the padded layout, or in token order with `row_tokens`
     const float* x_scale;    // [x_rows, k / 128]
     uint64_t x_rows;
+    const int32_t* row_tokens; // 64-row tiles: dense row -> x row (with the segment starts, dense and padded)
+    const int32_t* indptr;
+    const int32_t* pad_indptr;
     const uint8_t* w;        // e4m3 [groups, gated ? 2n : n, k]
     const float* w_scale;    // [groups, ceil(rows / 128), k / 128]
     uint32_t groups, n, k;
@@ -321,13 +325,15 @@ struct Fp8Gemm {
     const int32_t* tile_row0;
     const int32_t* tile_nrows;
     const int32_t* total_tiles;
+    int tables_ready;        // the tables were complete before the predecessor in the stream started
     uint32_t max_tiles;
-    uint32_t est_tiles;      // host-side estimate of *total_tiles, sizes the feature splits
-    uint32_t tile_rows;      // 16 (decode kernel) or 128 (token rows on the M side, fp8_rows.cu)
-    void* out;               // gated: u8 [x_rows, n]; else bf16 [x_rows, n]
-    float* out_scale;        // gated: f32 [x_rows, n / 128]
+    uint32_t tile_rows;      // 64 (fp8_stream.cu) or 128 (token rows on the M side, fp8_rows.cu; x rows gathered)
+    uint64_t out_rows;       // padded rows
+    void* out;               // gated: u8 [out_rows, n]; else bf16 [out_rows, n]
+    float* out_scale;        // gated: f32 [out_rows, n / 128]
 };
 cudaError_t launch_fp8_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** why_unsupported);
+cudaError_t launch_fp8_stream_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** why_unsupported);
 cudaError_t launch_fp8_rows_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** why_unsupported);
 
 // ---- device helpers ---------------------------------------------------------------

@@ -13,12 +13,15 @@
 //   smem        ring of stages: A 128 x 128 B, B 256 x 128 B; plain: + four 16-KB boxes staging the bf16 tile for
 //               TMA stores
 //   TMEM        two 256-column buffers: k block i + 1 is multiplied while k block i is promoted
-//   warps       0-7 promotion and epilogue (lane quadrant warp % 4, column half warp / 4), 8 producer, 9 MMA
+//   warps       0-7 promotion and epilogue (lane quadrant warp % 4, column half warp / 4), 8 producer, 9 MMA, 10-11
+//               note writers: they follow the tables and fetch the scales of the next unit
 //
 // Bound by operand delivery (48 KB per k block for 128 x 256 x 128 products) and the hand-over of the two buffers:
 // 0.76 us per k block, 0.63 without the loads. 4096 tokens x 128 experts top-8 (hidden 2048, intermediate 768):
-// gate_up 0.800 -> 0.159 ms, down 0.238 -> 0.088 ms against the decode kernel on 32-row tiles, which streamed every
-// weight through shared memory once per 32 rows.
+// gate_up 0.800 -> 0.156 ms, down 0.238 -> 0.087 ms against the decode kernel on 32-row tiles, which streamed every
+// weight through shared memory once per 32 rows. With the scales and tables fetched between the units by the
+// promotion warps, and whole token tiles moved for a few rows: layer of 1024 tokens 0.200 -> 0.177 ms, 2048 0.257 ->
+// 0.222 (4096: 0.377 -> 0.366).
 #include "tcgen05.cuh"
 
 #include <algorithm>
@@ -28,17 +31,22 @@ namespace {
 
 using namespace tc;
 
-constexpr int kFrThreads = 320;
+constexpr int kFrThreads = 384;
 constexpr uint32_t kFrN = 256;                        // weight rows per unit = MMA N
 constexpr uint32_t kFrStageBytes = 3 * kTileBytes;    // A tile + two B tiles
 constexpr uint32_t kFrMaxStages = 4;
 constexpr uint32_t kFrTmemCols = 512;
+constexpr uint32_t kFrMaxKBlocks = 32;                // k <= 4096
+constexpr uint32_t kFrMaxNotes = 2;
+constexpr uint32_t kFrBox = 32;                       // token rows of one copy
 
 enum : uint32_t {
     ERR_FR_FULL_WAIT = 0x58000001u,
     ERR_FR_EMPTY_WAIT = 0x58000002u,
     ERR_FR_ACC_FULL_WAIT = 0x58000003u,
     ERR_FR_ACC_EMPTY_WAIT = 0x58000004u,
+    ERR_FR_NOTE_FULL_WAIT = 0x58000005u,
+    ERR_FR_NOTE_EMPTY_WAIT = 0x58000006u,
 };
 
 struct Fp8RowsParams {
@@ -53,9 +61,27 @@ struct Fp8RowsParams {
     const int32_t* tile_row0;
     const int32_t* tile_nrows;
     const int32_t* total_tiles;
+    int tables_ready;      // the tables were complete before the predecessor in the stream started
     void* out;             // gated: e4m3 codes [rows, n]; plain: written through map_o
     float* out_scale;      // gated: f32 [rows, n / 128]
     uint32_t* err;
+};
+
+// What the other warps need to know about a unit.
+struct FrNote {
+    int row0, nrows, b_row, b_row2;
+    float ws[2][kFrMaxKBlocks];  // block scales of the two B tiles
+};
+
+template <bool GATED> struct FrSmem {
+    static constexpr uint32_t kStages = GATED ? kFrMaxStages : kFrMaxStages - 1;
+    static constexpr uint32_t kScaleRows = GATED ? 48 : 32; // k blocks of activation scales held, over all notes
+    static constexpr uint32_t kStaging = kStages * kFrStageBytes;               // plain: four 16-KB boxes
+    static constexpr uint32_t kScales = kStaging + (GATED ? 0 : 4 * kTileBytes); // [notes][k blocks][128] f32
+    static constexpr uint32_t kNotes = kScales + kScaleRows * 128 * 4;
+    static constexpr uint32_t kAmax = kNotes + kFrMaxNotes * static_cast<uint32_t>(sizeof(FrNote)); // gated: [2][128] f32
+    static constexpr uint32_t kBars = kAmax + (GATED ? 1024 : 0);
+    static constexpr uint32_t kBytes = kBars + (2 * kFrMaxStages + 4 + 2 * kFrMaxNotes) * 8 + 16;
 };
 
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t* r)
@@ -69,17 +95,22 @@ __global__ void __launch_bounds__(kFrThreads, 1)
 gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                      const __grid_constant__ CUtensorMap map_o, const Fp8RowsParams p)
 {
-    constexpr uint32_t kStages = GATED ? kFrMaxStages : kFrMaxStages - 1;
+    using S = FrSmem<GATED>;
+    constexpr uint32_t kStages = S::kStages;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    uint8_t* staging = smem + kStages * kFrStageBytes; // plain: four 16-KB boxes
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(staging + (GATED ? 0 : 4 * kTileBytes));
+    uint8_t* staging = smem + S::kStaging;
+    float* s_xs = reinterpret_cast<float*>(smem + S::kScales);
+    FrNote* s_note = reinterpret_cast<FrNote*>(smem + S::kNotes);
+    float* s_amax = reinterpret_cast<float*>(smem + S::kAmax);
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + S::kBars);
     uint64_t* empty_bar = full_bar + kFrMaxStages;
     uint64_t* acc_full = empty_bar + kFrMaxStages;
     uint64_t* acc_empty = acc_full + 2;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    uint64_t* note_full = acc_empty + 2;
+    uint64_t* note_empty = note_full + kFrMaxNotes;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(note_empty + kFrMaxNotes);
     volatile uint32_t* abort_flag = tmem_slot + 1;
-    float* s_amax = reinterpret_cast<float*>(tmem_slot + 4); // [2][128]
 
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31;
@@ -92,6 +123,10 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 8); // one arrival per promotion warp
+        }
+        for (uint32_t b = 0; b < kFrMaxNotes; ++b) {
+            mbar_init(&note_full[b], 2);  // the two writers
+            mbar_init(&note_empty[b], 9); // promotion warps, producer
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -107,41 +142,113 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    chain_begin();
+    const bool early = p.tables_ready && (warp == 8 || warp >= 10); // weights and tables are complete: no need to wait for them
+    if (!early)
+        chain_begin();
 
     // units of this CTA: every gridDim.x-th one. The CTAs of a round hold neighbouring units, so that a token tile
     // and the weights of an expert with several tiles are read by several SMs at about the same time
     const uint32_t total = static_cast<uint32_t>(*p.total_tiles) * p.units_per_tile;
+    const uint32_t notes = max(1u, min(kFrMaxNotes, S::kScaleRows / p.k_blocks));
+    // note of the next unit in turn; every reader takes each one and gives it back
+    uint32_t nt = 0, nph = 0;
+    const auto next_note = [&] {
+        if (++nt == notes) {
+            nt = 0;
+            nph ^= 1;
+        }
+    };
+    // the B tiles of a unit, as 128-row blocks of the expert: gate and up rows of the same features, or two successive
+    // blocks (the last unit of an odd count takes its own twice and drops the second result)
+    const auto b_block = [&](uint32_t nb) { return GATED ? nb : 2 * nb; };
+    const auto b_block2 = [&](uint32_t nb) { return GATED ? p.num_fb + nb : min(2 * nb + 1, p.num_fb - 1); };
 
-    if (warp == 8) {
+    if (warp >= 10) {
+        // -------------------------------------------------------- note writers --
+        const uint32_t i = threadIdx.x - 320;
+        bool waited = !early;
+        for (uint32_t u = blockIdx.x; u < total; u += gridDim.x, next_note()) {
+            const uint32_t tile = u / p.units_per_tile, nb = u % p.units_per_tile;
+            const int row0 = p.tile_row0[tile], nrows = p.tile_nrows[tile], expert = p.tile_expert[tile];
+            if (!waited)
+                chain_begin();
+            waited = true;
+            if (!__all_sync(0xffffffffu, mbar_wait(&note_empty[nt], nph ^ 1, abort_flag, p.err, ERR_FR_NOTE_EMPTY_WAIT)))
+                break;
+            FrNote& note = s_note[nt];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float* xs = p.x_scale + static_cast<size_t>(row0 + min(static_cast<int>(i) + 64 * h, nrows - 1)) * p.k_blocks;
+                for (uint32_t kb = 0; kb < p.k_blocks; ++kb)
+                    cp_async4(s_xs + (nt * p.k_blocks + kb) * 128 + i + 64 * h, xs + kb);
+            }
+            const uint32_t fb = warp == 10 ? b_block(nb) : b_block2(nb);
+            if (lane < p.k_blocks)
+                cp_async4(&note.ws[warp - 10][lane],
+                          p.w_scale + (static_cast<size_t>(expert) * (p.b_rows / 128) + fb) * p.k_blocks + lane);
+            if (i == 0) {
+                note.row0 = row0;
+                note.nrows = nrows;
+                note.b_row = expert * static_cast<int>(p.b_rows) + static_cast<int>(b_block(nb) * 128);
+                note.b_row2 = expert * static_cast<int>(p.b_rows) + static_cast<int>(b_block2(nb) * 128);
+            }
+            cp_async_wait();
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(&note_full[nt]);
+        }
+        if (!waited)
+            chain_begin();
+    } else if (warp == 8) {
         // ------------------------------------------------------------ producer --
-        if (lane == 0) {
-            uint32_t s = 0, ph = 0;
-            bool ok = true;
-            for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x) {
-                const uint32_t tile = u / p.units_per_tile, nb = u % p.units_per_tile;
-                const int row0 = p.tile_row0[tile];
-                const int b_row = p.tile_expert[tile] * static_cast<int>(p.b_rows)
-                    + static_cast<int>(nb * (GATED ? 128 : kFrN));
-                // the second B tile: the up rows of the features, or the next 128 features (the last unit of an odd
-                // count has none: it loads its own tile again and drops the result)
-                const bool second = GATED || (nb * kFrN + 128 < p.n);
-                const int b_row2 = b_row + (GATED ? static_cast<int>(p.n) : second ? 128 : 0);
-                for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
-                    if (!mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_FR_EMPTY_WAIT)) {
-                        ok = false;
-                        break;
+        // Lane 0 loads the weight tiles, lane j box j of the token tile: boxes past its last row are not moved.
+        uint32_t s = 0, ph = 0;
+        bool ok = true;
+        uint32_t ahead = 0; // k blocks of the first unit whose weights are on their way already
+        if (early) {
+            if (blockIdx.x < total && lane == 0) {
+                const uint32_t tile = blockIdx.x / p.units_per_tile, nb = blockIdx.x % p.units_per_tile;
+                const int b0 = p.tile_expert[tile] * static_cast<int>(p.b_rows);
+                for (; ahead < min(kStages, p.k_blocks); ++ahead) {
+                    uint8_t* sa = smem + ahead * kFrStageBytes;
+                    const int c0 = static_cast<int>(ahead * 128);
+                    mbar_expect_tx_only(&full_bar[ahead], 2 * kTileBytes);
+                    tma_load_2d(sa + kTileBytes, &map_w, &full_bar[ahead], c0, b0 + static_cast<int>(b_block(nb) * 128));
+                    tma_load_2d(sa + 2 * kTileBytes, &map_w, &full_bar[ahead], c0, b0 + static_cast<int>(b_block2(nb) * 128));
+                }
+            }
+            __syncwarp();
+            chain_begin();
+        }
+        for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x, next_note(), ahead = 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait<true>(&note_full[nt], nph, abort_flag, p.err, ERR_FR_NOTE_FULL_WAIT));
+            if (!ok)
+                break;
+            const FrNote& note = s_note[nt];
+            const int nrows = note.nrows, b_row = note.b_row, b_row2 = note.b_row2, row0 = note.row0;
+            const uint32_t boxes = (static_cast<uint32_t>(nrows) + kFrBox - 1) / kFrBox;
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(&note_empty[nt]);
+            for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
+                ok = __all_sync(0xffffffffu, mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_FR_EMPTY_WAIT));
+                if (!ok)
+                    break;
+                uint8_t* sa = smem + s * kFrStageBytes;
+                const int c0 = static_cast<int>(kb * 128);
+                if (lane == 0) {
+                    mbar_expect_tx(&full_bar[s], (kb < ahead ? 0 : 2 * kTileBytes) + boxes * kFrBox * 128);
+                    if (kb >= ahead) {
+                        tma_load_2d(sa + kTileBytes, &map_w, &full_bar[s], c0, b_row);
+                        tma_load_2d(sa + 2 * kTileBytes, &map_w, &full_bar[s], c0, b_row2);
                     }
-                    uint8_t* sa = smem + s * kFrStageBytes;
-                    mbar_expect_tx(&full_bar[s], kFrStageBytes);
-                    const int c0 = static_cast<int>(kb * 128);
-                    tma_load_2d(sa + kTileBytes, &map_w, &full_bar[s], c0, b_row);
-                    tma_load_2d(sa + 2 * kTileBytes, &map_w, &full_bar[s], c0, b_row2);
-                    tma_load_2d(sa, &map_x, &full_bar[s], c0, row0);
-                    if (++s == kStages) {
-                        s = 0;
-                        ph ^= 1;
-                    }
+                }
+                __syncwarp();
+                if (lane < boxes)
+                    tma_load_2d(sa + lane * kFrBox * 128, &map_x, &full_bar[s], c0, row0 + static_cast<int>(lane * kFrBox));
+                if (++s == kStages) {
+                    s = 0;
+                    ph ^= 1;
                 }
             }
         }
@@ -186,31 +293,24 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         constexpr uint32_t kSecond = GATED ? 128 : 64; // distance of the second 64 columns
         uint32_t b = 0, bph = 0;
         bool ok = true;
-        for (uint32_t u = blockIdx.x; u < total; u += gridDim.x) {
-            const uint32_t tile = u / p.units_per_tile, nb = u % p.units_per_tile;
-            const int expert = p.tile_expert[tile];
-            const uint32_t row0 = static_cast<uint32_t>(p.tile_row0[tile]);
-            const int nrows = p.tile_nrows[tile];
+        for (uint32_t u = blockIdx.x; u < total; u += gridDim.x, next_note()) {
+            ok = __all_sync(0xffffffffu, mbar_wait(&note_full[nt], nph, abort_flag, p.err, ERR_FR_NOTE_FULL_WAIT));
+            const FrNote& note = s_note[nt];
+            const uint32_t nb = u % p.units_per_tile;
+            const uint32_t row0 = static_cast<uint32_t>(note.row0);
+            const int nrows = note.nrows;
             const bool live = static_cast<int>(quad * 32) < nrows; // whole warps without a valid row only count along
-            const uint32_t w_blocks = p.b_rows / 128;
-            const uint32_t fb = GATED ? nb : min(2 * nb + half, p.num_fb - 1);
-            const float* xs = p.x_scale + static_cast<size_t>(row0 + r) * p.k_blocks;
-            const float* ws = p.w_scale + (static_cast<size_t>(expert) * w_blocks + fb) * p.k_blocks;
-            const float* wu = ws + static_cast<size_t>(GATED ? p.num_fb : 0) * p.k_blocks;
+            const uint32_t fb = GATED ? nb : 2 * nb + half;
+            const float* xs = s_xs + nt * p.k_blocks * 128 + r;
+            const float* ws = note.ws[GATED ? 0 : half];
             float acc[2][64];
 #pragma unroll
             for (int i = 0; i < 64; ++i)
                 acc[0][i] = acc[1][i] = 0.0f;
-            float xs_next = live ? xs[0] : 0.0f, ws_next = ws[0], wu_next = GATED ? wu[0] : 0.0f;
-            for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
-                const float s0 = ws_next * xs_next;
-                const float s1 = GATED ? wu_next * xs_next : s0;
-                if (kb + 1 < p.k_blocks) { // the factors of the next k block travel while this one is waited for
-                    xs_next = live ? xs[kb + 1] : 0.0f;
-                    ws_next = ws[kb + 1];
-                    if (GATED)
-                        wu_next = wu[kb + 1];
-                }
+            for (uint32_t kb = 0; kb < p.k_blocks && ok; ++kb) {
+                const float x = xs[kb * 128];
+                const float s0 = ws[kb] * x;
+                const float s1 = GATED ? note.ws[1][kb] * x : s0;
                 ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], bph, abort_flag, p.err, ERR_FR_ACC_FULL_WAIT));
                 if (!ok)
                     break;
@@ -235,6 +335,9 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
                 b ^= 1;
                 bph ^= b == 0;
             }
+            __syncwarp();
+            if (lane == 0)
+                mbar_arrive(&note_empty[nt]);
             if constexpr (GATED) {
                 // SwiGLU, then one e4m3 scale per token and 128 features: the two halves of a row are in the two
                 // warps of a lane quadrant, which exchange their maxima
@@ -326,8 +429,8 @@ cudaError_t launch_rows_instance(const CUtensorMap& mx, const CUtensorMap& mw, c
                                  const Fp8RowsParams& fp, uint32_t grid, cudaStream_t stream)
 {
     auto kernel = gemm_fp8_rows_kernel<GATED>;
-    constexpr size_t smem = 1024 + (GATED ? kFrMaxStages * kFrStageBytes
-                                          : (kFrMaxStages - 1) * kFrStageBytes + 4 * kTileBytes) + 2048;
+    constexpr size_t smem = 1024 + FrSmem<GATED>::kBytes;
+    static_assert(smem <= 227 * 1024);
     static bool configured[64] = {}; // per instantiation and device
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
@@ -359,15 +462,16 @@ cudaError_t launch_fp8_rows_gemm(const Fp8Gemm& g, cudaStream_t stream, const ch
     fp.tile_row0 = g.tile_row0;
     fp.tile_nrows = g.tile_nrows;
     fp.total_tiles = g.total_tiles;
+    fp.tables_ready = g.tables_ready;
     fp.out = g.out;
     fp.out_scale = g.out_scale;
     fp.err = device_error_word();
     CUtensorMap mx, mw, mo;
-    bool ok = make_operand_map(&mx, true, g.x, g.k, g.x_rows, g.k, 128)
+    bool ok = make_operand_map(&mx, true, g.x, g.k, g.x_rows, g.k, kFrBox)
         && make_operand_map(&mw, true, g.w, g.k, static_cast<uint64_t>(g.groups) * fp.b_rows, g.k, 128);
     mo = mx;
     if (ok && !g.gated)
-        ok = make_operand_map(&mo, false, g.out, g.n, g.x_rows, static_cast<uint64_t>(g.n) * 2, 128);
+        ok = make_operand_map(&mo, false, g.out, g.n, g.out_rows, static_cast<uint64_t>(g.n) * 2, 128);
     if (!ok) {
         if (why != nullptr)
             *why = "cuTensorMapEncodeTiled failed";

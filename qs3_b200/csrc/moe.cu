@@ -135,7 +135,7 @@ bool is_fp8_plan(const qsfi_moe_plan_desc& d)
 
 struct Fp8Workspace {
     RouteTables rt;    // token tiles of fp8_tile_rows rows
-    uint8_t* xq;       // [pad_rows, H] e4m3
+    uint8_t* xq;       // [pad_rows, H] e4m3, if the token rows are gathered by expert
     float* xq_s;       // [pad_rows, H/128]
     uint8_t* act;      // [pad_rows, I] e4m3
     float* act_s;      // [pad_rows, I/128]
@@ -151,8 +151,10 @@ Fp8Workspace carve_fp8(char* base, const qsfi_moe_plan_desc& d, uint32_t num_tok
                                     fp8_tile_rows(routes, d.local_num_experts));
     const size_t rows = w.rt.max_pad_rows;
     const size_t h = d.hidden_size, i = d.intermediate_size;
-    w.xq = carve<uint8_t>(base, off, rows * h);
-    w.xq_s = carve<float>(base, off, rows * (h / 128));
+    if (fp8_gather_first(routes, d.local_num_experts)) {
+        w.xq = carve<uint8_t>(base, off, rows * h);
+        w.xq_s = carve<float>(base, off, rows * (h / 128));
+    }
     w.act = carve<uint8_t>(base, off, rows * i);
     w.act_s = carve<float>(base, off, rows * (i / 128));
     w.y2 = carve<__nv_bfloat16>(base, off, rows * h);
@@ -171,7 +173,7 @@ struct LayerExtra {
     uint8_t* sh_xq_sf;
     uint8_t* sh_actq;       // [T128, Is/2]
     uint8_t* sh_actq_sf;
-    uint8_t* f8_x;          // FP8 plans with 128-row token tiles: hidden quantised in token order [T, H]
+    uint8_t* f8_x;          // FP8 plans: hidden quantised in token order [T, H]
     float* f8_s;            // [T, H/128]
     size_t bytes;
 };
@@ -192,8 +194,8 @@ LayerExtra carve_layer(char* base, size_t start, const qsfi_moe_plan_desc& d, ui
         x.sh_xq = carve<uint8_t>(base, off, t128 * h / 2);
         x.sh_xq_sf = carve<uint8_t>(base, off, qs3_nvfp4_tiled_scale_bytes(t128, h));
     }
-    if (is_fp8_plan(d) && fp8_tile_rows(num_tokens * d.top_k, d.local_num_experts) == kTileM) {
-        // a token meets top_k experts: quantised once here, its codes are gathered
+    if (is_fp8_plan(d)) {
+        // a token meets top_k experts: quantised once here
         x.f8_x = carve<uint8_t>(base, off, t * h);
         x.f8_s = carve<float>(base, off, t * (h / 128));
     }
@@ -500,12 +502,11 @@ qsfi_status run_routed_nvfp4(qsfi_context* ctx, const qsfi_moe_plan_desc& p, con
     return gemm_or_error(ctx, g2, "NVFP4 MoE down GEMM");
 }
 
-// Routed experts on FP8 operands; activation rows are already in w.xq / w.xq_s.
+// Routed experts on FP8 operands: activation rows gathered in w.xq / w.xq_s or (w.xq NULL) in token order.
 qsfi_status run_routed_fp8(qsfi_context* ctx, const qsfi_moe_plan_desc& p, const Fp8Workspace& w,
-                           uint32_t num_tokens, const uint8_t* gu, const float* gu_scale, const uint8_t* down,
+                           uint32_t num_tokens, const uint8_t* tokens, const float* token_s, bool tables_ready, const uint8_t* gu, const float* gu_scale, const uint8_t* down,
                            const float* down_scale)
 {
-    const uint32_t routes = num_tokens * p.top_k;
     const auto run = [&](const Fp8Gemm& g, const char* op) {
         const char* why = nullptr;
         cudaError_t err = launch_fp8_gemm(g, ctx->stream, &why);
@@ -517,7 +518,7 @@ qsfi_status run_routed_fp8(qsfi_context* ctx, const qsfi_moe_plan_desc& p, const
         return set_cuda_error(ctx, err, op);
     };
     Fp8Gemm g {};
-    g.x_rows = w.rt.max_pad_rows;
+    g.x_rows = g.out_rows = w.rt.max_pad_rows;
     g.groups = p.local_num_experts;
     g.tile_expert = w.rt.tile_expert;
     g.tile_row0 = w.rt.tile_row0;
@@ -525,11 +526,20 @@ qsfi_status run_routed_fp8(qsfi_context* ctx, const qsfi_moe_plan_desc& p, const
     g.total_tiles = w.rt.total_tiles;
     g.max_tiles = w.rt.max_tiles;
     g.tile_rows = w.rt.tile_rows;
-    g.est_tiles = std::min(p.local_num_experts, routes) + routes / w.rt.tile_rows;
     stage_mark(ctx->stream, STAGE_GATE_UP_GEMM);
     Fp8Gemm g1 = g;
-    g1.x = w.xq;
-    g1.x_scale = w.xq_s;
+    g1.tables_ready = tables_ready;
+    if (w.xq != nullptr) {
+        g1.x = w.xq;
+        g1.x_scale = w.xq_s;
+    } else {
+        g1.x = tokens;
+        g1.x_scale = token_s;
+        g1.x_rows = num_tokens;
+        g1.row_tokens = w.rt.row_tokens;
+        g1.indptr = w.rt.indptr;
+        g1.pad_indptr = w.rt.pad_indptr;
+    }
     g1.w = gu;
     g1.w_scale = gu_scale;
     g1.n = p.intermediate_size;
@@ -542,6 +552,7 @@ qsfi_status run_routed_fp8(qsfi_context* ctx, const qsfi_moe_plan_desc& p, const
         return status;
     stage_mark(ctx->stream, STAGE_DOWN_GEMM);
     Fp8Gemm g2 = g;
+    g2.tables_ready = 1;
     g2.x = w.act;
     g2.x_scale = w.act_s;
     g2.w = down;
@@ -1273,21 +1284,14 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
 
     const __nv_bfloat16* y2 = nullptr;
     if (fp8) {
-        // 4. quantise the routed rows: straight from the bf16 tokens in a decode batch (one launch), otherwise every
-        //    token once and then a gather of the codes; 5./6. grouped GEMMs
+        // 4. quantise every token once, and for larger batches gather the codes by expert; 5./6. grouped GEMMs
         stage_mark(st, STAGE_GATHER);
-        if (x.f8_x == nullptr) {
-            err = launch_fp8_gather_quantize(hidden, rt.route_prows, routes, p.top_k, p.hidden_size, wf.xq, wf.xq_s,
-                                             st);
-        } else {
-            err = launch_fp8_gather_quantize(hidden, nullptr, d->num_tokens, 1, p.hidden_size, x.f8_x, x.f8_s, st);
-            if (err == cudaSuccess)
-                err = launch_fp8_gather_rows(x.f8_x, x.f8_s, rt.route_prows, routes, p.top_k, p.hidden_size, wf.xq,
-                                             wf.xq_s, st);
-        }
+        err = launch_fp8_quantize_rows(hidden, d->num_tokens, p.hidden_size, x.f8_x, x.f8_s, st);
+        if (err == cudaSuccess && wf.xq != nullptr)
+            err = launch_fp8_gather_rows(x.f8_x, x.f8_s, rt.route_prows, routes, p.top_k, p.hidden_size, wf.xq, wf.xq_s, st);
         if (err != cudaSuccess)
             return set_cuda_error(ctx, err, "FP8 MoE gather");
-        status = run_routed_fp8(ctx, p, wf, d->num_tokens, static_cast<const uint8_t*>(d->gate_up_weight.data),
+        status = run_routed_fp8(ctx, p, wf, d->num_tokens, x.f8_x, x.f8_s, true, static_cast<const uint8_t*>(d->gate_up_weight.data),
                                 static_cast<const float*>(d->gate_up_scale_tiled.data),
                                 static_cast<const uint8_t*>(d->down_weight.data),
                                 static_cast<const float*>(d->down_scale_tiled.data));
@@ -1994,10 +1998,10 @@ qsfi_status qs3_fp8_quantize_act(qsfi_context* ctx, const qs3_fp8_quantize_act_d
     if ((reinterpret_cast<uintptr_t>(d->x.data) & 7u) != 0 || (reinterpret_cast<uintptr_t>(d->codes.data) & 3u) != 0)
         return set_invalid_arg(ctx, "FP8 activation quantiser tensors must be 8-byte aligned");
     return set_cuda_error(ctx,
-                          launch_fp8_gather_quantize(static_cast<const __nv_bfloat16*>(d->x.data), nullptr,
-                                                     static_cast<uint32_t>(rows), 1, static_cast<uint32_t>(k),
-                                                     static_cast<uint8_t*>(d->codes.data),
-                                                     static_cast<float*>(d->scale.data), ctx->stream),
+                          launch_fp8_quantize_rows(static_cast<const __nv_bfloat16*>(d->x.data),
+                                                   static_cast<uint32_t>(rows), static_cast<uint32_t>(k),
+                                                   static_cast<uint8_t*>(d->codes.data),
+                                                   static_cast<float*>(d->scale.data), ctx->stream),
                           "qs3_fp8_quantize_act");
 }
 
@@ -2076,14 +2080,14 @@ qsfi_status qs3_moe_execute_fp8(qsfi_context* ctx, const qsfi_moe_plan* plan, co
     cudaError_t err = launch_route_sort(static_cast<const int32_t*>(desc->topk_ids.data),
                                         static_cast<const float*>(desc->topk_weights.data), routes, p.top_k,
                                         p.local_expert_offset, p.local_num_experts, w.rt, st);
-    // gather the quantised token rows (codes and their scales) into expert order
-    if (err == cudaSuccess)
-        err = launch_fp8_gather_rows(static_cast<const uint8_t*>(desc->hidden.data),
-                                     static_cast<const float*>(desc->hidden_scale.data), w.rt.route_prows, routes,
-                                     p.top_k, p.hidden_size, w.xq, w.xq_s, st);
+    const uint8_t* hq = static_cast<const uint8_t*>(desc->hidden.data);
+    const float* hs = static_cast<const float*>(desc->hidden_scale.data);
+    // larger batches: the quantised token rows (codes and their scales) gathered into expert order
+    if (err == cudaSuccess && w.xq != nullptr)
+        err = launch_fp8_gather_rows(hq, hs, w.rt.route_prows, routes, p.top_k, p.hidden_size, w.xq, w.xq_s, st);
     if (err != cudaSuccess)
         return set_cuda_error(ctx, err, "FP8 MoE routing");
-    status = run_routed_fp8(ctx, p, w, desc->num_tokens, static_cast<const uint8_t*>(desc->gate_up_weight.data),
+    status = run_routed_fp8(ctx, p, w, desc->num_tokens, hq, hs, w.xq != nullptr, static_cast<const uint8_t*>(desc->gate_up_weight.data),
                             static_cast<const float*>(desc->gate_up_weight_scale.data),
                             static_cast<const uint8_t*>(desc->down_weight.data),
                             static_cast<const float*>(desc->down_weight_scale.data));

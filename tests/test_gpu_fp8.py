@@ -111,6 +111,30 @@ def test_execute_fp8_is_deterministic_and_linear_in_routing_weight(ops, ctx, ora
     assert np.array_equal(f32(outs[2]), 2.0 * f32(outs[0]))
 
 
+# one expert of `rows` rows beside emptier ones: edges of the 16-column MMA step, of the warps' 32-token halves and of the
+# tile; rows found through the tables (e = 16) and gathered (e = 2); odd numbers of feature blocks; scales of one and of
+# two units at a time (h = 4096)
+@pytest.mark.parametrize("rows", [1, 16, 17, 32, 33, 64, 65])
+@pytest.mark.parametrize("h,i,e", [(384, 384, 16), (640, 128, 2), (4096, 256, 16)])
+def test_fp8_rows_per_expert(ops, ctx, oracle, rows, h, i, e):
+    t = rows + 5
+    d = make_moe_inputs(46 + rows, t, h, e, i)
+    ids = np.where(np.arange(t) < rows, 0, 1 + np.arange(t) % (e - 1)).astype(np.int32).reshape(t, 1)
+    w = np.linspace(0.5, 1.5, t, dtype=np.float32).reshape(t, 1)
+    gu = ops.fp8_quantize_weight(ctx, to_dev(d["gate_up"]))
+    dn = ops.fp8_quantize_weight(ctx, to_dev(d["down"]))
+    hc, hs = ops.fp8_quantize_act(ctx, to_dev(d["hidden"]))
+    plan = _plan(ops, ctx, t, h, i, e, 1)
+    ws = torch.zeros(plan.workspace_size(t), dtype=torch.uint8, device="cuda")
+    out = torch.empty((t, h), dtype=torch.bfloat16, device="cuda")
+    ops.moe_execute_fp8(plan, hc, hs, to_dev(ids), to_dev(w), gu, dn, out, ws)
+    torch.cuda.synchronize()
+    assert ctx.read_device_error() == 0
+    ref = oracle.moe_fp8(to_np(hc), to_np(hs), ids, w, (to_np(gu.codes), to_np(gu.scale)),
+                         (to_np(dn.codes), to_np(dn.scale)))
+    _check(to_np(out), ref)
+
+
 @pytest.mark.parametrize("cfg", [
     dict(t=32, h=256, e=8, k=2, i=128),
     dict(t=64, h=2048, e=128, k=8, i=768),   # decode configuration
