@@ -15,9 +15,9 @@
 // (mostly padding) as weight bytes into shared memory and multiplied the padding; here a stage moves NT / 256 as
 // many. 33 tokens x 128 experts top-8 (hidden 2048, intermediate 768): gate_up 0.148 -> 0.114 (6.2 TB/s), down
 // 0.072 -> 0.059 ms; 2048 tokens x 512 experts top-10 (intermediate 512): gate_up 0.443 -> 0.370 (5.8 TB/s), down
-// 0.222 -> 0.174 ms. The token rows come by gather4 straight from the caller's tensor: a pass that copied each route's
-// row first, and the loads of rows that only pad a tile, cost 7 us of the 33-token layer (0.187 -> 0.180 ms) and 56 us of
-// the 2048-token one (0.680 -> 0.624). LM head, 2048 -> 151936: 1 row 0.151 -> 0.097 ms, 64 rows 0.116 -> 0.102, 128 rows 0.118 -> 0.113
+// 0.222 -> 0.174 ms. The token rows of experts with few of them come by gather4 straight from the caller's tensor: a pass
+// that copied each route's row first, and the loads of rows that only pad a tile, cost 7 us of the 33-token layer (0.187 ->
+// 0.180 ms) and 56 us of the 2048-token one (0.680 -> 0.624). LM head, 2048 -> 151936: 1 row 0.151 -> 0.097 ms, 64 rows 0.116 -> 0.102, 128 rows 0.118 -> 0.113
 // (0.131 -> 0.123 in a loop of seconds, where the board's 1000 W hold the clocks at 1.55 GHz).
 #include "tcgen05.cuh"
 
@@ -30,6 +30,7 @@ using namespace tc;
 
 constexpr int kBsThreads = 192;
 constexpr uint32_t kBsMaxStages = 6;
+constexpr uint32_t kBsBox = 32; // rows of one copy where the token rows lie together
 
 enum : uint32_t {
     ERR_BS_FULL_WAIT = 0x59000001u,
@@ -50,6 +51,8 @@ struct Bf16StreamParams {
     const int32_t* row_tokens; // NULL: A rows are the padded rows; else dense row -> A row
     const int32_t* indptr;     // with row_tokens: segment starts, dense and padded
     const int32_t* pad_indptr;
+    int gathered;              // rows of experts with more than kGatherRows rows are in map_g, padded
+    int tables_ready;      // the tables were complete before the predecessor in the stream started
     uint32_t dense_rows;   // no tile tables: one group, row tiles in order
     uint32_t half;         // weight rows of each of a unit's two tiles, 128 (dense: a multiple of 8 up to 128)
     __nv_bfloat16* out;    // [rows, n]
@@ -65,6 +68,7 @@ template <int NT> struct BsRing {
 template <int NT, bool GATED>
 __global__ void __launch_bounds__(kBsThreads, 1)
 gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                        const __grid_constant__ CUtensorMap map_g, // boxes of rows that lie together
                         const Bf16StreamParams p)
 {
     constexpr uint32_t kStageBytes = BsRing<NT>::kStageBytes;
@@ -105,7 +109,9 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    chain_begin();
+    const bool early = p.tables_ready && warp == 4; // weights and tables are complete: their loads need not wait
+    if (!early)
+        chain_begin();
 
     // unit i of this CTA: the CTAs of a round hold neighbouring units, so that a token tile (and the weights of an
     // expert with several tiles) is read by several SMs at about the same time
@@ -115,8 +121,8 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
 
     if (warp == 4) {
         // ------------------------------------------------------------ producer --
-        // Lane 0 loads the weight tiles, lane j rows 4 j .. 4 j + 3 of the token tile (gather4: the rows are found
-        // through the routing tables, so no gather pass is needed, and rows past the tile's last are not moved).
+        // Lane 0 loads the weight tiles, lane j part j of the token tile, a box of rows that lie together or four rows
+        // found through the routing tables (gather4: no gather pass). Parts past the tile's last row are not moved.
         uint32_t s = 0, ph = 0;
         bool ok = true;
         for (uint32_t i = 0; i < my_units && ok; ++i) {
@@ -127,14 +133,29 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             // rows of a tile past the last feature belong to something else and are dropped by the epilogue
             const int w_row = expert * static_cast<int>(p.b_rows) + static_cast<int>(nb * (GATED ? 1 : 2) * p.half);
             const int w_row2 = w_row + static_cast<int>(GATED ? p.n : p.half);
-            const int quads = (nrows + 3) / 4;
-            const int dense0 = p.row_tokens != nullptr ? p.indptr[expert] + row0 - p.pad_indptr[expert] : 0;
-            int row[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int j = min(static_cast<int>(lane) * 4 + q, nrows - 1);
-                row[q] = p.row_tokens != nullptr ? p.row_tokens[dense0 + j] : row0 + j;
+            uint32_t ahead = 0; // k blocks whose weights are on their way already
+            if (i == 0 && early) {
+                if (lane == 0) {
+                    for (; ahead < min(kNumStages, p.k_blocks); ++ahead) {
+                        uint8_t* sw = smem + ahead * kStageBytes;
+                        mbar_expect_tx_only(&full_bar[ahead], 2 * p.half * 128);
+                        tma_load_2d(sw, &map_w, &full_bar[ahead], static_cast<int>(ahead) * 64, w_row);
+                        tma_load_2d(sw + kTileBytes, &map_w, &full_bar[ahead], static_cast<int>(ahead) * 64, w_row2);
+                    }
+                }
+                __syncwarp();
+                chain_begin();
             }
+            bool boxes = true;
+            int row[4] = {};
+            if (p.row_tokens != nullptr) {
+                const int dense = p.indptr[expert], dense0 = dense + row0 - p.pad_indptr[expert];
+                boxes = p.gathered && p.indptr[expert + 1] - dense > static_cast<int>(kGatherRows);
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    row[q] = p.row_tokens[dense0 + min(static_cast<int>(lane) * 4 + q, nrows - 1)];
+            }
+            const uint32_t part_rows = boxes ? kBsBox : 4u, parts = (static_cast<uint32_t>(nrows) + part_rows - 1) / part_rows;
             for (uint32_t kb = 0; kb < p.k_blocks; ++kb) {
                 ok = __all_sync(0xffffffffu, mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_BS_EMPTY_WAIT));
                 if (!ok)
@@ -142,19 +163,28 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                 uint8_t* sw = smem + s * kStageBytes;
                 const int c0 = static_cast<int>(kb) * 64;
                 if (lane == 0) {
-                    mbar_expect_tx(&full_bar[s], 2 * p.half * 128 + static_cast<uint32_t>(quads) * 512);
-                    tma_load_2d(sw, &map_w, &full_bar[s], c0, w_row);
-                    tma_load_2d(sw + kTileBytes, &map_w, &full_bar[s], c0, w_row2);
+                    mbar_expect_tx(&full_bar[s], (kb < ahead ? 0 : 2 * p.half * 128) + parts * part_rows * 128);
+                    if (kb >= ahead) {
+                        tma_load_2d(sw, &map_w, &full_bar[s], c0, w_row);
+                        tma_load_2d(sw + kTileBytes, &map_w, &full_bar[s], c0, w_row2);
+                    }
                 }
                 __syncwarp();
-                if (static_cast<int>(lane) < quads)
-                    tma_gather4(sw + 2 * kTileBytes + lane * 512, &map_x, &full_bar[s], c0, row);
+                if (lane < parts) {
+                    uint8_t* dst = sw + 2 * kTileBytes + lane * part_rows * 128;
+                    if (boxes)
+                        tma_load_2d(dst, &map_g, &full_bar[s], c0, row0 + static_cast<int>(lane * kBsBox));
+                    else
+                        tma_gather4(dst, &map_x, &full_bar[s], c0, row);
+                }
                 if (++s == kNumStages) {
                     s = 0;
                     ph ^= 1;
                 }
             }
         }
+        if (early && my_units == 0)
+            chain_begin();
     } else if (warp == 5) {
         // ---------------------------------------------------------- MMA issuer --
         if (lane == 0) {
@@ -212,10 +242,8 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             tc_fence_after();
             const uint32_t src = tmem_base + lane_base + buf * 2 * NT;
             __nv_bfloat16* out = p.out + row0 * p.out_pitch + f;
-#pragma unroll
-            for (uint32_t c = 0; c < NT / 16; ++c) {
-                if (c * 16 >= nrows)
-                    break;
+#pragma unroll 1 // (short code: its first pass is fetched with HBM busy)
+            for (uint32_t c = 0; c * 16 < nrows; ++c) {
                 uint32_t va[16], vb[16];
                 tc_ld16(src + c * 16, va);
                 tc_ld16(src + NT + c * 16, vb);
@@ -257,7 +285,7 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
 }
 
 template <int NT, bool GATED>
-cudaError_t launch_stream_instance(const CUtensorMap& mw, const CUtensorMap& mx, const Bf16StreamParams& sp,
+cudaError_t launch_stream_instance(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mg, const Bf16StreamParams& sp,
                                    uint32_t grid, cudaStream_t stream)
 {
     auto kernel = gemm_bf16_stream_kernel<NT, GATED>;
@@ -274,7 +302,7 @@ cudaError_t launch_stream_instance(const CUtensorMap& mw, const CUtensorMap& mx,
         if (dev >= 0 && dev < 64)
             configured[dev] = true;
     }
-    return launch_chained(kernel, dim3(grid), kBsThreads, smem, stream, mw, mx, sp);
+    return launch_chained(kernel, dim3(grid), kBsThreads, smem, stream, mw, mx, mg, sp);
 }
 
 } // namespace
@@ -328,16 +356,27 @@ cudaError_t launch_bf16_stream_gemm(const GemmProblem& g, cudaStream_t stream, c
     sp.tile_nrows = g.tile_nrows;
     sp.total_tiles = g.total_tiles;
     sp.dense_rows = static_cast<uint32_t>(g.a_rows);
+    sp.tables_ready = g.tables_ready;
     sp.row_tokens = g.row_tokens;
     sp.indptr = g.indptr;
     sp.pad_indptr = g.pad_indptr;
+    sp.gathered = g.gathered != nullptr;
     sp.out = static_cast<__nv_bfloat16*>(g.out);
     sp.out_pitch = g.out_pitch_elems;
     sp.err = device_error_word();
     const uint32_t nt = g.tile_expert != nullptr ? g.tile_rows : g.a_rows <= 32 ? 32u : g.a_rows <= 64 ? 64u : 128u;
-    CUtensorMap mw, mx;
-    if (!make_operand_map(&mw, false, g.b, g.k, static_cast<uint64_t>(g.groups) * sp.b_rows, g.b_pitch_bytes, sp.half)
-        || !make_operand_map(&mx, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, 1)) {
+    CUtensorMap mw, mx, mg;
+    bool ok = make_operand_map(&mw, false, g.b, g.k, static_cast<uint64_t>(g.groups) * sp.b_rows, g.b_pitch_bytes, sp.half);
+    if (g.row_tokens == nullptr) {
+        ok = ok && make_operand_map(&mg, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, kBsBox);
+        mx = mg;
+    } else {
+        ok = ok && make_operand_map(&mx, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, 1);
+        mg = mx;
+        if (g.gathered != nullptr) // (as many rows as the tables have room for)
+            ok = ok && make_operand_map(&mg, false, g.gathered, g.k, static_cast<uint64_t>(g.max_tiles) * g.tile_rows, g.k * 2ull, kBsBox);
+    }
+    if (!ok) {
         if (why != nullptr)
             *why = "cuTensorMapEncodeTiled failed";
         return cudaErrorInvalidValue;
@@ -346,14 +385,14 @@ cudaError_t launch_bf16_stream_gemm(const GemmProblem& g, cudaStream_t stream, c
         std::min<uint64_t>((g.tile_expert != nullptr ? g.max_tiles : (g.a_rows + nt - 1) / nt) * static_cast<uint64_t>(sp.units_per_tile), device_sm_count()));
     switch (nt) {
     case 32:
-        return g.gated ? launch_stream_instance<32, true>(mw, mx, sp, grid, stream)
-                       : launch_stream_instance<32, false>(mw, mx, sp, grid, stream);
+        return g.gated ? launch_stream_instance<32, true>(mw, mx, mg, sp, grid, stream)
+                       : launch_stream_instance<32, false>(mw, mx, mg, sp, grid, stream);
     case 64:
-        return g.gated ? launch_stream_instance<64, true>(mw, mx, sp, grid, stream)
-                       : launch_stream_instance<64, false>(mw, mx, sp, grid, stream);
+        return g.gated ? launch_stream_instance<64, true>(mw, mx, mg, sp, grid, stream)
+                       : launch_stream_instance<64, false>(mw, mx, mg, sp, grid, stream);
     default:
-        return g.gated ? launch_stream_instance<128, true>(mw, mx, sp, grid, stream)
-                       : launch_stream_instance<128, false>(mw, mx, sp, grid, stream);
+        return g.gated ? launch_stream_instance<128, true>(mw, mx, mg, sp, grid, stream)
+                       : launch_stream_instance<128, false>(mw, mx, mg, sp, grid, stream);
     }
 }
 

@@ -140,6 +140,22 @@ cudaError_t launch_router_topk(const void* logits, int logits_bf16, const float*
 qsfi_status validate_router_desc(const qscu_router_topk_desc* d);
 
 // ---- permute / combine ----------------------------------------------------------
+// dst[padded row] = src[token] for the rows of experts with more than `min_rows` rows (row_bytes a multiple of 16).
+cudaError_t launch_gather_rows(const void* src, uint32_t row_bytes, const RouteTables& rt, uint32_t min_rows, void* dst,
+                               cudaStream_t stream);
+// The streaming kernels find an expert's token rows through the tables up to this many rows, and take more from a
+// gathered copy. A gather4 load occupies the copy engine for about 80 cycles: twelve stay well below the 1400 cycles in
+// which a stage's weights arrive from HBM, but the weights of an expert with several tiles come from L2, faster. bf16
+// layer, 128 experts top-8, in place / line at 64 / at 48 rows: 1024 tokens 0.325 / 0.306 / 0.266 ms, 2048 tokens 0.510 /
+// 0.335 / 0.335, 512 of a skewed router 0.213 / 0.190 / 0.178; all rows gathered: 512 experts top-10, 2048 tokens 0.630
+// -> 0.659.
+constexpr uint32_t kGatherRows = 48;
+// Whether a batch may have such experts and is large enough to look: the pass costs a few microseconds.
+inline bool gather_rows_pays(uint32_t num_tokens, uint32_t top_k, uint32_t experts)
+{
+    return num_tokens > kGatherRows && num_tokens * static_cast<uint64_t>(top_k) >= 8ull * experts;
+}
+
 struct CombineParams {
     const int32_t* route_prows;   // [T*K]
     const float* topk_weights;    // [T*K]
@@ -222,7 +238,9 @@ struct GemmProblem {
     const int32_t* indptr;
     const int32_t* pad_indptr;
     int a_scale_linear;
-    int tables_ready; // decode kernel only: the tile tables were complete before the predecessor in the stream started
+    const void* gathered; // bf16 streaming kernel, with row_tokens: padded-layout copy of the rows of experts with more
+                          // than kGatherRows rows, or NULL
+    int tables_ready; // NVFP4 decode and bf16 streaming kernels: the tile tables were complete before the predecessor in the stream started
     // decode kernel only: weights of a shared expert that is group number `groups` of the tile tables (NULL: none)
     const void* shared_b;
     const uint8_t* shared_b_scale_tiled;
@@ -299,24 +317,20 @@ cudaError_t launch_nvfp4_gather_tiles(const uint8_t* hidden_packed, const uint8_
 // ---- FP8 (e4m3, 128 x 128 weight blocks, per-token 128-element activation groups) ----
 // Rows of one token tile of the FP8 grouped GEMM for this many routes over this many experts.
 uint32_t fp8_tile_rows(uint32_t routes, uint32_t experts);
-// Whether the token rows are gathered by expert before the gate_up GEMM (otherwise it finds them itself).
-bool fp8_gather_first(uint32_t routes, uint32_t experts);
 // codes / scales = quantise(x) row by row (k a multiple of 128).
 cudaError_t launch_fp8_quantize_rows(const __nv_bfloat16* x, uint32_t rows, uint32_t k, uint8_t* codes, float* scales,
                                      cudaStream_t stream);
-// codes[prow] / scales[prow] = those of token route / top_k, already quantised (k a multiple of 128 up to 4096).
-cudaError_t launch_fp8_gather_rows(const uint8_t* codes, const float* scales, const int32_t* route_prows,
-                                   uint32_t routes, uint32_t top_k, uint32_t k, uint8_t* out_codes, float* out_scales,
-                                   cudaStream_t stream);
 cudaError_t launch_fp8_quantize_weight(const __nv_bfloat16* w, uint32_t experts, uint32_t rows, uint32_t k,
                                        uint8_t* codes, float* scales, cudaStream_t stream);
 struct Fp8Gemm {
     const uint8_t* x;        // e4m3 [x_rows, k]: rows in the padded layout, or in token order with `row_tokens`
     const float* x_scale;    // [x_rows, k / 128]
     uint64_t x_rows;
-    const int32_t* row_tokens; // 64-row tiles: dense row -> x row (with the segment starts, dense and padded)
+    const int32_t* row_tokens; // NULL: x rows are the padded rows; else dense row -> x row (with the segment starts)
     const int32_t* indptr;
     const int32_t* pad_indptr;
+    const uint8_t* gathered; // with row_tokens: padded-layout copy of the rows of experts with more than kGatherRows
+                             // rows (128-row tiles: of all), or NULL
     const uint8_t* w;        // e4m3 [groups, gated ? 2n : n, k]
     const float* w_scale;    // [groups, ceil(rows / 128), k / 128]
     uint32_t groups, n, k;
@@ -327,7 +341,7 @@ struct Fp8Gemm {
     const int32_t* total_tiles;
     int tables_ready;        // the tables were complete before the predecessor in the stream started
     uint32_t max_tiles;
-    uint32_t tile_rows;      // 64 (fp8_stream.cu) or 128 (token rows on the M side, fp8_rows.cu; x rows gathered)
+    uint32_t tile_rows;      // 64 (fp8_stream.cu) or 128 (token rows on the M side, fp8_rows.cu)
     uint64_t out_rows;       // padded rows
     void* out;               // gated: u8 [out_rows, n]; else bf16 [out_rows, n]
     float* out_scale;        // gated: f32 [out_rows, n / 128]

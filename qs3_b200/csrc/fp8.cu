@@ -1,6 +1,6 @@
 // FP8 block-scaled expert path (e4m3 weights with one f32 scale per 128 x 128 block,
-// e4m3 activations with one f32 scale per token per 128 elements): quantisers, the
-// gather of quantised rows and the choice of the grouped GEMM (tcgen05, kind::f8f6f4).
+// e4m3 activations with one f32 scale per token per 128 elements): quantisers
+// and the choice of the grouped GEMM (tcgen05, kind::f8f6f4).
 //
 // Upstream has no FP8 MoE surface (only the dtype enum values, qs_tensor.h:20-24); the
 // conventions are this library's and are restated by the CPU oracle:
@@ -75,37 +75,6 @@ fp8_quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, uint32_t rows, uin
         scales[unit] = s;
 }
 
-// codes[prow, :] / scales[prow, :] = those of token route / top_k, already quantised. A warp per route, all of a
-// row's loads in flight (k <= 4096: eight 16-byte vectors and one scale word per lane).
-__global__ void __launch_bounds__(256)
-fp8_gather_rows_kernel(const uint4* __restrict__ codes, const uint32_t* __restrict__ scales,
-                       const int32_t* __restrict__ route_prows, uint32_t routes, uint32_t top_k, uint32_t k,
-                       uint4* __restrict__ out_codes, uint32_t* __restrict__ out_scales)
-{
-    chain_begin();
-    const uint32_t route = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (route >= routes)
-        return;
-    const int prow = route_prows[route];
-    if (prow < 0)
-        return;
-    const uint32_t vecs = k / 16, groups = k / 128;
-    const uint4* src = codes + static_cast<size_t>(route / top_k) * vecs;
-    uint4* dst = out_codes + static_cast<size_t>(prow) * vecs;
-    const uint32_t sc = lane < groups ? scales[static_cast<size_t>(route / top_k) * groups + lane] : 0u;
-    uint4 v[8];
-#pragma unroll
-    for (uint32_t i = 0; i < 8; ++i)
-        if (lane + 32 * i < vecs)
-            v[i] = src[lane + 32 * i];
-#pragma unroll
-    for (uint32_t i = 0; i < 8; ++i)
-        if (lane + 32 * i < vecs)
-            dst[lane + 32 * i] = v[i];
-    if (lane < groups)
-        out_scales[static_cast<size_t>(prow) * groups + lane] = sc;
-}
-
 // One block per (k block, row block, expert): 128 x 128 weights -> codes + one scale. Sixteen lanes read the
 // 256 bytes of a row together, so a load or store instruction touches whole sectors. Bound by HBM: 2 bytes in,
 // 1 byte out per weight.
@@ -166,26 +135,6 @@ uint32_t fp8_tile_rows(uint32_t routes, uint32_t experts)
     // tiles: even routing 16 routes per expert 0.136 against 0.152 ms, 44: 0.164 against 0.172, 64: 0.186 against
     // 0.177; skewed routing 19: 0.102 against 0.103, 38: 0.139 against 0.137, 64: 0.182 against 0.160.
     return routes <= 40u * experts ? 64u : static_cast<uint32_t>(kTileM);
-}
-
-bool fp8_gather_first(uint32_t routes, uint32_t experts)
-{
-    // A gather4 load takes the copy engine about 80 cycles, so full token tiles come faster in boxes of 32 rows, after a
-    // pass that gathers them. Layer times without and with the pass (128 experts top-8): even routing 8 routes per
-    // expert 0.129 and 0.129 ms, 32: 0.148 and 0.153; skewed routing 4: 0.072 and 0.069, 12: 0.095 and 0.087, 25: 0.132
-    // and 0.117; 128-row tiles, 64 routes: 0.197 and 0.180, 256 routes: 0.490 and 0.364.
-    return routes > 8u * experts;
-}
-
-cudaError_t launch_fp8_gather_rows(const uint8_t* codes, const float* scales, const int32_t* route_prows,
-                                   uint32_t routes, uint32_t top_k, uint32_t k, uint8_t* out_codes, float* out_scales,
-                                   cudaStream_t stream)
-{
-    if (routes == 0)
-        return cudaSuccess;
-    return launch_chained(fp8_gather_rows_kernel, dim3((routes + 7) / 8), 256, 0, stream,
-                          reinterpret_cast<const uint4*>(codes), reinterpret_cast<const uint32_t*>(scales), route_prows,
-                          routes, top_k, k, reinterpret_cast<uint4*>(out_codes), reinterpret_cast<uint32_t*>(out_scales));
 }
 
 cudaError_t launch_fp8_quantize_rows(const __nv_bfloat16* x, uint32_t rows, uint32_t k, uint8_t* codes, float* scales,

@@ -61,6 +61,9 @@ struct Fp8RowsParams {
     const int32_t* tile_row0;
     const int32_t* tile_nrows;
     const int32_t* total_tiles;
+    const int32_t* row_tokens; // NULL: scales by padded row; else dense row -> row of x_scale
+    const int32_t* indptr;     // with row_tokens: segment starts, dense and padded
+    const int32_t* pad_indptr;
     int tables_ready;      // the tables were complete before the predecessor in the stream started
     void* out;             // gated: e4m3 codes [rows, n]; plain: written through map_o
     float* out_scale;      // gated: f32 [rows, n / 128]
@@ -170,6 +173,13 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         for (uint32_t u = blockIdx.x; u < total; u += gridDim.x, next_note()) {
             const uint32_t tile = u / p.units_per_tile, nb = u % p.units_per_tile;
             const int row0 = p.tile_row0[tile], nrows = p.tile_nrows[tile], expert = p.tile_expert[tile];
+            int row[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                row[h] = row0 + min(static_cast<int>(i) + 64 * h, nrows - 1);
+                if (p.row_tokens != nullptr)
+                    row[h] = p.row_tokens[p.indptr[expert] + row[h] - p.pad_indptr[expert]];
+            }
             if (!waited)
                 chain_begin();
             waited = true;
@@ -178,7 +188,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
             FrNote& note = s_note[nt];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const float* xs = p.x_scale + static_cast<size_t>(row0 + min(static_cast<int>(i) + 64 * h, nrows - 1)) * p.k_blocks;
+                const float* xs = p.x_scale + static_cast<size_t>(row[h]) * p.k_blocks;
                 for (uint32_t kb = 0; kb < p.k_blocks; ++kb)
                     cp_async4(s_xs + (nt * p.k_blocks + kb) * 128 + i + 64 * h, xs + kb);
             }
@@ -462,12 +472,15 @@ cudaError_t launch_fp8_rows_gemm(const Fp8Gemm& g, cudaStream_t stream, const ch
     fp.tile_row0 = g.tile_row0;
     fp.tile_nrows = g.tile_nrows;
     fp.total_tiles = g.total_tiles;
+    fp.row_tokens = g.row_tokens;
+    fp.indptr = g.indptr;
+    fp.pad_indptr = g.pad_indptr;
     fp.tables_ready = g.tables_ready;
     fp.out = g.out;
     fp.out_scale = g.out_scale;
     fp.err = device_error_word();
     CUtensorMap mx, mw, mo;
-    bool ok = make_operand_map(&mx, true, g.x, g.k, g.x_rows, g.k, kFrBox)
+    bool ok = make_operand_map(&mx, true, g.row_tokens != nullptr ? g.gathered : g.x, g.k, g.out_rows, g.k, kFrBox)
         && make_operand_map(&mw, true, g.w, g.k, static_cast<uint64_t>(g.groups) * fp.b_rows, g.k, 128);
     mo = mx;
     if (ok && !g.gated)

@@ -61,6 +61,7 @@ struct Fp8StreamParams {
     const int32_t* row_tokens; // NULL: x rows are the padded rows; else dense row -> x row
     const int32_t* indptr;     // with row_tokens: segment starts, dense and padded
     const int32_t* pad_indptr;
+    int gathered;              // rows of experts with more than kGatherRows rows are in map_g, padded
     int tables_ready;        // the tables were complete before the predecessor in the stream started
     void* out;               // gated: e4m3 codes [rows, n]; else bf16 [rows, n]
     float* out_scale;        // gated: f32 [rows, n / 128]
@@ -69,7 +70,7 @@ struct Fp8StreamParams {
 
 // What the other warps need to know about a unit.
 struct FsNote {
-    int row0, nrows, w_row, w_row2;
+    int row0, nrows, w_row, w_row2, boxes; // boxes: the token rows lie together (in map_g)
     int row[NT];                 // x row of each row of the tile (the last one's past the end)
     float ws[2][kFsMaxKBlocks];  // block scales of the two weight tiles
 };
@@ -86,6 +87,7 @@ struct FsSmem {
 template <bool GATED>
 __global__ void __launch_bounds__(kFsThreads, 1)
 gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                       const __grid_constant__ CUtensorMap map_g, // boxes of padded rows
                        const Fp8StreamParams p)
 {
     using S = FsSmem;
@@ -162,7 +164,13 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             // (the last plain unit of an odd feature-block count takes its own tile twice and drops the second result)
             const uint32_t fb2 = GATED ? p.num_fb + nb : min(2 * nb + 1, p.num_fb - 1);
             const int j = min(static_cast<int>(i % NT), nrows - 1);
-            const int row = p.row_tokens != nullptr ? p.row_tokens[p.indptr[expert] + row0 - p.pad_indptr[expert] + j] : row0 + j;
+            int row = row0 + j;
+            bool boxes = true;
+            if (p.row_tokens != nullptr) {
+                const int dense = p.indptr[expert];
+                row = p.row_tokens[dense + row - p.pad_indptr[expert]];
+                boxes = p.gathered && p.indptr[expert + 1] - dense > static_cast<int>(kGatherRows);
+            }
             if (!waited)
                 chain_begin();
             waited = true;
@@ -180,6 +188,7 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             if (i == 0) {
                 note.row0 = row0;
                 note.nrows = nrows;
+                note.boxes = boxes;
                 note.w_row = expert * static_cast<int>(p.b_rows) + static_cast<int>(fb * 128);
                 note.w_row2 = expert * static_cast<int>(p.b_rows) + static_cast<int>(fb2 * 128);
             }
@@ -218,8 +227,8 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 break;
             const FsNote& note = s_note[nt];
             const int nrows = note.nrows, w_row = note.w_row, w_row2 = note.w_row2, row0 = note.row0;
-            const uint32_t parts = static_cast<uint32_t>(p.row_tokens != nullptr ? (nrows + 3) / 4 : (nrows + kFsBox - 1) / kFsBox);
-            const uint32_t part_bytes = p.row_tokens != nullptr ? 512u : kFsBox * 128u;
+            const bool boxes = note.boxes;
+            const uint32_t part_rows = boxes ? kFsBox : 4u, parts = (static_cast<uint32_t>(nrows) + part_rows - 1) / part_rows;
             int row[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q)
@@ -234,7 +243,7 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 uint8_t* sw = smem + s * S::kStageBytes;
                 const int c0 = static_cast<int>(kb) * 128;
                 if (lane == 0) {
-                    mbar_expect_tx(&full_bar[s], (kb < ahead ? 0 : 2 * kTileBytes) + parts * part_bytes);
+                    mbar_expect_tx(&full_bar[s], (kb < ahead ? 0 : 2 * kTileBytes) + parts * part_rows * 128);
                     if (kb >= ahead) {
                         tma_load_2d(sw, &map_w, &full_bar[s], c0, w_row);
                         tma_load_2d(sw + kTileBytes, &map_w, &full_bar[s], c0, w_row2);
@@ -242,11 +251,11 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 }
                 __syncwarp();
                 if (lane < parts) {
-                    uint8_t* dst = sw + 2 * kTileBytes + lane * part_bytes;
-                    if (p.row_tokens != nullptr)
-                        tma_gather4(dst, &map_x, &full_bar[s], c0, row);
+                    uint8_t* dst = sw + 2 * kTileBytes + lane * part_rows * 128;
+                    if (boxes)
+                        tma_load_2d(dst, &map_g, &full_bar[s], c0, row0 + static_cast<int>(lane * kFsBox));
                     else
-                        tma_load_2d(dst, &map_x, &full_bar[s], c0, row0 + static_cast<int>(lane * kFsBox));
+                        tma_gather4(dst, &map_x, &full_bar[s], c0, row);
                 }
                 if (++s == kFsStages) {
                     s = 0;
@@ -414,8 +423,8 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 }
 
 template <bool GATED>
-cudaError_t launch_stream_instance(const CUtensorMap& mw, const CUtensorMap& mx, const Fp8StreamParams& fp, uint32_t grid,
-                                   cudaStream_t stream)
+cudaError_t launch_stream_instance(const CUtensorMap& mw, const CUtensorMap& mx, const CUtensorMap& mg,
+                                   const Fp8StreamParams& fp, uint32_t grid, cudaStream_t stream)
 {
     auto kernel = gemm_fp8_stream_kernel<GATED>;
     constexpr size_t smem = 1024 + FsSmem::kBytes;
@@ -431,7 +440,7 @@ cudaError_t launch_stream_instance(const CUtensorMap& mw, const CUtensorMap& mx,
         if (dev >= 0 && dev < 64)
             configured[dev] = true;
     }
-    return launch_chained(kernel, dim3(grid), kFsThreads, smem, stream, mw, mx, fp);
+    return launch_chained(kernel, dim3(grid), kFsThreads, smem, stream, mw, mx, mg, fp);
 }
 
 } // namespace
@@ -453,20 +462,31 @@ cudaError_t launch_fp8_stream_gemm(const Fp8Gemm& g, cudaStream_t stream, const 
     fp.row_tokens = g.row_tokens;
     fp.indptr = g.indptr;
     fp.pad_indptr = g.pad_indptr;
+    fp.gathered = g.gathered != nullptr;
     fp.tables_ready = g.tables_ready;
     fp.out = g.out;
     fp.out_scale = g.out_scale;
     fp.err = device_error_word();
-    CUtensorMap mw, mx;
-    if (!make_operand_map(&mw, true, g.w, g.k, static_cast<uint64_t>(g.groups) * fp.b_rows, g.k, 128)
-        || !make_operand_map(&mx, true, g.x, g.k, g.x_rows, g.k, g.row_tokens != nullptr ? 1u : kFsBox)) {
+    CUtensorMap mw, mx, mg;
+    bool ok = make_operand_map(&mw, true, g.w, g.k, static_cast<uint64_t>(g.groups) * fp.b_rows, g.k, 128);
+    if (g.row_tokens == nullptr) {
+        ok = ok && make_operand_map(&mg, true, g.x, g.k, g.x_rows, g.k, kFsBox);
+        mx = mg;
+    } else {
+        ok = ok && make_operand_map(&mx, true, g.x, g.k, g.x_rows, g.k, 1);
+        mg = mx;
+        if (g.gathered != nullptr)
+            ok = ok && make_operand_map(&mg, true, g.gathered, g.k, g.out_rows, g.k, kFsBox);
+    }
+    if (!ok) {
         if (why != nullptr)
             *why = "cuTensorMapEncodeTiled failed";
         return cudaErrorInvalidValue;
     }
     const uint32_t grid = static_cast<uint32_t>(
         std::min<uint64_t>(static_cast<uint64_t>(g.max_tiles) * fp.units_per_tile, device_sm_count()));
-    return g.gated ? launch_stream_instance<true>(mw, mx, fp, grid, stream) : launch_stream_instance<false>(mw, mx, fp, grid, stream);
+    return g.gated ? launch_stream_instance<true>(mw, mx, mg, fp, grid, stream)
+                   : launch_stream_instance<false>(mw, mx, mg, fp, grid, stream);
 }
 
 } // namespace qs3

@@ -70,6 +70,7 @@ bool upstream_bf16_workspace_bytes(const qsfi_moe_plan_desc& d, uint32_t num_tok
 
 struct Bf16Workspace {
     RouteTables rt;
+    __nv_bfloat16* expanded; // [pad_rows, H]: token rows gathered by expert, for large batches
     __nv_bfloat16* act;      // [pad_rows, I]
     __nv_bfloat16* y2;       // [pad_rows, H]
     size_t bytes;
@@ -82,6 +83,8 @@ Bf16Workspace carve_bf16(char* base, const qsfi_moe_plan_desc& d, uint32_t num_t
     size_t off = route_tables_carve(base, routes, d.local_num_experts, &w.rt,
                                     bf16_tile_rows(routes, d.local_num_experts));
     const size_t rows = w.rt.max_pad_rows;
+    if (gather_rows_pays(num_tokens, d.top_k, d.local_num_experts))
+        w.expanded = carve<__nv_bfloat16>(base, off, rows * d.hidden_size);
     w.act = carve<__nv_bfloat16>(base, off, rows * d.intermediate_size);
     w.y2 = carve<__nv_bfloat16>(base, off, rows * d.hidden_size);
     w.bytes = align_up(off, kWorkspaceAlign);
@@ -135,8 +138,7 @@ bool is_fp8_plan(const qsfi_moe_plan_desc& d)
 
 struct Fp8Workspace {
     RouteTables rt;    // token tiles of fp8_tile_rows rows
-    uint8_t* xq;       // [pad_rows, H] e4m3, if the token rows are gathered by expert
-    float* xq_s;       // [pad_rows, H/128]
+    uint8_t* xq;       // [pad_rows, H] e4m3: token rows gathered by expert, for large batches
     uint8_t* act;      // [pad_rows, I] e4m3
     float* act_s;      // [pad_rows, I/128]
     __nv_bfloat16* y2; // [pad_rows, H]
@@ -151,10 +153,8 @@ Fp8Workspace carve_fp8(char* base, const qsfi_moe_plan_desc& d, uint32_t num_tok
                                     fp8_tile_rows(routes, d.local_num_experts));
     const size_t rows = w.rt.max_pad_rows;
     const size_t h = d.hidden_size, i = d.intermediate_size;
-    if (fp8_gather_first(routes, d.local_num_experts)) {
+    if (w.rt.tile_rows == kTileM || gather_rows_pays(num_tokens, d.top_k, d.local_num_experts))
         w.xq = carve<uint8_t>(base, off, rows * h);
-        w.xq_s = carve<float>(base, off, rows * (h / 128));
-    }
     w.act = carve<uint8_t>(base, off, rows * i);
     w.act_s = carve<float>(base, off, rows * (i / 128));
     w.y2 = carve<__nv_bfloat16>(base, off, rows * h);
@@ -370,9 +370,16 @@ qsfi_status run_routed_bf16(qsfi_context* ctx, const qsfi_moe_plan_desc& p, cons
                             const __nv_bfloat16* hidden, uint32_t num_tokens,
                             const __nv_bfloat16* gate_up, const __nv_bfloat16* down)
 {
+    if (w.expanded != nullptr) {
+        const cudaError_t err = launch_gather_rows(hidden, p.hidden_size * 2, w.rt, kGatherRows, w.expanded, ctx->stream);
+        if (err != cudaSuccess)
+            return set_cuda_error(ctx, err, "MoE gather");
+    }
     stage_mark(ctx->stream, STAGE_GATE_UP_GEMM);
     GemmProblem g1 = grouped_problem(w.rt, p.local_num_experts);
-    g1.a = hidden; // token rows are read in place, through the routing tables
+    g1.gathered = w.expanded;
+    g1.tables_ready = w.expanded != nullptr; // the predecessor is the gather
+    g1.a = hidden; // token rows of experts with few of them are read in place, through the routing tables
     g1.a_rows = num_tokens;
     g1.row_tokens = w.rt.row_tokens;
     g1.indptr = w.rt.indptr;
@@ -391,6 +398,7 @@ qsfi_status run_routed_bf16(qsfi_context* ctx, const qsfi_moe_plan_desc& p, cons
         return status;
     stage_mark(ctx->stream, STAGE_DOWN_GEMM);
     GemmProblem g2 = grouped_problem(w.rt, p.local_num_experts);
+    g2.tables_ready = 1;
     g2.a = w.act;
     g2.a_pitch_bytes = static_cast<uint64_t>(p.intermediate_size) * 2;
     g2.b = down;
@@ -502,7 +510,8 @@ qsfi_status run_routed_nvfp4(qsfi_context* ctx, const qsfi_moe_plan_desc& p, con
     return gemm_or_error(ctx, g2, "NVFP4 MoE down GEMM");
 }
 
-// Routed experts on FP8 operands: activation rows gathered in w.xq / w.xq_s or (w.xq NULL) in token order.
+// Routed experts on FP8 operands, tokens quantised in token order (`tables_ready`: the routing tables were complete
+// before the predecessor in the stream started).
 qsfi_status run_routed_fp8(qsfi_context* ctx, const qsfi_moe_plan_desc& p, const Fp8Workspace& w,
                            uint32_t num_tokens, const uint8_t* tokens, const float* token_s, bool tables_ready, const uint8_t* gu, const float* gu_scale, const uint8_t* down,
                            const float* down_scale)
@@ -526,20 +535,22 @@ qsfi_status run_routed_fp8(qsfi_context* ctx, const qsfi_moe_plan_desc& p, const
     g.total_tiles = w.rt.total_tiles;
     g.max_tiles = w.rt.max_tiles;
     g.tile_rows = w.rt.tile_rows;
+    if (w.xq != nullptr) {
+        const cudaError_t err = launch_gather_rows(tokens, p.hidden_size, w.rt, w.rt.tile_rows == kTileM ? 0 : kGatherRows,
+                                                   w.xq, ctx->stream);
+        if (err != cudaSuccess)
+            return set_cuda_error(ctx, err, "FP8 MoE gather");
+    }
     stage_mark(ctx->stream, STAGE_GATE_UP_GEMM);
     Fp8Gemm g1 = g;
-    g1.tables_ready = tables_ready;
-    if (w.xq != nullptr) {
-        g1.x = w.xq;
-        g1.x_scale = w.xq_s;
-    } else {
-        g1.x = tokens;
-        g1.x_scale = token_s;
-        g1.x_rows = num_tokens;
-        g1.row_tokens = w.rt.row_tokens;
-        g1.indptr = w.rt.indptr;
-        g1.pad_indptr = w.rt.pad_indptr;
-    }
+    g1.tables_ready = tables_ready || w.xq != nullptr;
+    g1.x = tokens;
+    g1.x_scale = token_s;
+    g1.x_rows = num_tokens;
+    g1.row_tokens = w.rt.row_tokens;
+    g1.indptr = w.rt.indptr;
+    g1.pad_indptr = w.rt.pad_indptr;
+    g1.gathered = w.xq;
     g1.w = gu;
     g1.w_scale = gu_scale;
     g1.n = p.intermediate_size;
@@ -1284,13 +1295,11 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
 
     const __nv_bfloat16* y2 = nullptr;
     if (fp8) {
-        // 4. quantise every token once, and for larger batches gather the codes by expert; 5./6. grouped GEMMs
+        // 4. quantise every token once (token order); 5./6. grouped GEMMs
         stage_mark(st, STAGE_GATHER);
         err = launch_fp8_quantize_rows(hidden, d->num_tokens, p.hidden_size, x.f8_x, x.f8_s, st);
-        if (err == cudaSuccess && wf.xq != nullptr)
-            err = launch_fp8_gather_rows(x.f8_x, x.f8_s, rt.route_prows, routes, p.top_k, p.hidden_size, wf.xq, wf.xq_s, st);
         if (err != cudaSuccess)
-            return set_cuda_error(ctx, err, "FP8 MoE gather");
+            return set_cuda_error(ctx, err, "FP8 token quantiser");
         status = run_routed_fp8(ctx, p, wf, d->num_tokens, x.f8_x, x.f8_s, true, static_cast<const uint8_t*>(d->gate_up_weight.data),
                                 static_cast<const float*>(d->gate_up_scale_tiled.data),
                                 static_cast<const uint8_t*>(d->down_weight.data),
@@ -2082,12 +2091,9 @@ qsfi_status qs3_moe_execute_fp8(qsfi_context* ctx, const qsfi_moe_plan* plan, co
                                         p.local_expert_offset, p.local_num_experts, w.rt, st);
     const uint8_t* hq = static_cast<const uint8_t*>(desc->hidden.data);
     const float* hs = static_cast<const float*>(desc->hidden_scale.data);
-    // larger batches: the quantised token rows (codes and their scales) gathered into expert order
-    if (err == cudaSuccess && w.xq != nullptr)
-        err = launch_fp8_gather_rows(hq, hs, w.rt.route_prows, routes, p.top_k, p.hidden_size, w.xq, w.xq_s, st);
     if (err != cudaSuccess)
         return set_cuda_error(ctx, err, "FP8 MoE routing");
-    status = run_routed_fp8(ctx, p, w, desc->num_tokens, hq, hs, w.xq != nullptr, static_cast<const uint8_t*>(desc->gate_up_weight.data),
+    status = run_routed_fp8(ctx, p, w, desc->num_tokens, hq, hs, false, static_cast<const uint8_t*>(desc->gate_up_weight.data),
                             static_cast<const float*>(desc->gate_up_weight_scale.data),
                             static_cast<const uint8_t*>(desc->down_weight.data),
                             static_cast<const float*>(desc->down_weight_scale.data));

@@ -112,9 +112,9 @@ def test_execute_fp8_is_deterministic_and_linear_in_routing_weight(ops, ctx, ora
 
 
 # one expert of `rows` rows beside emptier ones: edges of the 16-column MMA step, of the warps' 32-token halves and of the
-# tile; rows found through the tables (e = 16) and gathered (e = 2); odd numbers of feature blocks; scales of one and of
-# two units at a time (h = 4096)
-@pytest.mark.parametrize("rows", [1, 16, 17, 32, 33, 64, 65])
+# tile; rows found through the tables and (e = 2, more than 48 rows) gathered; odd numbers of feature blocks; scales of
+# one and of two units at a time (h = 4096)
+@pytest.mark.parametrize("rows", [1, 16, 17, 32, 33, 48, 49, 64, 65])
 @pytest.mark.parametrize("h,i,e", [(384, 384, 16), (640, 128, 2), (4096, 256, 16)])
 def test_fp8_rows_per_expert(ops, ctx, oracle, rows, h, i, e):
     t = rows + 5

@@ -77,6 +77,17 @@ def test_matches_oracle(ops, oracle, cfg):
         assert np.array_equal(g, r)
 
 
+# one expert of `rows` rows beside emptier ones: read in place up to 48 rows, gathered beyond; 32-, 64- and 128-row tiles
+@pytest.mark.parametrize("rows,e", [(31, 16), (33, 2), (48, 2), (49, 2), (64, 2), (65, 6), (129, 2), (200, 2)])
+def test_rows_per_expert(ops, oracle, rows, e):
+    t, h, i = rows + 9, 328, 200
+    d = make_moe_inputs(5 + rows, t, h, e, i)
+    ids = np.where(np.arange(t) < rows, 0, 1 + np.arange(t) % (e - 1)).astype(np.int32).reshape(t, 1)
+    w = np.linspace(0.5, 1.5, t, dtype=np.float32).reshape(t, 1)
+    out, _, _ = _execute(ops, d["hidden"], ids, w, d["gate_up"], d["down"], e)
+    _check(out, oracle.moe_bf16(d["hidden"], ids, w, d["gate_up"], d["down"]))
+
+
 def test_expert_parallel_partials_sum_to_the_full_result(ops, oracle):
     t, h, e, k, i = 48, 256, 8, 2, 128
     d = make_moe_inputs(2, t, h, e, i)
