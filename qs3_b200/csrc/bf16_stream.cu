@@ -109,7 +109,9 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const bool early = p.tables_ready && warp == 4; // weights and tables are complete: their loads need not wait
+    // weights and tables are complete: a decode batch's loads need not wait (with skewed ends of a longer predecessor the
+    // CTAs would no longer read neighbouring rows together: down of 2048 tokens 0.177 -> 0.19 ms)
+    const bool early = NT == 32 && p.tables_ready && warp == 4;
     if (!early)
         chain_begin();
 
@@ -126,12 +128,13 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         uint32_t s = 0, ph = 0;
         bool ok = true;
         for (uint32_t i = 0; i < my_units && ok; ++i) {
-            const uint32_t u = blockIdx.x + i * gridDim.x, tile = u / p.units_per_tile, nb = u % p.units_per_tile;
+            const uint32_t u = blockIdx.x + i * gridDim.x, tile = u / p.units_per_tile;
+            const uint32_t f0 = u % p.units_per_tile * (GATED ? 1 : 2) * p.half;
             const int row0 = grouped ? p.tile_row0[tile] : static_cast<int>(tile * NT);
             const int nrows = grouped ? p.tile_nrows[tile] : static_cast<int>(min(static_cast<uint32_t>(NT), p.dense_rows - row0));
             const int expert = grouped ? p.tile_expert[tile] : 0;
             // rows of a tile past the last feature belong to something else and are dropped by the epilogue
-            const int w_row = expert * static_cast<int>(p.b_rows) + static_cast<int>(nb * (GATED ? 1 : 2) * p.half);
+            const int w_row = expert * static_cast<int>(p.b_rows) + static_cast<int>(f0);
             const int w_row2 = w_row + static_cast<int>(GATED ? p.n : p.half);
             uint32_t ahead = 0; // k blocks whose weights are on their way already
             if (i == 0 && early) {
@@ -146,9 +149,13 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                 __syncwarp();
                 chain_begin();
             }
-            bool boxes = true;
-            int row[4] = {};
-            if (p.row_tokens != nullptr) {
+            bool boxes = nrows > static_cast<int>(kGatherRows);
+            int row[4];
+            if (p.row_tokens == nullptr) { // (four rows of a small tile at a time, which moves no padding)
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    row[q] = row0 + min(static_cast<int>(lane) * 4 + q, nrows - 1);
+            } else {
                 const int dense = p.indptr[expert], dense0 = dense + row0 - p.pad_indptr[expert];
                 boxes = p.gathered && p.indptr[expert + 1] - dense > static_cast<int>(kGatherRows);
 #pragma unroll
@@ -228,12 +235,13 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         // ------------------------------------------------------------ epilogue --
         const uint32_t lane_base = (warp * 32) << 16;
         for (uint32_t i = 0; i < my_units; ++i) {
-            const uint32_t u = blockIdx.x + i * gridDim.x, tile = u / p.units_per_tile, nb = u % p.units_per_tile;
+            const uint32_t u = blockIdx.x + i * gridDim.x, tile = u / p.units_per_tile;
+            const uint32_t f0 = u % p.units_per_tile * (GATED ? 1 : 2) * p.half;
             const uint32_t buf = i & 1;
             const uint32_t row0 = grouped ? static_cast<uint32_t>(p.tile_row0[tile]) : tile * NT;
             const uint32_t nrows = grouped ? static_cast<uint32_t>(p.tile_nrows[tile]) : min(static_cast<uint32_t>(NT), p.dense_rows - row0);
             const uint32_t r = warp * 32 + lane; // weight row of each tile; rows past `half` hold nothing
-            const uint32_t f = nb * (GATED ? 1 : 2) * p.half + r; // plain: and f + half
+            const uint32_t f = f0 + r;           // plain: and f + half
             const bool live = r < p.half && f < p.n, live2 = r < p.half && f + p.half < p.n;
             const bool ready = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], (i >> 1) & 1, abort_flag, p.err,
                                                                  ERR_BS_ACC_FULL_WAIT));
@@ -366,16 +374,12 @@ cudaError_t launch_bf16_stream_gemm(const GemmProblem& g, cudaStream_t stream, c
     sp.err = device_error_word();
     const uint32_t nt = g.tile_expert != nullptr ? g.tile_rows : g.a_rows <= 32 ? 32u : g.a_rows <= 64 ? 64u : 128u;
     CUtensorMap mw, mx, mg;
-    bool ok = make_operand_map(&mw, false, g.b, g.k, static_cast<uint64_t>(g.groups) * sp.b_rows, g.b_pitch_bytes, sp.half);
-    if (g.row_tokens == nullptr) {
-        ok = ok && make_operand_map(&mg, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, kBsBox);
-        mx = mg;
-    } else {
-        ok = ok && make_operand_map(&mx, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, 1);
-        mg = mx;
-        if (g.gathered != nullptr) // (as many rows as the tables have room for)
-            ok = ok && make_operand_map(&mg, false, g.gathered, g.k, static_cast<uint64_t>(g.max_tiles) * g.tile_rows, g.k * 2ull, kBsBox);
-    }
+    const uint64_t w_rows = static_cast<uint64_t>(g.groups) * sp.b_rows;
+    const bool copy = g.row_tokens != nullptr && g.gathered != nullptr; // (as many rows as the tables have room for)
+    const bool ok = make_operand_map(&mw, false, g.b, g.k, w_rows, g.b_pitch_bytes, sp.half)
+        && make_operand_map(&mx, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, 1)
+        && make_operand_map(&mg, false, copy ? g.gathered : g.a, g.k, copy ? static_cast<uint64_t>(g.max_tiles) * g.tile_rows : g.a_rows,
+                            copy ? g.k * 2ull : g.a_pitch_bytes, kBsBox);
     if (!ok) {
         if (why != nullptr)
             *why = "cuTensorMapEncodeTiled failed";

@@ -456,31 +456,37 @@ route_sort_block_kernel(const int32_t* __restrict__ ids, const float* __restrict
     block_sort(s, weights, routes, top_k, experts, rt); // (starts with a barrier)
 }
 
-// dst[padded row] = src[token] for the tiles of experts with more than `min_rows` rows; a warp per row, four 16-byte
-// vectors per lane in flight. Bound by HBM and L2: rows * row bytes, read and written.
+// dst[padded row] = src[token] for the tiles of experts with more than `min_rows` rows; a block per 32 rows of a tile, a
+// warp per row, four 16-byte vectors per lane in flight. Bound by HBM and L2: rows * row bytes, read and written; where
+// few experts are heavy, by the blocks that find nothing to do (8 rows per block: 2048 tokens, 512 experts 0.008 ms).
+constexpr uint32_t kGatherBlockRows = 32;
+
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const uint4* __restrict__ src, uint32_t vec_per_row, RouteTables rt, int min_rows, uint4* __restrict__ dst)
 {
     chain_begin();
     const uint32_t tile = blockIdx.y, lane = threadIdx.x & 31;
-    const int j = static_cast<int>(blockIdx.x * 8 + (threadIdx.x >> 5));
-    if (static_cast<int>(tile) >= *rt.total_tiles || j >= rt.tile_nrows[tile])
+    if (static_cast<int>(tile) >= *rt.total_tiles)
         return;
-    const int expert = rt.tile_expert[tile], row = rt.tile_row0[tile] + j, dense0 = rt.indptr[expert];
+    const int expert = rt.tile_expert[tile], row0 = rt.tile_row0[tile], nrows = rt.tile_nrows[tile], dense0 = rt.indptr[expert];
     if (rt.indptr[expert + 1] - dense0 <= min_rows)
         return;
-    const uint4* s = src + static_cast<size_t>(rt.row_tokens[dense0 + row - rt.pad_indptr[expert]]) * vec_per_row;
-    uint4* d = dst + static_cast<size_t>(row) * vec_per_row;
-    for (uint32_t i0 = lane; i0 < vec_per_row; i0 += 128) {
-        uint4 v[4];
+    const int32_t* tokens = rt.row_tokens + dense0 + row0 - rt.pad_indptr[expert];
+    const int end = min(nrows, static_cast<int>((blockIdx.x + 1) * kGatherBlockRows));
+    for (int j = static_cast<int>(blockIdx.x * kGatherBlockRows + (threadIdx.x >> 5)); j < end; j += 8) {
+        const uint4* s = src + static_cast<size_t>(tokens[j]) * vec_per_row;
+        uint4* d = dst + static_cast<size_t>(row0 + j) * vec_per_row;
+        for (uint32_t i0 = lane; i0 < vec_per_row; i0 += 128) {
+            uint4 v[4];
 #pragma unroll
-        for (uint32_t q = 0; q < 4; ++q)
-            if (i0 + 32 * q < vec_per_row)
-                v[q] = s[i0 + 32 * q];
+            for (uint32_t q = 0; q < 4; ++q)
+                if (i0 + 32 * q < vec_per_row)
+                    v[q] = s[i0 + 32 * q];
 #pragma unroll
-        for (uint32_t q = 0; q < 4; ++q)
-            if (i0 + 32 * q < vec_per_row)
-                d[i0 + 32 * q] = v[q];
+            for (uint32_t q = 0; q < 4; ++q)
+                if (i0 + 32 * q < vec_per_row)
+                    d[i0 + 32 * q] = v[q];
+        }
     }
 }
 
@@ -1244,7 +1250,7 @@ cudaError_t launch_gather_rows(const void* src, uint32_t row_bytes, const RouteT
 {
     if (rt.max_tiles == 0)
         return cudaSuccess;
-    return launch_chained(gather_rows_kernel, dim3((rt.tile_rows + 7) / 8, rt.max_tiles), 256, 0, stream,
+    return launch_chained(gather_rows_kernel, dim3((rt.tile_rows + kGatherBlockRows - 1) / kGatherBlockRows, rt.max_tiles), 256, 0, stream,
                           static_cast<const uint4*>(src), row_bytes / 16, rt, static_cast<int>(min_rows),
                           static_cast<uint4*>(dst));
 }
