@@ -97,6 +97,11 @@ struct RouteTables {
     int32_t* tile_row0;    // [max_tiles] first padded row of the tile
     int32_t* tile_nrows;   // [max_tiles] valid rows in the tile
     int32_t* total_tiles;  // [1]
+    // Tables for either of two tile heights, chosen by the sort from the routes of each expert (NULL: `tile_rows` only):
+    // *alt_total_tiles counts the tiles if they have alt_tile_rows rows, *total_tiles if they have tile_rows, and the other
+    // one is 0, so that of two kernels launched one after the other one does the work.
+    int32_t* alt_total_tiles; // [1]
+    uint32_t alt_tile_rows, alt_max_tiles;
     // 256-row "pair tiles" for the CTA-pair GEMM (128-row plans only, NULL otherwise): an expert with t
     // row tiles gives t / 2 full pairs, listed from index 0 upwards, and t % 2 single (<= 128 rows),
     // listed from index max_tiles - 1 downwards; pair_counts = {full pairs, singles}
@@ -117,7 +122,7 @@ struct RouteTables {
 size_t route_tables_bytes(uint32_t routes, uint32_t experts);
 // Carves the tables out of `base` (may be NULL for sizing); returns bytes used.
 size_t route_tables_carve(char* base, uint32_t routes, uint32_t experts, RouteTables* out,
-                          uint32_t tile_rows = kTileM, uint32_t shared_rows = 0);
+                          uint32_t tile_rows = kTileM, uint32_t shared_rows = 0, uint32_t alt_tile_rows = 0);
 // Tokens to quantise (NVFP4) beside the sort.
 struct TokenQuant {
     const __nv_bfloat16* x; // [rows, k]
@@ -295,6 +300,10 @@ cudaError_t launch_nvfp4_pair_gemm(const GemmProblem& p, cudaStream_t stream, co
 cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);
 // Rows per token tile of an NVFP4 plan: 32 or 64 (decode kernel) when experts get few rows each, else 128.
 uint32_t nvfp4_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter);
+// Smaller tile height between which and 128 rows the sort shall choose, 0: none.
+uint32_t nvfp4_alt_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter);
+// Whether a sort of this size can choose between tile heights.
+bool route_sort_can_choose(uint32_t routes, uint32_t experts);
 bool gemm_tc_supported(const GemmProblem& p);
 // bf16 grouped GEMM of the routed experts, weights streamed as the M side (bf16_stream.cu), and the rows per token
 // tile of a bf16 plan.
@@ -365,6 +374,14 @@ __device__ __forceinline__ void chain_begin()
     chain_release();
 }
 
+// Work beside the main chain is launched unchained: a kernel that waits for its predecessor while it holds the shared
+// memory and registers of its SMs keeps the small kernels of the other stream out.
+extern thread_local bool launch_unchained;
+struct UnchainedScope {
+    UnchainedScope() { launch_unchained = true; }
+    ~UnchainedScope() { launch_unchained = false; }
+};
+
 template <typename... KArgs, typename... Args>
 cudaError_t launch_chained_cluster(void (*kernel)(KArgs...), uint32_t cluster, dim3 grid, uint32_t block, size_t smem,
                                    cudaStream_t stream, Args&&... args)
@@ -372,7 +389,7 @@ cudaError_t launch_chained_cluster(void (*kernel)(KArgs...), uint32_t cluster, d
     cudaLaunchConfig_t cfg {};
     cudaLaunchAttribute attr[2] = {};
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].val.programmaticStreamSerializationAllowed = launch_unchained ? 0 : 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim = { cluster, 1, 1 };
     cfg.gridDim = grid;

@@ -9,6 +9,9 @@
 
 namespace qs3 {
 
+thread_local bool launch_unchained = false;
+
+
 void clear_error(qsfi_error_info* err)
 {
     if (err == nullptr)

@@ -249,7 +249,7 @@ uint32_t splitk_choice(const GemmProblem& g)
     const uint32_t nt = splitk_tile_rows(g.a_rows);
     if (2 * splitk_tiles(g, nt) <= device_sm_count())
         return nt;
-    return nt == 64 && g.k >= 3072 && 2 * splitk_tiles(g, 128) <= device_sm_count() ? 128u : 0u;
+    return nt == 64 && g.k >= 2048 && 2 * splitk_tiles(g, 128) <= device_sm_count() ? 128u : 0u;
 }
 
 } // namespace

@@ -113,7 +113,8 @@ Nvfp4Workspace carve_nvfp4(char* base, const qsfi_moe_plan_desc& d, uint32_t num
     const uint32_t tile_rows = nvfp4_tile_rows(routes, d.local_num_experts, d.hidden_size, d.intermediate_size);
     // (64-row tiles of all tokens at the end of the CTAs' ranges made a long last round: 1021 tokens 0.283 against 0.232 ms)
     const bool merge = shared_inter == d.intermediate_size && tile_rows == 32;
-    size_t off = route_tables_carve(base, routes, d.local_num_experts, &w.rt, tile_rows, merge ? num_tokens : 0);
+    size_t off = route_tables_carve(base, routes, d.local_num_experts, &w.rt, tile_rows, merge ? num_tokens : 0,
+                                    nvfp4_alt_tile_rows(routes, d.local_num_experts, d.hidden_size, d.intermediate_size));
     const size_t rows = w.rt.max_pad_rows;
     const size_t h = d.hidden_size, i = d.intermediate_size, e = d.local_num_experts;
     if (w.rt.tile_rows == static_cast<uint32_t>(kTileM)) { // smaller tiles read the token rows in place
@@ -447,25 +448,35 @@ qsfi_status run_routed_nvfp4(qsfi_context* ctx, const qsfi_moe_plan_desc& p, con
     const float ga = act_global == 0.0f ? 1.0f : act_global;
     const float ga2 = act2_global == 0.0f ? 1.0f : act2_global;
     const bool in_place = w.rt.tile_rows != static_cast<uint32_t>(kTileM);
+    const bool either = w.rt.alt_total_tiles != nullptr; // the sort chose: of two kernels per GEMM one finds tiles
     if (!in_place) {
         const cudaError_t err = launch_nvfp4_gather_tiles(tokens, token_sf, w.rt, p.hidden_size, w.xq, w.xq_sf,
                                                           ctx->stream, sf_linear ? 0 : 1);
         if (err != cudaSuccess)
             return set_cuda_error(ctx, err, "NVFP4 MoE gather");
     }
+    const auto read_in_place = [&](GemmProblem& g) {
+        g.a = tokens;
+        g.a_scale_tiled = token_sf;
+        g.a_rows = num_tokens;
+        g.row_tokens = w.rt.row_tokens;
+        g.indptr = w.rt.indptr;
+        g.pad_indptr = w.rt.pad_indptr;
+        g.a_scale_linear = sf_linear;
+    };
+    const auto small_tiles = [&](GemmProblem& g) {
+        g.tile_rows = w.rt.alt_tile_rows;
+        g.total_tiles = w.rt.alt_total_tiles;
+        g.max_tiles = w.rt.alt_max_tiles;
+    };
     stage_mark(ctx->stream, STAGE_GATE_UP_GEMM);
     GemmProblem g1 = grouped_problem(w.rt, p.local_num_experts);
     g1.nvfp4 = 1;
-    g1.a = in_place ? tokens : w.xq;
+    g1.a = w.xq;
     g1.a_pitch_bytes = p.hidden_size / 2;
-    g1.a_scale_tiled = in_place ? token_sf : w.xq_sf;
-    if (in_place) {
-        g1.a_rows = num_tokens;
-        g1.row_tokens = w.rt.row_tokens;
-        g1.indptr = w.rt.indptr;
-        g1.pad_indptr = w.rt.pad_indptr;
-        g1.a_scale_linear = sf_linear;
-    }
+    g1.a_scale_tiled = w.xq_sf;
+    if (in_place)
+        read_in_place(g1);
     g1.b = wt.gu_packed;
     g1.b_pitch_bytes = p.hidden_size / 2;
     g1.b_scale_tiled = wt.gu_sf_tiled;
@@ -485,6 +496,11 @@ qsfi_status run_routed_nvfp4(qsfi_context* ctx, const qsfi_moe_plan_desc& p, con
     g1.shared_scale_up = wt.sh_gu_global_up;
     g1.out_global_scale = ga2;
     qsfi_status status = gemm_or_error(ctx, g1, "NVFP4 MoE gate_up GEMM");
+    if (status == QSFI_STATUS_OK && either) {
+        small_tiles(g1);
+        read_in_place(g1);
+        status = gemm_or_error(ctx, g1, "NVFP4 MoE gate_up GEMM");
+    }
     if (status != QSFI_STATUS_OK)
         return status;
     stage_mark(ctx->stream, STAGE_DOWN_GEMM);
@@ -507,6 +523,13 @@ qsfi_status run_routed_nvfp4(qsfi_context* ctx, const qsfi_moe_plan_desc& p, con
     g2.shared_b = wt.sh_d_packed;
     g2.shared_b_scale_tiled = wt.sh_d_sf_tiled;
     g2.shared_scale = wt.sh_d_global;
+    if (either) {
+        GemmProblem g3 = g2;
+        small_tiles(g3);
+        status = gemm_or_error(ctx, g3, "NVFP4 MoE down GEMM");
+        if (status != QSFI_STATUS_OK)
+            return status;
+    }
     return gemm_or_error(ctx, g2, "NVFP4 MoE down GEMM");
 }
 
@@ -1247,7 +1270,10 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
             ferr = cudaEventRecord(plan->ev_quant, side);
         if (ferr != cudaSuccess)
             return set_cuda_error(ctx, ferr, "NVFP4 MoE layer fork");
-        status = run_shared_nvfp4(side);
+        {
+            UnchainedScope alone;
+            status = run_shared_nvfp4(side);
+        }
         if (status != QSFI_STATUS_OK)
             return status;
         ferr = cudaEventRecord(plan->ev_shared, side);

@@ -533,11 +533,18 @@ uint32_t nvfp4_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uin
         && inter / 256 <= kSwMaxKBlocks;
     if (!fits)
         return static_cast<uint32_t>(kTileM);
-    // 32-row tiles while nearly every expert fits one; 64-row tiles up to where 128-row tiles of CTA pairs win. The
-    // second line depends on the skew, which the host does not know: with even routing (512 experts top-10) 64-row
-    // tiles win up to ~70 routes per expert (2200 tokens: 0.284 against 0.361 ms), with a Zipf-skewed router only up
-    // to ~22 (1021 tokens: 0.180 against 0.188 ms, 2048: 0.247 against 0.216), so the line lies where neither loses.
+    // 32-row tiles while nearly every expert fits one, 64-row tiles while they win whatever the skew (512 experts top-10:
+    // 1021 tokens of a skewed router 0.180 against 0.188 ms with 128-row tiles of CTA pairs, even routing 0.23 against 0.35)
     return routes <= 8 * experts ? 32u : routes <= 22 * experts ? 64u : static_cast<uint32_t>(kTileM);
+}
+
+uint32_t nvfp4_alt_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter)
+{
+    // Beyond that it depends on the skew, which only the sort sees; from 80 routes per expert on 64-row tiles never win.
+    return nvfp4_tile_rows(22 * experts, experts, hidden, inter) == 64 && routes > 22 * experts && routes <= 80 * experts
+            && route_sort_can_choose(routes, experts)
+        ? 64u
+        : 0u;
 }
 
 cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& g, cudaStream_t stream, const char** why)
