@@ -302,3 +302,25 @@ def test_64_row_token_tiles(ops, ctx, oracle, cfg):
     torch.cuda.synchronize()
     assert ctx.read_device_error() == 0
     _check(to_np(out), oracle.moe_nvfp4(hp, hs, ids, w, gu_ref, dn_ref, local_offset=off))
+
+
+@pytest.mark.parametrize("hot", [0.0, 1.0, 6.0])
+@pytest.mark.parametrize("t", [641, 700, 1280])
+def test_tile_height_chosen_by_the_sort(ops, ctx, oracle, t, hot):
+    """44 to 80 rows per expert: with even routing the sort lays out 64-row tiles, with a few hot experts 128-row ones."""
+    h, e, k, i = 256, 64, 4, 256
+    d = make_moe_inputs(47, t, h, e, i)
+    bias = np.where(np.arange(e) < 6, hot, 0.0).astype(np.float32)
+    gu, dn, _ = _quantise_all(ops, ctx, d, False)
+    plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=t, hidden_size=h, intermediate_size=i, num_experts=e, top_k=k,
+                                              backend=ops.capi.MOE_BACKEND_NVFP4))
+    out = torch.empty((t, h), dtype=torch.bfloat16, device="cuda")
+    ws = torch.zeros(plan.layer_workspace_size(t, 0), dtype=torch.uint8, device="cuda")
+    ids = torch.empty((t, k), dtype=torch.int32, device="cuda")
+    w = torch.empty((t, k), dtype=torch.float32, device="cuda")
+    ops.moe_layer_execute(plan, to_dev(d["hidden"]), to_dev(d["router"]), gu, dn, out, ws, router_bias=to_dev(bias),
+                          topk_ids=ids, topk_weights=w)
+    torch.cuda.synchronize()
+    assert ctx.read_device_error() == 0
+    hp, hs = oracle.nvfp4_quantize_act(d["hidden"], 1.0)
+    _check(to_np(out), oracle.moe_nvfp4(hp, hs, to_np(ids), to_np(w), _triple(gu), _triple(dn)))
