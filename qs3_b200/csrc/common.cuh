@@ -135,6 +135,12 @@ struct TokenQuant {
 cudaError_t launch_route_sort(const int32_t* topk_ids, const float* topk_weights, uint32_t routes,
                               uint32_t top_k, uint32_t local_offset, uint32_t experts,
                               const RouteTables& rt, cudaStream_t stream, const TokenQuant* quant = nullptr);
+// Top-k and sort of a small batch in one launch (f32 logits).
+bool router_sort_supported(uint32_t num_tokens, uint32_t num_experts, uint32_t top_k, uint32_t experts);
+cudaError_t launch_router_sort(const float* logits, const float* bias, int32_t* ids, float* weights, uint32_t num_tokens,
+                               uint32_t num_experts, uint32_t top_k, int sigmoid_score, int renormalize, float scaling,
+                               uint32_t local_offset, uint32_t experts, const RouteTables& rt, cudaStream_t stream,
+                               const TokenQuant* quant);
 
 // ---- router -----------------------------------------------------------------------
 // `bias` (optional f32 [num_experts]) is added to the logits before scoring.

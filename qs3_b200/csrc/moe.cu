@@ -1304,18 +1304,25 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
     // 2. top-k routing (src/model.rs:2092-2115)
     int32_t* ids = d->topk_ids.data != nullptr ? static_cast<int32_t*>(d->topk_ids.data) : x.topk_ids;
     float* wts = d->topk_weights.data != nullptr ? static_cast<float*>(d->topk_weights.data) : x.topk_weights;
-    cudaError_t err = launch_router_topk(logits, 0, static_cast<const float*>(d->router_bias.data), ids, wts,
-                                         d->num_tokens, p.num_experts, p.top_k,
-                                         d->score == QSCU_ROUTER_SCORE_SIGMOID, d->renormalize != 0,
-                                         d->routed_scaling_factor, st);
-    // 3. permutation
-    stage_mark(st, STAGE_ROUTE_SORT);
+    const float* bias = static_cast<const float*>(d->router_bias.data);
+    const int sigmoid = d->score == QSCU_ROUTER_SCORE_SIGMOID, renorm = d->renormalize != 0;
     const bool small_tiles = nvfp4 && rt.tile_rows != static_cast<uint32_t>(kTileM);
     TokenQuant tq { hidden, d->num_tokens, p.hidden_size, d->act_global_scale == 0.0f ? 1.0f : d->act_global_scale,
                     x.sh_xq, x.sh_xq_sf };
-    if (err == cudaSuccess)
-        err = launch_route_sort(ids, wts, routes, p.top_k, p.local_expert_offset, p.local_num_experts, rt, st,
-                                small_tiles && !fork && !prequant ? &tq : nullptr);
+    const TokenQuant* quant = small_tiles && !fork && !prequant ? &tq : nullptr;
+    cudaError_t err = cudaSuccess;
+    if (router_sort_supported(d->num_tokens, p.num_experts, p.top_k, p.local_num_experts)) { // 2. and 3. in one launch
+        err = launch_router_sort(logits, bias, ids, wts, d->num_tokens, p.num_experts, p.top_k, sigmoid, renorm,
+                                 d->routed_scaling_factor, p.local_expert_offset, p.local_num_experts, rt, st, quant);
+        stage_mark(st, STAGE_ROUTE_SORT);
+    } else {
+        err = launch_router_topk(logits, 0, bias, ids, wts, d->num_tokens, p.num_experts, p.top_k, sigmoid, renorm,
+                                 d->routed_scaling_factor, st);
+        // 3. permutation
+        stage_mark(st, STAGE_ROUTE_SORT);
+        if (err == cudaSuccess)
+            err = launch_route_sort(ids, wts, routes, p.top_k, p.local_expert_offset, p.local_num_experts, rt, st, quant);
+    }
     if (err != cudaSuccess)
         return set_cuda_error(ctx, err, "MoE routing");
 

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import bf16, f32, parse_floats, to_dev, to_np
+from helpers import bf16, f32, make_moe_inputs, parse_floats, to_dev, to_np
 
 pytestmark = pytest.mark.gpu
 
@@ -156,3 +156,30 @@ def test_shared_expert_gate_add(ops, oracle, golden):
         ops.shared_expert_gate_add_bf16(gate_t, to_dev(shared), out)
         ref = f32(oracle.shared_gate_add_bf16(np.array(case["gate"], np.float32), shared, out0))
         assert np.max(np.abs(f32(to_np(out)) - ref)) <= case["tolerance"]
+
+
+# sizes of the launch that routes and sorts a small batch: one token, a full block of warps, one more, more experts than
+# its larger batches take; part of the experts local
+@pytest.mark.parametrize("t,e,k,local", [(1, 8, 2, None), (16, 128, 8, None), (17, 128, 8, None), (8, 512, 10, (100, 300)),
+                                         (9, 512, 10, None), (3, 40, 4, (32, 8))])
+def test_router_and_sort_of_a_small_batch(ops, oracle, t, e, k, local):
+    h, i = 128, 64
+    off, le = local or (0, e)
+    d = make_moe_inputs(90 + t, t, h, e, i)
+    ctx = ops.Context()
+    plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=t, hidden_size=h, intermediate_size=i, num_experts=e, top_k=k,
+                                              local_expert_offset=off, local_num_experts=le))
+    ws = torch.zeros(plan.layer_workspace_size(t, 0), dtype=torch.uint8, device="cuda")
+    out = torch.empty((t, h), dtype=torch.bfloat16, device="cuda")
+    ids = torch.empty((t, k), dtype=torch.int32, device="cuda")
+    w = torch.empty((t, k), dtype=torch.float32, device="cuda")
+    logits = torch.empty((t, e), dtype=torch.float32, device="cuda")
+    ops.moe_layer_execute(plan, to_dev(d["hidden"]), to_dev(d["router"]), to_dev(d["gate_up"][off:off + le]),
+                          to_dev(d["down"][off:off + le]), out, ws, topk_ids=ids, topk_weights=w, router_logits=logits)
+    torch.cuda.synchronize()
+    ids_ref, w_ref = oracle.router_topk(to_np(logits), k, 0, True, 1.0)
+    assert np.array_equal(to_np(ids), ids_ref)
+    np.testing.assert_allclose(to_np(w), w_ref, rtol=1e-5)
+    tables = [to_np(x) for x in plan.routing_tables(ws, t)]
+    for g, r in zip(tables, oracle.route_sort(to_np(ids), to_np(w), off, le)):
+        assert np.array_equal(g, r)
