@@ -715,11 +715,12 @@ class SingleGpuLayer:
         if cfg.fp8:
             act_in = routes * (cfg.hidden + cfg.hidden // 128 * 4)
             act_out = routes * (cfg.inter + cfg.inter // 128 * 4)
-            kernel, nominal, fallback_ceiling = "gemm_fp8_kernel<16, gated>", 4500.0, 3413.0
+            kernel = "gemm_fp8_stream_kernel<gated>" if routes <= 40 * cfg.experts else "gemm_fp8_rows_kernel<gated>"
+            nominal, fallback_ceiling = 4500.0, 3413.0
         else:
             act_in = routes * (cfg.hidden // 2 + cfg.hidden // 16)
             act_out = routes * (cfg.inter // 2 + cfg.inter // 16)
-            decode = routes <= 16 * cfg.experts   # the plan's own rule for the swapped-operand kernel
+            decode = routes <= 22 * cfg.experts   # the plan's own rule for the swapped-operand kernel
             kernel = "gemm_nvfp4_swap_kernel<gated>" if decode else GATE_UP_KERNEL
             nominal, fallback_ceiling = 9000.0, 6642.0
         algo = hit * gu_bytes + act_in + act_out
@@ -794,7 +795,8 @@ GATE_UP_KERNEL = ("gemm_tc_astat_kernel<gated, swiglu_nvfp4>" if os.environ.get(
 TRAFFIC_RATIO = {"gemm_nvfp4_pair_kernel<gated, swiglu_nvfp4>": 1.07,
                  "gemm_tc_astat_kernel<gated, swiglu_nvfp4>": 1.02,
                  "gemm_nvfp4_swap_kernel<gated>": 1.00,
-                 "gemm_fp8_kernel<16, gated>": 1.02}
+                 "gemm_fp8_stream_kernel<gated>": 1.02,
+                 "gemm_fp8_rows_kernel<gated>": 1.02}
 
 
 def main():
