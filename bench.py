@@ -715,8 +715,7 @@ class SingleGpuLayer:
         if cfg.fp8:
             act_in = routes * (cfg.hidden + cfg.hidden // 128 * 4)
             act_out = routes * (cfg.inter + cfg.inter // 128 * 4)
-            kernel = "gemm_fp8_stream_kernel<gated>" if routes <= 40 * cfg.experts else "gemm_fp8_rows_kernel<gated>"
-            nominal, fallback_ceiling = 4500.0, 3413.0
+            kernel, nominal, fallback_ceiling = "gemm_fp8_stream_kernel<gated>", 4500.0, 3413.0
         else:
             act_in = routes * (cfg.hidden // 2 + cfg.hidden // 16)
             act_out = routes * (cfg.inter // 2 + cfg.inter // 16)
@@ -795,8 +794,7 @@ GATE_UP_KERNEL = ("gemm_tc_astat_kernel<gated, swiglu_nvfp4>" if os.environ.get(
 TRAFFIC_RATIO = {"gemm_nvfp4_pair_kernel<gated, swiglu_nvfp4>": 1.07,
                  "gemm_tc_astat_kernel<gated, swiglu_nvfp4>": 1.02,
                  "gemm_nvfp4_swap_kernel<gated>": 1.00,
-                 "gemm_fp8_stream_kernel<gated>": 1.02,
-                 "gemm_fp8_rows_kernel<gated>": 1.02}
+                 "gemm_fp8_stream_kernel<gated>": 1.00}
 
 
 def main():
