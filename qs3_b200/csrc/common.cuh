@@ -384,8 +384,9 @@ __device__ __forceinline__ void chain_begin()
 // memory and registers of its SMs keeps the small kernels of the other stream out.
 extern thread_local bool launch_unchained;
 struct UnchainedScope {
-    UnchainedScope() { launch_unchained = true; }
-    ~UnchainedScope() { launch_unchained = false; }
+    const bool before = launch_unchained;
+    explicit UnchainedScope(bool on = true) { launch_unchained = before || on; }
+    ~UnchainedScope() { launch_unchained = before; }
 };
 
 template <typename... KArgs, typename... Args>
