@@ -6,6 +6,8 @@
 
 #include <cooperative_groups.h>
 
+#include <utility>
+
 namespace qs3 {
 
 namespace {
@@ -28,6 +30,8 @@ quantize_weight_kernel(const __nv_bfloat16* __restrict__ w, uint32_t rows, uint3
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
+    // a block's shared memory may be written by a peer only once the block runs: awaited before the exchange, behind pass 1
+    auto started = cluster.barrier_arrive();
     const uint32_t rank = cluster.block_rank();
     const uint32_t e = blockIdx.x / kQwCluster;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -57,6 +61,7 @@ quantize_weight_kernel(const __nv_bfloat16* __restrict__ w, uint32_t rows, uint3
     if (lane == 0)
         s_part[warp] = m;
     __syncthreads();
+    cluster.barrier_wait(std::move(started));
     if (warp == 0) {
         m = lane < kQwThreads / 32 ? s_part[lane] : 0.0f;
 #pragma unroll
