@@ -131,7 +131,7 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < p.stages; ++s) {
             mbar_init(&full_bar[s], 1);
-            mbar_init(&empty_bar[s], 1);
+            mbar_init(&empty_bar[s], 2); // the MMAs of one issuer, and the other issuer has seen the stage
             mbar_init(&sf_ready[s], 1);
         }
         for (uint32_t b = 0; b < kSwMaxAcc; ++b) {
@@ -235,9 +235,11 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 }
                 if (ok && ((u - u0) & 1) != mine) {
                     // the other issuer's: its stages are waited for all the same, because a parity tells two
-                    // successive uses of a stage apart and no more
+                    // successive uses of a stage apart and no more, and no stage is refilled before both have
                     for (uint32_t kb = 0; kb < p.k_blocks && ok; ++kb) {
                         ok = mbar_wait<true>(&sf_ready[s], ph, abort_flag, p.err, ERR_SW_SF_WAIT);
+                        if (ok)
+                            mbar_arrive(&empty_bar[s]);
                         if (++s == p.stages) {
                             s = 0;
                             ph ^= 1;

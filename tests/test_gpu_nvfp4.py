@@ -264,6 +264,44 @@ def test_decode_batches_take_the_swapped_operand_kernel(ops, ctx, oracle, cfg):
     _check(to_np(out), ref)
 
 
+def _tile_height(ops, plan, ws, t):
+    """Rows of the token tiles in the tables of the last call: the padded segment starts follow the dense ones."""
+    counts, indptr, *_ = plan.routing_tables(ws, t)
+    view = ops.capi.RoutingView()
+    plan.ctx.check(plan.ctx._lib.qs3_moe_routing_tables(plan.ctx.handle, plan.handle, t, ws.data_ptr(), view))
+    at = view.indptr - ws.data_ptr() + 4 * len(indptr)
+    at = (at + 255) // 256 * 256
+    pad = to_np(ws[at:at + 4 * len(indptr)].view(torch.int32))
+    c = to_np(counts)
+    heights = [r for r in (32, 64, 128) if np.array_equal(np.diff(pad), (c + r - 1) // r * r)]
+    assert len(heights) == 1
+    return heights[0]
+
+
+# several feature blocks per CTA, so that both MMA issuers of the kernel work: a k of more blocks than the ring has stages
+# (2048 with 64-row tiles: eight over seven), of as many, and one of a single block
+@pytest.mark.parametrize("t,e,k,h,i,rows", [(100, 64, 8, 2048, 512, 64), (60, 64, 8, 2048, 512, 32),
+                                            (300, 128, 6, 256, 256, 64)])
+def test_swapped_operand_kernel_repeats(ops, ctx, oracle, t, e, k, h, i, rows):
+    d = make_moe_inputs(59, t, h, e, i)
+    gu, dn, _ = _quantise_all(ops, ctx, d, False)
+    plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=t, hidden_size=h, intermediate_size=i, num_experts=e, top_k=k,
+                                              backend=ops.capi.MOE_BACKEND_NVFP4))
+    hidden, router = to_dev(d["hidden"]), to_dev(d["router"])
+    ws = torch.zeros(plan.layer_workspace_size(t, 0), dtype=torch.uint8, device="cuda")
+    ids = torch.empty((t, k), dtype=torch.int32, device="cuda")
+    w = torch.empty((t, k), dtype=torch.float32, device="cuda")
+    outs = [torch.empty((t, h), dtype=torch.bfloat16, device="cuda") for _ in range(20)]
+    for out in outs:
+        ops.moe_layer_execute(plan, hidden, router, gu, dn, out, ws, topk_ids=ids, topk_weights=w)
+    torch.cuda.synchronize()
+    assert ctx.read_device_error() == 0
+    assert _tile_height(ops, plan, ws, t) == rows
+    hp, hs = oracle.nvfp4_quantize_act(d["hidden"], 1.0)
+    _check(to_np(outs[0]), oracle.moe_nvfp4(hp, hs, to_np(ids), to_np(w), _triple(gu), _triple(dn)))
+    assert all(torch.equal(out, outs[0]) for out in outs)
+
+
 @pytest.mark.parametrize("cfg", [
     dict(t=200, h=512, e=8, k=2, i=256, linear=False),   # 50 rows per expert: 64-row token tiles
     dict(t=61, h=2048, e=2, k=2, i=512, linear=True),    # 61 rows: a full k panel, a row group that is not full
