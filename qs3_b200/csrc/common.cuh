@@ -369,9 +369,11 @@ cudaError_t launch_fp8_rows_gemm(const Fp8Gemm& g, cudaStream_t stream, const ch
 #ifdef __CUDACC__
 // Chained launches (programmatic dependent launch): a kernel launched by launch_chained may start while its
 // predecessor in the stream still runs, so that launch latency, set-up and the fetch of its code overlap the
-// predecessor's tail. The rules: every thread of such a kernel executes chain_begin() before it touches global memory that
-// a predecessor reads or writes (and before it exits); chain_begin() first waits for the predecessor to complete, which has
+// predecessor's tail. The rules: every thread of such a kernel executes chain_begin() (or its two halves apart) before it touches
+// global memory that a predecessor reads or writes, and before it exits; it first waits for the predecessor to complete, which has
 // itself waited for its own, so at most two neighbouring kernels overlap and everything older is complete.
+// A kernel that allocates tensor memory does so before it releases its successor: a successor that sits on the same SM
+// allocates before it waits, and would hold the columns until the predecessor, which needs them, has completed.
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_begin()

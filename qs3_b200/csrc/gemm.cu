@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(kThreads)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const TcParams p)
 {
-    chain_begin();
+    chain_wait();
     // ---- which tile ----
     const uint32_t tile = blockIdx.y;
     int expert = 0, row0 = 0, nrows = 0;
@@ -96,6 +96,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    chain_release();
     const uint32_t tmem_sfa = tmem_base + kBN;
     const uint32_t tmem_sfb = tmem_base + kBN + 16;
 
@@ -245,7 +246,7 @@ gemm_tc_astat_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                      const __grid_constant__ CUtensorMap map_o, const TcParams p, const uint32_t stages,
                      const uint32_t nt_per_split, const uint32_t kbs)
 {
-    chain_begin();
+    chain_wait();
     const uint32_t tile = blockIdx.y;
     int expert = 0, row0 = 0, nrows = 0;
     if (p.tile_expert != nullptr) {
@@ -313,6 +314,7 @@ gemm_tc_astat_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    chain_release();
     const uint32_t tmem_sfa = tmem_base + 256;
     const uint32_t tmem_sfb = tmem_base + 384; // 16 columns per k block of every ring stage
     const uint32_t stage_bytes = kbs * kAsStageBytes;   // kbs k-blocks of B codes, then their scales
