@@ -19,6 +19,7 @@ SRC_DIR = os.path.join(PKG_DIR, "csrc")
 OBJ_DIR = os.path.join(SRC_DIR, "build")
 LIB_PATH = os.path.join(PKG_DIR, "libqs3moe.so")
 MARSHAL_PATH = os.path.join(PKG_DIR, "_marshal.so")
+MARSHAL_TAG_PATH = os.path.join(OBJ_DIR, "marshal.tag")
 CHECKED_LIB_PATH = os.path.join(PKG_DIR, "libqs3moe_checked.so")
 
 SOURCES = ["context.cu", "router.cu", "routing.cu", "gemm.cu", "gemm_api.cu", "nvfp4.cu", "moe.cu",
@@ -46,16 +47,33 @@ def _stale(target: str, deps: list[str]) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def marshal_tag() -> str:
+    """What the marshalling extension is built against beside its sources: torch's C++ interface and Python's."""
+    import importlib.metadata
+    import sysconfig
+    return f"{importlib.metadata.version('torch')} {sysconfig.get_config_var('SOABI')}"
+
+
+def _marshal_stale() -> bool:
+    if _stale(MARSHAL_PATH, [os.path.join(SRC_DIR, "marshal.cpp"), os.path.join(SRC_DIR, HEADERS[-1])]):
+        return True
+    if not os.path.exists(MARSHAL_TAG_PATH):
+        return True
+    with open(MARSHAL_TAG_PATH) as f:
+        return f.read() != marshal_tag()
+
+
 def build_marshal(force: bool = False) -> str:
     """Compile the Python extension that fills descriptors from torch tensors (``csrc/marshal.cpp``)."""
-    src = os.path.join(SRC_DIR, "marshal.cpp")
-    if force or _stale(MARSHAL_PATH, [src, os.path.join(SRC_DIR, HEADERS[-1])]):
+    if force or _marshal_stale():
         import sysconfig
 
         import torch
+        src = os.path.join(SRC_DIR, "marshal.cpp")
         base = os.path.dirname(torch.__file__)
         cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", src, "-o", MARSHAL_PATH,
                f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               f'-DQS3_TORCH_VERSION="{torch.__version__}"',
                *(f"-I{d}" for d in (os.path.join(base, "include"),
                                     os.path.join(base, "include", "torch", "csrc", "api", "include"),
                                     sysconfig.get_paths()["include"])),
@@ -63,6 +81,9 @@ def build_marshal(force: bool = False) -> str:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"g++ failed on {src}:\n{r.stdout}\n{r.stderr}")
+        os.makedirs(OBJ_DIR, exist_ok=True)
+        with open(MARSHAL_TAG_PATH, "w") as f:
+            f.write(marshal_tag())
     return MARSHAL_PATH
 
 

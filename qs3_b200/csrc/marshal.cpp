@@ -118,4 +118,12 @@ PyModuleDef module = { PyModuleDef_HEAD_INIT, "_marshal", nullptr, -1, methods, 
 
 } // namespace
 
-PyMODINIT_FUNC PyInit__marshal() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__marshal()
+{
+    PyObject* m = PyModule_Create(&module);
+    if (m != nullptr && PyModule_AddStringConstant(m, "torch_version", QS3_TORCH_VERSION) != 0) {
+        Py_DECREF(m);
+        return nullptr;
+    }
+    return m;
+}

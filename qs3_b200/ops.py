@@ -21,7 +21,10 @@ from . import capi
 try:
     from . import _marshal
 except ImportError as exc:
-    raise RuntimeError("qs3_b200/_marshal.so is missing: build it with `python -m qs3_b200._build`") from exc
+    raise RuntimeError(f"cannot load qs3_b200/_marshal.so ({exc}): build it with `python -m qs3_b200._build`") from exc
+if _marshal.torch_version != torch.__version__:   # it reads tensors by torch's C++ interface
+    raise RuntimeError(f"qs3_b200/_marshal.so was built for torch {_marshal.torch_version}, not {torch.__version__}: "
+                       "rebuild it with `python -m qs3_b200._build`")
 
 _STATUS_NAMES = {0: "Ok", 1: "InvalidArgument", 2: "Unsupported", 3: "OutOfMemory",
                  4: "CudaError", 5: "BackendError", 6: "InternalError"}

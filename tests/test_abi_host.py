@@ -319,3 +319,29 @@ def test_reference_arm_layer_shapes_equal_the_workload_constants():
         for field in ("name", "tokens", "hidden", "experts", "top_k", "inter", "shared_inter", "nvfp4", "zipf_s",
                       "fp8", "dtype_name"):
             assert getattr(a, field) == getattr(b, field), (name, field)
+
+
+def test_marshalling_extension_follows_torch_and_python(tmp_path, monkeypatch):
+    """Its binary is tied to torch's C++ interface and Python's: another version of either makes it stale, and a binary that
+    does not load or was built for another torch says so."""
+    import subprocess
+    import sys
+
+    from qs3_b200 import _build
+    assert not _build._marshal_stale()
+    monkeypatch.setattr(_build, "marshal_tag", lambda: "another torch")
+    assert _build._marshal_stale()
+
+    def fails(body):
+        code = f"import sys, types\n{body}\nfrom qs3_b200 import ops\n"
+        r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+        assert r.returncode != 0
+        return r.stderr
+    assert "built for torch 0.1" in fails(
+        "m = types.ModuleType('_marshal'); m.torch_version = '0.1'\n"
+        "import qs3_b200; qs3_b200._marshal = sys.modules['qs3_b200._marshal'] = m")
+    assert "undefined symbol: x" in fails(
+        "class Broken:\n"
+        "    def find_spec(self, name, *a):\n"
+        "        if name == 'qs3_b200._marshal': raise ImportError('undefined symbol: x')\n"
+        "sys.meta_path.insert(0, Broken())")
