@@ -119,8 +119,9 @@ struct RouteTables {
     uint32_t shared_rows;
 };
 
+constexpr uint32_t kAltMaxRoutes = 80; // routes per expert up to which the sort chooses between tile heights
 size_t route_tables_bytes(uint32_t routes, uint32_t experts);
-// Carves the tables out of `base` (may be NULL for sizing); returns bytes used.
+// Carves the tables out of `base` (may be NULL for sizing); returns bytes used, never fewer for more routes.
 size_t route_tables_carve(char* base, uint32_t routes, uint32_t experts, RouteTables* out,
                           uint32_t tile_rows = kTileM, uint32_t shared_rows = 0, uint32_t alt_tile_rows = 0);
 // Tokens to quantise (NVFP4) beside the sort.
@@ -306,7 +307,7 @@ cudaError_t launch_nvfp4_pair_gemm(const GemmProblem& p, cudaStream_t stream, co
 cudaError_t launch_nvfp4_swap_gemm(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);
 // Rows per token tile of an NVFP4 plan: 32 or 64 (decode kernel) when experts get few rows each, else 128.
 uint32_t nvfp4_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter);
-// Smaller tile height between which and 128 rows the sort shall choose, 0: none.
+// Smaller tile height between which and 128 rows the sort chooses up to kAltMaxRoutes routes per expert, 0: none.
 uint32_t nvfp4_alt_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter);
 // Whether a sort of this size can choose between tile heights.
 bool route_sort_can_choose(uint32_t routes, uint32_t experts);

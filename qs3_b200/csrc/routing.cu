@@ -1281,12 +1281,16 @@ size_t route_tables_carve(char* base, uint32_t routes, uint32_t experts, RouteTa
     rt.max_pad_rows = static_cast<uint32_t>(max_pad_rows);
     rt.max_tiles = static_cast<uint32_t>(max_pad_rows / tile_rows);
     uint32_t tiles = rt.max_tiles; // room in the tables
+    // A plan keeps the room of the largest choice beyond it: a workspace for many tokens serves fewer as well.
+    const bool alt = alt_tile_rows != 0 && routes <= kAltMaxRoutes * experts;
     if (alt_tile_rows != 0) {
-        rt.alt_tile_rows = alt_tile_rows;
-        rt.alt_max_tiles = static_cast<uint32_t>(align_up(routes, alt_tile_rows) / alt_tile_rows + seg);
-        tiles = rt.alt_max_tiles > tiles ? rt.alt_max_tiles : tiles;
-        const uint32_t alt_rows = rt.alt_max_tiles * alt_tile_rows; // (fewer than with the larger tiles, rounding aside)
-        rt.max_pad_rows = alt_rows > rt.max_pad_rows ? alt_rows : rt.max_pad_rows;
+        const uint32_t alt_routes = alt ? routes : kAltMaxRoutes * experts;
+        const uint32_t alt_tiles = static_cast<uint32_t>(align_up(alt_routes, alt_tile_rows) / alt_tile_rows + seg);
+        tiles = alt_tiles > tiles ? alt_tiles : tiles;
+        if (alt) { // (no more padded rows than with the larger tiles)
+            rt.alt_tile_rows = alt_tile_rows;
+            rt.alt_max_tiles = alt_tiles;
+        }
     }
     rt.route_blocks = (routes + kSortChunk - 1) / kSortChunk;
     rt.counts = carve<int32_t>(base, off, experts);
@@ -1300,8 +1304,10 @@ size_t route_tables_carve(char* base, uint32_t routes, uint32_t experts, RouteTa
     rt.tile_row0 = carve<int32_t>(base, off, tiles);
     rt.tile_nrows = carve<int32_t>(base, off, tiles);
     rt.total_tiles = carve<int32_t>(base, off, 1);
-    if (alt_tile_rows != 0)
-        rt.alt_total_tiles = carve<int32_t>(base, off, 1);
+    if (alt_tile_rows != 0) {
+        int32_t* const alt_total = carve<int32_t>(base, off, 1);
+        rt.alt_total_tiles = alt ? alt_total : nullptr;
+    }
     if (tile_rows == static_cast<uint32_t>(kTileM)) {
         rt.pair_expert = carve<int32_t>(base, off, rt.max_tiles);
         rt.pair_row0 = carve<int32_t>(base, off, rt.max_tiles);

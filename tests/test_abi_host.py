@@ -345,3 +345,28 @@ def test_marshalling_extension_follows_torch_and_python(tmp_path, monkeypatch):
         "    def find_spec(self, name, *a):\n"
         "        if name == 'qs3_b200._marshal': raise ImportError('undefined symbol: x')\n"
         "sys.meta_path.insert(0, Broken())")
+
+
+@pytest.mark.parametrize("backend", ["STAGED_BF16", "NVFP4", "FP8_BLOCKSCALE"])
+@pytest.mark.parametrize("experts,top_k", [(1, 1), (8, 2), (50, 8), (127, 10)])
+def test_workspace_of_many_tokens_serves_fewer(lib, ctx, backend, experts, top_k):
+    """Every layout change with the batch (tile heights, gathered copies, small sorts) included: 100 routes per expert
+    cover them all."""
+    b = getattr(capi, f"MOE_BACKEND_{backend}")
+    dt = {"STAGED_BF16": capi.DTYPE_BF16, "NVFP4": capi.DTYPE_NVFP4_E2M1, "FP8_BLOCKSCALE": capi.DTYPE_FP8_E4M3}[backend]
+    tokens = 100 * experts // top_k + 1
+    d = _plan_desc(backend=b, max_num_tokens=tokens, intermediate_size=256, num_experts=experts, local_num_experts=experts,
+                   top_k=top_k, activation_dtype=dt, weight_dtype=dt)
+    plan, n = C.c_void_p(), C.c_size_t()
+    assert lib.qsfi_moe_plan_create(ctx, C.byref(d), C.byref(plan)) == capi.STATUS_OK
+    try:
+        for size in (lambda t: lib.qsfi_moe_workspace_size(ctx, plan, t, C.byref(n)),
+                     lambda t: lib.qs3_moe_layer_workspace_size(ctx, plan, t, 0, C.byref(n)),
+                     lambda t: lib.qs3_moe_layer_workspace_size(ctx, plan, t, 256, C.byref(n))):
+            largest = 0
+            for t in range(1, tokens + 1):
+                assert size(t) == capi.STATUS_OK
+                assert n.value >= largest, t
+                largest = n.value
+    finally:
+        lib.qsfi_moe_plan_destroy(plan)
