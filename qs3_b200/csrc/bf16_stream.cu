@@ -315,8 +315,34 @@ cudaError_t launch_stream_instance(const CUtensorMap& mw, const CUtensorMap& mx,
 
 } // namespace
 
-uint32_t bf16_tile_rows(uint32_t routes, uint32_t experts)
+bool bf16_one_tile_per_cta(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter)
 {
+    // Few experts give the streaming kernel fewer units than SMs, each of 256 weight rows with the epilogue of a whole
+    // token tile at its end and, up to kGatherRows rows, gather4 loads that HBM no longer hides. Tiles of 128 x 128, two CTAs
+    // per SM, are shorter; beyond about a round of them, and for few rows, where the weights decide, streaming wins.
+    // Routed experts alone (hidden, experts top-k, intermediate; tokens: streaming / one tile per CTA, us):
+    //   2048, 8 top-2, 512     100: 38 / 32, 150: 46 / 32, 1000: 61 / 46, 2500: 97 / 87, 4000: 109 / 106
+    //   2048, 8 top-2, 1024    100: 43 / 47, 150: 52 / 45, 1000: 70 / 56, 2500: 121 / 120
+    //   1024, 4 top-1, 512     64: 26 / 26, 150: 33 / 26, 1000: 46 / 28, 4000: 53 / 40
+    //   2048, 16 top-4, 768    150: 51 / 55, 300: 73 / 56, 1000: 103 / 94, 1500: 121 / 121, 4000: 219 / 245
+    //   2048, 32 top-4, 512    300: 61 / 70, 600: 81 / 71, 1500: 105 / 108
+    // With a short k that epilogue does not hide behind the k loop of the next unit either, once an expert has the rows for
+    // whole tiles:
+    //   1024, 64 top-6, 512    600: 69 / 79, 1500: 111 / 113, 2500: 138 / 131, 6000: 269 / 255
+    //   512, 256 top-8, 512    1000: 100 / 150, 2000: 144 / 155, 2500: 165 / 160, 6000: 296 / 270
+    //   512, 64 top-8, 256     300: 36 / 36, 600: 50 / 37, 4000: 132 / 107
+    //   256, 128 top-8, 128    300: 28 / 32, 600: 34 / 32, 1500: 48 / 35
+    const uint64_t rows = (routes + experts - 1) / experts;
+    const uint64_t ctas = (rows + kTileM - 1) / kTileM * experts * ((inter + 63) / 64);
+    if (hidden <= 1024 && rows >= 16 + hidden * hidden / 5400)
+        return true;
+    return rows > 16 && 10 * ctas <= 26 * kSmCount && (rows - 16) * 2 * kSmCount >= 36 * ctas;
+}
+
+uint32_t bf16_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter)
+{
+    if (bf16_one_tile_per_cta(routes, experts, hidden, inter))
+        return static_cast<uint32_t>(kTileM);
     // Token bytes per weight byte grow with the tile, weight passes with the tiles of an expert. Layer times, 128
     // experts top-8: 8 routes per expert 0.239 ms with 32-row against 0.243 with 64-row tiles, 32 routes of a skewed
     // router 0.229 against 0.203; 64 routes 0.287 with 64-row against 0.291 with 128-row tiles, 128 routes 0.380
@@ -334,7 +360,7 @@ bool bf16_stream_gemm_supported(const GemmProblem& g)
         return plain && !g.gated && g.groups == 1 && g.epilogue == EPI_STORE_BF16 && g.a_rows <= 64
             && (g.n + 255) / 256 >= device_sm_count();
     }
-    return plain && (g.tile_rows == 32 || g.tile_rows == 64 || g.tile_rows == 128)
+    return plain && !g.one_tile_per_cta && (g.tile_rows == 32 || g.tile_rows == 64 || g.tile_rows == 128)
         && (g.gated ? g.epilogue == EPI_SWIGLU_BF16 : g.epilogue == EPI_STORE_BF16);
 }
 

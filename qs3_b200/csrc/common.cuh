@@ -38,6 +38,7 @@ namespace qs3 {
 
 constexpr size_t kWorkspaceAlign = 256;
 constexpr int kTileM = 128; // rows of one tensor-core tile; expert segments are padded to it
+constexpr uint32_t kSmCount = 148; // of the device, for rules that decide a workspace's layout: its size is asked for without one
 
 // ---- error plumbing (upstream qsfi_context.cu:10-101) -------------------------
 void clear_error(qsfi_error_info* err);
@@ -252,6 +253,7 @@ struct GemmProblem {
     int a_scale_linear;
     const void* gathered; // bf16 streaming kernel, with row_tokens: padded-layout copy of the rows of experts with more
                           // than kGatherRows rows, or NULL
+    int one_tile_per_cta; // bf16: not the streaming kernel
     int tables_ready; // NVFP4 decode and bf16 streaming kernels: the tile tables were complete before the predecessor in the stream started
     // decode kernel only: weights of a shared expert that is group number `groups` of the tile tables (NULL: none)
     const void* shared_b;
@@ -316,7 +318,10 @@ bool gemm_tc_supported(const GemmProblem& p);
 // tile of a bf16 plan.
 bool bf16_stream_gemm_supported(const GemmProblem& p);
 cudaError_t launch_bf16_stream_gemm(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);
-uint32_t bf16_tile_rows(uint32_t routes, uint32_t experts);
+uint32_t bf16_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter);
+// Whether the grouped GEMMs of a bf16 plan run as one 128 x 128 tile per CTA (gemm_tc_kernel) on a gathered copy of all
+// routed rows.
+bool bf16_one_tile_per_cta(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter);
 
 // ---- NVFP4 ----------------------------------------------------------------------
 // Token rows in token order -> e2m1 codes and scales tiled by token row.

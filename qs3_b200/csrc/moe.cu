@@ -70,9 +70,10 @@ bool upstream_bf16_workspace_bytes(const qsfi_moe_plan_desc& d, uint32_t num_tok
 
 struct Bf16Workspace {
     RouteTables rt;
-    __nv_bfloat16* expanded; // [pad_rows, H]: token rows gathered by expert, for large batches
+    __nv_bfloat16* expanded; // [pad_rows, H]: token rows gathered by expert, for large batches and one_tile_per_cta
     __nv_bfloat16* act;      // [pad_rows, I]
     __nv_bfloat16* y2;       // [pad_rows, H]
+    bool one_tile_per_cta;
     size_t bytes;
 };
 
@@ -81,9 +82,10 @@ Bf16Workspace carve_bf16(char* base, const qsfi_moe_plan_desc& d, uint32_t num_t
     Bf16Workspace w {};
     const uint32_t routes = num_tokens * d.top_k;
     size_t off = route_tables_carve(base, routes, d.local_num_experts, &w.rt,
-                                    bf16_tile_rows(routes, d.local_num_experts));
+                                    bf16_tile_rows(routes, d.local_num_experts, d.hidden_size, d.intermediate_size));
     const size_t rows = w.rt.max_pad_rows;
-    if (gather_rows_pays(num_tokens, d.top_k, d.local_num_experts))
+    w.one_tile_per_cta = bf16_one_tile_per_cta(routes, d.local_num_experts, d.hidden_size, d.intermediate_size);
+    if (w.one_tile_per_cta || gather_rows_pays(num_tokens, d.top_k, d.local_num_experts))
         w.expanded = carve<__nv_bfloat16>(base, off, rows * d.hidden_size);
     w.act = carve<__nv_bfloat16>(base, off, rows * d.intermediate_size);
     w.y2 = carve<__nv_bfloat16>(base, off, rows * d.hidden_size);
@@ -372,19 +374,25 @@ qsfi_status run_routed_bf16(qsfi_context* ctx, const qsfi_moe_plan_desc& p, cons
                             const __nv_bfloat16* gate_up, const __nv_bfloat16* down)
 {
     if (w.expanded != nullptr) {
-        const cudaError_t err = launch_gather_rows(hidden, p.hidden_size * 2, w.rt, kGatherRows, w.expanded, ctx->stream);
+        const cudaError_t err = launch_gather_rows(hidden, p.hidden_size * 2, w.rt, w.one_tile_per_cta ? 0 : kGatherRows,
+                                                   w.expanded, ctx->stream);
         if (err != cudaSuccess)
             return set_cuda_error(ctx, err, "MoE gather");
     }
     stage_mark(ctx->stream, STAGE_GATE_UP_GEMM);
     GemmProblem g1 = grouped_problem(w.rt, p.local_num_experts);
-    g1.gathered = w.expanded;
-    g1.tables_ready = w.expanded != nullptr; // the predecessor is the gather
-    g1.a = hidden; // token rows of experts with few of them are read in place, through the routing tables
-    g1.a_rows = num_tokens;
-    g1.row_tokens = w.rt.row_tokens;
-    g1.indptr = w.rt.indptr;
-    g1.pad_indptr = w.rt.pad_indptr;
+    g1.one_tile_per_cta = w.one_tile_per_cta;
+    if (w.one_tile_per_cta) {
+        g1.a = w.expanded;
+    } else {
+        g1.gathered = w.expanded;
+        g1.tables_ready = w.expanded != nullptr; // the predecessor is the gather
+        g1.a = hidden; // token rows of experts with few of them are read in place, through the routing tables
+        g1.a_rows = num_tokens;
+        g1.row_tokens = w.rt.row_tokens;
+        g1.indptr = w.rt.indptr;
+        g1.pad_indptr = w.rt.pad_indptr;
+    }
     g1.a_pitch_bytes = static_cast<uint64_t>(p.hidden_size) * 2;
     g1.b = gate_up;
     g1.b_pitch_bytes = static_cast<uint64_t>(p.hidden_size) * 2;
@@ -399,6 +407,7 @@ qsfi_status run_routed_bf16(qsfi_context* ctx, const qsfi_moe_plan_desc& p, cons
         return status;
     stage_mark(ctx->stream, STAGE_DOWN_GEMM);
     GemmProblem g2 = grouped_problem(w.rt, p.local_num_experts);
+    g2.one_tile_per_cta = w.one_tile_per_cta;
     g2.tables_ready = 1;
     g2.a = w.act;
     g2.a_pitch_bytes = static_cast<uint64_t>(p.intermediate_size) * 2;

@@ -525,10 +525,10 @@ router_sort_block_kernel(RouterParams r, uint32_t top_k, uint32_t local_offset, 
     block_sort(s, r.weights, r.num_tokens * top_k, top_k, experts, rt); // (starts with a barrier)
 }
 
-// dst[padded row] = src[token] for the tiles of experts with more than `min_rows` rows; a block per 32 rows of a tile, a
-// warp per row, four 16-byte vectors per lane in flight. Bound by HBM and L2: rows * row bytes, read and written; where
-// few experts are heavy, by the blocks that find nothing to do (8 rows per block: 2048 tokens, 512 experts 0.008 ms).
-constexpr uint32_t kGatherBlockRows = 32;
+// dst[padded row] = src[token] for the tiles of experts with more than `min_rows` rows; a block per 32 rows of a tile (8 where
+// those blocks fit the device at once), a warp per row, four 16-byte vectors per lane in flight. Bound by HBM and L2: rows *
+// row bytes, read and written; where few experts are heavy, by the blocks that find nothing to do (8 rows per block: 2048
+// tokens, 512 experts 0.008 ms).
 
 __global__ void __launch_bounds__(256)
 gather_rows_kernel(const uint4* __restrict__ src, uint32_t vec_per_row, RouteTables rt, int min_rows, uint4* __restrict__ dst)
@@ -541,8 +541,9 @@ gather_rows_kernel(const uint4* __restrict__ src, uint32_t vec_per_row, RouteTab
     if (rt.indptr[expert + 1] - dense0 <= min_rows)
         return;
     const int32_t* tokens = rt.row_tokens + dense0 + row0 - rt.pad_indptr[expert];
-    const int end = min(nrows, static_cast<int>((blockIdx.x + 1) * kGatherBlockRows));
-    for (int j = static_cast<int>(blockIdx.x * kGatherBlockRows + (threadIdx.x >> 5)); j < end; j += 8) {
+    const uint32_t block_rows = rt.tile_rows / gridDim.x;
+    const int end = min(nrows, static_cast<int>((blockIdx.x + 1) * block_rows));
+    for (int j = static_cast<int>(blockIdx.x * block_rows + (threadIdx.x >> 5)); j < end; j += 8) {
         const uint4* s = src + static_cast<size_t>(tokens[j]) * vec_per_row;
         uint4* d = dst + static_cast<size_t>(row0 + j) * vec_per_row;
         for (uint32_t i0 = lane; i0 < vec_per_row; i0 += 128) {
@@ -1369,7 +1370,8 @@ cudaError_t launch_gather_rows(const void* src, uint32_t row_bytes, const RouteT
 {
     if (rt.max_tiles == 0)
         return cudaSuccess;
-    return launch_chained(gather_rows_kernel, dim3((rt.tile_rows + kGatherBlockRows - 1) / kGatherBlockRows, rt.max_tiles), 256, 0, stream,
+    const uint32_t block_rows = rt.max_tiles * (rt.tile_rows / 8) <= 8 * kSmCount ? 8 : 32;
+    return launch_chained(gather_rows_kernel, dim3(rt.tile_rows / block_rows, rt.max_tiles), 256, 0, stream,
                           static_cast<const uint4*>(src), row_bytes / 16, rt, static_cast<int>(min_rows),
                           static_cast<uint4*>(dst));
 }

@@ -105,6 +105,22 @@ def to_np(t):
     return t.numpy().copy()
 
 
+def tile_height(plan, ws, t):
+    """Rows of the token tiles in the tables of the plan's last call: the padded segment starts follow the dense ones."""
+    import torch
+    from qs3_b200 import capi
+    counts, indptr, *_ = plan.routing_tables(ws, t)
+    view = capi.RoutingView()
+    plan.ctx.check(plan.ctx._lib.qs3_moe_routing_tables(plan.ctx.handle, plan.handle, t, ws.data_ptr(), view))
+    at = view.indptr - ws.data_ptr() + 4 * len(indptr)
+    at = (at + 255) // 256 * 256
+    pad = to_np(ws[at:at + 4 * len(indptr)].view(torch.int32))
+    c = to_np(counts)
+    heights = [r for r in (32, 64, 128) if np.array_equal(np.diff(pad), (c + r - 1) // r * r)]
+    assert len(heights) == 1
+    return heights[0]
+
+
 # ------------------------------------------------------- synthetic checkpoints ---
 
 _ST_ITEMSIZE = {"F64": 8, "F32": 4, "F16": 2, "BF16": 2, "I64": 8, "I32": 4, "I16": 2, "I8": 1, "U8": 1,

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import bf16, f32, make_moe_inputs, max_abs, moe_case_arrays, rel_l2, to_dev, to_np
+from helpers import bf16, f32, make_moe_inputs, max_abs, moe_case_arrays, rel_l2, tile_height, to_dev, to_np
 
 pytestmark = pytest.mark.gpu
 
@@ -59,8 +59,11 @@ def _check(out, ref):
     dict(t=77, h=72, e=5, k=3, i=40),        # ragged k and n tails on the tensor-core kernel
     dict(t=300, h=512, e=16, k=4, i=192),    # several row tiles per expert
     dict(t=64, h=1024, e=64, k=8, i=256, hot=True),
-    dict(t=97, h=264, e=6, k=2, i=136),      # 64-row token tiles; features one block past the weight tiles
-    dict(t=400, h=128, e=4, k=2, i=264),     # 128-row token tiles, several per expert; plain n of half a unit
+    dict(t=97, h=264, e=6, k=2, i=136),      # few experts: one tile per CTA on gathered rows; features past the tiles
+    dict(t=400, h=128, e=4, k=2, i=264),     # the same, several tiles per expert
+    dict(t=3000, h=72, e=90, k=1, i=64),     # the same, more tiles than the gather takes with small blocks
+    dict(t=44, h=264, e=6, k=2, i=136),      # streamed, 64-row token tiles; features one block past the weight tiles
+    dict(t=1040, h=1032, e=8, k=1, i=1608),  # streamed, 128-row token tiles, several per expert; plain n of half a unit
 ])
 def test_matches_oracle(ops, oracle, cfg):
     t, h, e, k, i = cfg["t"], cfg["h"], cfg["e"], cfg["k"], cfg["i"]
@@ -77,14 +80,18 @@ def test_matches_oracle(ops, oracle, cfg):
         assert np.array_equal(g, r)
 
 
-# one expert of `rows` rows beside emptier ones: read in place up to 48 rows, gathered beyond; 32-, 64- and 128-row tiles
-@pytest.mark.parametrize("rows,e", [(31, 16), (33, 2), (48, 2), (49, 2), (64, 2), (65, 6), (129, 2), (200, 2)])
-def test_rows_per_expert(ops, oracle, rows, e):
+# one expert of `rows` rows beside emptier ones. Streamed with 32- and 64-row tiles: read in place up to 48 rows, gathered
+# beyond; with few experts for the rows one 128-row tile per CTA on a gathered copy
+@pytest.mark.parametrize("rows,e,height", [(31, 16, 32), (33, 3, 64), (48, 4, 64), (49, 4, 64), (64, 5, 64), (65, 5, 64),
+                                           (129, 9, 64), (200, 14, 64), (33, 2, 128), (48, 2, 128), (49, 2, 128),
+                                           (64, 2, 128), (65, 2, 128), (129, 2, 128), (200, 2, 128), (65, 6, 64)])
+def test_rows_per_expert(ops, oracle, rows, e, height):
     t, h, i = rows + 9, 328, 200
     d = make_moe_inputs(5 + rows, t, h, e, i)
     ids = np.where(np.arange(t) < rows, 0, 1 + np.arange(t) % (e - 1)).astype(np.int32).reshape(t, 1)
     w = np.linspace(0.5, 1.5, t, dtype=np.float32).reshape(t, 1)
-    out, _, _ = _execute(ops, d["hidden"], ids, w, d["gate_up"], d["down"], e)
+    out, plan, ws = _execute(ops, d["hidden"], ids, w, d["gate_up"], d["down"], e)
+    assert tile_height(plan, ws, t) == height
     _check(out, oracle.moe_bf16(d["hidden"], ids, w, d["gate_up"], d["down"]))
 
 

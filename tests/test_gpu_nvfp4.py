@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import bf16, f32, make_moe_inputs, max_abs, rel_l2, to_dev, to_np, zipf_bias
+from helpers import bf16, f32, make_moe_inputs, max_abs, rel_l2, tile_height, to_dev, to_np, zipf_bias
 
 pytestmark = pytest.mark.gpu
 
@@ -264,20 +264,6 @@ def test_decode_batches_take_the_swapped_operand_kernel(ops, ctx, oracle, cfg):
     _check(to_np(out), ref)
 
 
-def _tile_height(ops, plan, ws, t):
-    """Rows of the token tiles in the tables of the last call: the padded segment starts follow the dense ones."""
-    counts, indptr, *_ = plan.routing_tables(ws, t)
-    view = ops.capi.RoutingView()
-    plan.ctx.check(plan.ctx._lib.qs3_moe_routing_tables(plan.ctx.handle, plan.handle, t, ws.data_ptr(), view))
-    at = view.indptr - ws.data_ptr() + 4 * len(indptr)
-    at = (at + 255) // 256 * 256
-    pad = to_np(ws[at:at + 4 * len(indptr)].view(torch.int32))
-    c = to_np(counts)
-    heights = [r for r in (32, 64, 128) if np.array_equal(np.diff(pad), (c + r - 1) // r * r)]
-    assert len(heights) == 1
-    return heights[0]
-
-
 # several feature blocks per CTA, so that both MMA issuers of the kernel work: a k of more blocks than the ring has stages
 # (2048 with 64-row tiles: eight over seven), of as many, and one of a single block
 @pytest.mark.parametrize("t,e,k,h,i,rows", [(100, 64, 8, 2048, 512, 64), (60, 64, 8, 2048, 512, 32),
@@ -296,7 +282,7 @@ def test_swapped_operand_kernel_repeats(ops, ctx, oracle, t, e, k, h, i, rows):
         ops.moe_layer_execute(plan, hidden, router, gu, dn, out, ws, topk_ids=ids, topk_weights=w)
     torch.cuda.synchronize()
     assert ctx.read_device_error() == 0
-    assert _tile_height(ops, plan, ws, t) == rows
+    assert tile_height(plan, ws, t) == rows
     hp, hs = oracle.nvfp4_quantize_act(d["hidden"], 1.0)
     _check(to_np(outs[0]), oracle.moe_nvfp4(hp, hs, to_np(ids), to_np(w), _triple(gu), _triple(dn)))
     assert all(torch.equal(out, outs[0]) for out in outs)
