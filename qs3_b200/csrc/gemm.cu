@@ -2,6 +2,7 @@
 //   gemm_tc_kernel        tcgen05, one 128 x 128 tile per CTA: gated dense bf16 problems and ragged k, NVFP4 with
 //                         k > 2048 (grouped bf16 problems go to bf16_stream.cu, larger dense ones to gemm_dense.cu)
 //   gemm_tc_astat_kernel  tcgen05, NVFP4 with the A panel resident in shared memory (k <= 2048)
+//   gemm_skinny_kernel    CUDA cores, f32 result of at most 64 rows and few features
 //   gemm_simt_kernel      CUDA cores, shapes the tensor-core tiles cannot address
 // launch_gemm() at the end picks one of these, a kernel of gemm_splitk.cu, gemm_dense.cu, gemm_pair.cu or bf16_stream.cu, or the
 // decode kernel of nvfp4_decode.cu.
@@ -735,6 +736,82 @@ bool pair_down_enabled()
     return enabled;
 }
 
+// ---- skinny bf16 GEMM: few rows, few features, f32 result ------------------------------------
+//
+// out[t, n] = sum_k A[t, k] * B[n, k] for a handful of rows (router logits of a decode batch over few experts): every
+// output feature gets a block; a warp keeps its slice of the weight row in registers and walks two rows of A
+// (L2-resident), lanes split k, one shuffle reduction per output. Latency-bound; against split-k with compensated sums, k =
+// 2048: 16 rows x 128 3.3 / 5.2 us, 64 x 64 5.6 / 6.4, 1 x 256 3.3 / 4.3, beyond 256 blocks 16 x 384 7.5 / 5.3. k = 256 stays
+// here whatever the features: so short a sum is closer than the tensor core's (64 x 128: 5.5e-8 against 6.0e-8).
+constexpr uint32_t kSkinnyWarps = 8;
+constexpr uint32_t kSkinnyRowsPerWarp = 2;
+constexpr uint32_t kSkinnyMaxChunks = 16; // k <= 4096, in 256-element chunks (8 per lane)
+
+__global__ void __launch_bounds__(kSkinnyWarps * 32)
+gemm_skinny_kernel(const __nv_bfloat16* __restrict__ a, uint64_t a_pitch, const __nv_bfloat16* __restrict__ b,
+                   uint64_t b_pitch, uint32_t rows, uint32_t k, float* __restrict__ out, uint64_t out_pitch,
+                   float alpha, float beta, const float* __restrict__ bias)
+{
+    chain_begin();
+    const uint32_t n = blockIdx.x;
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t chunks = k / 256;
+    const uint4* wrow = reinterpret_cast<const uint4*>(b + static_cast<uint64_t>(n) * b_pitch);
+    uint4 wv[kSkinnyMaxChunks];
+#pragma unroll
+    for (uint32_t c = 0; c < kSkinnyMaxChunks; ++c)
+        wv[c] = c < chunks ? wrow[c * 32 + lane] : make_uint4(0, 0, 0, 0);
+    const uint32_t row0 = (blockIdx.y * kSkinnyWarps + warp) * kSkinnyRowsPerWarp;
+    for (uint32_t r = row0; r < min(rows, row0 + kSkinnyRowsPerWarp); ++r) {
+        const uint4* xrow = reinterpret_cast<const uint4*>(a + static_cast<uint64_t>(r) * a_pitch);
+        float acc = 0.0f;
+#pragma unroll
+        for (uint32_t c = 0; c < kSkinnyMaxChunks; ++c) {
+            if (c < chunks) {
+                const uint4 xv = xrow[c * 32 + lane];
+                const uint32_t xs[4] = { xv.x, xv.y, xv.z, xv.w };
+                const uint32_t ws[4] = { wv[c].x, wv[c].y, wv[c].z, wv[c].w };
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    acc = fmaf(bf16_bits_to_f32(xs[j] & 0xffffu), bf16_bits_to_f32(ws[j] & 0xffffu), acc);
+                    acc = fmaf(bf16_bits_to_f32(xs[j] >> 16), bf16_bits_to_f32(ws[j] >> 16), acc);
+                }
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) {
+            float* o = out + static_cast<uint64_t>(r) * out_pitch + n;
+            float v = acc * (alpha == 0.0f ? 1.0f : alpha);
+            if (beta != 0.0f)
+                v += beta * *o;
+            if (bias != nullptr)
+                v += bias[n];
+            *o = v;
+        }
+    }
+}
+
+// Dense bf16 problem with f32 output whose rows would not fill one tensor-core tile.
+bool skinny_supported(const GemmProblem& g)
+{
+    return !g.nvfp4 && !g.gated && g.epilogue == EPI_STORE_F32 && g.tile_expert == nullptr && g.groups == 1
+        && g.group_scale == nullptr && g.a_rows <= 64 && g.k % 256 == 0 && g.k / 256 <= kSkinnyMaxChunks
+        && aligned16(g.a) && aligned16(g.b) && g.a_pitch_bytes % 16 == 0 && g.b_pitch_bytes % 16 == 0
+        && (g.k == 256 || g.n * ((g.a_rows + 15) / 16) <= 256);
+}
+
+cudaError_t launch_skinny(const GemmProblem& g, cudaStream_t stream)
+{
+    const uint32_t rows = static_cast<uint32_t>(g.a_rows);
+    const UnchainedScope plain; // (a chained start of so short a kernel: 1 x 2048 x 256 0.0038 against 0.0036 ms)
+    const dim3 grid(g.n, (rows + kSkinnyWarps * kSkinnyRowsPerWarp - 1) / (kSkinnyWarps * kSkinnyRowsPerWarp));
+    return launch_chained(gemm_skinny_kernel, grid, kSkinnyWarps * 32, 0, stream, static_cast<const __nv_bfloat16*>(g.a),
+                          g.a_pitch_bytes / 2, static_cast<const __nv_bfloat16*>(g.b), g.b_pitch_bytes / 2, rows, g.k,
+                          static_cast<float*>(g.out), g.out_pitch_elems, g.alpha, g.beta, g.bias);
+}
+
 TcParams make_params(const GemmProblem& g)
 {
     TcParams tp {};
@@ -867,6 +944,8 @@ cudaError_t launch_gemm(const GemmProblem& g, cudaStream_t stream, const char** 
             *why = "more than 65535 row tiles";
         return cudaErrorNotSupported;
     }
+    if (skinny_supported(g))
+        return launch_skinny(g, stream);
     if (gemm_splitk_supported(g))
         return launch_gemm_splitk(g, stream, why);
     if (gemm_dense_bf16_supported(g))

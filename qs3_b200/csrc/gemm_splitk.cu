@@ -7,12 +7,21 @@
 //   grid    (splits, ceil(n / 128), ceil(m / NT)), clusters of `splits` CTAs
 //   tile    128 weight rows (M side) x NT rows of A (N side, 16..128): accumulator lane = feature, column = row
 //   smem    ring of stages: B 128 x 64 + A NT x 64; then the f32 partial tile [NT][128] (the ring is idle by then)
-//   warps   0-3 accumulator -> shared memory, 4 producer (TMA), 5 MMA issuer; all six sum and store
+//   warps   0-3 (and 6 upwards) accumulator -> shared memory, 4 producer (TMA), 5 MMA issuer; all sum and store
+//
+// f32 results of few rows: the tensor core truncates what it adds to an accumulator, about 1.5e-8 of the result for every
+// instruction in the chain. So two instructions at most meet in an accumulator (each k block fills two), and warps add them
+// up in registers, compensated, as do the sums over the ranks. Error against 64 bits (2-norm) and time of 2048 x 512:
+//   rows                            1          16         64
+//   one chain per rank              24e-8 4.4  24e-8 4.4  23e-8 5.7 us
+//   short chains, compensated       6.3e-8 4.9 6.0e-8 5.6 6.0e-8 6.8
+//   CUDA cores, a block per feature 7.5e-8 5.6 8.1e-8 8.5 7.9e-8 28.6 (gemm_skinny_kernel: few features)
+// and of 65000 features, where no tile is split, 64 rows: one chain 2.1e-6 56 us, compensated 5.8e-8 103, CUDA cores 7.9e-8
+// 3710.
 //
 // Bound by latency: launch, one trip to HBM for the weights (and, at decode sizes, the code), two cluster barriers.
-// Router logits, hidden 2048: 512 experts, 1 token 0.0065 -> 0.0056 ms (a block per expert on CUDA cores), 128 tokens
-// 0.0153 -> 0.0098 (split over grid.z with a reduction pass), 1021 tokens 0.0194 -> 0.0112; 128 experts, 64 tokens
-// 0.0120 -> 0.0072, 4096 tokens 0.0204 -> 0.0128.
+// Router logits, hidden 2048: 512 experts, 128 tokens 0.0153 -> 0.0098 ms (split over grid.z with a reduction pass), 1021
+// tokens 0.0194 -> 0.0112; 128 experts, 4096 tokens 0.0204 -> 0.0128.
 #include "tcgen05.cuh"
 
 #include <cooperative_groups.h>
@@ -24,7 +33,6 @@ namespace {
 
 using namespace tc;
 
-constexpr int kSkThreads = 192;
 constexpr uint32_t kSkStages = 4;
 constexpr uint32_t kSkMaxSplits = 8; // the largest portable cluster
 constexpr uint32_t kSkPitch = 132; // floats per row of the partial tile
@@ -33,6 +41,7 @@ enum : uint32_t {
     ERR_SK_FULL_WAIT = 0x5a000001u,
     ERR_SK_EMPTY_WAIT = 0x5a000002u,
     ERR_SK_ACC_WAIT = 0x5a000003u,
+    ERR_SK_ACC_EMPTY_WAIT = 0x5a000004u,
 };
 
 struct SplitkParams {
@@ -52,8 +61,46 @@ template <int NT> struct SkSmem {
     static constexpr uint32_t kBytes = kRing > kPartial ? kRing : kPartial;
 };
 
-template <int NT, bool F32>
-__global__ void __launch_bounds__(kSkThreads)
+// How the products of a row are summed (see above).
+enum SkSum { SUM_CHAIN = 0, SUM_SHORT_CHAINS = 1, SUM_COMPENSATED = 2 };
+
+// Tensor-memory buffers: short chains two accumulators per k block, in turn; else one accumulator for all of k.
+template <int NT, int SUM> struct SkTmem {
+    static constexpr uint32_t kBufs = SUM == SUM_CHAIN ? 1 : NT <= 32 ? 4 : 2;
+    static constexpr uint32_t kUsed = SUM == SUM_CHAIN ? NT : 2 * NT * kBufs;
+    static constexpr uint32_t kCols = kUsed < 32 ? 32 : kUsed;
+    // warps that empty them, in fours, one per quarter of the lanes; compensated sums take a warp for 16 columns
+    static constexpr uint32_t kAdders = SUM == SUM_COMPENSATED ? NT / 4 : 4;
+    static constexpr uint32_t kThreads = (kAdders + 2) * 32;
+    static constexpr uint32_t kMine = NT * 4 / kAdders; // columns of an adding warp
+};
+
+// Compensated (Kahan) sums of two neighbouring values at a time: s - c is the sum of the values added so far to within a
+// rounding of it. An infinity makes c a NaN: a plain sum beside it tells.
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+constexpr uint64_t kNegate2 = 0x8000000080000000ull;
+__device__ __forceinline__ void kahan2(uint64_t& s, uint64_t& c, uint64_t x)
+{
+    const uint64_t y = add2(x, c ^ kNegate2), t = add2(s, y);
+    c = add2(add2(t, s ^ kNegate2), y ^ kNegate2);
+    s = t;
+}
+__device__ __forceinline__ void kahan(float& s, float& c, float x)
+{
+    const float y = __fadd_rn(x, -c), t = __fadd_rn(s, y);
+    c = __fadd_rn(__fadd_rn(t, -s), -y);
+    s = t;
+}
+__device__ __forceinline__ float half2(uint64_t v, uint32_t i) { return __uint_as_float(static_cast<uint32_t>(v >> (32 * i))); }
+__device__ __forceinline__ uint64_t pack2(uint32_t a, uint32_t b) { return static_cast<uint64_t>(b) << 32 | a; }
+
+template <int NT, bool F32, int SUM>
+__global__ void __launch_bounds__(SkTmem<NT, SUM>::kThreads)
 gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_a,
                    const SplitkParams p)
 {
@@ -61,15 +108,18 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = cluster.block_rank(), splits = cluster.num_blocks();
     constexpr uint32_t kStageBytes = SkSmem<NT>::kStageBytes;
-    constexpr uint32_t kTmemCols = NT < 32 ? 32 : NT;
+    constexpr uint32_t kTmemCols = SkTmem<NT, SUM>::kCols, kBufs = SkTmem<NT, SUM>::kBufs;
+    constexpr uint32_t kAdders = SkTmem<NT, SUM>::kAdders, kMine = SkTmem<NT, SUM>::kMine;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    float* part = reinterpret_cast<float*>(smem); // [NT][kSkPitch], after the ring
+    float* part = reinterpret_cast<float*>(smem); // [NT][kSkPitch], after the ring; short chains: and what to subtract, the same
+    constexpr uint32_t kRest = NT * kSkPitch;
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + SkSmem<NT>::kBytes);
     uint64_t* empty_bar = full_bar + kSkStages;
-    uint64_t* acc_bar = empty_bar + kSkStages;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_bar + 1);
+    uint64_t* acc_full = empty_bar + kSkStages;
+    uint64_t* acc_empty = acc_full + kBufs; // short chains
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + kBufs);
     volatile uint32_t* abort_flag = tmem_slot + 1;
 
     const uint32_t warp = threadIdx.x >> 5;
@@ -82,7 +132,10 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
-        mbar_init(acc_bar, 1);
+        for (uint32_t b = 0; b < kBufs; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], kAdders);
+        }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -122,7 +175,11 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
                 = (1u << 4) | (1u << 7) | (1u << 10) | ((static_cast<uint32_t>(NT) >> 3) << 17) | ((kBM >> 4) << 24);
             bool ok = true;
             for (uint32_t i = 0; i < kb1 - kb0; ++i) {
-                const uint32_t s = i % kSkStages, ph = (i / kSkStages) & 1;
+                const uint32_t s = i % kSkStages, ph = (i / kSkStages) & 1, b = i % kBufs;
+                if (SUM != SUM_CHAIN && !mbar_wait<true>(&acc_empty[b], ((i / kBufs) & 1) ^ 1, abort_flag, p.err, ERR_SK_ACC_EMPTY_WAIT)) {
+                    ok = false;
+                    break;
+                }
                 if (!mbar_wait<true>(&full_bar[s], ph, abort_flag, p.err, ERR_SK_FULL_WAIT)) {
                     ok = false;
                     break;
@@ -132,31 +189,87 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
                 const uint64_t db = operand_desc(sb), da = operand_desc(sb + kTileBytes);
 #pragma unroll
                 for (uint32_t j = 0; j < 4; ++j)
-                    tc_mma_bf16(tmem_base, db + 2 * j, da + 2 * j, kIdesc, (i > 0 || j > 0) ? 1u : 0u);
+                    tc_mma_bf16(SUM != SUM_CHAIN ? tmem_base + (2 * b + j / 2) * NT : tmem_base, db + 2 * j, da + 2 * j, kIdesc,
+                                (SUM != SUM_CHAIN ? j % 2 : i + j) > 0 ? 1u : 0u);
                 tc_commit(&empty_bar[s]);
+                if (SUM != SUM_CHAIN)
+                    tc_commit(&acc_full[b]);
             }
-            if (ok)
-                tc_commit(acc_bar);
+            if (ok && SUM == SUM_CHAIN)
+                tc_commit(acc_full);
         }
     } else {
-        // ------------------------------------- accumulator -> partial tile in smem --
-        ready = __all_sync(0xffffffffu, mbar_wait(acc_bar, 0, abort_flag, p.err, ERR_SK_ACC_WAIT));
-        tc_fence_after();
-        if (ready) { // every load has been consumed: the ring is free
-            const bool some = kb1 > kb0; // a rank past the end of k adds zeros
+        // ------------------------------------- accumulators -> partial tile in smem --
+        // this warp's lanes, and its first column
+        const uint32_t quarter = warp % 4, c0 = (warp < 4 ? 0 : (warp - 2) / 4) * kMine;
+        const uint32_t lanes = tmem_base + ((quarter * 32) << 16) + c0;
+        float* const mine = part + c0 * kSkPitch + quarter * 32 + lane;
+        if constexpr (SUM != SUM_CHAIN) {
+            constexpr bool KAHAN = SUM == SUM_COMPENSATED;
+            constexpr uint32_t kKept = KAHAN ? kMine / 2 : 1;
+            uint64_t plain[kMine / 2], sum[kKept] = {}, rest[kKept] = {};
 #pragma unroll
-            for (uint32_t c = 0; c < NT / 16; ++c) {
-                if (m0 + c * 16 >= p.m)
+            for (uint32_t t = 0; t < kMine / 2; ++t)
+                plain[t] = 0;
+            for (uint32_t i = 0; i < kb1 - kb0; ++i) {
+                const uint32_t b = i % kBufs;
+                ready = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], (i / kBufs) & 1, abort_flag, p.err, ERR_SK_ACC_WAIT));
+                if (!ready)
                     break;
-                uint32_t v[16];
-                tc_ld16(tmem_base + ((warp * 32) << 16) + c * 16, v);
-                tc_ld_wait();
+                tc_fence_after();
 #pragma unroll
-                for (uint32_t t = 0; t < 16; ++t)
-                    part[(c * 16 + t) * kSkPitch + warp * 32 + lane] = some ? __uint_as_float(v[t]) : 0.0f;
+                for (uint32_t c = 0; c < kMine / 16; ++c) {
+                    if (m0 + c0 + c * 16 < p.m) { // uniform
+                        uint32_t v[16], w[16];
+                        tc_ld16(lanes + 2 * b * NT + c * 16, v);
+                        tc_ld16(lanes + (2 * b + 1) * NT + c * 16, w);
+                        tc_ld_wait();
+#pragma unroll
+                        for (uint32_t t = 0; t < 8; ++t) {
+                            const uint64_t x = add2(pack2(v[2 * t], v[2 * t + 1]), pack2(w[2 * t], w[2 * t + 1]));
+                            plain[c * 8 + t] = add2(plain[c * 8 + t], x);
+                            if constexpr (KAHAN)
+                                kahan2(sum[c * 8 + t], rest[c * 8 + t], x);
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0)
+                    mbar_arrive(&acc_empty[b]);
             }
+            // every load of this CTA has been consumed (all adding warps have seen the last block): the ring is free
+            ready = group_all(1, kAdders * 32, ready);
+#pragma unroll
+            for (uint32_t t = 0; t < kMine; ++t)
+                if (ready && m0 + c0 + t < p.m) {
+                    const float whole = half2(plain[t / 2], t % 2);
+                    mine[t * kSkPitch] = whole;
+                    if constexpr (KAHAN) {
+                        if (isfinite(whole))
+                            mine[t * kSkPitch] = half2(sum[t / 2], t % 2);
+                        mine[kRest + t * kSkPitch] = isfinite(whole) ? half2(rest[t / 2], t % 2) : 0.0f;
+                    }
+                }
+        } else {
+            ready = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.err, ERR_SK_ACC_WAIT));
+            tc_fence_after();
+            if (ready) { // every load has been consumed: the ring is free
+                const bool some = kb1 > kb0; // a rank past the end of k adds zeros
+#pragma unroll
+                for (uint32_t c = 0; c < NT / 16; ++c) {
+                    if (m0 + c * 16 >= p.m)
+                        break;
+                    uint32_t v[16];
+                    tc_ld16(lanes + c * 16, v);
+                    tc_ld_wait();
+#pragma unroll
+                    for (uint32_t t = 0; t < 16; ++t)
+                        mine[(c * 16 + t) * kSkPitch] = some ? __uint_as_float(v[t]) : 0.0f;
+                }
+            }
+            tc_fence_before();
         }
-        tc_fence_before();
     }
     cluster.sync(); // every partial tile is complete
     // rows of the tile are dealt out over the cluster's warps; a lane sums four features over the ranks, in order
@@ -164,12 +277,21 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
     const float alpha = p.alpha == 0.0f ? 1.0f : p.alpha;
     const uint32_t rows = min(static_cast<uint32_t>(NT), p.m - m0);
     const uint32_t f = n0 + lane * 4;
-    for (uint32_t t = rank * (kSkThreads / 32) + warp; t < rows && *abort_flag == 0; t += splits * (kSkThreads / 32)) {
+    constexpr uint32_t kWarps = kAdders + 2;
+    for (uint32_t t = rank * kWarps + warp; t < rows && *abort_flag == 0; t += splits * kWarps) {
         float4 v[kSkMaxSplits];
 #pragma unroll
         for (uint32_t s = 0; s < kSkMaxSplits; ++s)
             v[s] = s < splits ? *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, s) + t * kSkPitch + lane * 4)
                               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float4 r[SUM == SUM_COMPENSATED ? kSkMaxSplits : 1]; // (all loads on their way before the sums)
+        if constexpr (SUM == SUM_COMPENSATED) {
+#pragma unroll
+            for (uint32_t s = 0; s < kSkMaxSplits; ++s)
+                r[s] = s < splits
+                    ? *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, s) + kRest + t * kSkPitch + lane * 4)
+                    : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
         float a[4] = { v[0].x, v[0].y, v[0].z, v[0].w };
 #pragma unroll
         for (uint32_t s = 1; s < kSkMaxSplits; ++s) {
@@ -177,6 +299,21 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
             a[1] += v[s].y;
             a[2] += v[s].z;
             a[3] += v[s].w;
+        }
+        if constexpr (SUM == SUM_COMPENSATED) {
+            float sum[4] = { v[0].x, v[0].y, v[0].z, v[0].w }, rest[4] = {}, low[4] = { r[0].x, r[0].y, r[0].z, r[0].w };
+#pragma unroll
+            for (uint32_t s = 1; s < kSkMaxSplits; ++s) {
+                const float x[4] = { v[s].x, v[s].y, v[s].z, v[s].w }, y[4] = { r[s].x, r[s].y, r[s].z, r[s].w };
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q) {
+                    kahan(sum[q], rest[q], x[q]);
+                    low[q] += y[q];
+                }
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q)
+                a[q] = isfinite(a[q]) ? sum[q] - (rest[q] + low[q]) : a[q];
         }
         const uint64_t at = static_cast<uint64_t>(m0 + t) * p.out_pitch + f;
         const uint32_t left = f < p.n ? min(4u, p.n - f) : 0u;
@@ -214,12 +351,12 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
     }
 }
 
-template <int NT, bool F32>
+template <int NT, bool F32, int SUM>
 cudaError_t launch_splitk_instance(const CUtensorMap& mb, const CUtensorMap& ma, const SplitkParams& sp, dim3 grid,
                                    cudaStream_t stream)
 {
-    auto kernel = gemm_splitk_kernel<NT, F32>;
-    constexpr size_t smem = 1024 + SkSmem<NT>::kBytes + 128;
+    auto kernel = gemm_splitk_kernel<NT, F32, SUM>;
+    constexpr size_t smem = 1024 + SkSmem<NT>::kBytes + 256;
     static bool configured[64] = {}; // per instantiation and device
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
@@ -232,21 +369,43 @@ cudaError_t launch_splitk_instance(const CUtensorMap& mb, const CUtensorMap& ma,
         if (dev >= 0 && dev < 64)
             configured[dev] = true;
     }
-    return launch_chained_cluster(kernel, grid.x, grid, kSkThreads, smem, stream, mb, ma, sp);
+    return launch_chained_cluster(kernel, grid.x, grid, SkTmem<NT, SUM>::kThreads, smem, stream, mb, ma, sp);
 }
 
-// Rows of A per tile: the fewest MMA columns that hold them, 64 above that (128 x 4096 x 2048: 0.0125 ms against
-// 0.0145 with 128) as long as every tile can still be split.
-uint32_t splitk_tile_rows(uint64_t m) { return m <= 16 ? 16u : m <= 32 ? 32u : 64u; }
-
 uint64_t splitk_tiles(const GemmProblem& g, uint32_t nt) { return (g.n + 127ull) / 128 * ((g.a_rows + nt - 1) / nt); }
+
+// Rows of A per tile: the fewest MMA columns that hold them, 64 above that (128 x 4096 x 2048: 0.0125 ms against
+// 0.0145 with 128) as long as every tile can still be split. Compensated sums in smaller tiles as long as each can be split in
+// four: adding up is what they wait for (64 x 2048 x 512: 0.0054 ms, with 32 rows 0.0066).
+uint32_t splitk_tile_rows(const GemmProblem& g)
+{
+    if (g.epilogue == EPI_STORE_F32 && g.a_rows <= 64)
+        for (uint32_t nt = 16; nt < 64; nt *= 2)
+            if (4 * splitk_tiles(g, nt) <= device_sm_count())
+                return nt;
+    return g.a_rows <= 16 ? 16u : g.a_rows <= 32 ? 32u : 64u;
+}
+
+// Compensated sums for f32 results of decode batches, which the CUDA cores summed before; short chains for router logits of
+// up to a few row tiles. A larger batch's had one chain over all of k before this kernel, and adding up outside the
+// tensor core takes longer than the loads where every SM has a tile (4096 x 2048 x 8: 0.0128 against 0.0120 ms).
+SkSum splitk_sum(const GemmProblem& g, uint32_t nt)
+{
+    if (g.epilogue != EPI_STORE_F32)
+        return SUM_CHAIN;
+    return g.a_rows <= 64 ? SUM_COMPENSATED : nt == 64 && splitk_tiles(g, 128) <= 18 ? SUM_SHORT_CHAINS : SUM_CHAIN;
+}
 
 // Tile rows of a problem that this kernel takes, 0: it does not. At least two CTAs per tile without exceeding one CTA
 // per SM, since more tiles fill the device as they are; a long k is split with 128-row tiles too (2048 x 4096 x 512:
 // 0.0207 against 0.0269 ms for the 128 x 256 kernel, but 512 x 2048 x 2048: 0.0163 against 0.0145).
 uint32_t splitk_choice(const GemmProblem& g)
 {
-    const uint32_t nt = splitk_tile_rows(g.a_rows);
+    const uint32_t nt = splitk_tile_rows(g);
+    if (g.epilogue == EPI_STORE_F32 && g.a_rows <= 64) // whatever the tiles: for its sums
+        return nt;
+    if (g.a_rows > 64 && g.k < 512) // nothing to split (1021 x 256 x 8: 0.0058 against 0.0046 ms in one tile per CTA)
+        return 0;
     if (2 * splitk_tiles(g, nt) <= device_sm_count())
         return nt;
     return nt == 64 && g.k >= 2048 && 2 * splitk_tiles(g, 128) <= device_sm_count() ? 128u : 0u;
@@ -290,12 +449,19 @@ cudaError_t launch_gemm_splitk(const GemmProblem& g, cudaStream_t stream, const 
         return cudaErrorInvalidValue;
     }
     const dim3 grid(splits, (g.n + 127) / 128, static_cast<uint32_t>((g.a_rows + nt - 1) / nt));
-    const bool f32 = g.epilogue == EPI_STORE_F32;
-    switch (nt) {
-    case 16: return f32 ? launch_splitk_instance<16, true>(mb, ma, sp, grid, stream) : launch_splitk_instance<16, false>(mb, ma, sp, grid, stream);
-    case 32: return f32 ? launch_splitk_instance<32, true>(mb, ma, sp, grid, stream) : launch_splitk_instance<32, false>(mb, ma, sp, grid, stream);
-    case 64: return f32 ? launch_splitk_instance<64, true>(mb, ma, sp, grid, stream) : launch_splitk_instance<64, false>(mb, ma, sp, grid, stream);
-    default: return f32 ? launch_splitk_instance<128, true>(mb, ma, sp, grid, stream) : launch_splitk_instance<128, false>(mb, ma, sp, grid, stream);
+    const auto launch = [&](auto kernel) { return kernel(mb, ma, sp, grid, stream); };
+    if (g.epilogue != EPI_STORE_F32)
+        return launch(nt == 16 ? launch_splitk_instance<16, false, SUM_CHAIN>
+            : nt == 32         ? launch_splitk_instance<32, false, SUM_CHAIN>
+            : nt == 64         ? launch_splitk_instance<64, false, SUM_CHAIN>
+                               : launch_splitk_instance<128, false, SUM_CHAIN>);
+    switch (splitk_sum(g, nt)) {
+    case SUM_COMPENSATED:
+        return launch(nt == 16 ? launch_splitk_instance<16, true, SUM_COMPENSATED>
+            : nt == 32         ? launch_splitk_instance<32, true, SUM_COMPENSATED>
+                               : launch_splitk_instance<64, true, SUM_COMPENSATED>);
+    case SUM_SHORT_CHAINS: return launch(launch_splitk_instance<64, true, SUM_SHORT_CHAINS>);
+    default: return launch(nt == 64 ? launch_splitk_instance<64, true, SUM_CHAIN> : launch_splitk_instance<128, true, SUM_CHAIN>);
     }
 }
 

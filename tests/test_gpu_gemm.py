@@ -130,6 +130,35 @@ def test_splitk_kernel(gemm, shape, beta):
     assert torch.equal(again, out)
 
 
+# f32 results of few rows: on the CUDA cores (few features), split k with 16-, 32- and 64-row tiles, a k tail, more tiles
+# than SMs. A sum in one tensor-core chain truncates in every instruction and is off by 2e-6 at k = 2048; chains of two
+# instructions (at most 2^-23 of the value each, half of that on average) and a rounding stay within 1e-7.
+@pytest.mark.parametrize("shape", [(1, 2048, 128), (64, 1024, 64), (1, 2048, 512), (17, 576, 300), (33, 2048, 512),
+                                   (64, 2048, 1100), (24, 2056, 4096), (40, 2048, 5000), (64, 512, 38000)])
+def test_f32_sums_of_few_rows(gemm, shape):
+    rows, k, n = shape
+    g = torch.Generator(device="cuda").manual_seed(rows + k + n)
+    x = torch.randn((rows, k), generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn((n, k), generator=g, device="cuda") * 0.02).to(torch.bfloat16)
+    out = torch.empty((rows, n), dtype=torch.float32, device="cuda")
+    gemm.gemm_bf16(x, w, out)
+    want = x.double() @ w.double().t()
+    assert float((out.double() - want).norm()) <= 1e-7 * float(want.norm())
+    # an infinity stays one, two of different sign make a NaN, and other rows and columns keep their sums
+    x2, w2 = x.clone(), w.clone()
+    x2[0, k - 1] = float("inf")
+    x2[rows - 1, 3] = float("-inf")
+    w2[5, 70] = float("inf")
+    again = torch.empty_like(out)
+    gemm.gemm_bf16(x2, w2, again)
+    special = ~torch.isfinite(again)
+    ref = x2.double() @ w2.double().t()
+    assert torch.equal(special, ~torch.isfinite(ref))
+    assert torch.equal(torch.isnan(again), torch.isnan(ref))
+    assert torch.equal(again[special & ~torch.isnan(ref)].double(), ref[special & ~torch.isnan(ref)])
+    assert torch.equal(again[~special], out[~special])
+
+
 # at most 128 rows and more than 148 units of features: weights streamed as the M side, unit height chosen for full
 # rounds (37889 = 148 * 256 + 1 features: the last unit holds one), every row tile height
 @pytest.mark.parametrize("rows,k,n", [(1, 64, 37889), (33, 200, 40000), (128, 128, 50007)])
