@@ -741,7 +741,7 @@ bool pair_down_enabled()
 // out[t, n] = sum_k A[t, k] * B[n, k] for a handful of rows (router logits of a decode batch over few experts): every
 // output feature gets a block; a warp keeps its slice of the weight row in registers and walks two rows of A
 // (L2-resident), lanes split k, one shuffle reduction per output. Latency-bound; against split-k with compensated sums, k =
-// 2048: 16 rows x 128 3.3 / 5.2 us, 64 x 64 5.6 / 6.4, 1 x 256 3.3 / 4.3, beyond 256 blocks 16 x 384 7.5 / 5.3. k = 256 stays
+// 2048: 16 rows x 128 3.1 / 4.8 us, 64 x 64 5.4 / 5.0, 1 x 256 3.3 / 4.3, beyond 256 blocks 16 x 384 7.5 / 5.0. k = 256 stays
 // here whatever the features: so short a sum is closer than the tensor core's (64 x 128: 5.5e-8 against 6.0e-8).
 constexpr uint32_t kSkinnyWarps = 8;
 constexpr uint32_t kSkinnyRowsPerWarp = 2;
@@ -805,7 +805,6 @@ bool skinny_supported(const GemmProblem& g)
 cudaError_t launch_skinny(const GemmProblem& g, cudaStream_t stream)
 {
     const uint32_t rows = static_cast<uint32_t>(g.a_rows);
-    const UnchainedScope plain; // (a chained start of so short a kernel: 1 x 2048 x 256 0.0038 against 0.0036 ms)
     const dim3 grid(g.n, (rows + kSkinnyWarps * kSkinnyRowsPerWarp - 1) / (kSkinnyWarps * kSkinnyRowsPerWarp));
     return launch_chained(gemm_skinny_kernel, grid, kSkinnyWarps * 32, 0, stream, static_cast<const __nv_bfloat16*>(g.a),
                           g.a_pitch_bytes / 2, static_cast<const __nv_bfloat16*>(g.b), g.b_pitch_bytes / 2, rows, g.k,

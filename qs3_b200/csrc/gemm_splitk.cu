@@ -14,9 +14,9 @@
 // up in registers, compensated, as do the sums over the ranks. Error against 64 bits (2-norm) and time of 2048 x 512:
 //   rows                            1          16         64
 //   one chain per rank              24e-8 4.4  24e-8 4.4  23e-8 5.7 us
-//   short chains, compensated       6.3e-8 4.9 6.0e-8 5.6 6.0e-8 6.8
+//   short chains, compensated       6.8e-8 4.4 6.5e-8 5.0 6.6e-8 5.8
 //   CUDA cores, a block per feature 7.5e-8 5.6 8.1e-8 8.5 7.9e-8 28.6 (gemm_skinny_kernel: few features)
-// and of 65000 features, where no tile is split, 64 rows: one chain 2.1e-6 56 us, compensated 5.8e-8 103, CUDA cores 7.9e-8
+// and of 65000 features, where no tile is split, 64 rows: one chain 2.1e-6 56 us, compensated 5.8e-8 98, CUDA cores 7.9e-8
 // 3710.
 //
 // Bound by latency: launch, one trip to HBM for the weights (and, at decode sizes, the code), two cluster barriers.
@@ -113,8 +113,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    float* part = reinterpret_cast<float*>(smem); // [NT][kSkPitch], after the ring; short chains: and what to subtract, the same
-    constexpr uint32_t kRest = NT * kSkPitch;
+    float* part = reinterpret_cast<float*>(smem); // [NT][kSkPitch], after the ring
     uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + SkSmem<NT>::kBytes);
     uint64_t* empty_bar = full_bar + kSkStages;
     uint64_t* acc_full = empty_bar + kSkStages;
@@ -244,12 +243,8 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
             for (uint32_t t = 0; t < kMine; ++t)
                 if (ready && m0 + c0 + t < p.m) {
                     const float whole = half2(plain[t / 2], t % 2);
-                    mine[t * kSkPitch] = whole;
-                    if constexpr (KAHAN) {
-                        if (isfinite(whole))
-                            mine[t * kSkPitch] = half2(sum[t / 2], t % 2);
-                        mine[kRest + t * kSkPitch] = isfinite(whole) ? half2(rest[t / 2], t % 2) : 0.0f;
-                    }
+                    mine[t * kSkPitch]
+                        = KAHAN && isfinite(whole) ? half2(sum[KAHAN ? t / 2 : 0], t % 2) - half2(rest[KAHAN ? t / 2 : 0], t % 2) : whole;
                 }
         } else {
             ready = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, abort_flag, p.err, ERR_SK_ACC_WAIT));
@@ -284,14 +279,6 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
         for (uint32_t s = 0; s < kSkMaxSplits; ++s)
             v[s] = s < splits ? *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, s) + t * kSkPitch + lane * 4)
                               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        float4 r[SUM == SUM_COMPENSATED ? kSkMaxSplits : 1]; // (all loads on their way before the sums)
-        if constexpr (SUM == SUM_COMPENSATED) {
-#pragma unroll
-            for (uint32_t s = 0; s < kSkMaxSplits; ++s)
-                r[s] = s < splits
-                    ? *reinterpret_cast<const float4*>(cluster.map_shared_rank(part, s) + kRest + t * kSkPitch + lane * 4)
-                    : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
         float a[4] = { v[0].x, v[0].y, v[0].z, v[0].w };
 #pragma unroll
         for (uint32_t s = 1; s < kSkMaxSplits; ++s) {
@@ -301,19 +288,18 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
             a[3] += v[s].w;
         }
         if constexpr (SUM == SUM_COMPENSATED) {
-            float sum[4] = { v[0].x, v[0].y, v[0].z, v[0].w }, rest[4] = {}, low[4] = { r[0].x, r[0].y, r[0].z, r[0].w };
+            float sum[4] = { v[0].x, v[0].y, v[0].z, v[0].w }, rest[4] = {};
 #pragma unroll
             for (uint32_t s = 1; s < kSkMaxSplits; ++s) {
-                const float x[4] = { v[s].x, v[s].y, v[s].z, v[s].w }, y[4] = { r[s].x, r[s].y, r[s].z, r[s].w };
+                const float x[4] = { v[s].x, v[s].y, v[s].z, v[s].w };
 #pragma unroll
                 for (uint32_t q = 0; q < 4; ++q) {
                     kahan(sum[q], rest[q], x[q]);
-                    low[q] += y[q];
                 }
             }
 #pragma unroll
             for (uint32_t q = 0; q < 4; ++q)
-                a[q] = isfinite(a[q]) ? sum[q] - (rest[q] + low[q]) : a[q];
+                a[q] = isfinite(a[q]) ? sum[q] - rest[q] : a[q];
         }
         const uint64_t at = static_cast<uint64_t>(m0 + t) * p.out_pitch + f;
         const uint32_t left = f < p.n ? min(4u, p.n - f) : 0u;
@@ -376,7 +362,7 @@ uint64_t splitk_tiles(const GemmProblem& g, uint32_t nt) { return (g.n + 127ull)
 
 // Rows of A per tile: the fewest MMA columns that hold them, 64 above that (128 x 4096 x 2048: 0.0125 ms against
 // 0.0145 with 128) as long as every tile can still be split. Compensated sums in smaller tiles as long as each can be split in
-// four: adding up is what they wait for (64 x 2048 x 512: 0.0054 ms, with 32 rows 0.0066).
+// four: adding up is what they wait for (33 x 2048 x 512: 0.0054 ms, with 32 rows 0.0066).
 uint32_t splitk_tile_rows(const GemmProblem& g)
 {
     if (g.epilogue == EPI_STORE_F32 && g.a_rows <= 64)
@@ -436,9 +422,11 @@ cudaError_t launch_gemm_splitk(const GemmProblem& g, cudaStream_t stream, const 
     sp.err = device_error_word();
     const uint32_t nt = splitk_choice(g);
     const uint64_t tiles = splitk_tiles(g, nt);
-    // as many splits as fit one CTA per SM, two k blocks each at least
+    // as many splits as fit one CTA per SM, two k blocks each at least; none for compensated sums of a short k, which a
+    // rounding per rank would leave further off (64 x 512 x 512: 6.4e-8, 5.8e-8 unsplit, on CUDA cores 6.2e-8)
     uint32_t splits = 1;
-    while (splits < kSkMaxSplits && 2 * splits * tiles <= device_sm_count() && 2 * (2 * splits) <= sp.k_blocks)
+    while (splits < kSkMaxSplits && 2 * splits * tiles <= device_sm_count() && 2 * (2 * splits) <= sp.k_blocks
+           && (splitk_sum(g, nt) != SUM_COMPENSATED || sp.k_blocks > 8))
         splits *= 2;
     sp.kb_per_split = (sp.k_blocks + splits - 1) / splits;
     CUtensorMap mb, ma;
