@@ -6,6 +6,7 @@
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <utility>
 
 namespace qs3 {
@@ -22,6 +23,72 @@ constexpr uint32_t kQwCluster = 16;
 constexpr uint32_t kQwThreads = 512;
 constexpr uint32_t kQwChunk = 512;   // k elements of one unit of pass 2: a 16-element block per lane
 constexpr uint32_t kQwPitch = 36;    // bytes per row of the scale staging (odd word count: no bank conflicts)
+
+__device__ __forceinline__ float global_scale_of(float amax) { return amax > 0.0f ? __fdiv_rn(amax, 6.0f * 448.0f) : 1.0f; }
+
+// Units of 128 tiled rows x kQwChunk elements of expert `e`, every `step`-th from `first`; a warp takes eight rows, a lane one
+// block of a row. `s_code` is 128 * kQwPitch bytes of shared memory.
+__device__ __forceinline__ void quantize_units(const __nv_bfloat16* __restrict__ w, uint32_t e, uint32_t rows, uint32_t k, float g,
+                                               uint8_t* __restrict__ packed, uint8_t* __restrict__ scale_linear,
+                                               uint8_t* __restrict__ scale_tiled, uint64_t tiled_bytes, int gated,
+                                               uint32_t first, uint32_t step, uint8_t* s_code)
+{
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t kb_per_row = k / 16, kgroups = k / 64;
+    const uint32_t k_chunks = (k + kQwChunk - 1) / kQwChunk;
+    const uint32_t units = (rows + 127) / 128 * k_chunks;
+    for (uint32_t unit = first; unit < units; unit += step) {
+        const uint32_t rb = unit / k_chunks, kc = unit % k_chunks;
+        const uint32_t kb = kc * (kQwChunk / 16) + lane;
+        constexpr uint32_t kRows = 128 / (kQwThreads / 32);
+#pragma unroll
+        for (uint32_t i0 = 0; i0 < kRows; i0 += 4) {
+            uint4 va[4], vb[4];
+            uint64_t grow[4];
+            bool live[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t tr = warp + (i0 + q) * (kQwThreads / 32); // row of the tile
+                const uint32_t row = gated ? rb * 64 + (tr & 63) + (tr >= 64 ? rows / 2 : 0) : rb * 128 + tr;
+                live[q] = row < rows && kb < kb_per_row;
+                grow[q] = static_cast<uint64_t>(e) * rows + row;
+                const uint4* p = reinterpret_cast<const uint4*>(w + grow[q] * k + static_cast<uint64_t>(kb) * 16);
+                va[q] = live[q] ? p[0] : make_uint4(0, 0, 0, 0);
+                vb[q] = live[q] ? p[1] : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                float x[16];
+                unpack16_bf16(va[q], vb[q], x);
+                const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
+                const float block_amax = bf16x2_max(bf16x2_amax(bf16x2_amax(zero, va[q]), vb[q]));
+                uint32_t lo, hi;
+                const uint8_t code = quantize_block16(x, block_amax, g, &lo, &hi);
+                if (live[q]) {
+                    *reinterpret_cast<uint2*>(packed + grow[q] * (k / 2) + static_cast<uint64_t>(kb) * 8) = make_uint2(lo, hi);
+                    if (scale_linear != nullptr)
+                        scale_linear[grow[q] * kb_per_row + kb] = code;
+                }
+                s_code[(warp + (i0 + q) * (kQwThreads / 32)) * kQwPitch + lane] = live[q] ? code : 0;
+            }
+        }
+        __syncthreads();
+        if (scale_tiled != nullptr && threadIdx.x < 256) {
+            // thread = (k group, lane of the scale tile): rows lane, lane + 32, lane + 64, lane + 96
+            const uint32_t kg = kc * (kQwChunk / 64) + warp;
+            if (kg < kgroups) {
+                uint32_t word[4];
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q)
+                    word[q] = *reinterpret_cast<const uint32_t*>(s_code + (lane + 32 * q) * kQwPitch + warp * 4);
+                *reinterpret_cast<uint4*>(scale_tiled + static_cast<uint64_t>(e) * tiled_bytes
+                                          + (static_cast<uint64_t>(rb) * kgroups + kg) * 512 + lane * 16)
+                    = make_uint4(word[0], word[1], word[2], word[3]);
+            }
+        }
+        __syncthreads(); // the staging is reused by the next unit
+    }
+}
 
 __global__ void __launch_bounds__(kQwThreads, 2)
 quantize_weight_kernel(const __nv_bfloat16* __restrict__ w, uint32_t rows, uint32_t k, float* __restrict__ global_scale,
@@ -76,65 +143,59 @@ quantize_weight_kernel(const __nv_bfloat16* __restrict__ w, uint32_t rows, uint3
 #pragma unroll
     for (uint32_t r = 0; r < kQwCluster; ++r)
         amax = fmaxf(amax, s_amax[r]);
-    const float g = amax > 0.0f ? __fdiv_rn(amax, 6.0f * 448.0f) : 1.0f;
+    const float g = global_scale_of(amax);
     if (rank == 0 && threadIdx.x == 0)
         global_scale[e] = g;
 
-    // pass 2: units of 128 tiled rows x kQwChunk elements; a warp takes eight rows, a lane one block of a row
-    const uint32_t kb_per_row = k / 16, kgroups = k / 64;
-    const uint32_t k_chunks = (k + kQwChunk - 1) / kQwChunk;
-    const uint32_t units = (rows + 127) / 128 * k_chunks;
-    for (uint32_t unit = rank; unit < units; unit += kQwCluster) {
-        const uint32_t rb = unit / k_chunks, kc = unit % k_chunks;
-        const uint32_t kb = kc * (kQwChunk / 16) + lane;
-        constexpr uint32_t kRows = 128 / (kQwThreads / 32);
+    // pass 2
+    quantize_units(w, e, rows, k, g, packed, scale_linear, scale_tiled, tiled_bytes, gated, rank, kQwCluster, s_code);
+}
+
+// The same over the whole grid, blockIdx.y = expert, for experts too few and too large for their clusters: bound by HBM, 1 x
+// 32768 x 2048 0.401 -> 0.063 ms (3.5 TB/s; the second pass comes from L2 where the weights fit it).
+// amax_bits[e] = bits of the expert's amax (non-negative floats order like their bit patterns), zeroed before.
+__global__ void __launch_bounds__(kQwThreads)
+expert_amax_kernel(const __nv_bfloat16* __restrict__ w, uint64_t per_expert, uint32_t* __restrict__ amax_bits)
+{
+    const uint4* src = reinterpret_cast<const uint4*>(w + blockIdx.y * per_expert);
+    const uint64_t vecs = per_expert / 8, step = static_cast<uint64_t>(gridDim.x) * kQwThreads;
+    __nv_bfloat162 m2 = __floats2bfloat162_rn(0.0f, 0.0f);
+    for (uint64_t i0 = static_cast<uint64_t>(blockIdx.x) * kQwThreads + threadIdx.x; i0 < vecs; i0 += 4 * step) {
+        uint4 v[4];
 #pragma unroll
-        for (uint32_t i0 = 0; i0 < kRows; i0 += 4) {
-            uint4 va[4], vb[4];
-            uint64_t grow[4];
-            bool live[4];
+        for (int q = 0; q < 4; ++q)
+            v[q] = i0 + q * step < vecs ? src[i0 + q * step] : make_uint4(0, 0, 0, 0);
 #pragma unroll
-            for (uint32_t q = 0; q < 4; ++q) {
-                const uint32_t tr = warp + (i0 + q) * (kQwThreads / 32); // row of the tile
-                const uint32_t row = gated ? rb * 64 + (tr & 63) + (tr >= 64 ? rows / 2 : 0) : rb * 128 + tr;
-                live[q] = row < rows && kb < kb_per_row;
-                grow[q] = static_cast<uint64_t>(e) * rows + row;
-                const uint4* p = reinterpret_cast<const uint4*>(w + grow[q] * k + static_cast<uint64_t>(kb) * 16);
-                va[q] = live[q] ? p[0] : make_uint4(0, 0, 0, 0);
-                vb[q] = live[q] ? p[1] : make_uint4(0, 0, 0, 0);
-            }
-#pragma unroll
-            for (uint32_t q = 0; q < 4; ++q) {
-                float x[16];
-                unpack16_bf16(va[q], vb[q], x);
-                const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
-                const float block_amax = bf16x2_max(bf16x2_amax(bf16x2_amax(zero, va[q]), vb[q]));
-                uint32_t lo, hi;
-                const uint8_t code = quantize_block16(x, block_amax, g, &lo, &hi);
-                if (live[q]) {
-                    *reinterpret_cast<uint2*>(packed + grow[q] * (k / 2) + static_cast<uint64_t>(kb) * 8) = make_uint2(lo, hi);
-                    if (scale_linear != nullptr)
-                        scale_linear[grow[q] * kb_per_row + kb] = code;
-                }
-                s_code[(warp + (i0 + q) * (kQwThreads / 32)) * kQwPitch + lane] = live[q] ? code : 0;
-            }
-        }
-        __syncthreads();
-        if (scale_tiled != nullptr && threadIdx.x < 256) {
-            // thread = (k group, lane of the scale tile): rows lane, lane + 32, lane + 64, lane + 96
-            const uint32_t kg = kc * (kQwChunk / 64) + warp;
-            if (kg < kgroups) {
-                uint32_t word[4];
-#pragma unroll
-                for (uint32_t q = 0; q < 4; ++q)
-                    word[q] = *reinterpret_cast<const uint32_t*>(s_code + (lane + 32 * q) * kQwPitch + warp * 4);
-                *reinterpret_cast<uint4*>(scale_tiled + static_cast<uint64_t>(e) * tiled_bytes
-                                          + (static_cast<uint64_t>(rb) * kgroups + kg) * 512 + lane * 16)
-                    = make_uint4(word[0], word[1], word[2], word[3]);
-            }
-        }
-        __syncthreads(); // the staging is reused by the next unit
+        for (int q = 0; q < 4; ++q)
+            m2 = bf16x2_amax(m2, v[q]);
     }
+    const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(bf16x2_max(m2)));
+    __shared__ uint32_t s_part[kQwThreads / 32];
+    if ((threadIdx.x & 31) == 0)
+        s_part[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const uint32_t all = __reduce_max_sync(0xffffffffu, threadIdx.x < kQwThreads / 32 ? s_part[threadIdx.x] : 0u);
+        if (threadIdx.x == 0)
+            atomicMax(amax_bits + blockIdx.y, all);
+    }
+}
+
+__global__ void finish_global_scale_kernel(float* scale, uint32_t experts)
+{
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < experts)
+        scale[e] = global_scale_of(scale[e]);
+}
+
+__global__ void __launch_bounds__(kQwThreads, 2)
+quantize_weight_flat_kernel(const __nv_bfloat16* __restrict__ w, uint32_t rows, uint32_t k, const float* __restrict__ global_scale,
+                            uint8_t* __restrict__ packed, uint8_t* __restrict__ scale_linear,
+                            uint8_t* __restrict__ scale_tiled, uint64_t tiled_bytes, int gated)
+{
+    __shared__ __align__(16) uint8_t s_code[128 * kQwPitch];
+    quantize_units(w, blockIdx.y, rows, k, global_scale[blockIdx.y], packed, scale_linear, scale_tiled, tiled_bytes, gated,
+                   blockIdx.x, gridDim.x, s_code);
 }
 
 // Activation rows to the declared (linear) layout; one thread per block.
@@ -249,6 +310,15 @@ uint32_t blocks_for(uint64_t total, uint32_t threads)
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Fewer blocks than SMs and more than a few microseconds' work for each: the whole grid per expert instead of a cluster,
+// which costs a memset and two launches. Experts x bytes of each, cluster / whole grid in us: 1 x 4 MB 14 / 13, 1 x 17
+// 44 / 14, 1 x 134 401 / 63, 4 x 8 25 / 18, 4 x 67 223 / 109, 8 x 8 37 / 27, 12 x 8 47 / 50, 16 x 34 278 / 254, 20 x 34
+// 302 / 330.
+bool quantize_flat_pays(uint64_t experts, uint64_t per_expert)
+{
+    return experts * kQwCluster < kSmCount && per_expert > (2u << 20);
+}
+
 } // namespace
 
 cudaError_t launch_nvfp4_quantize_rows(const __nv_bfloat16* x, uint32_t rows, uint32_t k, float global_scale,
@@ -323,7 +393,27 @@ qsfi_status qs3_nvfp4_quantize_weight(qsfi_context* ctx, const qs3_nvfp4_quantiz
         || (d->scale_tiled.data != nullptr && !aligned16(d->scale_tiled.data)))
         return set_invalid_arg(ctx, "NVFP4 quantisation buffers must be 16-byte aligned");
 
-    // rows of the last 128-row block that do not exist get scale 0 from the kernel itself
+    // rows of the last 128-row block that do not exist get scale 0 from the kernels themselves
+    const uint64_t per_expert = static_cast<uint64_t>(rows) * k;
+    if (quantize_flat_pays(static_cast<uint64_t>(experts), per_expert)) {
+        cudaStream_t st = ctx->stream;
+        const uint32_t want = 2 * kSmCount, e32 = static_cast<uint32_t>(experts);
+        const uint64_t units = (rows + 127) / 128 * ((k + kQwChunk - 1) / kQwChunk);
+        cudaError_t err = cudaMemsetAsync(d->global_scale.data, 0, sizeof(float) * e32, st);
+        if (err != cudaSuccess)
+            return set_cuda_error(ctx, err, "cudaMemsetAsync global_scale");
+        expert_amax_kernel<<<dim3((2 * want + e32 - 1) / e32, e32), kQwThreads, 0, st>>>(
+            static_cast<const __nv_bfloat16*>(d->weight.data), per_expert, static_cast<uint32_t*>(d->global_scale.data));
+        finish_global_scale_kernel<<<1, 32, 0, st>>>(static_cast<float*>(d->global_scale.data), e32);
+        quantize_weight_flat_kernel<<<dim3(static_cast<uint32_t>(std::min<uint64_t>(units, (want + e32 - 1) / e32)), e32),
+                                      kQwThreads, 0, st>>>(
+            static_cast<const __nv_bfloat16*>(d->weight.data), static_cast<uint32_t>(rows), static_cast<uint32_t>(k),
+            static_cast<const float*>(d->global_scale.data), static_cast<uint8_t*>(d->packed.data),
+            static_cast<uint8_t*>(d->scale_linear.data), static_cast<uint8_t*>(d->scale_tiled.data), tiled_bytes,
+            static_cast<int>(d->gated_rows != 0));
+        note_launch(3);
+        return set_cuda_error(ctx, cudaGetLastError(), "qs3_nvfp4_quantize_weight");
+    }
     static bool configured[64] = {};
     const int dev = ctx->device_ordinal;
     if (dev < 0 || dev >= 64 || !configured[dev]) {

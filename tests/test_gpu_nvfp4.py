@@ -54,9 +54,10 @@ def test_weight_quantiser_and_scale_tiling_are_bit_exact(ops, ctx, oracle, gated
 
 # one block, a k that is no multiple of the 512-element unit, a last row block that is not full, more experts
 # than clusters run at a time; many experts so small that most blocks of a cluster have nothing to read before they
-# exchange their maxima
+# exchange their maxima; few experts large enough for the whole grid each, a k tail and a row tail among them
 @pytest.mark.parametrize("e,rows,k,gated", [(1, 128, 64, True), (2, 384, 576, True), (3, 200, 832, False),
-                                            (40, 128, 1024, False), (600, 128, 64, True)])
+                                            (40, 128, 1024, False), (600, 128, 64, True), (2, 2048, 1088, True),
+                                            (1, 2056, 1024, False)])
 def test_weight_quantiser_edges(ops, ctx, oracle, e, rows, k, gated):
     rng = np.random.default_rng(rows + k)
     w = bf16(rng.standard_normal((e, rows, k), dtype=np.float32) * 0.02)
