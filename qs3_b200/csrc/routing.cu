@@ -305,7 +305,7 @@ route_place_kernel(const int32_t* __restrict__ ids, const float* __restrict__ we
 constexpr uint32_t kBlockSortThreads = 512;
 constexpr uint32_t kBlockSortWarps = kBlockSortThreads / 32;
 constexpr uint32_t kBlockSortRoutes = 2560; // 4000 routes: 0.0160 ms, with the three kernels 0.0148
-constexpr uint32_t kBlockSortExperts = 896; // the shared memory stays below 48 KB
+constexpr uint32_t kBlockSortExperts = 1024; // two per thread; the shared memory stays below 48 KB
 
 size_t block_sort_smem(uint32_t experts)
 {

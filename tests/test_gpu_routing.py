@@ -106,7 +106,8 @@ def _route_tables(ops, ids_np, w_np, experts, local_offset, local_experts):
     dict(t=2049, k=8, e=128), dict(t=300, k=3, e=4096, skew=True), dict(t=64, k=2, e=16, one_expert=True),
     dict(t=200, k=6, e=32, local=(8, 8)), dict(t=200, k=6, e=32, local=(24, 8)),
     # the one-block sort: its most routes and experts (two experts a thread), and one route more
-    dict(t=256, k=10, e=896), dict(t=2560, k=1, e=513), dict(t=2561, k=1, e=512), dict(t=100, k=3, e=897),
+    dict(t=256, k=10, e=896), dict(t=2560, k=1, e=513), dict(t=2561, k=1, e=512), dict(t=100, k=3, e=897), dict(t=250, k=8, e=1024),
+    dict(t=1, k=1, e=1025),
 ])
 def test_route_permutation_is_bit_exact(ops, oracle, case):
     t, k, e = case["t"], case["k"], case["e"]
