@@ -477,9 +477,10 @@ cudaError_t launch_gemm_dense_bf16(const GemmProblem& g, cudaStream_t stream, co
         }
     }
     const uint32_t tiles_n = (g.n + bn - 1) / bn;
-    // Several row tiles read a B panel from neighbouring SMs; over many rounds a chained start, which lets the next problem
-    // begin on the SMs that are done first, sets them out of step (156 rows x 151936 columns: 0.152 against 0.146 ms).
-    const UnchainedScope in_step(tiles_m > 1 && static_cast<uint64_t>(tiles_m) * tiles_n >= 4ull * device_sm_count());
+    // Several row tiles read a B panel from neighbouring SMs; over several rounds a chained start, which lets the next problem
+    // begin on the SMs that are done first, sets them out of step (156 rows x 2048 x 151936, 8 rounds: 0.152 against 0.146 ms;
+    // 300 x 4096 x 50000, 4 rounds: 0.129 against 0.125). In one or two it pays (1000 x 512 x 8192: 0.0114, unchained 0.0123).
+    const UnchainedScope in_step(tiles_m > 1 && static_cast<uint64_t>(tiles_m) * tiles_n > 3ull * device_sm_count());
     CUtensorMap ma, mb;
     if (!make_operand_map(&ma, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, kBM)
         || !make_operand_map(&mb, false, g.b, g.k, g.n, g.b_pitch_bytes, pair ? 128 : bn / 2)) {
