@@ -11,6 +11,7 @@ error classes: a failing call raises :class:`Qs3Error` carrying the
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import struct
 from dataclasses import dataclass
 
@@ -88,16 +89,17 @@ _MOE_FP8_EXECUTE_DESC = _layout(capi.MoeFp8ExecuteDesc, ("hidden", capi.DTYPE_FP
     ("down_weight", capi.DTYPE_FP8_E4M3), "down_weight_scale", "out", "workspace")
 
 
-def _layer_layout(gate_up_fp8, down_fp8):
+@functools.lru_cache(maxsize=None)
+def _layer_layout(gate_up_fp8, down_fp8, shared_gate_up_fp8, shared_down_fp8):
     weight = lambda n, fp8: ((f"{n}_weight", capi.DTYPE_FP8_E4M3 if fp8 else None),
                              (f"{n}_scale_tiled", None, 0) if fp8 else f"{n}_scale_tiled", f"{n}_global_scale")
     return _layout(capi.MoeLayerDesc, "hidden", "router_weight", "router_bias", *weight("gate_up", gate_up_fp8),
-                   *weight("down", down_fp8), *weight("shared_gate_up", False), *weight("shared_down", False),
+                   *weight("down", down_fp8), *weight("shared_gate_up", shared_gate_up_fp8),
+                   *weight("shared_down", shared_down_fp8),
                    "shared_gate_weight", "out", "topk_ids", "topk_weights", "router_logits", "workspace",
                    "hidden_packed", "hidden_scale_tiled", "residual_inout", "next_norm_weight")
 
 
-_MOE_LAYER_DESC = {(g, d): _layer_layout(g, d) for g in (False, True) for d in (False, True)}
 _QSCB_GEMM_DESC = _layout(capi.QscbGemmDesc, "x", "weight", "out")
 _RMSNORM_DESC = _layout(capi.RmsnormDesc, "x", "weight", "out")
 _FUSED_ADD_RMSNORM_DESC = _layout(capi.FusedAddRmsnormDesc, "x", "residual_inout", "weight", "out")
@@ -487,9 +489,12 @@ def moe_layer_execute(plan: MoePlan, hidden, router_weight, gate_up, down, out, 
     if shared is not None:
         sgu, sdn, shared_gate = _weight_tensors(shared.gate_up), _weight_tensors(shared.down), shared.gate_weight
         d.shared_intermediate_size = shared.intermediate_size
-    _fill(d, _MOE_LAYER_DESC[isinstance(gate_up, Fp8Weight), isinstance(down, Fp8Weight)], hidden, router_weight,
-          router_bias, *_weight_tensors(gate_up), *_weight_tensors(down), *sgu, *sdn, shared_gate, out, topk_ids,
-          topk_weights, router_logits, workspace, hidden_packed, hidden_scale_tiled, residual_inout, next_norm_weight)
+    layout = _layer_layout(isinstance(gate_up, Fp8Weight), isinstance(down, Fp8Weight),
+                           shared is not None and isinstance(shared.gate_up, Fp8Weight),
+                           shared is not None and isinstance(shared.down, Fp8Weight))
+    _fill(d, layout, hidden, router_weight, router_bias, *_weight_tensors(gate_up), *_weight_tensors(down), *sgu, *sdn,
+          shared_gate, out, topk_ids, topk_weights, router_logits, workspace, hidden_packed, hidden_scale_tiled,
+          residual_inout, next_norm_weight)
     d.score = score
     d.renormalize = 1 if renormalize else 0
     d.routed_scaling_factor = routed_scaling_factor

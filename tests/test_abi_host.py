@@ -370,3 +370,24 @@ def test_workspace_of_many_tokens_serves_fewer(lib, ctx, backend, experts, top_k
                 largest = n.value
     finally:
         lib.qsfi_moe_plan_destroy(plan)
+
+
+def test_fp8_layer_refuses_a_shared_expert_of_any_kind():
+    import torch
+
+    from qs3_b200 import ops
+    ctx = ops.Context(-1)
+    plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=4, hidden_size=256, intermediate_size=256, num_experts=2, top_k=1,
+                                              backend=capi.MOE_BACKEND_FP8_BLOCKSCALE))
+
+    def fp8(e, rows, k):
+        return ops.Fp8Weight(torch.zeros((e, rows, k), dtype=torch.uint8), torch.zeros((e, rows // 128, k // 128)))
+
+    def bf16(*shape):
+        return torch.zeros(shape, dtype=torch.bfloat16)
+    for gate_up, down in ((fp8(1, 512, 256), fp8(1, 256, 256)), (bf16(1, 512, 256), bf16(1, 256, 256))):
+        with pytest.raises(ops.Qs3Error, match="does not take a shared expert") as e:
+            ops.moe_layer_execute(plan, bf16(4, 256), bf16(2, 256), fp8(2, 512, 256), fp8(2, 256, 256), bf16(4, 256),
+                                  torch.zeros(1 << 20, dtype=torch.uint8),
+                                  shared=ops.SharedExpert(gate_up, down, bf16(1, 256), 256))
+        assert e.value.status == capi.STATUS_UNSUPPORTED
