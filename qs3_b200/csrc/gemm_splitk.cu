@@ -360,12 +360,14 @@ cudaError_t launch_splitk_instance(const CUtensorMap& mb, const CUtensorMap& ma,
 
 uint64_t splitk_tiles(const GemmProblem& g, uint32_t nt) { return (g.n + 127ull) / 128 * ((g.a_rows + nt - 1) / nt); }
 
+bool splitk_compensated(const GemmProblem& g) { return g.epilogue == EPI_STORE_F32 && g.a_rows <= 64; }
+
 // Rows of A per tile: the fewest MMA columns that hold them, 64 above that (128 x 4096 x 2048: 0.0125 ms against
 // 0.0145 with 128) as long as every tile can still be split. Compensated sums in smaller tiles as long as each can be split in
 // four: adding up is what they wait for (33 x 2048 x 512: 0.0054 ms, with 32 rows 0.0066).
 uint32_t splitk_tile_rows(const GemmProblem& g)
 {
-    if (g.epilogue == EPI_STORE_F32 && g.a_rows <= 64)
+    if (splitk_compensated(g))
         for (uint32_t nt = 16; nt < 64; nt *= 2)
             if (4 * splitk_tiles(g, nt) <= device_sm_count())
                 return nt;
@@ -379,7 +381,9 @@ SkSum splitk_sum(const GemmProblem& g, uint32_t nt)
 {
     if (g.epilogue != EPI_STORE_F32)
         return SUM_CHAIN;
-    return g.a_rows <= 64 ? SUM_COMPENSATED : nt == 64 && splitk_tiles(g, 128) <= 18 ? SUM_SHORT_CHAINS : SUM_CHAIN;
+    return splitk_compensated(g) ? SUM_COMPENSATED
+        : nt == 64 && splitk_tiles(g, 128) <= 18 ? SUM_SHORT_CHAINS
+                                                 : SUM_CHAIN;
 }
 
 // Tile rows of a problem that this kernel takes, 0: it does not. At least two CTAs per tile without exceeding one CTA
@@ -388,7 +392,7 @@ SkSum splitk_sum(const GemmProblem& g, uint32_t nt)
 uint32_t splitk_choice(const GemmProblem& g)
 {
     const uint32_t nt = splitk_tile_rows(g);
-    if (g.epilogue == EPI_STORE_F32 && g.a_rows <= 64) // whatever the tiles: for its sums
+    if (splitk_compensated(g) && g.k <= 4096) // whatever the tiles (longer sums were a chain: 64 x 7168 x 16384 0.071 / 0.056 ms)
         return nt;
     if (g.a_rows > 64 && g.k < 512) // nothing to split (1021 x 256 x 8: 0.0058 against 0.0046 ms in one tile per CTA)
         return 0;
