@@ -159,9 +159,11 @@ def test_f32_sums_of_few_rows(gemm, shape):
     assert torch.equal(again[~special], out[~special])
 
 
-# at most 128 rows and more than 148 units of features: weights streamed as the M side, unit height chosen for full
-# rounds (37889 = 148 * 256 + 1 features: the last unit holds one), every row tile height
-@pytest.mark.parametrize("rows,k,n", [(1, 64, 37889), (33, 200, 40000), (128, 128, 50007)])
+# at most 64 rows and at least 148 units of features: weights streamed as the M side, unit height chosen for full
+# rounds (37889 = 148 * 256 + 1 features: the last unit holds one), both row tile heights, rows in fours up to 48 and in
+# boxes of 32 beyond (the second partly past the end); 128 rows: the dense kernel with a width chosen the same way
+@pytest.mark.parametrize("rows,k,n", [(1, 64, 37889), (33, 200, 40000), (48, 64, 37633), (49, 128, 37700), (63, 200, 40000),
+                                      (64, 72, 50007), (128, 128, 50007)])
 def test_feature_streaming_kernel(gemm, rows, k, n):
     rng = np.random.default_rng(rows + k)
     x = bf16(rng.standard_normal((rows, k), dtype=np.float32))

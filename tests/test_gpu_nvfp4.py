@@ -83,6 +83,11 @@ def _quantise_all(ops, ctx, d, shared):
     return gu, dn, sh
 
 
+def _hot_bias(e):
+    """Router bias that sends a route of every token to expert 3."""
+    return np.where(np.arange(e) == 3, 10.0, 0.0).astype(np.float32)
+
+
 def _triple(q):
     return to_np(q.packed), to_np(q.scale_linear), to_np(q.global_scale)
 
@@ -234,17 +239,19 @@ def test_gate_and_up_rows_with_separate_global_scales(ops, ctx, oracle):
 
 
 @pytest.mark.parametrize("cfg", [
-    dict(t=16, h=512, e=64, k=4, i=256, s=256),                 # a few rows per expert, most experts empty
-    dict(t=128, h=2048, e=128, k=10, i=512, s=512, bias=True),  # decode batch of the prefill layer's shape
-    dict(t=40, h=256, e=4, k=2, i=256, s=0),                    # 80 routes on 4 experts: several 32-row tiles each
+    dict(t=16, h=512, e=64, k=4, i=256, s=256, rows=32),        # a few rows per expert, most experts empty
+    dict(t=100, h=2048, e=128, k=10, i=512, s=512, bias=True, rows=32),  # decode batch of the prefill layer's shape
+    dict(t=128, h=2048, e=128, k=10, i=512, s=512, bias=True, rows=64),
+    dict(t=40, h=256, e=16, k=2, i=256, s=0, hot=True, rows=32),         # an expert with 40 rows: two tiles
+    dict(t=40, h=256, e=4, k=2, i=256, s=0, rows=64),
 ])
 def test_decode_batches_take_the_swapped_operand_kernel(ops, ctx, oracle, cfg):
-    """With at most 16 routes per expert on average the plan pads expert segments to 32 rows and
-    the grouped GEMMs run with the weights as the M side of the MMA; same results as the oracle."""
+    """Up to 8 routes per expert on average the plan pads expert segments to 32 rows, up to 22 to 64, and the grouped GEMMs
+    run with the weights as the M side of the MMA (a shared expert joins them with 32-row tiles); same results as the
+    oracle."""
     t, h, e, k, i, s = cfg["t"], cfg["h"], cfg["e"], cfg["k"], cfg["i"], cfg["s"]
-    assert t * k <= 16 * e or e == 4
     d = make_moe_inputs(41, t, h, e, i, s)
-    bias = zipf_bias(e, d["rng"]) if cfg.get("bias") else None
+    bias = zipf_bias(e, d["rng"]) if cfg.get("bias") else _hot_bias(e) if cfg.get("hot") else None
     gu, dn, sh = _quantise_all(ops, ctx, d, bool(s))
     plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=t, hidden_size=h, intermediate_size=i,
                                               num_experts=e, top_k=k, backend=ops.capi.MOE_BACKEND_NVFP4))
@@ -258,6 +265,7 @@ def test_decode_batches_take_the_swapped_operand_kernel(ops, ctx, oracle, cfg):
                           act_global_scale=0.5, act2_global_scale=0.25, topk_ids=ids_t, topk_weights=w_t)
     torch.cuda.synchronize()
     assert ctx.read_device_error() == 0
+    assert tile_height(plan, ws, t) == cfg["rows"]
     hp, hs = oracle.nvfp4_quantize_act(d["hidden"], 0.5)
     shared_ref = dict(gu=_triple(sh[0]), d=_triple(sh[1]), gate_w=d["sh_gate"]) if s else None
     ref = oracle.moe_nvfp4(hp, hs, to_np(ids_t), to_np(w_t), _triple(gu), _triple(dn), act_global=0.5,
@@ -290,14 +298,19 @@ def test_swapped_operand_kernel_repeats(ops, ctx, oracle, t, e, k, h, i, rows):
 
 
 @pytest.mark.parametrize("cfg", [
-    dict(t=200, h=512, e=8, k=2, i=256, linear=False),   # 50 rows per expert: 64-row token tiles
-    dict(t=61, h=2048, e=2, k=2, i=512, linear=True),    # 61 rows: a full k panel, a row group that is not full
-    dict(t=33, h=2048, e=2, k=2, i=256, linear=True),    # one row in the second 32-row half
-    dict(t=90, h=256, e=8, k=2, i=256, linear=True, local=(3, 4)),
+    dict(t=60, h=512, e=8, k=2, i=256, linear=False, rows=64),
+    dict(t=61, h=2048, e=8, k=2, i=512, linear=True, hot=True, rows=64),  # 61 rows: a row group that is not full
+    dict(t=33, h=2048, e=4, k=2, i=256, linear=True, hot=True, rows=64),  # one row in the second 32-row half
+    dict(t=70, h=256, e=8, k=2, i=256, linear=False, hot=True, rows=64),  # a second tile of six rows
+    dict(t=40, h=256, e=8, k=2, i=256, linear=True, local=(3, 4), rows=64),
+    dict(t=200, h=512, e=8, k=2, i=256, linear=False, rows=128),
+    dict(t=61, h=2048, e=2, k=2, i=512, linear=True, rows=128),
+    dict(t=33, h=2048, e=2, k=2, i=256, linear=True, rows=128),
+    dict(t=90, h=256, e=8, k=2, i=256, linear=True, local=(3, 4), rows=128),
 ])
 def test_64_row_token_tiles(ops, ctx, oracle, cfg):
-    """More than a decode batch's rows per expert, still too few for 128-row tiles: token rows read in place
-    from tiled (layer call) and row-major (declared call) scales."""
+    """More than a decode batch's rows per expert, still too few for 128-row tiles (which the last ones take): token rows
+    read in place from tiled (layer call) and row-major (declared call) scales."""
     t, h, e, k, i = (cfg[n] for n in ("t", "h", "e", "k", "i"))
     off, le = cfg.get("local", (0, e))
     d = make_moe_inputs(43, t, h, e, i)
@@ -306,7 +319,8 @@ def test_64_row_token_tiles(ops, ctx, oracle, cfg):
     plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=t, hidden_size=h, intermediate_size=i, num_experts=e,
                                               top_k=k, local_expert_offset=off, local_num_experts=le,
                                               backend=ops.capi.MOE_BACKEND_NVFP4))
-    ids, w = oracle.router_topk(oracle.gemm_bf16(d["hidden"], d["router"], "f32"), k, 0, True, 1.0)
+    bias = _hot_bias(e) if cfg.get("hot") else np.zeros(e, np.float32)
+    ids, w = oracle.router_topk(oracle.gemm_bf16(d["hidden"], d["router"], "f32") + bias, k, 0, True, 1.0)
     out = torch.empty((t, h), dtype=torch.bfloat16, device="cuda")
     hp, hs = oracle.nvfp4_quantize_act(d["hidden"], 1.0)
     gu_ref, dn_ref = _triple(gu), _triple(dn)
@@ -322,31 +336,67 @@ def test_64_row_token_tiles(ops, ctx, oracle, cfg):
         ws = torch.zeros(plan.layer_workspace_size(t, 0), dtype=torch.uint8, device="cuda")
         ids_t = torch.empty((t, k), dtype=torch.int32, device="cuda")
         w_t = torch.empty((t, k), dtype=torch.float32, device="cuda")
-        ops.moe_layer_execute(plan, to_dev(d["hidden"]), to_dev(d["router"]), gu, dn, out, ws, topk_ids=ids_t,
-                              topk_weights=w_t)
+        ops.moe_layer_execute(plan, to_dev(d["hidden"]), to_dev(d["router"]), gu, dn, out, ws, router_bias=to_dev(bias),
+                              topk_ids=ids_t, topk_weights=w_t)
         ids, w = to_np(ids_t), to_np(w_t)
     torch.cuda.synchronize()
     assert ctx.read_device_error() == 0
+    assert tile_height(plan, ws, t) == cfg["rows"]
     _check(to_np(out), oracle.moe_nvfp4(hp, hs, ids, w, gu_ref, dn_ref, local_offset=off))
 
 
-@pytest.mark.parametrize("hot", [0.0, 1.0, 6.0])
-@pytest.mark.parametrize("t", [641, 700, 1280])
-def test_tile_height_chosen_by_the_sort(ops, ctx, oracle, t, hot):
-    """44 to 80 rows per expert: with even routing the sort lays out 64-row tiles, with a few hot experts 128-row ones."""
+def _chosen_height(ids, e):
+    """The sort's choice between 64- and 128-row tiles: fewer tiles, a 64-row one counted as 5 and a 128-row one as 7."""
+    counts = np.bincount(ids.ravel(), minlength=e)
+    return 64 if 5 * np.sum((counts + 63) // 64) < 7 * np.sum((counts + 127) // 128) else 128
+
+
+@pytest.mark.parametrize("t,hot,rows", [(641, 0.0, 64), (700, 0.0, 64), (1280, 0.0, 128), (641, 1.0, 64), (700, 1.0, 64),
+                                        (1280, 1.0, 64), (641, 6.0, 128), (700, 6.0, 128), (1200, 6.0, 128)])
+@pytest.mark.parametrize("s", [0, 256])
+def test_tile_height_chosen_by_the_sort(ops, ctx, oracle, t, hot, rows, s):
+    """40 to 80 rows per expert: 64-row tiles where they are not too many, alone and beside a shared expert (side stream)."""
     h, e, k, i = 256, 64, 4, 256
-    d = make_moe_inputs(47, t, h, e, i)
+    d = make_moe_inputs(47, t, h, e, i, s)
     bias = np.where(np.arange(e) < 6, hot, 0.0).astype(np.float32)
-    gu, dn, _ = _quantise_all(ops, ctx, d, False)
+    gu, dn, sh = _quantise_all(ops, ctx, d, bool(s))
     plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=t, hidden_size=h, intermediate_size=i, num_experts=e, top_k=k,
                                               backend=ops.capi.MOE_BACKEND_NVFP4))
     out = torch.empty((t, h), dtype=torch.bfloat16, device="cuda")
-    ws = torch.zeros(plan.layer_workspace_size(t, 0), dtype=torch.uint8, device="cuda")
+    ws = torch.zeros(plan.layer_workspace_size(t, s), dtype=torch.uint8, device="cuda")
     ids = torch.empty((t, k), dtype=torch.int32, device="cuda")
     w = torch.empty((t, k), dtype=torch.float32, device="cuda")
+    shared = ops.SharedExpert(sh[0], sh[1], to_dev(d["sh_gate"]), s) if s else None
     ops.moe_layer_execute(plan, to_dev(d["hidden"]), to_dev(d["router"]), gu, dn, out, ws, router_bias=to_dev(bias),
-                          topk_ids=ids, topk_weights=w)
+                          shared=shared, topk_ids=ids, topk_weights=w)
     torch.cuda.synchronize()
     assert ctx.read_device_error() == 0
+    assert _chosen_height(to_np(ids), e) == rows == tile_height(plan, ws, t)
     hp, hs = oracle.nvfp4_quantize_act(d["hidden"], 1.0)
-    _check(to_np(out), oracle.moe_nvfp4(hp, hs, to_np(ids), to_np(w), _triple(gu), _triple(dn)))
+    shared_ref = dict(gu=_triple(sh[0]), d=_triple(sh[1]), gate_w=d["sh_gate"]) if s else None
+    _check(to_np(out), oracle.moe_nvfp4(hp, hs, to_np(ids), to_np(w), _triple(gu), _triple(dn), shared=shared_ref,
+                                        hidden_bf16=d["hidden"]))
+
+
+@pytest.mark.parametrize("hot,rows", [(0.0, 64), (6.0, 128)])
+def test_tile_height_chosen_in_the_declared_call(ops, ctx, oracle, hot, rows):
+    t, h, e, k, i = 700, 256, 64, 4, 256
+    d = make_moe_inputs(53, t, h, e, i)
+    bias = np.where(np.arange(e) < 6, hot, 0.0).astype(np.float32)
+    ids, w = oracle.router_topk(oracle.gemm_bf16(d["hidden"], d["router"], "f32") + bias, k, 0, True, 1.0)
+
+    def quantise(x):  # this call has no gate_up global scale: quantised against 1, weights scaled up
+        q = oracle.nvfp4_quantize_act(bf16(f32(x) * 8.0).reshape(-1, x.shape[2]), 1.0)
+        return tuple(v.reshape(e, x.shape[1], -1) for v in q) + (np.ones(e, np.float32),)
+    gu, dn = quantise(d["gate_up"]), quantise(d["down"])
+    hp, hs = oracle.nvfp4_quantize_act(d["hidden"], 1.0)
+    plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=t, hidden_size=h, intermediate_size=i, num_experts=e, top_k=k,
+                                              backend=ops.capi.MOE_BACKEND_NVFP4))
+    ws = torch.zeros(plan.workspace_size(t), dtype=torch.uint8, device="cuda")
+    out = torch.empty((t, h), dtype=torch.bfloat16, device="cuda")
+    ops.moe_execute_nvfp4(plan, to_dev(hp), to_dev(hs), to_dev(ids), to_dev(w), *map(to_dev, gu[:2]), *map(to_dev, dn[:2]),
+                          out, ws)
+    torch.cuda.synchronize()
+    assert ctx.read_device_error() == 0
+    assert _chosen_height(ids, e) == rows == tile_height(plan, ws, t)
+    _check(to_np(out), oracle.moe_nvfp4(hp, hs, ids, w, gu, dn))
