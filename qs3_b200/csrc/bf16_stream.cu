@@ -1,6 +1,6 @@
 // Grouped bf16 GEMM of the routed experts: weight streaming with the operands swapped (weight rows are the M side of
 // the MMA, the expert's token tile of NT padded rows the N side). The plain variant also takes dense problems of at
-// most 128 rows with many features (the LM head of a decode batch): one row tile, no tables.
+// most 64 rows with many features (the LM head of a decode batch): one row tile, no tables.
 //
 //   unit   one token tile x 256 weight rows of its expert: gated: 128 gate rows and the 128 up rows of the same
 //          features (two accumulators with the same lanes, so SwiGLU needs no exchange); plain: 256 features
@@ -17,8 +17,7 @@
 // 0.072 -> 0.059 ms; 2048 tokens x 512 experts top-10 (intermediate 512): gate_up 0.443 -> 0.370 (5.8 TB/s), down
 // 0.222 -> 0.174 ms. The token rows of experts with few of them come by gather4 straight from the caller's tensor: a pass
 // that copied each route's row first, and the loads of rows that only pad a tile, cost 7 us of the 33-token layer (0.187 ->
-// 0.180 ms) and 56 us of the 2048-token one (0.680 -> 0.624). LM head, 2048 -> 151936: 1 row 0.151 -> 0.097 ms, 64 rows 0.116 -> 0.102, 128 rows 0.118 -> 0.113
-// (0.131 -> 0.123 in a loop of seconds, where the board's 1000 W hold the clocks at 1.55 GHz).
+// 0.180 ms) and 56 us of the 2048-token one (0.680 -> 0.624). LM head, 2048 -> 151936: 1 row 0.151 -> 0.097 ms, 64 rows 0.116 -> 0.102.
 #include "tcgen05.cuh"
 
 #include <algorithm>
@@ -398,7 +397,7 @@ cudaError_t launch_bf16_stream_gemm(const GemmProblem& g, cudaStream_t stream, c
     sp.out = static_cast<__nv_bfloat16*>(g.out);
     sp.out_pitch = g.out_pitch_elems;
     sp.err = device_error_word();
-    const uint32_t nt = g.tile_expert != nullptr ? g.tile_rows : g.a_rows <= 32 ? 32u : g.a_rows <= 64 ? 64u : 128u;
+    const uint32_t nt = g.tile_expert != nullptr ? g.tile_rows : g.a_rows <= 32 ? 32u : 64u;
     CUtensorMap mw, mx, mg;
     const uint64_t w_rows = static_cast<uint64_t>(g.groups) * sp.b_rows;
     const bool copy = g.row_tokens != nullptr && g.gathered != nullptr; // (as many rows as the tables have room for)

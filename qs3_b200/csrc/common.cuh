@@ -50,6 +50,9 @@ qsfi_status set_cuda_error(qsfi_context* ctx, cudaError_t err, const char* op);
 qsfi_status activate_context(qsfi_context* ctx);
 qsfi_status status_from_cuda(cudaError_t err);
 
+// SMs of the current device.
+uint32_t device_sm_count();
+
 // Device-side error word shared by the tensor-core kernels (one per device).
 uint32_t* device_error_word();
 

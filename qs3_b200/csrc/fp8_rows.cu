@@ -1,11 +1,10 @@
-// FP8 block-scaled grouped GEMM for experts with more rows than a decode batch gives them (fp8.cu has the kernel
+// FP8 block-scaled grouped GEMM for experts with more rows than a decode batch gives them (fp8_stream.cu has the kernel
 // for those): token rows are the M side of the MMA again.
 //
 // A 128 x 256 output tile per unit: 128 token rows of one expert x 256 weight rows (gated: 128 gate rows and the
-// 128 up rows of the same features). The block scales are promoted outside the tensor core as in the decode
+// 128 up rows of the same features). The block scales are promoted outside the tensor core as in the streaming
 // kernel, but with tokens in the tensor-memory lanes a lane needs ONE factor per k block and 128-feature block
-// (x_scale[token] * w_scale[block]), so promoting an element is a single FMA without any shared-memory operand:
-// 128 x 256 partials cost eight warps about 300 cycles against the ~690 cycles of their four MMAs.
+// (x_scale[token] * w_scale[block]), so promoting an element is a single FMA without any shared-memory operand.
 //
 //   persistent  one CTA per SM, every gridDim.x-th (token tile, feature block) unit: the CTAs of a round hold
 //               neighbouring units, so a token tile and the weights of an expert with several tiles are read by
@@ -16,8 +15,8 @@
 //   warps       0-7 promotion and epilogue (lane quadrant warp % 4, column half warp / 4), 8 producer, 9 MMA, 10-11
 //               note writers: they follow the tables and fetch the scales of the next unit
 //
-// Bound by operand delivery (48 KB per k block for 128 x 256 x 128 products) and the hand-over of the two buffers:
-// 0.76 us per k block, 0.63 without the loads. 4096 tokens x 128 experts top-8 (hidden 2048, intermediate 768):
+// Bound by the promotion (one tensor-memory read in flight per warp) and the hand-over of the two buffers: 0.76 us per k
+// block, 0.63 without the loads, against 0.35 (690 cycles) for its four MMAs. 4096 tokens x 128 experts top-8 (hidden 2048, intermediate 768):
 // gate_up 0.800 -> 0.156 ms, down 0.238 -> 0.087 ms against the decode kernel on 32-row tiles, which streamed every
 // weight through shared memory once per 32 rows. With the scales and tables fetched between the units by the
 // promotion warps, and whole token tiles moved for a few rows: layer of 1024 tokens 0.200 -> 0.177 ms, 2048 0.257 ->
@@ -64,7 +63,6 @@ struct Fp8RowsParams {
     const int32_t* row_tokens; // NULL: scales by padded row; else dense row -> row of x_scale
     const int32_t* indptr;     // with row_tokens: segment starts, dense and padded
     const int32_t* pad_indptr;
-    int tables_ready;      // the tables were complete before the predecessor in the stream started
     void* out;             // gated: e4m3 codes [rows, n]; plain: written through map_o
     float* out_scale;      // gated: f32 [rows, n / 128]
     uint32_t* err;
@@ -145,7 +143,8 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const bool early = p.tables_ready && (warp == 8 || warp >= 10); // weights and tables are complete: no need to wait for them
+    // weights and tables (the predecessor is the gather or the gate_up GEMM) are complete: who reads only them need not wait
+    const bool early = warp == 8 || warp >= 10;
     if (!early)
         chain_begin();
 
@@ -169,7 +168,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     if (warp >= 10) {
         // -------------------------------------------------------- note writers --
         const uint32_t i = threadIdx.x - 320;
-        bool waited = !early;
+        bool waited = false;
         for (uint32_t u = blockIdx.x; u < total; u += gridDim.x, next_note()) {
             const uint32_t tile = u / p.units_per_tile, nb = u % p.units_per_tile;
             const int row0 = p.tile_row0[tile], nrows = p.tile_nrows[tile], expert = p.tile_expert[tile];
@@ -215,21 +214,19 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         uint32_t s = 0, ph = 0;
         bool ok = true;
         uint32_t ahead = 0; // k blocks of the first unit whose weights are on their way already
-        if (early) {
-            if (blockIdx.x < total && lane == 0) {
-                const uint32_t tile = blockIdx.x / p.units_per_tile, nb = blockIdx.x % p.units_per_tile;
-                const int b0 = p.tile_expert[tile] * static_cast<int>(p.b_rows);
-                for (; ahead < min(kStages, p.k_blocks); ++ahead) {
-                    uint8_t* sa = smem + ahead * kFrStageBytes;
-                    const int c0 = static_cast<int>(ahead * 128);
-                    mbar_expect_tx_only(&full_bar[ahead], 2 * kTileBytes);
-                    tma_load_2d(sa + kTileBytes, &map_w, &full_bar[ahead], c0, b0 + static_cast<int>(b_block(nb) * 128));
-                    tma_load_2d(sa + 2 * kTileBytes, &map_w, &full_bar[ahead], c0, b0 + static_cast<int>(b_block2(nb) * 128));
-                }
+        if (blockIdx.x < total && lane == 0) {
+            const uint32_t tile = blockIdx.x / p.units_per_tile, nb = blockIdx.x % p.units_per_tile;
+            const int b0 = p.tile_expert[tile] * static_cast<int>(p.b_rows);
+            for (; ahead < min(kStages, p.k_blocks); ++ahead) {
+                uint8_t* sa = smem + ahead * kFrStageBytes;
+                const int c0 = static_cast<int>(ahead * 128);
+                mbar_expect_tx_only(&full_bar[ahead], 2 * kTileBytes);
+                tma_load_2d(sa + kTileBytes, &map_w, &full_bar[ahead], c0, b0 + static_cast<int>(b_block(nb) * 128));
+                tma_load_2d(sa + 2 * kTileBytes, &map_w, &full_bar[ahead], c0, b0 + static_cast<int>(b_block2(nb) * 128));
             }
-            __syncwarp();
-            chain_begin();
         }
+        __syncwarp();
+        chain_begin();
         for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x, next_note(), ahead = 0) {
             ok = __all_sync(0xffffffffu, mbar_wait<true>(&note_full[nt], nph, abort_flag, p.err, ERR_FR_NOTE_FULL_WAIT));
             if (!ok)
@@ -475,10 +472,14 @@ cudaError_t launch_fp8_rows_gemm(const Fp8Gemm& g, cudaStream_t stream, const ch
     fp.row_tokens = g.row_tokens;
     fp.indptr = g.indptr;
     fp.pad_indptr = g.pad_indptr;
-    fp.tables_ready = g.tables_ready;
     fp.out = g.out;
     fp.out_scale = g.out_scale;
     fp.err = device_error_word();
+    if (!g.tables_ready) {
+        if (why != nullptr)
+            *why = "the FP8 GEMM of 128-row tiles reads its tables before its predecessor ends";
+        return cudaErrorNotSupported;
+    }
     CUtensorMap mx, mw, mo;
     bool ok = make_operand_map(&mx, true, g.row_tokens != nullptr ? g.gathered : g.x, g.k, g.out_rows, g.k, kFrBox)
         && make_operand_map(&mw, true, g.w, g.k, static_cast<uint64_t>(g.groups) * fp.b_rows, g.k, 128);

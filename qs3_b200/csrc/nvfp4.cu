@@ -1,6 +1,6 @@
 // NVFP4 quantisers and scale-layout kernels: weight preparation (the layout the
 // upstream weight loader never produced, src/weight_loader.rs:33-66), activation
-// quantisation fused with the token gather, and linear -> tiled scale re-tiling.
+// quantisation in token order, the gather of its codes by expert, and linear -> tiled scale re-tiling.
 #include "common.cuh"
 #include "nvfp4.cuh"
 

@@ -301,7 +301,7 @@ route_place_kernel(const int32_t* __restrict__ ids, const float* __restrict__ we
 // ---- counting sort of up to kBlockSortRoutes routes by one block ------------------------------------------------
 // Everything stays in shared memory between the routes' local expert ids (`ids`, -1: not local) and the tables: per-warp
 // histograms by match_any, prefix over the warps, one packed block scan (routes in the low, tiles in the high
-// half), stable placement. Stable in route index, like the three kernels of routing.cu, whose tables these are.
+// half), stable placement. Stable in route index, like the three kernels above, whose tables these are.
 constexpr uint32_t kBlockSortThreads = 512;
 constexpr uint32_t kBlockSortWarps = kBlockSortThreads / 32;
 constexpr uint32_t kBlockSortRoutes = 2560; // 4000 routes: 0.0160 ms, with the three kernels 0.0148
@@ -1380,9 +1380,9 @@ cudaError_t launch_combine(const CombineParams& p, cudaStream_t stream)
 {
     if (p.num_tokens == 0)
         return cudaSuccess;
-    // one block per token while the blocks fit two waves (600 tokens: 0.0137 against 0.0142 ms, 1021: 0.019 against
-    // 0.014)
-    const bool spread = p.num_tokens <= 592;
+    // one block per token while the blocks fit two waves of two per SM (600 tokens: 0.0137 against 0.0142 ms, 1021: 0.019
+    // against 0.014)
+    const bool spread = p.num_tokens <= 4 * device_sm_count();
     const uint32_t blocks = spread ? p.num_tokens : (p.num_tokens + 3) / 4;
     if (p.residual != nullptr) {
         if (p.hidden_size > kCombineThreads * 8 || p.skip_empty)

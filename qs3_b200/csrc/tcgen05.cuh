@@ -55,7 +55,6 @@ struct TcParams {
 } // namespace tc
 bool make_operand_map(CUtensorMap* map, bool bytes_type, const void* base, uint64_t inner_elems, uint64_t rows,
                       uint64_t pitch_bytes, uint32_t box_rows);
-uint32_t device_sm_count();
 namespace tc {
 
 // ---- PTX wrappers -------------------------------------------------------------------
