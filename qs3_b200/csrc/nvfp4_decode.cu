@@ -542,8 +542,9 @@ uint32_t nvfp4_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uin
 
 uint32_t nvfp4_alt_tile_rows(uint32_t routes, uint32_t experts, uint32_t hidden, uint32_t inter)
 {
-    // Beyond that it depends on the skew, which only the sort sees; from 80 routes per expert on (kAltMaxRoutes) 64-row
-    // tiles never win.
+    // Beyond that it depends on the skew, which only the sort sees, by the cost of a tile of either kind (routing.cu: both
+    // measured at 512 experts of 2048 x 512). From 80 routes per expert on (kAltMaxRoutes) evenly routed experts have one
+    // 128-row tile for two of 64 or two for three, and those come out ahead.
     return nvfp4_tile_rows(22 * experts, experts, hidden, inter) == 64 && routes > 22 * experts
             && route_sort_can_choose(routes, experts)
         ? 64u
