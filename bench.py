@@ -793,7 +793,7 @@ GATE_UP_KERNEL = ("gemm_tc_astat_kernel<gated, swiglu_nvfp4>" if os.environ.get(
                   else "gemm_nvfp4_pair_kernel<gated, swiglu_nvfp4>")
 TRAFFIC_RATIO = {"gemm_nvfp4_pair_kernel<gated, swiglu_nvfp4>": 1.07,
                  "gemm_tc_astat_kernel<gated, swiglu_nvfp4>": 1.02,
-                 "gemm_nvfp4_swap_kernel<gated>": 1.00,
+                 "gemm_nvfp4_swap_kernel<gated>": 1.01,
                  "gemm_fp8_stream_kernel<gated>": 1.00}
 
 
