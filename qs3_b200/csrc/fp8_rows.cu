@@ -12,15 +12,18 @@
 //   smem        ring of stages: A 128 x 128 B, B 256 x 128 B; plain: + four 16-KB boxes staging the bf16 tile for
 //               TMA stores
 //   TMEM        two 256-column buffers: k block i + 1 is multiplied while k block i is promoted
-//   warps       0-7 promotion and epilogue (lane quadrant warp % 4, column half warp / 4), 8 producer, 9 MMA, 10-11
+//   warps       0-15 promotion and epilogue (lane quadrant warp % 4, column quarter warp / 4), 16 producer, 17 MMA, 18-19
 //               note writers: they follow the tables and fetch the scales of the next unit
 //
-// Bound by the promotion (one tensor-memory read in flight per warp) and the hand-over of the two buffers: 0.76 us per k
-// block, 0.63 without the loads, against 0.35 (690 cycles) for its four MMAs. 4096 tokens x 128 experts top-8 (hidden 2048, intermediate 768):
-// gate_up 0.800 -> 0.156 ms, down 0.238 -> 0.087 ms against the decode kernel on 32-row tiles, which streamed every
-// weight through shared memory once per 32 rows. With the scales and tables fetched between the units by the
-// promotion warps, and whole token tiles moved for a few rows: layer of 1024 tokens 0.200 -> 0.177 ms, 2048 0.257 ->
-// 0.222 (4096: 0.377 -> 0.366).
+// Bound by operand delivery: a k block is 48 KB, which an SM takes in at 75 GB/s, 0.64 us, against 0.35 (690 cycles) for
+// its four MMAs. 4096 tokens x 128 experts top-8 (hidden 2048, intermediate 768): gate_up 0.800 -> 0.156 ms, down 0.238
+// -> 0.087 ms against the decode kernel on 32-row tiles, which streamed every weight through shared memory once per 32
+// rows. With the scales and tables fetched between the units by the promotion warps, and whole token tiles moved for a
+// few rows: layer of 1024 tokens 0.200 -> 0.177 ms, 2048 0.257 -> 0.222 (4096: 0.377 -> 0.366). Eight promotion warps
+// with one tensor-memory read in flight each and an FMA per element took as long as the operands; four warps per
+// scheduler, two elements per FMA and the buffer given back as soon as it is read: 1024 tokens 0.180 -> 0.174 ms, 2048
+// 0.218 -> 0.211, 4096 0.380 -> 0.374. (Pairs of CTAs with half of B each, 32 KB a k block, were slower, 0.341 -> 0.389 ms:
+// a buffer's way to the other CTA and back takes longer than the two buffers cover.)
 #include "tcgen05.cuh"
 
 #include <algorithm>
@@ -30,7 +33,8 @@ namespace {
 
 using namespace tc;
 
-constexpr int kFrThreads = 384;
+constexpr uint32_t kFrAdders = 16;                    // promotion warps
+constexpr int kFrThreads = (kFrAdders + 4) * 32;
 constexpr uint32_t kFrN = 256;                        // weight rows per unit = MMA N
 constexpr uint32_t kFrStageBytes = 3 * kTileBytes;    // A tile + two B tiles
 constexpr uint32_t kFrMaxStages = 4;
@@ -80,16 +84,20 @@ template <bool GATED> struct FrSmem {
     static constexpr uint32_t kStaging = kStages * kFrStageBytes;               // plain: four 16-KB boxes
     static constexpr uint32_t kScales = kStaging + (GATED ? 0 : 4 * kTileBytes); // [notes][k blocks][128] f32
     static constexpr uint32_t kNotes = kScales + kScaleRows * 128 * 4;
-    static constexpr uint32_t kAmax = kNotes + kFrMaxNotes * static_cast<uint32_t>(sizeof(FrNote)); // gated: [2][128] f32
-    static constexpr uint32_t kBars = kAmax + (GATED ? 1024 : 0);
+    static constexpr uint32_t kAmax = kNotes + kFrMaxNotes * static_cast<uint32_t>(sizeof(FrNote)); // gated: [4][128] f32
+    static constexpr uint32_t kBars = kAmax + (GATED ? 2048 : 0);
     static constexpr uint32_t kBytes = kBars + (2 * kFrMaxStages + 4 + 2 * kFrMaxNotes) * 8 + 16;
 };
 
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t* r)
+// a * b + c of two values, each as fmaf
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c)
 {
-    tc_ld16(taddr, r);
-    tc_ld16(taddr + 16, r + 16);
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
+__device__ __forceinline__ uint64_t pack2(uint32_t a, uint32_t b) { return static_cast<uint64_t>(b) << 32 | a; }
+__device__ __forceinline__ float part2(uint64_t v, uint32_t i) { return __uint_as_float(static_cast<uint32_t>(v >> (32 * i))); }
 
 template <bool GATED>
 __global__ void __launch_bounds__(kFrThreads, 1)
@@ -123,17 +131,17 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 8); // one arrival per promotion warp
+            mbar_init(&acc_empty[b], kFrAdders); // one arrival per promotion warp
         }
         for (uint32_t b = 0; b < kFrMaxNotes; ++b) {
-            mbar_init(&note_full[b], 2);  // the two writers
-            mbar_init(&note_empty[b], 9); // promotion warps, producer
+            mbar_init(&note_full[b], 2);              // the two writers
+            mbar_init(&note_empty[b], kFrAdders + 1); // promotion warps, producer
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 9) {
+    if (warp == kFrAdders + 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(kFrTmemCols)
                      : "memory");
@@ -144,7 +152,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // weights and tables (the predecessor is the gather or the gate_up GEMM) are complete: who reads only them need not wait
-    const bool early = warp == 8 || warp >= 10;
+    const bool early = warp == kFrAdders || warp >= kFrAdders + 2;
     if (!early)
         chain_begin();
 
@@ -165,9 +173,9 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     const auto b_block = [&](uint32_t nb) { return GATED ? nb : 2 * nb; };
     const auto b_block2 = [&](uint32_t nb) { return GATED ? p.num_fb + nb : min(2 * nb + 1, p.num_fb - 1); };
 
-    if (warp >= 10) {
+    if (warp >= kFrAdders + 2) {
         // -------------------------------------------------------- note writers --
-        const uint32_t i = threadIdx.x - 320;
+        const uint32_t i = threadIdx.x - (kFrAdders + 2) * 32, w = i / 32;
         bool waited = false;
         for (uint32_t u = blockIdx.x; u < total; u += gridDim.x, next_note()) {
             const uint32_t tile = u / p.units_per_tile, nb = u % p.units_per_tile;
@@ -191,9 +199,9 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
                 for (uint32_t kb = 0; kb < p.k_blocks; ++kb)
                     cp_async4(s_xs + (nt * p.k_blocks + kb) * 128 + i + 64 * h, xs + kb);
             }
-            const uint32_t fb = warp == 10 ? b_block(nb) : b_block2(nb);
+            const uint32_t fb = w == 0 ? b_block(nb) : b_block2(nb);
             if (lane < p.k_blocks)
-                cp_async4(&note.ws[warp - 10][lane],
+                cp_async4(&note.ws[w][lane],
                           p.w_scale + (static_cast<size_t>(expert) * (p.b_rows / 128) + fb) * p.k_blocks + lane);
             if (i == 0) {
                 note.row0 = row0;
@@ -208,7 +216,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         }
         if (!waited)
             chain_begin();
-    } else if (warp == 8) {
+    } else if (warp == kFrAdders) {
         // ------------------------------------------------------------ producer --
         // Lane 0 loads the weight tiles, lane j box j of the token tile: boxes past its last row are not moved.
         uint32_t s = 0, ph = 0;
@@ -259,7 +267,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
                 }
             }
         }
-    } else if (warp == 9) {
+    } else if (warp == kFrAdders + 1) {
         // ---------------------------------------------------------- MMA issuer --
         if (lane == 0) {
             // M = 128 tokens, N = 256 weight rows, e4m3 x e4m3 -> f32, both operands K-major
@@ -293,11 +301,11 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
         }
     } else {
         // ------------------------------------------------- promotion, epilogue --
-        const uint32_t quad = warp & 3, half = warp >> 2;
+        const uint32_t quad = warp & 3, part = warp >> 2;
         const uint32_t r = quad * 32 + lane; // token row of the tile = TMEM lane
-        // columns of this warp: gated 64 gate columns and the 64 up columns of the same features; plain 128 columns
-        const uint32_t col0 = (quad * 32) << 16 | (GATED ? half * 64 : half * 128);
-        constexpr uint32_t kSecond = GATED ? 128 : 64; // distance of the second 64 columns
+        // columns of this warp: gated 32 gate columns and the 32 up columns of the same features; plain 64 columns
+        const uint32_t col0 = (quad * 32) << 16 | part * (GATED ? 32 : 64);
+        constexpr uint32_t kSecond = GATED ? 128 : 32; // distance of the second 32 columns
         uint32_t b = 0, bph = 0;
         bool ok = true;
         for (uint32_t u = blockIdx.x; u < total; u += gridDim.x, next_note()) {
@@ -307,17 +315,16 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
             const uint32_t row0 = static_cast<uint32_t>(note.row0);
             const int nrows = note.nrows;
             const bool live = static_cast<int>(quad * 32) < nrows; // whole warps without a valid row only count along
-            const uint32_t fb = GATED ? nb : 2 * nb + half;
             const float* xs = s_xs + nt * p.k_blocks * 128 + r;
-            const float* ws = note.ws[GATED ? 0 : half];
-            float acc[2][64];
+            const float* ws = note.ws[GATED ? 0 : part / 2];
+            uint64_t acc[2][16]; // two neighbouring columns each
 #pragma unroll
-            for (int i = 0; i < 64; ++i)
-                acc[0][i] = acc[1][i] = 0.0f;
+            for (int i = 0; i < 16; ++i)
+                acc[0][i] = acc[1][i] = 0;
             for (uint32_t kb = 0; kb < p.k_blocks && ok; ++kb) {
-                const float x = xs[kb * 128];
-                const float s0 = ws[kb] * x;
-                const float s1 = GATED ? note.ws[1][kb] * x : s0;
+                const uint32_t x = __float_as_uint(xs[kb * 128]);
+                const uint32_t f0 = __float_as_uint(ws[kb] * __uint_as_float(x));
+                const uint32_t f1 = GATED ? __float_as_uint(note.ws[1][kb] * __uint_as_float(x)) : f0;
                 ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[b], bph, abort_flag, p.err, ERR_FR_ACC_FULL_WAIT));
                 if (!ok)
                     break;
@@ -326,19 +333,24 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
                     const uint32_t src = tmem_base + b * kFrN + col0;
 #pragma unroll
                     for (uint32_t c = 0; c < 4; ++c) {
-                        uint32_t v[32];
-                        tc_ld32(src + (c >> 1) * kSecond + (c & 1) * 32, v);
+                        uint32_t v[16];
+                        tc_ld16(src + (c >> 1) * kSecond + (c & 1) * 16, v);
                         tc_ld_wait();
+                        if (c == 3) { // the buffer has been read: the next k block may be multiplied into it
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0)
+                                mbar_arrive(&acc_empty[b]);
+                        }
+                        const uint64_t f = (c >> 1) ? pack2(f1, f1) : pack2(f0, f0);
 #pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            acc[c >> 1][(c & 1) * 32 + i]
-                                = fmaf(__uint_as_float(v[i]), (c >> 1) ? s1 : s0, acc[c >> 1][(c & 1) * 32 + i]);
+                        for (int i = 0; i < 8; ++i)
+                            acc[c >> 1][(c & 1) * 8 + i]
+                                = fma2(pack2(v[2 * i], v[2 * i + 1]), f, acc[c >> 1][(c & 1) * 8 + i]);
                     }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0)
+                } else if (lane == 0) {
                     mbar_arrive(&acc_empty[b]);
+                }
                 b ^= 1;
                 bph ^= b == 0;
             }
@@ -346,72 +358,74 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
             if (lane == 0)
                 mbar_arrive(&note_empty[nt]);
             if constexpr (GATED) {
-                // SwiGLU, then one e4m3 scale per token and 128 features: the two halves of a row are in the two
+                // SwiGLU, then one e4m3 scale per token and 128 features: the four quarters of a row are in the four
                 // warps of a lane quadrant, which exchange their maxima
+                float act[32];
                 float amax = 0.0f;
 #pragma unroll
-                for (int i = 0; i < 64; ++i) {
-                    const float g = acc[0][i];
-                    acc[0][i] = __fdividef(g, 1.0f + __expf(-g)) * acc[1][i];
-                    amax = fmaxf(amax, fabsf(acc[0][i]));
+                for (int i = 0; i < 32; ++i) {
+                    const float g = part2(acc[0][i / 2], i % 2);
+                    act[i] = __fdividef(g, 1.0f + __expf(-g)) * part2(acc[1][i / 2], i % 2);
+                    amax = fmaxf(amax, fabsf(act[i]));
                 }
-                s_amax[half * 128 + r] = amax;
-                ok = group_all(1 + quad, 64, ok); // the two warps stop together
+                s_amax[part * 128 + r] = amax;
+                ok = group_all(1 + quad, 128, ok); // the four warps stop together
                 if (!ok)
                     break;
-                amax = fmaxf(amax, s_amax[(half ^ 1) * 128 + r]);
-                asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory"); // both have read: the next unit may write
+#pragma unroll
+                for (uint32_t q = 0; q < 4; ++q)
+                    amax = fmaxf(amax, s_amax[q * 128 + r]);
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + quad) : "memory"); // all have read: the next unit may write
                 if (static_cast<int>(r) < nrows) {
                     const float sc = fmaxf(__fdiv_rn(amax, 448.0f), 1.0e-30f);
                     const float inv = __fdiv_rn(1.0f, sc);
-                    uint8_t* out = static_cast<uint8_t*>(p.out) + static_cast<size_t>(row0 + r) * p.n + fb * 128 + half * 64;
+                    uint8_t* out = static_cast<uint8_t*>(p.out) + static_cast<size_t>(row0 + r) * p.n + nb * 128 + part * 32;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
+                    for (int i = 0; i < 2; ++i) {
                         uint32_t w[4];
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             w[j] = 0;
 #pragma unroll
                             for (int q = 0; q < 4; ++q)
-                                w[j] |= static_cast<uint32_t>(f32_to_e4m3_sat(__fmul_rn(acc[0][16 * i + 4 * j + q], inv)))
+                                w[j] |= static_cast<uint32_t>(f32_to_e4m3_sat(__fmul_rn(act[16 * i + 4 * j + q], inv)))
                                     << (8 * q);
                         }
                         reinterpret_cast<uint4*>(out)[i] = make_uint4(w[0], w[1], w[2], w[3]);
                     }
-                    if (half == 0)
-                        p.out_scale[static_cast<size_t>(row0 + r) * p.num_fb + fb] = sc;
+                    if (part == 0)
+                        p.out_scale[static_cast<size_t>(row0 + r) * p.num_fb + nb] = sc;
                 }
             } else {
-                // bf16 rows through shared memory and TMA stores (64-column boxes). Every row of the tile is written:
-                // rows past the segment end are padding rows of the same expert.
-                ok = group_all(1 + half, 128, ok);
+                // bf16 rows through shared memory and TMA stores (a 64-column box for the four warps of a part). Every
+                // row of the tile is written: rows past the segment end are padding rows of the same expert.
+                ok = group_all(1 + part, 128, ok);
                 if (!ok)
                     break;
                 const bool issuer = quad == 0 && lane == 0;
-                if (issuer) // the half's previous boxes have left the staging
+                if (issuer) // the part's previous box has left the staging
                     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");
+                uint8_t* row_smem = staging + part * kTileBytes + r * 128;
 #pragma unroll
-                for (uint32_t c = 0; c < 2; ++c) {
-                    uint8_t* row_smem = staging + (half * 2 + c) * kTileBytes + r * 128;
+                for (uint32_t q = 0; q < 8; ++q) {
+                    uint32_t w[4];
 #pragma unroll
-                    for (uint32_t q = 0; q < 8; ++q) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-                            w[i] = pack_bf16x2(acc[c][8 * q + 2 * i], acc[c][8 * q + 2 * i + 1]);
-                        *reinterpret_cast<uint4*>(row_smem + ((q ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+                    for (uint32_t i = 0; i < 4; ++i) {
+                        const uint64_t v = acc[q / 4][(q % 4) * 4 + i];
+                        w[i] = pack_bf16x2(part2(v, 0), part2(v, 1));
                     }
+                    *reinterpret_cast<uint4*>(row_smem + ((q ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("bar.sync %0, 128;" ::"r"(1 + half) : "memory");
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + part) : "memory");
                 if (issuer) {
-                    const uint32_t n0 = nb * kFrN + half * 128;
-                    for (uint32_t c = 0; c < 2 && n0 < p.n; ++c)
+                    const uint32_t n0 = nb * kFrN + part * 64;
+                    if (n0 < p.n)
                         asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
                                          reinterpret_cast<uint64_t>(&map_o)),
-                                     "r"(smem_u32(staging + (half * 2 + c) * kTileBytes)),
-                                     "r"(static_cast<int>(n0 + c * 64)), "r"(static_cast<int>(row0))
+                                     "r"(smem_u32(staging + part * kTileBytes)), "r"(static_cast<int>(n0)),
+                                     "r"(static_cast<int>(row0))
                                      : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
@@ -424,7 +438,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
     // ---- teardown ----
     tc_fence_before();
     __syncthreads();
-    if (warp == 9) {
+    if (warp == kFrAdders + 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kFrTmemCols)
                      : "memory");
