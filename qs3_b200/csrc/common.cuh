@@ -23,15 +23,20 @@ struct qsfi_context {
     size_t host_int_workspace_bytes;
     uint64_t scratch_generation;
     qsfi_error_info last_error;
+    // (after upstream's fields) Side stream of the whole-layer call, taken on first use: the token quantiser and the shared
+    // expert run there beside the router chain. Each context has its own, so that calls of several contexts on one plan
+    // do not meet in an event.
+    struct qs3_side_stream* side;
+};
+
+struct qs3_side_stream {
+    int device;
+    cudaStream_t stream;
+    cudaEvent_t fork, quant, shared; // fork / join with the context's stream
 };
 
 struct qsfi_moe_plan {
     qsfi_moe_plan_desc desc;
-    // Side stream of the whole-layer call, created on first use: the token quantiser and the
-    // shared expert run there beside the router chain (fork / join with the three events).
-    mutable cudaStream_t side_stream = nullptr;
-    mutable cudaEvent_t ev_fork = nullptr, ev_quant = nullptr, ev_shared = nullptr;
-    mutable int side_state = 0; // 0 not tried, 1 ready, -1 unavailable
 };
 
 namespace qs3 {
@@ -49,6 +54,9 @@ qsfi_status set_unsupported(qsfi_context* ctx, const char* fmt, ...);
 qsfi_status set_cuda_error(qsfi_context* ctx, cudaError_t err, const char* op);
 qsfi_status activate_context(qsfi_context* ctx);
 qsfi_status status_from_cuda(cudaError_t err);
+
+// The context's side stream, NULL when none can be had; given back with the context.
+qs3_side_stream* side_stream(qsfi_context* ctx);
 
 // SMs of the current device.
 uint32_t device_sm_count();

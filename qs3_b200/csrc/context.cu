@@ -6,11 +6,85 @@
 #include <atomic>
 #include <mutex>
 #include <new>
+#include <vector>
 
 namespace qs3 {
 
 thread_local bool launch_unchained = false;
 
+namespace {
+
+// Side streams of destroyed contexts, for the next ones: creating one and its events takes about 0.2 ms, which the first
+// layer call of every context paid.
+constexpr size_t kSideStreamsKept = 8;
+std::mutex side_mutex;
+std::vector<qs3_side_stream*>& side_free = *new std::vector<qs3_side_stream*>; // (contexts may outlive static objects)
+
+void destroy_side(qs3_side_stream* s)
+{
+    for (cudaEvent_t ev : { s->fork, s->quant, s->shared })
+        if (ev != nullptr)
+            cudaEventDestroy(ev);
+    if (s->stream != nullptr)
+        cudaStreamDestroy(s->stream);
+    delete s;
+}
+
+void give_back(qs3_side_stream* s)
+{
+    if (s == nullptr)
+        return;
+    // (what still runs on it only delays its next user; one that is being captured is of no use to others)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+        std::lock_guard<std::mutex> lock(side_mutex);
+        if (side_free.size() < kSideStreamsKept) {
+            side_free.push_back(s);
+            return;
+        }
+    }
+    destroy_side(s);
+}
+
+} // namespace
+
+qs3_side_stream* side_stream(qsfi_context* ctx)
+{
+    int device = -1;
+    if (cudaGetDevice(&device) != cudaSuccess)
+        return nullptr;
+    if (ctx->side != nullptr) {
+        if (ctx->side->device == device)
+            return ctx->side;
+        give_back(ctx->side); // a context of no device of its own, used on another one
+        ctx->side = nullptr;
+    }
+    {
+        std::lock_guard<std::mutex> lock(side_mutex);
+        for (auto it = side_free.begin(); it != side_free.end(); ++it)
+            if ((*it)->device == device) {
+                ctx->side = *it;
+                side_free.erase(it);
+                return ctx->side;
+            }
+    }
+    qs3_side_stream* s = new (std::nothrow) qs3_side_stream {};
+    if (s == nullptr)
+        return nullptr;
+    s->device = device;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed; // the first call of a context may be one that is captured
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const bool made = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) == cudaSuccess
+        && cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess
+        && cudaEventCreateWithFlags(&s->quant, cudaEventDisableTiming) == cudaSuccess
+        && cudaEventCreateWithFlags(&s->shared, cudaEventDisableTiming) == cudaSuccess;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (made)
+        return ctx->side = s;
+    cudaGetLastError();
+    destroy_side(s);
+    return nullptr;
+}
 
 void clear_error(qsfi_error_info* err)
 {
@@ -199,6 +273,7 @@ void qsfi_context_destroy(qsfi_context* ctx)
             cudaSetDevice(ctx->device_ordinal);
         cudaFree(ctx->float_workspace);
     }
+    give_back(ctx->side);
     delete ctx;
 }
 

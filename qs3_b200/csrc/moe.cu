@@ -350,23 +350,6 @@ qsfi_status gemm_or_error(qsfi_context* ctx, const GemmProblem& g, const char* o
     return gemm_on_stream(ctx, g, op, ctx->stream);
 }
 
-// Side stream and events of a plan (see qsfi_moe_plan); false when they cannot be had, in
-// which case the layer runs on the context's stream alone.
-bool plan_side_stream(const qsfi_moe_plan* plan)
-{
-    if (plan->side_state == 0) {
-        plan->side_state = -1;
-        if (cudaStreamCreateWithFlags(&plan->side_stream, cudaStreamNonBlocking) == cudaSuccess
-            && cudaEventCreateWithFlags(&plan->ev_fork, cudaEventDisableTiming) == cudaSuccess
-            && cudaEventCreateWithFlags(&plan->ev_quant, cudaEventDisableTiming) == cudaSuccess
-            && cudaEventCreateWithFlags(&plan->ev_shared, cudaEventDisableTiming) == cudaSuccess)
-            plan->side_state = 1;
-        else
-            cudaGetLastError();
-    }
-    return plan->side_state == 1;
-}
-
 // Routed experts in bf16 on rows already described by `rt`:
 // gate_up GEMM + SwiGLU -> down GEMM. Leaves Y2 in w.y2.
 qsfi_status run_routed_bf16(qsfi_context* ctx, const qsfi_moe_plan_desc& p, const Bf16Workspace& w,
@@ -726,16 +709,6 @@ qsfi_status qsfi_moe_plan_create(qsfi_context* ctx, const qsfi_moe_plan_desc* de
 
 void qsfi_moe_plan_destroy(qsfi_moe_plan* plan)
 {
-    if (plan == nullptr)
-        return;
-    if (plan->ev_fork != nullptr)
-        cudaEventDestroy(plan->ev_fork);
-    if (plan->ev_quant != nullptr)
-        cudaEventDestroy(plan->ev_quant);
-    if (plan->ev_shared != nullptr)
-        cudaEventDestroy(plan->ev_shared);
-    if (plan->side_stream != nullptr)
-        cudaStreamDestroy(plan->side_stream);
     delete plan;
 }
 
@@ -1260,34 +1233,67 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
         s2.group_scale = static_cast<const float*>(d->shared_down_global_scale.data);
         return gemm_on_stream(ctx, s2, "NVFP4 shared down GEMM", stream);
     };
+    const auto run_shared_bf16 = [&](cudaStream_t stream) -> qsfi_status {
+        // shared expert, src/model.rs:2174-2228, with SiLU*mul fused into the first GEMM
+        stage_mark(st, STAGE_SHARED);
+        GemmProblem s1 {};
+        s1.a = hidden;
+        s1.a_rows = d->num_tokens;
+        s1.a_pitch_bytes = static_cast<uint64_t>(h) * 2;
+        s1.b = d->shared_gate_up_weight.data;
+        s1.b_pitch_bytes = static_cast<uint64_t>(h) * 2;
+        s1.groups = 1;
+        s1.n = is;
+        s1.k = p.hidden_size;
+        s1.gated = 1;
+        s1.epilogue = EPI_SWIGLU_BF16;
+        s1.out = x.sh_act;
+        s1.out_pitch_elems = is;
+        const qsfi_status st1 = gemm_on_stream(ctx, s1, "shared gate_up GEMM", stream);
+        if (st1 != QSFI_STATUS_OK)
+            return st1;
+        GemmProblem s2 {};
+        s2.a = x.sh_act;
+        s2.a_rows = d->num_tokens;
+        s2.a_pitch_bytes = static_cast<uint64_t>(is) * 2;
+        s2.b = d->shared_down_weight.data;
+        s2.b_pitch_bytes = static_cast<uint64_t>(is) * 2;
+        s2.groups = 1;
+        s2.n = p.hidden_size;
+        s2.k = is;
+        s2.epilogue = EPI_STORE_BF16;
+        s2.out = x.sh_out;
+        s2.out_pitch_elems = p.hidden_size;
+        return gemm_on_stream(ctx, s2, "shared down GEMM", stream);
+    };
     // With a shared expert, the token quantiser and the shared expert's two GEMMs depend on
-    // the tokens only: they run on the plan's side stream beside the router chain (logits
+    // the tokens only: they run on the context's side stream beside the router chain (logits
     // GEMM, top-k, sort) and join the main stream where their results are consumed. The
     // per-stage recorder needs one timeline, so a profiled call stays on the main stream.
     // (In a decode batch it joins the grouped GEMMs instead and the quantiser runs beside the sort: no fork.)
     const bool merged = rt.shared_rows != 0;
-    const bool fork = nvfp4 && shared && !merged && !stage_recording() && plan_side_stream(plan);
+    const bool fork = shared && !merged && !stage_recording() && side_stream(ctx) != nullptr;
     if (fork) {
-        cudaStream_t side = plan->side_stream;
-        cudaError_t ferr = cudaEventRecord(plan->ev_fork, st);
+        cudaStream_t side = ctx->side->stream;
+        cudaError_t ferr = cudaEventRecord(ctx->side->fork, st);
         if (ferr == cudaSuccess)
-            ferr = cudaStreamWaitEvent(side, plan->ev_fork, 0);
-        if (ferr == cudaSuccess && !prequant)
+            ferr = cudaStreamWaitEvent(side, ctx->side->fork, 0);
+        if (ferr == cudaSuccess && nvfp4 && !prequant)
             ferr = launch_nvfp4_quantize_rows(hidden, d->num_tokens, p.hidden_size, d->act_global_scale, x.sh_xq,
                                               x.sh_xq_sf, side);
-        if (ferr == cudaSuccess)
-            ferr = cudaEventRecord(plan->ev_quant, side);
+        if (ferr == cudaSuccess && nvfp4)
+            ferr = cudaEventRecord(ctx->side->quant, side);
         if (ferr != cudaSuccess)
-            return set_cuda_error(ctx, ferr, "NVFP4 MoE layer fork");
+            return set_cuda_error(ctx, ferr, "MoE layer fork");
         {
             UnchainedScope alone;
-            status = run_shared_nvfp4(side);
+            status = nvfp4 ? run_shared_nvfp4(side) : run_shared_bf16(side);
         }
         if (status != QSFI_STATUS_OK)
             return status;
-        ferr = cudaEventRecord(plan->ev_shared, side);
+        ferr = cudaEventRecord(ctx->side->shared, side);
         if (ferr != cudaSuccess)
-            return set_cuda_error(ctx, ferr, "NVFP4 MoE layer fork");
+            return set_cuda_error(ctx, ferr, "MoE layer fork");
     }
 
     stage_mark(st, STAGE_ROUTER_GEMM);
@@ -1354,7 +1360,7 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
         //    or with the routed rows read in place
         stage_mark(st, STAGE_GATHER);
         if (fork)
-            err = cudaStreamWaitEvent(st, plan->ev_quant, 0);
+            err = cudaStreamWaitEvent(st, ctx->side->quant, 0);
         else if (!prequant && !small_tiles)
             err = launch_nvfp4_quantize_rows(hidden, d->num_tokens, p.hidden_size, d->act_global_scale, x.sh_xq,
                                              x.sh_xq_sf, st);
@@ -1386,7 +1392,7 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
             // 7. shared expert
             stage_mark(st, STAGE_SHARED);
             if (fork) {
-                err = cudaStreamWaitEvent(st, plan->ev_shared, 0);
+                err = cudaStreamWaitEvent(st, ctx->side->shared, 0);
                 if (err != cudaSuccess)
                     return set_cuda_error(ctx, err, "NVFP4 MoE layer join");
             } else {
@@ -1404,37 +1410,12 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
             return status;
         y2 = wb.y2;
         if (shared) {
-            // shared expert, src/model.rs:2174-2228, with SiLU*mul fused into the first GEMM
-            stage_mark(st, STAGE_SHARED);
-            GemmProblem s1 {};
-            s1.a = hidden;
-            s1.a_rows = d->num_tokens;
-            s1.a_pitch_bytes = static_cast<uint64_t>(h) * 2;
-            s1.b = d->shared_gate_up_weight.data;
-            s1.b_pitch_bytes = static_cast<uint64_t>(h) * 2;
-            s1.groups = 1;
-            s1.n = is;
-            s1.k = p.hidden_size;
-            s1.gated = 1;
-            s1.epilogue = EPI_SWIGLU_BF16;
-            s1.out = x.sh_act;
-            s1.out_pitch_elems = is;
-            status = gemm_or_error(ctx, s1, "shared gate_up GEMM");
-            if (status != QSFI_STATUS_OK)
-                return status;
-            GemmProblem s2 {};
-            s2.a = x.sh_act;
-            s2.a_rows = d->num_tokens;
-            s2.a_pitch_bytes = static_cast<uint64_t>(is) * 2;
-            s2.b = d->shared_down_weight.data;
-            s2.b_pitch_bytes = static_cast<uint64_t>(is) * 2;
-            s2.groups = 1;
-            s2.n = p.hidden_size;
-            s2.k = is;
-            s2.epilogue = EPI_STORE_BF16;
-            s2.out = x.sh_out;
-            s2.out_pitch_elems = p.hidden_size;
-            status = gemm_or_error(ctx, s2, "shared down GEMM");
+            if (fork)
+                err = cudaStreamWaitEvent(st, ctx->side->shared, 0);
+            if (err != cudaSuccess)
+                return set_cuda_error(ctx, err, "MoE layer join");
+            if (!fork)
+                status = run_shared_bf16(st);
             if (status != QSFI_STATUS_OK)
                 return status;
         }
@@ -1540,7 +1521,7 @@ qsfi_status qs3_moe_ep_route(qsfi_context* ctx, const qsfi_moe_plan* plan, const
         || (quantise && !aligned16(d->hidden_packed.data)))
         return set_invalid_arg(ctx, "MoE tensors must be 16-byte aligned");
 
-    // The token quantiser depends on the tokens only: it runs on the plan's side stream beside the
+    // The token quantiser depends on the tokens only: it runs on the context's side stream beside the
     // router GEMM and the top-k and joins before the call returns its stream to the caller.
     qs3_nvfp4_quantize_act_desc q {};
     q.x = d->hidden;
@@ -1549,19 +1530,19 @@ qsfi_status qs3_moe_ep_route(qsfi_context* ctx, const qsfi_moe_plan* plan, const
     q.global_scale = d->act_global_scale;
     q.rows = d->num_tokens;
     cudaStream_t main_stream = ctx->stream;
-    const bool fork = quantise && !stage_recording() && plan_side_stream(plan);
+    const bool fork = quantise && !stage_recording() && side_stream(ctx) != nullptr;
     if (fork) {
-        cudaError_t ferr = cudaEventRecord(plan->ev_fork, main_stream);
+        cudaError_t ferr = cudaEventRecord(ctx->side->fork, main_stream);
         if (ferr == cudaSuccess)
-            ferr = cudaStreamWaitEvent(plan->side_stream, plan->ev_fork, 0);
+            ferr = cudaStreamWaitEvent(ctx->side->stream, ctx->side->fork, 0);
         if (ferr != cudaSuccess)
             return set_cuda_error(ctx, ferr, "MoE route fork");
-        ctx->stream = plan->side_stream;
+        ctx->stream = ctx->side->stream;
         status = qs3_nvfp4_quantize_act(ctx, &q);
         ctx->stream = main_stream;
         if (status != QSFI_STATUS_OK)
             return status;
-        ferr = cudaEventRecord(plan->ev_quant, plan->side_stream);
+        ferr = cudaEventRecord(ctx->side->quant, ctx->side->stream);
         if (ferr != cudaSuccess)
             return set_cuda_error(ctx, ferr, "MoE route fork");
     }
@@ -1595,7 +1576,7 @@ qsfi_status qs3_moe_ep_route(qsfi_context* ctx, const qsfi_moe_plan* plan, const
     if (err != cudaSuccess)
         return set_cuda_error(ctx, err, "MoE routing");
     if (fork)
-        return set_cuda_error(ctx, cudaStreamWaitEvent(main_stream, plan->ev_quant, 0), "MoE route join");
+        return set_cuda_error(ctx, cudaStreamWaitEvent(main_stream, ctx->side->quant, 0), "MoE route join");
     if (quantise)
         return qs3_nvfp4_quantize_act(ctx, &q);
     return QSFI_STATUS_OK;
