@@ -148,6 +148,16 @@ struct TokenQuant {
 cudaError_t launch_route_sort(const int32_t* topk_ids, const float* topk_weights, uint32_t routes,
                               uint32_t top_k, uint32_t local_offset, uint32_t experts,
                               const RouteTables& rt, cudaStream_t stream, const TokenQuant* quant = nullptr);
+// Router scores of a few tokens, for kernels that route them on the way.
+struct RouterParams {
+    const float* logits; // [num_tokens, num_experts]
+    const float* bias;   // optional [num_experts]
+    int32_t* ids;        // out [num_tokens, top_k]
+    float* weights;
+    uint32_t num_tokens, num_experts;
+    int sigmoid_score, renormalize;
+    float scaling;
+};
 // Top-k and sort of a small batch in one launch (f32 logits).
 bool router_sort_supported(uint32_t num_tokens, uint32_t num_experts, uint32_t top_k, uint32_t experts);
 cudaError_t launch_router_sort(const float* logits, const float* bias, int32_t* ids, float* weights, uint32_t num_tokens,
@@ -381,6 +391,40 @@ struct Fp8Gemm {
 cudaError_t launch_fp8_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** why_unsupported);
 cudaError_t launch_fp8_stream_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** why_unsupported);
 cudaError_t launch_fp8_rows_gemm(const Fp8Gemm& g, cudaStream_t stream, const char** why_unsupported);
+
+// ---- experts of a handful of tokens as matrix-vector products (gemv.cu) ----
+enum GemvFormat { GEMV_BF16 = 0, GEMV_FP8 = 1, GEMV_NVFP4 = 2 };
+struct GemvWeights { // of the routed experts, or of the shared one
+    const uint8_t *gate_up, *down;               // [experts, 2 inter, hidden], [experts, hidden, inter]
+    const void *gate_up_scale, *down_scale;      // NVFP4: tiled block scales; FP8: f32 block scales
+    const float *gate_up_global, *gate_up_global_up, *down_global; // NVFP4, optional
+};
+struct GemvParams {
+    const __nv_bfloat16* hidden;  // [tokens, hidden]
+    const uint8_t* hidden_packed; // NVFP4: the tokens' codes, with scales tiled by token row (NULL: quantised here)
+    const uint8_t* hidden_sf;
+    const int32_t* ids;           // [tokens, top_k], given or written by the router of the same launch
+    const float* weights;
+    uint32_t num_tokens, hidden_size, inter, top_k, experts, local_offset;
+    uint32_t shared;              // 1: a shared expert of the same intermediate size follows the routed slots
+    int early;                    // the predecessor in the stream writes nothing but the logits
+    GemvWeights routed, shared_weights;
+    float act_global, act2_global;
+    uint8_t* act;                 // [tokens * slots, inter]: bf16, f32 (FP8), e2m1 codes (NVFP4) with act_scale [.., inter / 16]
+    uint8_t* act_scale;
+    const __nv_bfloat16* shared_gate; // [hidden]
+    __nv_bfloat16* out;           // [tokens, hidden]; or, with y2, the slots' rows, to be combined by a later launch:
+    __nv_bfloat16* y2;            // row route_prows[route], the shared expert's in y2_shared at *shared_row0 (NULL: 0) + token
+    __nv_bfloat16* y2_shared;
+    const int32_t *route_prows, *shared_row0;
+};
+// Bytes of `act` for that many tokens.
+inline size_t gemv_act_bytes(int fmt, size_t rows, size_t inter) { return rows * inter * (fmt == GEMV_BF16 ? 2 : fmt == GEMV_FP8 ? 4 : 1) / (fmt == GEMV_NVFP4 ? 2 : 1); }
+// Whether such a call is taken. `num_experts`: of the router.
+bool gemv_supported(int fmt, uint32_t num_tokens, uint32_t top_k, uint32_t num_experts, uint32_t experts, uint32_t hidden,
+                    uint32_t inter, uint32_t shared_inter);
+// `router`: routes the tokens first (NULL: ids and weights are given). Fills the tables of `rt` on the way.
+cudaError_t launch_gemv(int fmt, const GemvParams& p, const RouterParams* router, const RouteTables& rt, cudaStream_t stream);
 
 // ---- device helpers ---------------------------------------------------------------
 #ifdef __CUDACC__

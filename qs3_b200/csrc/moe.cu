@@ -829,6 +829,23 @@ qsfi_status qsfi_moe_execute_bf16(qsfi_context* ctx, const qsfi_moe_plan* plan,
         return status;
     Bf16Workspace w = carve_bf16(static_cast<char*>(desc->workspace.data), p, desc->num_tokens);
     const uint32_t routes = desc->num_tokens * p.top_k;
+    if (gemv_supported(GEMV_BF16, desc->num_tokens, p.top_k, 1, p.local_num_experts, p.hidden_size, p.intermediate_size, 0)) {
+        GemvParams g {};
+        g.hidden = static_cast<const __nv_bfloat16*>(desc->hidden.data);
+        g.ids = static_cast<const int32_t*>(desc->topk_ids.data);
+        g.weights = static_cast<const float*>(desc->topk_weights.data);
+        g.num_tokens = desc->num_tokens;
+        g.hidden_size = p.hidden_size;
+        g.inter = p.intermediate_size;
+        g.top_k = p.top_k;
+        g.experts = p.local_num_experts;
+        g.local_offset = p.local_expert_offset;
+        g.routed.gate_up = static_cast<const uint8_t*>(desc->gate_up_weight.data);
+        g.routed.down = static_cast<const uint8_t*>(desc->down_weight.data);
+        g.act = reinterpret_cast<uint8_t*>(w.act);
+        g.out = static_cast<__nv_bfloat16*>(desc->out.data);
+        return set_cuda_error(ctx, launch_gemv(GEMV_BF16, g, nullptr, w.rt, ctx->stream), "qsfi_moe_execute_bf16");
+    }
     cudaError_t err = launch_route_sort(static_cast<const int32_t*>(desc->topk_ids.data),
                                         static_cast<const float*>(desc->topk_weights.data), routes, p.top_k,
                                         p.local_expert_offset, p.local_num_experts, w.rt, ctx->stream);
@@ -1272,7 +1289,19 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
     // per-stage recorder needs one timeline, so a profiled call stays on the main stream.
     // (In a decode batch it joins the grouped GEMMs instead and the quantiser runs beside the sort: no fork.)
     const bool merged = rt.shared_rows != 0;
-    const bool fork = shared && !merged && !stage_recording() && side_stream(ctx) != nullptr;
+    // a handful of tokens: no grouped GEMMs (a shared expert of another size, or beside larger NVFP4 tiles, keeps them)
+    const int gemv_fmt = nvfp4 ? GEMV_NVFP4 : fp8 ? GEMV_FP8 : GEMV_BF16;
+    const size_t slot_rows = routes + (shared ? d->num_tokens : 0u);
+    const size_t act_room = static_cast<size_t>(rt.max_pad_rows) * p.intermediate_size / (nvfp4 ? 2 : 1) * (nvfp4 || fp8 ? 1 : 2);
+    // (a result in the tokens' place would be written while other blocks still read them for the gate)
+    const char *xb = static_cast<const char*>(d->hidden.data), *ob = static_cast<const char*>(d->out.data);
+    const ptrdiff_t token_bytes = static_cast<ptrdiff_t>(t * h * 2);
+    const bool in_place = xb < ob + token_bytes && ob < xb + token_bytes;
+    const bool gemv = (!nvfp4 || !shared || merged) && !(shared && in_place)
+        && gemv_supported(gemv_fmt, d->num_tokens, p.top_k, p.num_experts, p.local_num_experts, p.hidden_size,
+                          p.intermediate_size, shared ? is : 0)
+        && gemv_act_bytes(gemv_fmt, slot_rows, p.intermediate_size) <= act_room;
+    const bool fork = shared && !merged && !gemv && !stage_recording() && side_stream(ctx) != nullptr;
     if (fork) {
         cudaStream_t side = ctx->side->stream;
         cudaError_t ferr = cudaEventRecord(ctx->side->fork, st);
@@ -1326,7 +1355,59 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
                     x.sh_xq, x.sh_xq_sf };
     const TokenQuant* quant = small_tiles && !fork && !prequant ? &tq : nullptr;
     cudaError_t err = cudaSuccess;
-    if (router_sort_supported(d->num_tokens, p.num_experts, p.top_k, p.local_num_experts)) { // 2. and 3. in one launch
+    if (gemv) { // 2. to 8. of a handful of tokens
+        stage_mark(st, STAGE_GATE_UP_GEMM);
+        GemvParams g {};
+        g.hidden = hidden;
+        g.hidden_packed = prequant ? x.sh_xq : nullptr;
+        g.hidden_sf = x.sh_xq_sf;
+        g.ids = ids;
+        g.weights = wts;
+        g.num_tokens = d->num_tokens;
+        g.hidden_size = p.hidden_size;
+        g.inter = p.intermediate_size;
+        g.top_k = p.top_k;
+        g.experts = p.local_num_experts;
+        g.local_offset = p.local_expert_offset;
+        g.shared = shared;
+        g.early = 1;
+        g.routed.gate_up = static_cast<const uint8_t*>(d->gate_up_weight.data);
+        g.routed.down = static_cast<const uint8_t*>(d->down_weight.data);
+        g.routed.gate_up_scale = d->gate_up_scale_tiled.data;
+        g.routed.down_scale = d->down_scale_tiled.data;
+        g.shared_weights.gate_up = static_cast<const uint8_t*>(d->shared_gate_up_weight.data);
+        g.shared_weights.down = static_cast<const uint8_t*>(d->shared_down_weight.data);
+        if (nvfp4) {
+            g.routed.gate_up_global = static_cast<const float*>(d->gate_up_global_scale.data);
+            g.routed.gate_up_global_up = gate_up_global_up(d->gate_up_global_scale, p.local_num_experts);
+            g.routed.down_global = static_cast<const float*>(d->down_global_scale.data);
+            g.shared_weights.gate_up_scale = d->shared_gate_up_scale_tiled.data;
+            g.shared_weights.down_scale = d->shared_down_scale_tiled.data;
+            if (shared) {
+                g.shared_weights.gate_up_global = static_cast<const float*>(d->shared_gate_up_global_scale.data);
+                g.shared_weights.gate_up_global_up = gate_up_global_up(d->shared_gate_up_global_scale, 1);
+                g.shared_weights.down_global = static_cast<const float*>(d->shared_down_global_scale.data);
+            }
+        }
+        g.act_global = d->act_global_scale == 0.0f ? 1.0f : d->act_global_scale;
+        g.act2_global = d->act2_global_scale == 0.0f ? 1.0f : d->act2_global_scale;
+        g.act = nvfp4 ? wn.act : fp8 ? wf.act : reinterpret_cast<uint8_t*>(wb.act);
+        g.act_scale = wn.act_sf;
+        g.shared_gate = static_cast<const __nv_bfloat16*>(d->shared_gate_weight.data);
+        g.out = static_cast<__nv_bfloat16*>(d->out.data);
+        if (post_norm) {
+            g.y2 = nvfp4 ? wn.y2 : fp8 ? wf.y2 : wb.y2;
+            g.y2_shared = merged ? g.y2 : x.sh_out;
+            g.route_prows = rt.route_prows;
+            g.shared_row0 = merged ? rt.pad_indptr + p.local_num_experts : nullptr;
+        }
+        const RouterParams router { logits, bias, ids, wts, d->num_tokens, p.num_experts, sigmoid, renorm, d->routed_scaling_factor };
+        err = launch_gemv(gemv_fmt, g, &router, rt, st);
+        if (err != cudaSuccess || !post_norm) {
+            stage_mark(st, STAGE_END);
+            return set_cuda_error(ctx, err, "qs3_moe_layer_execute");
+        }
+    } else if (router_sort_supported(d->num_tokens, p.num_experts, p.top_k, p.local_num_experts)) { // 2. and 3. in one launch
         err = launch_router_sort(logits, bias, ids, wts, d->num_tokens, p.num_experts, p.top_k, sigmoid, renorm,
                                  d->routed_scaling_factor, p.local_expert_offset, p.local_num_experts, rt, st, quant);
         stage_mark(st, STAGE_ROUTE_SORT);
@@ -1342,7 +1423,9 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
         return set_cuda_error(ctx, err, "MoE routing");
 
     const __nv_bfloat16* y2 = nullptr;
-    if (fp8) {
+    if (gemv) {
+        y2 = nvfp4 ? wn.y2 : fp8 ? wf.y2 : wb.y2;
+    } else if (fp8) {
         // 4. quantise every token once (token order); 5./6. grouped GEMMs
         stage_mark(st, STAGE_GATHER);
         err = launch_fp8_quantize_rows(hidden, d->num_tokens, p.hidden_size, x.f8_x, x.f8_s, st);
