@@ -24,7 +24,7 @@ CHECKED_LIB_PATH = os.path.join(PKG_DIR, "libqs3moe_checked.so")
 
 SOURCES = ["context.cu", "router.cu", "routing.cu", "gemm.cu", "gemm_api.cu", "nvfp4.cu", "moe.cu",
            "peak_probe.cu", "fp8.cu", "fp8_rows.cu", "fp8_stream.cu", "bf16_stream.cu", "gemv.cu", "norm.cu", "loader.cu", "nvfp4_decode.cu", "gemm_dense.cu", "gemm_splitk.cu", "gemm_pair.cu", "failure.cu"]
-HEADERS = ["common.cuh", "nvfp4.cuh", "tcgen05.cuh", "topk.cuh", "route_sort.cuh", os.path.join("..", "..", "include", "qs3_moe.h")]
+HEADERS = ["common.cuh", "nvfp4.cuh", "tcgen05.cuh", "topk.cuh", "route_sort.cuh", "fp8.cuh", os.path.join("..", "..", "include", "qs3_moe.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -136,13 +136,14 @@ size_t route_tables_bytes(uint32_t routes, uint32_t experts);
 // Carves the tables out of `base` (may be NULL for sizing); returns bytes used, never fewer for more routes.
 size_t route_tables_carve(char* base, uint32_t routes, uint32_t experts, RouteTables* out,
                           uint32_t tile_rows = kTileM, uint32_t shared_rows = 0, uint32_t alt_tile_rows = 0);
-// Tokens to quantise (NVFP4) beside the sort.
+// Tokens to quantise beside the sort: NVFP4, or FP8 with row-major scales.
 struct TokenQuant {
     const __nv_bfloat16* x; // [rows, k]
     uint32_t rows, k;
     float global_scale;
     uint8_t* packed;
     uint8_t* scale_tiled;
+    float* fp8_scale; // NULL: NVFP4
 };
 // Counting sort of the routes by local expert, stable in route index.
 cudaError_t launch_route_sort(const int32_t* topk_ids, const float* topk_weights, uint32_t routes,

@@ -9,6 +9,7 @@
 // 128 x 128 block scales are not a tcgen05 block-scale format, so every 128-wide k block is accumulated on its own in
 // tensor memory and promoted into f32 registers as acc += partial * (w_scale[block] * x_scale[token, k block]):
 // fp8_stream.cu (weight streaming, experts with few rows) and fp8_rows.cu (token rows on the M side).
+#include "fp8.cuh"
 #include "tcgen05.cuh"
 
 #include <algorithm>
@@ -21,58 +22,13 @@ using namespace tc;
 
 // ---- quantisers -------------------------------------------------------------------------
 
-__device__ __forceinline__ float fp8_scale_of(float amax)
-{
-    return fmaxf(__fdiv_rn(amax, 448.0f), 1.0e-30f);
-}
-
-__device__ __forceinline__ uint32_t pack_e4m3x4(const float* f, float inv)
-{
-    uint32_t r = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        r |= static_cast<uint32_t>(f32_to_e4m3_sat(__fmul_rn(f[i], inv))) << (8 * i);
-    return r;
-}
-
 // codes[row, :] / scales[row, :] = quantise(x[row, :]); 16 lanes per (row, 128-element group), eight elements per lane.
 __global__ void __launch_bounds__(256)
 fp8_quantize_rows_kernel(const __nv_bfloat16* __restrict__ x, uint32_t rows, uint32_t k, uint8_t* __restrict__ codes,
                          float* __restrict__ scales)
 {
     chain_begin();
-    const uint32_t groups = k / 128;
-    const uint64_t unit = static_cast<uint64_t>(blockIdx.x) * 16 + (threadIdx.x >> 4);
-    const uint32_t sub = threadIdx.x & 15;
-    const bool live = unit < static_cast<uint64_t>(rows) * groups;
-    const size_t at = static_cast<size_t>(unit) * 128 + sub * 8; // rows and groups follow each other without gaps
-    uint2 v2[2] = { make_uint2(0, 0), make_uint2(0, 0) };
-    if (live) { // (the entry points promise 8-byte aligned rows)
-        const uint2* src = reinterpret_cast<const uint2*>(x + at);
-        v2[0] = src[0];
-        v2[1] = src[1];
-    }
-    const uint32_t w[4] = { v2[0].x, v2[0].y, v2[1].x, v2[1].y };
-    float f[8];
-    float amax = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        f[2 * j] = bf16_bits_to_f32(w[j] & 0xffffu);
-        f[2 * j + 1] = bf16_bits_to_f32(w[j] >> 16);
-        amax = fmaxf(amax, fmaxf(fabsf(f[2 * j]), fabsf(f[2 * j + 1])));
-    }
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1)
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if (!live)
-        return;
-    const float s = fp8_scale_of(amax);
-    const float inv = __fdiv_rn(1.0f, s);
-    uint32_t* dst = reinterpret_cast<uint32_t*>(codes + at);
-    dst[0] = pack_e4m3x4(f, inv);
-    dst[1] = pack_e4m3x4(f + 4, inv);
-    if (sub == 0)
-        scales[unit] = s;
+    fp8_quantize_groups(x, rows, k, codes, scales, static_cast<uint64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5));
 }
 
 // One block per (k block, row block, expert): 128 x 128 weights -> codes + one scale. Sixteen lanes read the

@@ -525,10 +525,9 @@ qsfi_status run_routed_nvfp4(qsfi_context* ctx, const qsfi_moe_plan_desc& p, con
     return gemm_or_error(ctx, g2, "NVFP4 MoE down GEMM");
 }
 
-// Routed experts on FP8 operands, tokens quantised in token order (`tables_ready`: the routing tables were complete
-// before the predecessor in the stream started).
+// Routed experts on FP8 operands, tokens quantised in token order.
 qsfi_status run_routed_fp8(qsfi_context* ctx, const qsfi_moe_plan_desc& p, const Fp8Workspace& w,
-                           uint32_t num_tokens, const uint8_t* tokens, const float* token_s, bool tables_ready, const uint8_t* gu, const float* gu_scale, const uint8_t* down,
+                           uint32_t num_tokens, const uint8_t* tokens, const float* token_s, const uint8_t* gu, const float* gu_scale, const uint8_t* down,
                            const float* down_scale)
 {
     const auto run = [&](const Fp8Gemm& g, const char* op) {
@@ -558,7 +557,7 @@ qsfi_status run_routed_fp8(qsfi_context* ctx, const qsfi_moe_plan_desc& p, const
     }
     stage_mark(ctx->stream, STAGE_GATE_UP_GEMM);
     Fp8Gemm g1 = g;
-    g1.tables_ready = tables_ready || w.xq != nullptr;
+    g1.tables_ready = w.xq != nullptr; // the predecessor is the gather
     g1.x = tokens;
     g1.x_scale = token_s;
     g1.x_rows = num_tokens;
@@ -1352,8 +1351,8 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
     const int sigmoid = d->score == QSCU_ROUTER_SCORE_SIGMOID, renorm = d->renormalize != 0;
     const bool small_tiles = nvfp4 && rt.tile_rows != static_cast<uint32_t>(kTileM);
     TokenQuant tq { hidden, d->num_tokens, p.hidden_size, d->act_global_scale == 0.0f ? 1.0f : d->act_global_scale,
-                    x.sh_xq, x.sh_xq_sf };
-    const TokenQuant* quant = small_tiles && !fork && !prequant ? &tq : nullptr;
+                    fp8 ? x.f8_x : x.sh_xq, x.sh_xq_sf, fp8 ? x.f8_s : nullptr };
+    const TokenQuant* quant = fp8 || (small_tiles && !fork && !prequant) ? &tq : nullptr;
     cudaError_t err = cudaSuccess;
     if (gemv) { // 2. to 8. of a handful of tokens
         stage_mark(st, STAGE_GATE_UP_GEMM);
@@ -1426,12 +1425,9 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
     if (gemv) {
         y2 = nvfp4 ? wn.y2 : fp8 ? wf.y2 : wb.y2;
     } else if (fp8) {
-        // 4. quantise every token once (token order); 5./6. grouped GEMMs
+        // 4. the tokens, quantised beside the sort; 5./6. grouped GEMMs
         stage_mark(st, STAGE_GATHER);
-        err = launch_fp8_quantize_rows(hidden, d->num_tokens, p.hidden_size, x.f8_x, x.f8_s, st);
-        if (err != cudaSuccess)
-            return set_cuda_error(ctx, err, "FP8 token quantiser");
-        status = run_routed_fp8(ctx, p, wf, d->num_tokens, x.f8_x, x.f8_s, true, static_cast<const uint8_t*>(d->gate_up_weight.data),
+        status = run_routed_fp8(ctx, p, wf, d->num_tokens, x.f8_x, x.f8_s, static_cast<const uint8_t*>(d->gate_up_weight.data),
                                 static_cast<const float*>(d->gate_up_scale_tiled.data),
                                 static_cast<const uint8_t*>(d->down_weight.data),
                                 static_cast<const float*>(d->down_scale_tiled.data));
@@ -2199,7 +2195,7 @@ qsfi_status qs3_moe_execute_fp8(qsfi_context* ctx, const qsfi_moe_plan* plan, co
     const float* hs = static_cast<const float*>(desc->hidden_scale.data);
     if (err != cudaSuccess)
         return set_cuda_error(ctx, err, "FP8 MoE routing");
-    status = run_routed_fp8(ctx, p, w, desc->num_tokens, hq, hs, false, static_cast<const uint8_t*>(desc->gate_up_weight.data),
+    status = run_routed_fp8(ctx, p, w, desc->num_tokens, hq, hs, static_cast<const uint8_t*>(desc->gate_up_weight.data),
                             static_cast<const float*>(desc->gate_up_weight_scale.data),
                             static_cast<const uint8_t*>(desc->down_weight.data),
                             static_cast<const float*>(desc->down_weight_scale.data));

@@ -4,6 +4,7 @@
 #include "common.cuh"
 #include "route_sort.cuh"
 #include "topk.cuh"
+#include "fp8.cuh"
 #include "nvfp4.cuh"
 
 #include <algorithm>
@@ -280,6 +281,14 @@ route_place_kernel(const int32_t* __restrict__ ids, const float* __restrict__ we
     route_place_body(ids, weights, routes, top_k, local_offset, experts, rt, s_hist, blockIdx.x);
 }
 
+__device__ __forceinline__ void quantize_beside(const TokenQuant& q, uint64_t warp)
+{
+    if (q.fp8_scale != nullptr)
+        fp8_quantize_groups(q.x, q.rows, q.k, q.packed, q.fp8_scale, warp);
+    else
+        quantize_row_chunk(q.x, q.rows, q.k, q.global_scale, q.packed, q.scale_tiled, warp);
+}
+
 // All three steps in one block for a decode batch's routes: 1280 routes over 512 experts 0.0129 ->
 // 0.0078 ms, 10 routes 0.0058 -> 0.0042 against 256 threads with global histograms.
 __global__ void __launch_bounds__(kBlockSortThreads)
@@ -288,8 +297,7 @@ route_sort_block_kernel(const int32_t* __restrict__ ids, const float* __restrict
 {
     chain_begin();
     if (blockIdx.x > 0) { // the other blocks quantise the tokens meanwhile
-        quantize_row_chunk(quant.x, quant.rows, quant.k, quant.global_scale, quant.packed, quant.scale_tiled,
-                           static_cast<uint64_t>(blockIdx.x - 1) * kBlockSortWarps + (threadIdx.x >> 5));
+        quantize_beside(quant, static_cast<uint64_t>(blockIdx.x - 1) * kBlockSortWarps + (threadIdx.x >> 5));
         return;
     }
     extern __shared__ __align__(16) uint8_t s_dyn[];
@@ -307,8 +315,7 @@ router_sort_block_kernel(RouterParams r, uint32_t top_k, uint32_t local_offset, 
 {
     chain_begin();
     if (blockIdx.x > 0) {
-        quantize_row_chunk(quant.x, quant.rows, quant.k, quant.global_scale, quant.packed, quant.scale_tiled,
-                           static_cast<uint64_t>(blockIdx.x - 1) * kBlockSortWarps + (threadIdx.x >> 5));
+        quantize_beside(quant, static_cast<uint64_t>(blockIdx.x - 1) * kBlockSortWarps + (threadIdx.x >> 5));
         return;
     }
     extern __shared__ __align__(16) uint8_t s_dyn[];
@@ -1043,12 +1050,13 @@ bool route_sort_can_choose(uint32_t routes, uint32_t experts)
 
 namespace {
 
-// Blocks of the one-block sorts beyond the first: a warp per 512 elements to quantise.
+// Blocks of the one-block sorts beyond the first: a warp per 512 elements to quantise (FP8: 256).
 uint32_t quant_blocks(const TokenQuant* quant)
 {
     if (quant == nullptr)
         return 0;
-    const uint64_t units = static_cast<uint64_t>(quant->rows) * ((quant->k + 511) / 512);
+    const uint64_t units = quant->fp8_scale != nullptr ? (static_cast<uint64_t>(quant->rows) * (quant->k / 128) + 1) / 2
+                                                       : static_cast<uint64_t>(quant->rows) * ((quant->k + 511) / 512);
     return static_cast<uint32_t>((units + kBlockSortWarps - 1) / kBlockSortWarps);
 }
 
@@ -1142,8 +1150,10 @@ cudaError_t launch_route_sort(const int32_t* topk_ids, const float* topk_weights
                               rt, quant != nullptr ? *quant : TokenQuant {});
     }
     if (quant != nullptr) {
-        const cudaError_t err = launch_nvfp4_quantize_rows(quant->x, quant->rows, quant->k, quant->global_scale,
-                                                           quant->packed, quant->scale_tiled, stream);
+        const cudaError_t err = quant->fp8_scale != nullptr
+            ? launch_fp8_quantize_rows(quant->x, quant->rows, quant->k, quant->packed, quant->fp8_scale, stream)
+            : launch_nvfp4_quantize_rows(quant->x, quant->rows, quant->k, quant->global_scale, quant->packed,
+                                         quant->scale_tiled, stream);
         if (err != cudaSuccess)
             return err;
     }
