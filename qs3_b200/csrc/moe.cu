@@ -856,6 +856,7 @@ qsfi_status qsfi_moe_execute_bf16(qsfi_context* ctx, const qsfi_moe_plan* plan,
     if (status != QSFI_STATUS_OK)
         return status;
     CombineParams cp {};
+    cp.early = 1; // after the down GEMM
     cp.route_prows = w.rt.route_prows;
     cp.topk_weights = static_cast<const float*>(desc->topk_weights.data);
     cp.expert_out = w.y2;
@@ -977,6 +978,7 @@ qsfi_status qsfi_moe_execute_nvfp4(qsfi_context* ctx, const qsfi_moe_plan* plan,
     if (status != QSFI_STATUS_OK)
         return status;
     CombineParams cp {};
+    cp.early = 1; // after the down GEMM
     cp.route_prows = w.rt.route_prows;
     cp.topk_weights = static_cast<const float*>(desc->topk_weights.data);
     cp.expert_out = w.y2;
@@ -1503,6 +1505,7 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
     // 8. weighted combine (+ sigmoid-gated shared expert)
     stage_mark(st, STAGE_COMBINE);
     CombineParams cp {};
+    cp.early = 1; // after the down GEMM
     cp.route_prows = rt.route_prows;
     cp.topk_weights = wts;
     cp.expert_out = y2;
@@ -2202,6 +2205,7 @@ qsfi_status qs3_moe_execute_fp8(qsfi_context* ctx, const qsfi_moe_plan* plan, co
     if (status != QSFI_STATUS_OK)
         return status;
     CombineParams cp {};
+    cp.early = 1; // after the down GEMM
     cp.route_prows = w.rt.route_prows;
     cp.topk_weights = static_cast<const float*>(desc->topk_weights.data);
     cp.expert_out = w.y2;

@@ -697,7 +697,8 @@ __global__ void __launch_bounds__(kCombineThreads, TOKENS == 1 ? 2 : 4) combine_
     __shared__ float s_w[TOKENS][32];
     __shared__ float s_dot[TOKENS][kGroup / 32];
     __shared__ int s_any[TOKENS];
-    chain_begin();
+    if (!p.early)
+        chain_begin();
     const uint32_t group = threadIdx.x / kGroup, gl = threadIdx.x % kGroup;
     const uint32_t token = blockIdx.x * TOKENS + group;
     const bool live = token < p.num_tokens;
@@ -745,6 +746,8 @@ __global__ void __launch_bounds__(kCombineThreads, TOKENS == 1 ? 2 : 4) combine_
         if (lane == 0)
             s_dot[group][gl / 32] = dot;
     }
+    if (p.early) // all of the above is older than the predecessor
+        chain_begin();
     __syncthreads();
     if (!live || (p.skip_empty && !s_any[group]))
         return; // no local route: the row stays unwritten and is never read
@@ -797,7 +800,8 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_norm_kernel(Combin
     __shared__ float s_dot[TOKENS][kGroup / 32];
     __shared__ float s_sq[TOKENS][kGroup / 32];
     __shared__ int s_any[TOKENS];
-    chain_begin();
+    if (!p.early)
+        chain_begin();
     const uint32_t group = threadIdx.x / kGroup, gl = threadIdx.x % kGroup;
     const uint32_t token = blockIdx.x * TOKENS + group;
     const bool live = token < p.num_tokens;
@@ -842,6 +846,15 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_norm_kernel(Combin
         if (lane == 0)
             s_dot[group][gl / 32] = dot;
     }
+    const uint4* nw = reinterpret_cast<const uint4*>(p.norm_weight);
+    uint4* res = reinterpret_cast<uint4*>(p.residual) + static_cast<size_t>(live ? token : 0) * vec_per_row;
+    uint4 own_res = make_uint4(0, 0, 0, 0), own_nw = make_uint4(0, 0, 0, 0); // one token per block: a thread has one chunk
+    if (TOKENS == 1 && live && gl < vec_per_row) {
+        own_res = res[gl];
+        own_nw = nw[gl];
+    }
+    if (p.early) // all of the above is older than the predecessor
+        chain_begin();
     __syncthreads();
     float gate = 0.0f;
     if (p.shared_out != nullptr) {
@@ -853,7 +866,6 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_norm_kernel(Combin
     }
 
     const uint32_t n_valid = live ? static_cast<uint32_t>(s_any[group]) : 0u;
-    uint4* res = reinterpret_cast<uint4*>(p.residual) + static_cast<size_t>(live ? token : 0) * vec_per_row;
     float vals[TOKENS][8]; // chunks gl, gl + kGroup, ... of the row
     float sum_sq = 0.0f;
 #pragma unroll
@@ -867,7 +879,7 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_norm_kernel(Combin
                 continue;
             if (p.shared_out != nullptr)
                 add_shared(p, token, vec_per_row, i, gate, acc);
-            const uint4 rv = res[i];
+            const uint4 rv = TOKENS == 1 ? own_res : res[i];
             const uint32_t rs[4] = { rv.x, rv.y, rv.z, rv.w };
             uint32_t o[4];
 #pragma unroll
@@ -898,13 +910,12 @@ __global__ void __launch_bounds__(kCombineThreads, 2) combine_norm_kernel(Combin
         total += s_sq[group][w];
     const float inv_rms = 1.0f / sqrtf(total / static_cast<float>(p.hidden_size) + p.norm_eps);
     uint4* out = reinterpret_cast<uint4*>(p.out) + static_cast<size_t>(token) * vec_per_row;
-    const uint4* nw = reinterpret_cast<const uint4*>(p.norm_weight);
 #pragma unroll
     for (uint32_t c = 0; c < TOKENS; ++c) {
         const uint32_t i = gl + c * kGroup;
         if (i >= vec_per_row)
             continue;
-        const uint4 wv = nw[i];
+        const uint4 wv = TOKENS == 1 ? own_nw : nw[i];
         const uint32_t ws[4] = { wv.x, wv.y, wv.z, wv.w };
         uint32_t o[4];
 #pragma unroll
