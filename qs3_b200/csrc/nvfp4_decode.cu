@@ -161,9 +161,10 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     const uint32_t xsf_cols = 4 * p.kgroups;
 
     // The tables of the down projection are older than its predecessor (the gate_up GEMM, whose start means that the
-    // sort is complete), and weights are older still: its producer fills the ring before it waits. Every other role
-    // touches what the predecessor wrote.
-    if (!p.tables_ready || warp != 4)
+    // sort is complete), and weights are older still: its producer fills the ring before it waits, its panel loaders look up
+    // their first tile. Every other role touches what the predecessor wrote.
+    const bool early = p.tables_ready && (warp == 4 || (warp >= 7 && warp <= 10));
+    if (!early)
         chain_begin();
 
     // this CTA's units: feature blocks [u0, u1) of the tiles in order
@@ -325,10 +326,17 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         }
     } else if (warp >= 7 && warp <= 10) {
         // ------------------------------------------------------- panel loaders --
-        const uint32_t t = threadIdx.x - 7 * 32;
+        // A warp takes every fourth row, a lane one or two vectors of it; scale words by (row, k group), each thread the same
+        // row throughout. Few instructions: a warp of its own per scheduler runs them one after the other, and with
+        // divisions per vector the first tile took 4 us to ask for and 2 to store, with the ring full and HBM idle
+        // (first MMA 8.9 -> 4.0 us after the predecessor's end in the down kernel of 128 tokens).
+        const uint32_t t = threadIdx.x - 7 * 32, lw = t >> 5;
         const uint32_t vecs = p.k_blocks * 8;      // 16-byte vectors per row
+        const uint32_t halves = vecs > 32 ? 2 : 1; // vectors of a row per lane
+        const uint32_t sj = t % NT, kg0 = t / NT;  // this thread's scale words: row, first k group
+        constexpr uint32_t kKgStep = kSwLoaders / NT;
         uint32_t i = 0;
-        bool ok = true;
+        bool ok = true, waited = !early;
         for (uint32_t u = u0; u < u1 && ok; u = (u / p.num_fb + 1) * p.num_fb, ++i) {
             const uint32_t tile = u / p.num_fb;
             const uint32_t row0 = static_cast<uint32_t>(p.tile_row0[tile]);
@@ -341,51 +349,54 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 if (expert != p.shared_group)
                     rows = p.row_tokens + p.indptr[expert] + first;
             }
-            const auto src_row = [&](uint32_t j) -> uint64_t {
-                return rows != nullptr ? static_cast<uint64_t>(rows[j]) : static_cast<uint64_t>(first) + j;
-            };
+            // source rows of the tile's rows lane and lane + 32
+            uint32_t src[NT / 32];
+#pragma unroll
+            for (uint32_t h = 0; h < NT / 32; ++h) {
+                const uint32_t j = lane + 32 * h;
+                src[h] = j >= nrows ? 0u : rows != nullptr ? static_cast<uint32_t>(rows[j]) : first + j;
+            }
+            if (!waited)
+                chain_begin();
+            waited = true;
             // the tile's codes (the first kSwBatch vectors a thread) and scale words travel together
-            const uint32_t items = nrows * vecs, words = p.kgroups * NT;
+            const uint32_t items = (nrows + 3) / 4 * halves; // of a warp
             uint4 v[kSwBatch];
             const auto load_codes = [&](uint32_t c0) {
 #pragma unroll
                 for (uint32_t q = 0; q < kSwBatch; ++q) {
-                    const uint32_t c = c0 + q * kSwLoaders + t;
-                    if (c < items)
-                        v[q] = *reinterpret_cast<const uint4*>(p.x + src_row(c / vecs) * (vecs * 16) + (c % vecs) * 16);
+                    const uint32_t c = c0 + q, j = lw + 4 * (halves == 2 ? c >> 1 : c), vec = lane + (halves == 2 ? (c & 1) * 32 : 0);
+                    const uint32_t r = __shfl_sync(0xffffffffu, NT == 64 && j >= 32 ? src[NT / 32 - 1] : src[0], j & 31);
+                    if (j < nrows && vec < vecs)
+                        v[q] = *reinterpret_cast<const uint4*>(p.x + static_cast<uint64_t>(r) * (vecs * 16) + vec * 16);
                 }
             };
             const auto store_codes = [&](uint32_t c0) {
 #pragma unroll
                 for (uint32_t q = 0; q < kSwBatch; ++q) {
-                    const uint32_t c = c0 + q * kSwLoaders + t;
-                    if (c < items) {
-                        const uint32_t j = c / vecs, col = c % vecs;
-                        *reinterpret_cast<uint4*>(panel + (col >> 3) * kPanelTile + j * 128 + (((col & 7) ^ (j & 7)) << 4)) = v[q];
-                    }
+                    const uint32_t c = c0 + q, j = lw + 4 * (halves == 2 ? c >> 1 : c), vec = lane + (halves == 2 ? (c & 1) * 32 : 0);
+                    if (j < nrows && vec < vecs)
+                        *reinterpret_cast<uint4*>(panel + (vec >> 3) * kPanelTile + j * 128 + (((vec & 7) ^ (j & 7)) << 4)) = v[q];
                 }
             };
             load_codes(0);
-            // scale words: (row, k group), a warp takes the rows of one k group
-            for (uint32_t c0 = t; c0 < words; c0 += 8 * kSwLoaders) {
+            const uint64_t sr = NT == 64 && (lw & 1) ? src[NT / 32 - 1] : src[0]; // of row sj
+            const uint8_t* sf = p.x_sf + (p.x_sf_linear ? sr * (p.kgroups * 4) : tiled_scale_offset(sr, 0, p.kgroups));
+            const uint32_t sf_step = p.x_sf_linear ? 4 : 512; // bytes between k groups
+            for (uint32_t k0 = kg0; k0 < p.kgroups; k0 += 8 * kKgStep) {
                 uint32_t w[8];
 #pragma unroll
                 for (uint32_t q = 0; q < 8; ++q) {
-                    const uint32_t c = c0 + q * kSwLoaders, j = c % NT, kg = c / NT;
-                    w[q] = 0;
-                    if (c < words && j < nrows) {
-                        const uint64_t r = src_row(j);
-                        w[q] = *reinterpret_cast<const uint32_t*>(
-                            p.x_sf + (p.x_sf_linear ? r * (p.kgroups * 4) + kg * 4 : tiled_scale_offset(r, 4ull * kg, p.kgroups)));
-                    }
+                    const uint32_t kg = k0 + q * kKgStep;
+                    w[q] = kg < p.kgroups && sj < nrows ? *reinterpret_cast<const uint32_t*>(sf + kg * sf_step) : 0u;
                 }
-                if (c0 == t && i >= 1)
+                if (k0 == kg0 && i >= 1)
                     ok = mbar_wait(psf_free, (i - 1) & 1, abort_flag, p.err, ERR_SW_PANEL_FREE_WAIT);
 #pragma unroll
                 for (uint32_t q = 0; q < 8; ++q) {
-                    const uint32_t c = c0 + q * kSwLoaders, j = c % NT, kg = c / NT;
-                    if (c < words && ok)
-                        *reinterpret_cast<uint32_t*>(panel_sf + kg * 512 + (j & 31) * 16 + (j >> 5) * 4) = w[q];
+                    const uint32_t kg = k0 + q * kKgStep;
+                    if (kg < p.kgroups && ok)
+                        *reinterpret_cast<uint32_t*>(panel_sf + kg * 512 + (sj & 31) * 16 + (sj >> 5) * 4) = w[q];
                 }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // tcgen05.cp reads through the async proxy
@@ -396,7 +407,9 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 mbar_arrive(psf_full);
             if (i >= 1)
                 ok = mbar_wait(panel_free, (i - 1) & 1, abort_flag, p.err, ERR_SW_PANEL_FREE_WAIT);
-            for (uint32_t c0 = 0; c0 < items && ok; c0 += kSwBatch * kSwLoaders) {
+            // (every lane of a warp shuffles in load_codes: whether the wait gave up is decided for the warp)
+            ok = __all_sync(0xffffffffu, ok);
+            for (uint32_t c0 = 0; c0 < items && ok; c0 += kSwBatch) {
                 if (c0 != 0)
                     load_codes(c0);
                 store_codes(c0);
@@ -406,6 +419,8 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             if (ok && t == 0)
                 mbar_arrive(panel_full);
         }
+        if (!waited)
+            chain_begin();
     } else {
         // ------------------------------------------------------------ epilogue --
         const uint32_t lane_base = (warp * 32) << 16;
