@@ -137,7 +137,7 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             const int w_row2 = w_row + static_cast<int>(GATED ? p.n : p.half);
             uint32_t ahead = 0; // k blocks whose weights are on their way already
             if (i == 0 && early) {
-                if (lane == 0) {
+                if (elect_one()) {
                     for (; ahead < min(kNumStages, p.k_blocks); ++ahead) {
                         uint8_t* sw = smem + ahead * kStageBytes;
                         mbar_expect_tx_only(&full_bar[ahead], 2 * p.half * 128);
@@ -168,7 +168,7 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                     break;
                 uint8_t* sw = smem + s * kStageBytes;
                 const int c0 = static_cast<int>(kb) * 64;
-                if (lane == 0) {
+                if (elect_one()) {
                     mbar_expect_tx(&full_bar[s], (kb < ahead ? 0 : 2 * p.half * 128) + parts * part_rows * 128);
                     if (kb >= ahead) {
                         tma_load_2d(sw, &map_w, &full_bar[s], c0, w_row);
@@ -193,7 +193,7 @@ gemm_bf16_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             chain_begin();
     } else if (warp == 5) {
         // ---------------------------------------------------------- MMA issuer --
-        if (lane == 0) {
+        if (elect_one()) {
             // M = 128 weight rows, N = NT tokens, bf16 x bf16 -> f32, both operands K-major
             constexpr uint32_t kIdesc
                 = (1u << 4) | (1u << 7) | (1u << 10) | ((static_cast<uint32_t>(NT) >> 3) << 17) | ((kBM >> 4) << 24);

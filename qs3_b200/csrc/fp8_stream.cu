@@ -207,7 +207,7 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         bool ok = true;
         uint32_t ahead = 0; // k blocks of the first unit whose weights are on their way already
         if (early) {
-            if (blockIdx.x < total && lane == 0) {
+            if (blockIdx.x < total && elect_one()) {
                 const uint32_t tile = blockIdx.x / p.units_per_tile, nb = blockIdx.x % p.units_per_tile;
                 const uint32_t fb = GATED ? nb : 2 * nb, fb2 = GATED ? p.num_fb + nb : min(2 * nb + 1, p.num_fb - 1);
                 const int w0 = p.tile_expert[tile] * static_cast<int>(p.b_rows);
@@ -242,7 +242,7 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                     break;
                 uint8_t* sw = smem + s * S::kStageBytes;
                 const int c0 = static_cast<int>(kb) * 128;
-                if (lane == 0) {
+                if (elect_one()) {
                     mbar_expect_tx(&full_bar[s], (kb < ahead ? 0 : 2 * kTileBytes) + parts * part_rows * 128);
                     if (kb >= ahead) {
                         tma_load_2d(sw, &map_w, &full_bar[s], c0, w_row);
@@ -265,7 +265,7 @@ gemm_fp8_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         }
     } else if (warp == 9) {
         // ---------------------------------------------------------- MMA issuer --
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t s = 0, ph = 0, b = 0, bph = 0;
             bool ok = true;
             for (uint32_t u = blockIdx.x; u < total && ok; u += gridDim.x, next_note()) {

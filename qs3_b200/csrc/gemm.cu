@@ -103,7 +103,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
     if (warp == 4) {
         // ------------------------------------------------------------ producer --
-        if (lane == 0) {
+        if (elect_one()) {
             const int b_row = expert * static_cast<int>(p.b_rows) + static_cast<int>(n0);
             const uint8_t* sfa_src = NVFP4
                 ? p.sfa + (static_cast<uint64_t>(row0 >> 7) * p.kgroups) * 512
@@ -139,7 +139,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
     } else if (warp == 5) {
         // ---------------------------------------------------------- MMA issuer --
-        if (lane == 0) {
+        if (elect_one()) {
             // instruction descriptor: M = 128, N = 128, both operands K-major
             constexpr uint32_t kIdesc = NVFP4
                 ? ((1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((kBM >> 4) << 24))
@@ -323,7 +323,7 @@ gemm_tc_astat_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
     if (warp == 8) {
         // ------------------------------------------------------------ producer --
-        if (lane == 0) {
+        if (elect_one()) {
             // the A panel and its scales, once
             mbar_expect_tx(panel_bar, kb_count * (kTileBytes + kSfBytes));
             for (uint32_t kb = 0; kb < kb_count; ++kb)
@@ -366,7 +366,7 @@ gemm_tc_astat_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
     } else if (warp == 9) {
         // ---------------------------------------------------------- MMA issuer --
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((kBN >> 3) << 17) | ((kBM >> 4) << 24);
             // the copier has put the A scales into tensor memory (which also means the A panel has landed)
             bool ok = mbar_wait<true>(sfa_ready, 0, abort_flag, p.err, ERR_AS_PANEL_WAIT);
@@ -412,7 +412,7 @@ gemm_tc_astat_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
     } else if (warp == 10) {
         // -------------------------------------------------------- scale copier --
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = mbar_wait<true>(panel_bar, 0, abort_flag, p.err, ERR_AS_PANEL_WAIT);
             if (ok) {
                 tc_fence_after();

@@ -86,7 +86,7 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
     if (warp == 8) {
         // ------------------------------------------------------------ producer --
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t s = 0, ph = 0;
             bool ok = true;
             for (uint32_t t = blockIdx.x; t < total && ok; t += gridDim.x) {
@@ -112,7 +112,7 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
     } else if (warp == 9) {
         // ---------------------------------------------------------- MMA issuer --
-        if (lane == 0) {
+        if (elect_one()) {
             // M = 128, N = bn, bf16 x bf16 -> f32, both operands K-major
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((bn >> 3) << 17) | ((kBM >> 4) << 24);
             uint32_t s = 0, ph = 0, u = 0;
@@ -282,7 +282,7 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
     if (warp == 8) {
         // ------------------------------------------------------------ producer --
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t s = 0, ph = 0;
             bool ok = true;
             for (uint32_t t = pair; t < total && ok; t += pairs) {
@@ -312,7 +312,7 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
     } else if (warp == 9) {
         // ---------------------------------------------------------- MMA issuer --
-        if (rank == 0 && lane == 0) {
+        if (rank == 0 && elect_one()) {
             // M = 256 (128 rows in each CTA), N = 256 (128 B rows from each CTA)
             constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
             uint32_t s = 0, ph = 0, u = 0;

@@ -470,7 +470,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         // loaded as soon as the last column tile of the current unit is done with block kb, so a panel
         // trails the previous unit's last column tile by one k block instead of waiting for its end. The
         // panel stream is polled, never waited for, so that it cannot hold up the ring.
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t p_unit = cluster_id, p_no = 0, p_kb = 0, p_slot0 = 0, p_par = 0;
             Unit pu;
             bool p_have = load_unit(pp, p_unit, sc, &pu);
@@ -603,7 +603,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         // tcgen05.cp costs its issuing thread 50-70 cycles apiece; the eight copies of a stage's B scales
         // (plus four of A scales in a unit's first column tile) from one thread take longer than the
         // stage's four MMAs, so the two 128-row halves of the B scales have a copier thread each.
-        if (kPgBN == 256 && rank == 0 && lane == 0) {
+        if (kPgBN == 256 && rank == 0 && elect_one()) {
             uint32_t s = 0, ph = 0;
             bool ok = true;
             Unit un;
@@ -636,7 +636,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
     } else if (warp == 9) {
         // ---------------------------------------------------------- MMA issuer --
-        if (rank == 0 && lane == 0) {
+        if (rank == 0 && elect_one()) {
             constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((kPgBN >> 3) << 17) | ((256u >> 4) << 24);
             const uint32_t a_addr = smem_u32(a_panel);
             uint32_t s = 0, ph = 0, unit_no = 0, tile_no = 0, sfi = 0;
@@ -714,7 +714,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         // -------------------------------------------------------- scale copier --
         // Same order as the MMA issuer consumes: per stage, in a unit's first column tile the A scales of
         // the stage's k block first (both CTAs' staging -> their own tensor memory), then the stage's B scales.
-        if (rank == 0 && lane == 0) {
+        if (rank == 0 && elect_one()) {
             uint32_t s = 0, ph = 0, unit_no = 0, sfi = 0;
             bool ok = true;
             Unit un;

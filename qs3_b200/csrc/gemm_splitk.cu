@@ -154,7 +154,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
     bool ready = true;
     if (warp == 4) {
         // ------------------------------------------------------------ producer --
-        if (lane == 0) {
+        if (elect_one()) {
             for (uint32_t i = 0; i < kb1 - kb0; ++i) {
                 const uint32_t s = i % kSkStages, ph = (i / kSkStages) & 1;
                 if (!mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_SK_EMPTY_WAIT))
@@ -168,7 +168,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
         }
     } else if (warp == 5) {
         // ---------------------------------------------------------- MMA issuer --
-        if (lane == 0) {
+        if (elect_one()) {
             // M = 128 weight rows, N = NT rows of A, bf16 x bf16 -> f32, both operands K-major
             constexpr uint32_t kIdesc
                 = (1u << 4) | (1u << 7) | (1u << 10) | ((static_cast<uint32_t>(NT) >> 3) << 17) | ((kBM >> 4) << 24);

@@ -176,7 +176,7 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 
     if (warp == 4) {
         // ------------------------------------------------------------ producer --
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t s = 0, ph = 0;
             bool ok = true;
             uint32_t tile = tile_first, fb = fb_first;
@@ -217,7 +217,7 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         // --------------------------------------------------------- MMA issuers --
         // Alternate feature blocks: one thread's instructions, waits and commits take longer than the weights of a
         // feature block with a short k (down of a 128-token batch: one issuer 0.056 ms, two 0.050).
-        if (lane == 0) {
+        if (elect_one()) {
             // M = 128 weight rows, N = NT tokens, e2m1 x e2m1 with e4m3 block scales, f32 accumulate
             constexpr uint32_t kIdesc
                 = (1u << 7) | (1u << 10) | ((static_cast<uint32_t>(NT) >> 3) << 17) | ((kBM >> 4) << 24);
@@ -287,7 +287,7 @@ gemm_nvfp4_swap_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         }
     } else if (warp == 6) {
         // -------------------------------------------------------- scale copier --
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t s = 0, ph = 0, fb = fb_first, i = 0;
             bool ok = true;
             for (uint32_t u = u0; u < u1 && ok; ++u) {
