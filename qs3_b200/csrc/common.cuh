@@ -321,10 +321,19 @@ struct GemmProblem {
 cudaError_t launch_gemm(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);
 // Dense bf16 problems with few output tiles: k split over the CTAs of a cluster (gemm_splitk.cu).
 bool gemm_splitk_supported(const GemmProblem& p);
-cudaError_t launch_gemm_splitk(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);
+// `rows` of A per tile, 0: this kernel's own choice.
+cudaError_t launch_gemm_splitk(const GemmProblem& p, uint32_t rows, cudaStream_t stream, const char** why_unsupported);
+float gemm_splitk_estimate(const GemmProblem& p, uint32_t rows); // microseconds, bf16 results
 // Persistent 128 x 256 kernel for dense bf16 problems with more than 64 rows (gemm_dense.cu).
 bool gemm_dense_bf16_supported(const GemmProblem& p);
-cudaError_t launch_gemm_dense_bf16(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);
+enum DenseKernel : uint32_t { DENSE_ONE, DENSE_PAIR, DENSE_SPLIT };
+struct DenseChoice {
+    DenseKernel kernel;
+    uint32_t width; // columns of a tile; DENSE_SPLIT: rows of A
+};
+DenseChoice gemm_dense_choice(const GemmProblem& p);
+// DENSE_ONE and DENSE_PAIR
+cudaError_t launch_gemm_dense_bf16(const GemmProblem& p, DenseChoice choice, cudaStream_t stream, const char** why_unsupported);
 // NVFP4 GEMM on CTA pairs (256 x 256 instructions, weights cross L2 -> SM once per 256 rows; gemm_pair.cu).
 bool nvfp4_pair_gemm_supported(const GemmProblem& p);
 cudaError_t launch_nvfp4_pair_gemm(const GemmProblem& p, cudaStream_t stream, const char** why_unsupported);

@@ -848,6 +848,22 @@ bool make_operand_map(CUtensorMap* map, bool bytes_type, const void* base, uint6
     return make_map(map, bytes_type, base, inner_elems, rows, pitch_bytes, box_rows);
 }
 
+bool make_output_map(CUtensorMap* map, bool f32, void* out, uint64_t cols, uint64_t rows, uint64_t pitch_elems)
+{
+    EncodeTiledFn fn = encode_tiled_fn();
+    const uint64_t bytes = f32 ? 4 : 2;
+    if (fn == nullptr || !aligned16(out) || pitch_elems * bytes % 16 != 0 || cols * bytes % 16 != 0)
+        return false;
+    const cuuint64_t dims[2] = { cols, rows };
+    const cuuint64_t strides[1] = { pitch_elems * bytes };
+    const cuuint32_t box[2] = { static_cast<cuuint32_t>(64 / bytes), 32 };
+    const cuuint32_t estr[2] = { 1, 1 };
+    return fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, out, dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE)
+        == CUDA_SUCCESS;
+}
+
 uint32_t device_sm_count() { return sm_count(); }
 
 bool make_scale_tile_map(CUtensorMap* map, const void* base, uint64_t tiles, uint32_t box_tiles)
@@ -945,10 +961,15 @@ cudaError_t launch_gemm(const GemmProblem& g, cudaStream_t stream, const char** 
     }
     if (skinny_supported(g))
         return launch_skinny(g, stream);
-    if (gemm_splitk_supported(g))
-        return launch_gemm_splitk(g, stream, why);
-    if (gemm_dense_bf16_supported(g))
-        return launch_gemm_dense_bf16(g, stream, why);
+    const bool dense = gemm_dense_bf16_supported(g);
+    if ((!dense || g.epilogue == EPI_STORE_F32) && gemm_splitk_supported(g))
+        return launch_gemm_splitk(g, 0, stream, why);
+    if (dense) {
+        const DenseChoice choice = gemm_dense_choice(g);
+        if (choice.kernel == DENSE_SPLIT)
+            return launch_gemm_splitk(g, choice.width, stream, why);
+        return launch_gemm_dense_bf16(g, choice, stream, why);
+    }
     if (pair_kernel_wanted(g))
         return launch_nvfp4_pair_gemm(g, stream, why);
     if (gemm_tc_supported(g)) {

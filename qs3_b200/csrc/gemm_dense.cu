@@ -6,13 +6,12 @@
 //
 //   persistent   one CTA per SM walks the output tiles (row tile fastest, so the CTAs of a wave
 //                share one or two B panels through L2)
-//   128 x 256    tcgen05.mma kind::f16 with N = 256: the widest single-CTA instruction; or fewer columns where
-//                that fills the last round of the SMs (151936 features: 594 tiles of 256 columns leave two tiles to a
-//                fifth round, 208 columns fill five)
+//   128 x bn     tcgen05.mma kind::f16 with N = bn columns, 32 to 256 (256: the widest single-CTA instruction), as many as
+//                gemm_dense_choice() finds quickest
 //   TMEM         two 256-column f32 accumulators: the epilogue of tile i (eight warps, two per
 //                lane quadrant) overlaps the main loop of tile i + 1
-//   smem         ring of four stages, each A 128 x 64 bf16 (16 KB) + B 256 x 64 bf16 (32 KB),
-//                filled by TMA with the 128-byte swizzle
+//   smem         192 KB ring of stages, each A 128 x 64 bf16 (16 KB) + B bn x 64, filled by TMA with the 128-byte swizzle;
+//                32 KB through which the output goes (dense_epilogue)
 //
 // Rows past the end of A or B are zero-filled by TMA and masked in the epilogue. Every wait is
 // bounded; on expiry the kernel records a code and leaves through the normal teardown.
@@ -29,10 +28,15 @@ using namespace tc;
 
 constexpr int kDnThreads = 320; // warps 0-7 epilogue, 8 producer, 9 MMA issuer
 constexpr uint32_t kDnBN = 256;
-constexpr uint32_t kDnStageBytes = 3 * kTileBytes; // A tile + two B tiles
-constexpr uint32_t kDnStages = 4;
+constexpr uint32_t kDnRing = 12 * kTileBytes; // stages of an A tile + bn rows of B: four of 256 rows, up to eight of fewer
+constexpr uint32_t kDnMaxStages = 8;
+__host__ __device__ constexpr uint32_t dense_stages(uint32_t bn)
+{
+    return kDnRing / (kTileBytes + bn * 128) < kDnMaxStages ? kDnRing / (kTileBytes + bn * 128) : kDnMaxStages;
+}
 constexpr uint32_t kDnTmemCols = 512;
-constexpr uint64_t kDnMinTiles = 64;
+constexpr uint32_t kDnOutBytes = 2048;            // staging of a warp's 32 rows x 64 bytes of output
+constexpr uint32_t kDnStaging = 8 * 2 * kDnOutBytes; // two per epilogue warp
 
 enum : uint32_t {
     ERR_DN_FULL_WAIT = 0x55000001u,
@@ -41,26 +45,100 @@ enum : uint32_t {
     ERR_DN_ACC_EMPTY_WAIT = 0x55000004u,
 };
 
-template <int EPI>
+// Epilogue of one output tile: 128 accumulator lanes (rows from row0) x bn columns (from col0), by eight warps, two per
+// quarter of the lanes. A lane holds a row, so a warp's store of 16 bytes a lane touches 32 rows, and every 32-byte sector
+// is written twice; of a short k this takes longer than the products. With TMA a warp gathers 64 bytes of each of its rows
+// in shared memory (64-byte swizzle, no bank conflicts) and has them written, two such stores in flight: 4096 x 512 x 8192
+// 50 -> 39 us, 3001 x 2048 x 4096 42.5 -> 40.9. The last columns of a tile are taken as the last 64 bytes, which may write some
+// columns twice, with the same values; rows and columns past the end are clipped. beta reads the output, and an output that
+// TMA cannot address is stored row by row.
+template <int EPI, bool TMA>
+__device__ __forceinline__ void dense_epilogue(const TcParams& p, const CUtensorMap* map_o, uint8_t* staging, uint32_t& stores,
+                                               uint32_t tmem_acc, uint32_t warp, uint32_t lane, uint32_t row0, uint32_t col0,
+                                               uint32_t bn)
+{
+    const uint32_t quad = warp & 3, half = warp >> 2;
+    if constexpr (!TMA) {
+        // the tile's columns as a problem of their own: this epilogue works in units of 128 of them
+        TcParams q = p;
+        q.n = min(bn, p.n - col0);
+        q.out = static_cast<uint8_t*>(p.out) + static_cast<uint64_t>(col0) * (EPI == EPI_STORE_F32 ? 4 : 2);
+        if (p.bias != nullptr)
+            q.bias = p.bias + col0;
+        const int nrows = static_cast<int>(min(static_cast<uint32_t>(kBM), p.dense_rows - row0));
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h)
+            epilogue_tile<false, EPI, 2>(q, tmem_acc + h * kBN, quad, lane, 0, static_cast<int>(row0), nrows, h, half);
+        return;
+    }
+    if (row0 + quad * 32 >= p.dense_rows)
+        return;
+    constexpr uint32_t kCols = EPI == EPI_STORE_F32 ? 16 : 32;
+    const uint32_t cols = min(bn, p.n - col0);
+    const float scale = p.alpha == 0.0f ? 1.0f : p.alpha;
+    for (uint32_t c = half * kCols; c < cols; c += 2 * kCols) {
+        const uint32_t at = min(c, bn - kCols);
+        uint32_t v[kCols];
+        tc_ld16(tmem_acc + ((quad * 32) << 16) + at, v);
+        if constexpr (kCols == 32)
+            tc_ld16(tmem_acc + ((quad * 32) << 16) + at + 16, v + 16);
+        tc_ld_wait();
+        float f[kCols];
+#pragma unroll
+        for (uint32_t i = 0; i < kCols; ++i) {
+            f[i] = __uint_as_float(v[i]) * scale;
+            if (p.bias != nullptr && col0 + at + i < p.n)
+                f[i] += p.bias[col0 + at + i];
+        }
+        uint8_t* buf = staging + (stores++ & 1) * kDnOutBytes;
+        if (lane == 0) // the store before the last has left its buffer
+            asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        __syncwarp();
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            uint4 w;
+            if constexpr (EPI == EPI_STORE_F32)
+                w = make_uint4(__float_as_uint(f[4 * j]), __float_as_uint(f[4 * j + 1]), __float_as_uint(f[4 * j + 2]),
+                               __float_as_uint(f[4 * j + 3]));
+            else
+                w = make_uint4(pack_bf16x2(f[8 * j], f[8 * j + 1]), pack_bf16x2(f[8 * j + 2], f[8 * j + 3]),
+                               pack_bf16x2(f[8 * j + 4], f[8 * j + 5]), pack_bf16x2(f[8 * j + 6], f[8 * j + 7]));
+            *reinterpret_cast<uint4*>(buf + lane * 64 + ((j ^ (lane >> 1 & 3)) << 4)) = w;
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
+                             reinterpret_cast<uint64_t>(map_o)),
+                         "r"(smem_u32(buf)), "r"(col0 + at), "r"(row0 + quad * 32)
+                         : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+    }
+}
+
+template <int EPI, bool TMA>
 __global__ void __launch_bounds__(kDnThreads, 1)
 gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                       const TcParams p, const uint32_t tiles_m, const uint32_t tiles_n, const uint32_t bn)
+                       const __grid_constant__ CUtensorMap map_o, const TcParams p, const uint32_t tiles_m, const uint32_t tiles_n, const uint32_t bn)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kDnStages * kDnStageBytes);
-    uint64_t* empty_bar = full_bar + kDnStages;
-    uint64_t* acc_full = empty_bar + kDnStages;
+    uint8_t* staging = smem + kDnRing; // [8 warps][2]
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(staging + (TMA ? kDnStaging : 0));
+    uint64_t* empty_bar = full_bar + kDnMaxStages;
+    uint64_t* acc_full = empty_bar + kDnMaxStages;
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     volatile uint32_t* abort_flag = tmem_slot + 1;
+    const uint32_t stage_bytes = kTileBytes + bn * 128, stages = dense_stages(bn);
 
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t total = tiles_m * tiles_n;
 
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < kDnStages; ++s) {
+        for (uint32_t s = 0; s < stages; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
@@ -97,13 +175,13 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                         ok = false;
                         break;
                     }
-                    uint8_t* sa = smem + s * kDnStageBytes;
-                    mbar_expect_tx(&full_bar[s], kTileBytes + bn * 128);
+                    uint8_t* sa = smem + s * stage_bytes;
+                    mbar_expect_tx(&full_bar[s], stage_bytes);
                     const int c0 = static_cast<int>(kb) * 64;
                     tma_load_2d(sa, &map_a, &full_bar[s], c0, row0);
                     tma_load_2d(sa + kTileBytes, &map_b, &full_bar[s], c0, col0);
                     tma_load_2d(sa + kTileBytes + bn * 64, &map_b, &full_bar[s], c0, col0 + static_cast<int>(bn / 2));
-                    if (++s == kDnStages) {
+                    if (++s == stages) {
                         s = 0;
                         ph ^= 1;
                     }
@@ -129,14 +207,14 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(smem + s * kDnStageBytes);
+                    const uint32_t sa = smem_u32(smem + s * stage_bytes);
                     const uint64_t da = operand_desc(sa);
                     const uint64_t db = operand_desc(sa + kTileBytes); // bn rows: two tiles back to back
 #pragma unroll
                     for (uint32_t j = 0; j < 4; ++j)
                         tc_mma_bf16(d, da + 2 * j, db + 2 * j, idesc, (kb > 0 || j > 0) ? 1u : 0u);
                     tc_commit(&empty_bar[s]);
-                    if (++s == kDnStages) {
+                    if (++s == stages) {
                         s = 0;
                         ph ^= 1;
                     }
@@ -147,7 +225,7 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
     } else {
         // ------------------------------------------------------------ epilogue --
-        uint32_t u = 0;
+        uint32_t u = 0, stores = 0;
         for (uint32_t t = blockIdx.x; t < total; t += gridDim.x, ++u) {
             const uint32_t buf = u & 1;
             const bool ready = __all_sync(
@@ -155,24 +233,15 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             if (!ready)
                 break;
             tc_fence_after();
-            const int row0 = static_cast<int>((t % tiles_m) * kBM);
-            const int nrows = min(kBM, static_cast<int>(p.dense_rows) - row0);
-            // the tile's columns as a problem of their own: the epilogue works in units of 128 of them
-            const uint32_t col0 = (t / tiles_m) * bn;
-            TcParams q = p;
-            q.n = min(bn, p.n - col0);
-            q.out = static_cast<uint8_t*>(p.out) + static_cast<uint64_t>(col0) * (EPI == EPI_STORE_F32 ? 4 : 2);
-            if (p.bias != nullptr)
-                q.bias = p.bias + col0;
-#pragma unroll
-            for (uint32_t h = 0; h < 2; ++h)
-                epilogue_tile<false, EPI, 2>(q, tmem_base + buf * kDnBN + h * kBN, warp & 3, lane, 0, row0, nrows, h,
-                                             warp >> 2);
+            dense_epilogue<EPI, TMA>(p, &map_o, staging + warp * 2 * kDnOutBytes, stores, tmem_base + buf * kDnBN, warp, lane,
+                                (t % tiles_m) * kBM, (t / tiles_m) * bn, bn);
             tc_fence_before();
             __syncwarp();
             if (lane == 0)
                 mbar_arrive(&acc_empty[buf]);
         }
+        if (lane == 0)
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); // the stores have left shared memory
     }
 
     tc_fence_before();
@@ -201,7 +270,6 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 constexpr uint32_t kPrKbs = 2;                              // k blocks (of 64) per stage
 constexpr uint32_t kPrStageBytes = kPrKbs * 2 * kTileBytes; // per CTA and k block: A 128 x 64, B 128 x 64
 constexpr uint32_t kPrStages = 3;
-constexpr uint64_t kPrMinTiles = 74;
 
 __device__ __forceinline__ uint32_t cluster_addr(const void* local, uint32_t cta_rank)
 {
@@ -231,10 +299,11 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster_addr)
                  : "memory");
 }
 
-template <int EPI>
+template <int EPI, bool TMA>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kDnThreads, 1)
 gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                       const TcParams p, const uint32_t tiles_m, const uint32_t tiles_n)
+                       const __grid_constant__ CUtensorMap map_o, const TcParams p, const uint32_t tiles_m,
+                       const uint32_t tiles_n, const uint32_t bn)
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -242,7 +311,8 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + kPrStages * kPrStageBytes);
+    uint8_t* staging = smem + kPrStages * kPrStageBytes; // [8 warps][2]
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(staging + (TMA ? kDnStaging : 0));
     uint64_t* empty_bar = full_bar + kPrStages;
     uint64_t* acc_full = empty_bar + kPrStages;
     uint64_t* acc_empty = acc_full + 2;
@@ -287,7 +357,7 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             bool ok = true;
             for (uint32_t t = pair; t < total && ok; t += pairs) {
                 const int row0 = static_cast<int>((t % tiles_m) * 256 + rank * 128);
-                const int col0 = static_cast<int>((t / tiles_m) * 256 + rank * 128);
+                const int col0 = static_cast<int>((t / tiles_m) * bn + rank * (bn / 2));
                 for (uint32_t kb = 0; kb < p.k_blocks; kb += kPrKbs) {
                     if (!mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_DN_EMPTY_WAIT)) {
                         ok = false;
@@ -296,7 +366,7 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                     const uint32_t nkb = min(kPrKbs, p.k_blocks - kb);
                     uint8_t* sa = smem + s * kPrStageBytes;
                     if (rank == 0)
-                        mbar_expect_tx(&full_bar[s], nkb * 4 * kTileBytes); // both CTAs' A and B tiles
+                        mbar_expect_tx(&full_bar[s], nkb * (2 * kTileBytes + bn * 128)); // both CTAs' A and B tiles
                     const uint32_t bar = cluster_addr(&full_bar[s], 0);
                     for (uint32_t q = 0; q < nkb; ++q) {
                         const int c0 = static_cast<int>(kb + q) * 64;
@@ -313,8 +383,8 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     } else if (warp == 9) {
         // ---------------------------------------------------------- MMA issuer --
         if (rank == 0 && elect_one()) {
-            // M = 256 (128 rows in each CTA), N = 256 (128 B rows from each CTA)
-            constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
+            // M = 256 (128 rows in each CTA), N = bn (half of the B rows from each CTA)
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((bn >> 3) << 17) | ((256u >> 4) << 24);
             uint32_t s = 0, ph = 0, u = 0;
             bool ok = true;
             for (uint32_t t = pair; t < total && ok; t += pairs, ++u) {
@@ -339,7 +409,7 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                             const uint32_t acc = (kb + q > 0 || j > 0) ? 1u : 0u;
                             asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t"
                                          "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, q;\n\t}" ::"r"(d),
-                                         "l"(da + 2 * j), "l"(db + 2 * j), "r"(kIdesc), "r"(acc)
+                                         "l"(da + 2 * j), "l"(db + 2 * j), "r"(idesc), "r"(acc)
                                          : "memory");
                         }
                     }
@@ -358,7 +428,7 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
     } else {
         // ------------------------------------------------------------ epilogue --
-        uint32_t u = 0;
+        uint32_t u = 0, stores = 0;
         for (uint32_t t = pair; t < total; t += pairs, ++u) {
             const uint32_t buf = u & 1;
             const bool ready = __all_sync(
@@ -366,18 +436,17 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             if (!ready)
                 break;
             tc_fence_after();
-            const int row0 = static_cast<int>((t % tiles_m) * 256 + rank * 128);
-            const int nrows = min(kBM, static_cast<int>(p.dense_rows) - row0);
-            const uint32_t nt = (t / tiles_m) * 2;
-#pragma unroll
-            for (uint32_t h = 0; h < 2; ++h)
-                epilogue_tile<false, EPI, 2>(p, tmem_base + buf * kDnBN + h * kBN, warp & 3, lane, 0, row0, nrows,
-                                             nt + h, warp >> 2);
+            const uint32_t row0 = (t % tiles_m) * 256 + rank * 128;
+            if (row0 < p.dense_rows)
+                dense_epilogue<EPI, TMA>(p, &map_o, staging + warp * 2 * kDnOutBytes, stores, tmem_base + buf * kDnBN, warp, lane, row0,
+                                    (t / tiles_m) * bn, bn);
             tc_fence_before();
             __syncwarp();
             if (lane == 0)
                 mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0));
         }
+        if (lane == 0)
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); // the stores have left shared memory
     }
 
     tc_fence_before();
@@ -389,12 +458,12 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
 }
 
-template <int EPI>
-cudaError_t launch_pair_instance(const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& tp, uint32_t tiles_m,
-                                 uint32_t tiles_n, cudaStream_t stream)
+template <int EPI, bool TMA>
+cudaError_t launch_pair_instance(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const TcParams& tp,
+                                 uint32_t tiles_m, uint32_t tiles_n, uint32_t bn, cudaStream_t stream)
 {
-    auto kernel = gemm_dense_pair_kernel<EPI>;
-    constexpr size_t smem = 1024 + kPrStages * kPrStageBytes + 256;
+    auto kernel = gemm_dense_pair_kernel<EPI, TMA>;
+    constexpr size_t smem = 1024 + kPrStages * kPrStageBytes + (TMA ? kDnStaging : 0) + 256;
     static bool configured[64] = {};
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
@@ -408,15 +477,15 @@ cudaError_t launch_pair_instance(const CUtensorMap& ma, const CUtensorMap& mb, c
             configured[dev] = true;
     }
     const uint32_t pairs = std::min(tiles_m * tiles_n, device_sm_count() / 2);
-    return launch_chained(kernel, dim3(2 * pairs), kDnThreads, smem, stream, ma, mb, tp, tiles_m, tiles_n);
+    return launch_chained(kernel, dim3(2 * pairs), kDnThreads, smem, stream, ma, mb, mo, tp, tiles_m, tiles_n, bn);
 }
 
-template <int EPI>
-cudaError_t launch_dense_instance(const CUtensorMap& ma, const CUtensorMap& mb, const TcParams& tp, uint32_t tiles_m,
-                                  uint32_t tiles_n, uint32_t bn, cudaStream_t stream)
+template <int EPI, bool TMA>
+cudaError_t launch_dense_instance(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const TcParams& tp,
+                                  uint32_t tiles_m, uint32_t tiles_n, uint32_t bn, cudaStream_t stream)
 {
-    auto kernel = gemm_dense_bf16_kernel<EPI>;
-    constexpr size_t smem = 1024 + kDnStages * kDnStageBytes + 256;
+    auto kernel = gemm_dense_bf16_kernel<EPI, TMA>;
+    constexpr size_t smem = 1024 + kDnRing + (TMA ? kDnStaging : 0) + 256;
     static bool configured[64] = {};
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
@@ -430,23 +499,60 @@ cudaError_t launch_dense_instance(const CUtensorMap& ma, const CUtensorMap& mb, 
             configured[dev] = true;
     }
     const uint32_t grid = std::min(tiles_m * tiles_n, device_sm_count());
-    return launch_chained(kernel, dim3(grid), kDnThreads, smem, stream, ma, mb, tp, tiles_m, tiles_n, bn);
+    return launch_chained(kernel, dim3(grid), kDnThreads, smem, stream, ma, mb, mo, tp, tiles_m, tiles_n, bn);
 }
 
 } // namespace
 
 bool gemm_dense_bf16_supported(const GemmProblem& g)
 {
-    return !g.nvfp4 && !g.gated && g.tile_expert == nullptr && g.groups == 1 && g.a_rows > 64 && g.k % 64 == 0
-        && g.k >= 64 && g.n >= 128 && (g.epilogue == EPI_STORE_BF16 || g.epilogue == EPI_STORE_F32)
+    return !g.nvfp4 && !g.gated && g.tile_expert == nullptr && g.groups == 1 && g.group_scale == nullptr && g.a_rows > 64
+        && g.k % 64 == 0 && g.k >= 64 && g.n >= 128 && (g.epilogue == EPI_STORE_BF16 || g.epilogue == EPI_STORE_F32)
         && (reinterpret_cast<uintptr_t>(g.a) & 15u) == 0 && (reinterpret_cast<uintptr_t>(g.b) & 15u) == 0
         && g.a_pitch_bytes % 16 == 0 && g.b_pitch_bytes % 16 == 0
-        && (g.a_rows + kBM - 1) / kBM * ((g.n + kDnBN - 1) / kDnBN) < (1ull << 31)
-        // with fewer tiles than this the 128 x 128 kernel spreads the problem over more SMs
-        && (g.a_rows + kBM - 1) / kBM * ((g.n + kDnBN - 1) / kDnBN) >= kDnMinTiles;
+        && (g.a_rows + kBM - 1) / kBM * ((g.n + 31ull) / 32) < (1ull << 31);
 }
 
-cudaError_t launch_gemm_dense_bf16(const GemmProblem& g, cudaStream_t stream, const char** why)
+// What computes a dense problem of more than 64 rows: the kernel, and the columns (rows of A for the split one) of a tile, by
+// an estimate of its time in microseconds. Fitted to 72..3001 rows, k 512..4096, 512..8192 features, operands from HBM, which it
+// meets within a tenth; what it has to get right is the order. A CTA's operands come through a ring that holds 192 KB, a trip
+// of 1.1 us, so a k block takes 1.1 us / stages however few SMs work: narrow tiles are quick by themselves, wide ones move
+// fewer bytes, and the rounds of the SMs decide between them.
+//   one CTA per tile of 128 x c   2.9 + c / 80 + rounds (1 + k blocks (1.1 / stages + 0.0003 c))
+//   a pair of CTAs, 256 x c       6.8 + rounds (1.5 + k blocks (0.15 + 0.00062 c)), a round not under the 3.5 c / 256 that
+//                                 its output takes
+//   split k (gemm_splitk.cu)      bf16 results only: f32 results have their own choice there
+// Before, by the number of 128 x 256 tiles: 300 x 4096 x 4096 27.1 -> 18.0 us, 1200 x 4096 x 4096 46.3 -> 37.6,
+// 800 x 4096 x 2048 26.0 -> 18.0, 200 x 512 x 2048 6.9 -> 5.7, 2000 x 512 x 8192 26.9 -> 23.
+DenseChoice gemm_dense_choice(const GemmProblem& g)
+{
+    const uint32_t sms = device_sm_count();
+    const float kb = static_cast<float>(g.k / 64);
+    const auto rounds = [](uint64_t tiles, uint32_t at_once) { return static_cast<float>((tiles + at_once - 1) / at_once); };
+    const uint64_t tiles_m = (g.a_rows + kBM - 1) / kBM, pair_m = (g.a_rows + 255) / 256;
+    DenseChoice best { DENSE_ONE, kDnBN };
+    float least = 1e30f;
+    const auto offer = [&](DenseKernel kernel, uint32_t width, float time) {
+        if (time < least) {
+            least = time;
+            best = { kernel, width };
+        }
+    };
+    for (uint32_t c = kDnBN; c >= 32; c -= 16) {
+        const float r = rounds(tiles_m * ((g.n + c - 1) / c), sms);
+        offer(DENSE_ONE, c, 2.9f + 0.0125f * c + r * (1.0f + kb * (1.1f / dense_stages(c) + 0.0003f * c)));
+    }
+    for (uint32_t c = 256; c >= 128; c -= 32) {
+        const float r = rounds(pair_m * ((g.n + c - 1) / c), sms / 2);
+        offer(DENSE_PAIR, c, 6.8f + r * (1.5f + std::max(kb * (0.15f + 0.00062f * c), 3.5f * c / 256)));
+    }
+    if (g.epilogue == EPI_STORE_BF16)
+        for (uint32_t nt : { 64u, 96u, 128u })
+            offer(DENSE_SPLIT, nt, gemm_splitk_estimate(g, nt));
+    return best;
+}
+
+cudaError_t launch_gemm_dense_bf16(const GemmProblem& g, DenseChoice choice, cudaStream_t stream, const char** why)
 {
     TcParams tp {};
     tp.n = g.n;
@@ -460,39 +566,32 @@ cudaError_t launch_gemm_dense_bf16(const GemmProblem& g, cudaStream_t stream, co
     tp.bias = g.bias;
     tp.err = device_error_word();
     const uint32_t tiles_m = static_cast<uint32_t>((g.a_rows + kBM - 1) / kBM);
-    // enough 256 x 256 tiles to give every CTA pair work: two SMs per tile, B shared between them
-    const uint32_t pair_m = static_cast<uint32_t>((g.a_rows + 255) / 256), pair_n = (g.n + 255) / 256;
-    const bool pair = static_cast<uint64_t>(pair_m) * pair_n >= kPrMinTiles && g.a_rows >= 1024;
-    // columns per tile: rounds of the SMs x columns, the narrower tiles charged for moving A more often
-    uint32_t bn = kDnBN;
-    if (!pair) {
-        uint64_t best = ~0ull;
-        for (uint32_t c = kDnBN; c >= 160; c -= 16) {
-            const uint64_t tiles = static_cast<uint64_t>(tiles_m) * ((g.n + c - 1) / c);
-            const uint64_t cost = (tiles + device_sm_count() - 1) / device_sm_count() * (c + 128);
-            if (cost < best) {
-                best = cost;
-                bn = c;
-            }
-        }
-    }
-    const uint32_t tiles_n = (g.n + bn - 1) / bn;
+    const bool pair = choice.kernel == DENSE_PAIR;
+    const uint32_t pair_m = static_cast<uint32_t>((g.a_rows + 255) / 256);
+    const uint32_t bn = choice.width, tiles_n = (g.n + bn - 1) / bn;
     // Several row tiles read a B panel from neighbouring SMs; over several rounds a chained start, which lets the next problem
     // begin on the SMs that are done first, sets them out of step (156 rows x 2048 x 151936, 8 rounds: 0.152 against 0.146 ms;
     // 300 x 4096 x 50000, 4 rounds: 0.129 against 0.125). In one or two it pays (1000 x 512 x 8192: 0.0114, unchained 0.0123).
     const UnchainedScope in_step(tiles_m > 1 && static_cast<uint64_t>(tiles_m) * tiles_n > 3ull * device_sm_count());
     CUtensorMap ma, mb;
     if (!make_operand_map(&ma, false, g.a, g.k, g.a_rows, g.a_pitch_bytes, kBM)
-        || !make_operand_map(&mb, false, g.b, g.k, g.n, g.b_pitch_bytes, pair ? 128 : bn / 2)) {
+        || !make_operand_map(&mb, false, g.b, g.k, g.n, g.b_pitch_bytes, bn / 2)) {
         if (why != nullptr)
             *why = "cuTensorMapEncodeTiled failed";
         return cudaErrorInvalidValue;
     }
+    CUtensorMap mo = ma;
+    const bool f32 = g.epilogue == EPI_STORE_F32;
+    // In a single round nothing hides the way through shared memory, and a smaller block starts sooner: 200 x 512 x 4096
+    // 5.0 us, stored directly 4.7; 845 x 512 x 4096 8.3 / 7.6. Not so f32 results (1021 x 2048 x 512: 8.9 / 9.3).
+    const bool several = pair || f32 || static_cast<uint64_t>(tiles_m) * tiles_n > device_sm_count();
+    const bool tma = several && g.beta == 0.0f && make_output_map(&mo, f32, g.out, g.n, g.a_rows, g.out_pitch_elems);
+    const auto launch = [&](auto kernel, uint32_t rows) { return kernel(ma, mb, mo, tp, rows, tiles_n, bn, stream); };
     if (pair)
-        return g.epilogue == EPI_STORE_F32 ? launch_pair_instance<EPI_STORE_F32>(ma, mb, tp, pair_m, pair_n, stream)
-                                           : launch_pair_instance<EPI_STORE_BF16>(ma, mb, tp, pair_m, pair_n, stream);
-    return g.epilogue == EPI_STORE_F32 ? launch_dense_instance<EPI_STORE_F32>(ma, mb, tp, tiles_m, tiles_n, bn, stream)
-                                       : launch_dense_instance<EPI_STORE_BF16>(ma, mb, tp, tiles_m, tiles_n, bn, stream);
+        return tma ? launch(f32 ? launch_pair_instance<EPI_STORE_F32, true> : launch_pair_instance<EPI_STORE_BF16, true>, pair_m)
+                   : launch(f32 ? launch_pair_instance<EPI_STORE_F32, false> : launch_pair_instance<EPI_STORE_BF16, false>, pair_m);
+    return tma ? launch(f32 ? launch_dense_instance<EPI_STORE_F32, true> : launch_dense_instance<EPI_STORE_BF16, true>, tiles_m)
+               : launch(f32 ? launch_dense_instance<EPI_STORE_F32, false> : launch_dense_instance<EPI_STORE_BF16, false>, tiles_m);
 }
 
 } // namespace qs3

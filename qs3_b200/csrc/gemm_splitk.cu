@@ -33,7 +33,8 @@ namespace {
 
 using namespace tc;
 
-constexpr uint32_t kSkStages = 4;
+constexpr uint32_t kSkMaxStages = 8;
+constexpr uint32_t kSkRing = 192 * 1024; // shared memory of the stages, at most
 constexpr uint32_t kSkMaxSplits = 8; // the largest portable cluster
 constexpr uint32_t kSkPitch = 132; // floats per row of the partial tile
 
@@ -47,6 +48,7 @@ enum : uint32_t {
 struct SplitkParams {
     uint32_t m, n;
     uint32_t k_blocks, kb_per_split;
+    uint32_t stages;
     void* out;
     uint64_t out_pitch;
     float alpha, beta;
@@ -56,9 +58,12 @@ struct SplitkParams {
 
 template <int NT> struct SkSmem {
     static constexpr uint32_t kStageBytes = kTileBytes + NT * 128;
-    static constexpr uint32_t kRing = kSkStages * kStageBytes;
     static constexpr uint32_t kPartial = NT * kSkPitch * 4;
-    static constexpr uint32_t kBytes = kRing > kPartial ? kRing : kPartial;
+    static constexpr uint32_t kMostStages = kSkRing / kStageBytes < kSkMaxStages ? kSkRing / kStageBytes : kSkMaxStages;
+    __host__ __device__ static uint32_t bytes(uint32_t stages)
+    {
+        return stages * kStageBytes > kPartial ? stages * kStageBytes : kPartial;
+    }
 };
 
 // How the products of a row are summed (see above).
@@ -68,7 +73,7 @@ enum SkSum { SUM_CHAIN = 0, SUM_SHORT_CHAINS = 1, SUM_COMPENSATED = 2 };
 template <int NT, int SUM> struct SkTmem {
     static constexpr uint32_t kBufs = SUM == SUM_CHAIN ? 1 : NT <= 32 ? 4 : 2;
     static constexpr uint32_t kUsed = SUM == SUM_CHAIN ? NT : 2 * NT * kBufs;
-    static constexpr uint32_t kCols = kUsed < 32 ? 32 : kUsed;
+    static constexpr uint32_t kCols = kUsed <= 32 ? 32 : kUsed <= 64 ? 64 : kUsed <= 128 ? 128 : 256; // a power of two
     // warps that empty them, in fours, one per quarter of the lanes; compensated sums take a warp for 16 columns
     static constexpr uint32_t kAdders = SUM == SUM_COMPENSATED ? NT / 4 : 4;
     static constexpr uint32_t kThreads = (kAdders + 2) * 32;
@@ -114,9 +119,9 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     float* part = reinterpret_cast<float*>(smem); // [NT][kSkPitch], after the ring
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + SkSmem<NT>::kBytes);
-    uint64_t* empty_bar = full_bar + kSkStages;
-    uint64_t* acc_full = empty_bar + kSkStages;
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + SkSmem<NT>::bytes(p.stages));
+    uint64_t* empty_bar = full_bar + kSkMaxStages;
+    uint64_t* acc_full = empty_bar + kSkMaxStages;
     uint64_t* acc_empty = acc_full + kBufs; // short chains
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + kBufs);
     volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -127,7 +132,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
     const uint32_t kb0 = min(rank * p.kb_per_split, p.k_blocks), kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
 
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < kSkStages; ++s) {
+        for (uint32_t s = 0; s < p.stages; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
@@ -155,8 +160,8 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
     if (warp == 4) {
         // ------------------------------------------------------------ producer --
         if (elect_one()) {
+            uint32_t s = 0, ph = 0;
             for (uint32_t i = 0; i < kb1 - kb0; ++i) {
-                const uint32_t s = i % kSkStages, ph = (i / kSkStages) & 1;
                 if (!mbar_wait<true>(&empty_bar[s], ph ^ 1, abort_flag, p.err, ERR_SK_EMPTY_WAIT))
                     break;
                 uint8_t* sb = smem + s * kStageBytes;
@@ -164,6 +169,10 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
                 const int c0 = static_cast<int>(kb0 + i) * 64;
                 tma_load_2d(sb, &map_b, &full_bar[s], c0, static_cast<int>(n0));
                 tma_load_2d(sb + kTileBytes, &map_a, &full_bar[s], c0, static_cast<int>(m0));
+                if (++s == p.stages) {
+                    s = 0;
+                    ph ^= 1;
+                }
             }
         }
     } else if (warp == 5) {
@@ -173,8 +182,9 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
             constexpr uint32_t kIdesc
                 = (1u << 4) | (1u << 7) | (1u << 10) | ((static_cast<uint32_t>(NT) >> 3) << 17) | ((kBM >> 4) << 24);
             bool ok = true;
+            uint32_t s = 0, ph = 0;
             for (uint32_t i = 0; i < kb1 - kb0; ++i) {
-                const uint32_t s = i % kSkStages, ph = (i / kSkStages) & 1, b = i % kBufs;
+                const uint32_t b = i % kBufs;
                 if (SUM != SUM_CHAIN && !mbar_wait<true>(&acc_empty[b], ((i / kBufs) & 1) ^ 1, abort_flag, p.err, ERR_SK_ACC_EMPTY_WAIT)) {
                     ok = false;
                     break;
@@ -193,6 +203,10 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
                 tc_commit(&empty_bar[s]);
                 if (SUM != SUM_CHAIN)
                     tc_commit(&acc_full[b]);
+                if (++s == p.stages) {
+                    s = 0;
+                    ph ^= 1;
+                }
             }
             if (ok && SUM == SUM_CHAIN)
                 tc_commit(acc_full);
@@ -337,19 +351,31 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
     }
 }
 
+// A CTA alone on its SM takes as many stages as the k blocks of a rank can use (72 x 4096 x 4096: four stages 0.0163 ms,
+// eight 0.0136). Two share an SM when there are more tiles than SMs, and when clusters of four or eight would take most of the
+// SMs, since not every one finds its SMs free side by side then (33 x 4096 x 2048, 16 clusters of eight: 0.0133 ms with eight
+// stages, 0.0090 with four; 809 x 4096 x 512, 36 of four: 0.0159 against 0.0118 with fewer tiles).
+uint32_t splitk_stages(uint32_t nt, uint64_t tiles, uint32_t splits, uint32_t kb_per_split)
+{
+    const uint64_t ctas = tiles * splits, sms = device_sm_count();
+    const bool alone = ctas <= (splits < 4 ? sms : splits == 4 ? sms * 7 / 8 : sms * 3 / 4);
+    return std::min({ alone ? kSkMaxStages : 4u, kSkRing / (kTileBytes + nt * 128), kb_per_split });
+}
+
 template <int NT, bool F32, int SUM>
-cudaError_t launch_splitk_instance(const CUtensorMap& mb, const CUtensorMap& ma, const SplitkParams& sp, dim3 grid,
+cudaError_t launch_splitk_instance(const CUtensorMap& mb, const CUtensorMap& ma, SplitkParams sp, dim3 grid,
                                    cudaStream_t stream)
 {
     auto kernel = gemm_splitk_kernel<NT, F32, SUM>;
-    constexpr size_t smem = 1024 + SkSmem<NT>::kBytes + 256;
+    sp.stages = splitk_stages(NT, static_cast<uint64_t>(grid.y) * grid.z, grid.x, sp.kb_per_split);
+    const size_t smem = 1024 + SkSmem<NT>::bytes(sp.stages) + 256, most = 1024 + SkSmem<NT>::bytes(SkSmem<NT>::kMostStages) + 256;
     static bool configured[64] = {}; // per instantiation and device
     int dev = 0;
     cudaError_t err = cudaGetDevice(&dev);
     if (err != cudaSuccess)
         return err;
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most));
         if (err != cudaSuccess)
             return err;
         if (dev >= 0 && dev < 64)
@@ -386,6 +412,19 @@ SkSum splitk_sum(const GemmProblem& g, uint32_t nt)
                                                  : SUM_CHAIN;
 }
 
+// As many splits as fit one CTA per SM, two k blocks each at least; none for compensated sums of a short k, which a
+// rounding per rank would leave further off (64 x 512 x 512: 6.4e-8, 5.8e-8 unsplit, on CUDA cores 6.2e-8).
+uint32_t splitk_splits(const GemmProblem& g, uint32_t nt)
+{
+    const uint64_t tiles = splitk_tiles(g, nt);
+    const uint32_t k_blocks = (g.k + 63) / 64;
+    uint32_t splits = 1;
+    while (splits < kSkMaxSplits && 2 * splits * tiles <= device_sm_count() && 2 * (2 * splits) <= k_blocks
+           && (splitk_sum(g, nt) != SUM_COMPENSATED || k_blocks > 8))
+        splits *= 2;
+    return splits;
+}
+
 // Tile rows of a problem that this kernel takes, 0: it does not. At least two CTAs per tile without exceeding one CTA
 // per SM, since more tiles fill the device as they are; a long k is split with 128-row tiles too (2048 x 4096 x 512:
 // 0.0207 against 0.0269 ms for the 128 x 256 kernel, but 512 x 2048 x 2048: 0.0163 against 0.0145).
@@ -412,7 +451,17 @@ bool gemm_splitk_supported(const GemmProblem& g)
         && splitk_choice(g) != 0;
 }
 
-cudaError_t launch_gemm_splitk(const GemmProblem& g, cudaStream_t stream, const char** why)
+// 200 x 4096 x 2048, 64 rows a tile: 11.8 us both; 130 x 4096 x 2048, 96 rows: 11.1, measured 10.5.
+float gemm_splitk_estimate(const GemmProblem& g, uint32_t nt)
+{
+    if (splitk_tiles(g, nt) > device_sm_count())
+        return 1e30f;
+    const uint32_t splits = splitk_splits(g, nt), kbs = ((g.k + 63) / 64 + splits - 1) / splits;
+    const uint32_t stages = splitk_stages(nt, splitk_tiles(g, nt), splits, 8);
+    return 4.6f + 0.028f * nt + kbs * (1.1f / stages + 0.0003f * nt + 0.01f);
+}
+
+cudaError_t launch_gemm_splitk(const GemmProblem& g, uint32_t rows, cudaStream_t stream, const char** why)
 {
     SplitkParams sp {};
     sp.m = static_cast<uint32_t>(g.a_rows);
@@ -424,14 +473,9 @@ cudaError_t launch_gemm_splitk(const GemmProblem& g, cudaStream_t stream, const 
     sp.beta = g.beta;
     sp.bias = g.bias;
     sp.err = device_error_word();
-    const uint32_t nt = splitk_choice(g);
+    const uint32_t nt = rows != 0 ? rows : splitk_choice(g);
     const uint64_t tiles = splitk_tiles(g, nt);
-    // as many splits as fit one CTA per SM, two k blocks each at least; none for compensated sums of a short k, which a
-    // rounding per rank would leave further off (64 x 512 x 512: 6.4e-8, 5.8e-8 unsplit, on CUDA cores 6.2e-8)
-    uint32_t splits = 1;
-    while (splits < kSkMaxSplits && 2 * splits * tiles <= device_sm_count() && 2 * (2 * splits) <= sp.k_blocks
-           && (splitk_sum(g, nt) != SUM_COMPENSATED || sp.k_blocks > 8))
-        splits *= 2;
+    const uint32_t splits = splitk_splits(g, nt);
     sp.kb_per_split = (sp.k_blocks + splits - 1) / splits;
     CUtensorMap mb, ma;
     if (!make_operand_map(&mb, false, g.b, g.k, g.n, g.b_pitch_bytes, 128)
@@ -446,6 +490,7 @@ cudaError_t launch_gemm_splitk(const GemmProblem& g, cudaStream_t stream, const 
         return launch(nt == 16 ? launch_splitk_instance<16, false, SUM_CHAIN>
             : nt == 32         ? launch_splitk_instance<32, false, SUM_CHAIN>
             : nt == 64         ? launch_splitk_instance<64, false, SUM_CHAIN>
+            : nt == 96         ? launch_splitk_instance<96, false, SUM_CHAIN>
                                : launch_splitk_instance<128, false, SUM_CHAIN>);
     switch (splitk_sum(g, nt)) {
     case SUM_COMPENSATED:

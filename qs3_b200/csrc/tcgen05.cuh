@@ -55,6 +55,9 @@ struct TcParams {
 } // namespace tc
 bool make_operand_map(CUtensorMap* map, bool bytes_type, const void* base, uint64_t inner_elems, uint64_t rows,
                       uint64_t pitch_bytes, uint32_t box_rows);
+// Row-major output [rows, cols] written by TMA in boxes of 32 rows x 64 bytes (64-byte swizzle). False: not addressable
+// (TMA clips a row in units of 16 bytes: columns that end inside one would write past it).
+bool make_output_map(CUtensorMap* map, bool f32, void* out, uint64_t cols, uint64_t rows, uint64_t pitch_elems);
 namespace tc {
 
 // ---- PTX wrappers -------------------------------------------------------------------

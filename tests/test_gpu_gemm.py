@@ -204,3 +204,30 @@ def test_dense_kernel_edges_and_epilogue(gemm, shape, out_dtype):
     else:
         assert np.all(np.abs(got[:, :n] - want) <= np.abs(want) * 2.0 ** -7 + 2e-3)
     assert np.all(got[:, n:] == 5.0)
+
+
+# Outputs gathered in shared memory and written by TMA: last tiles of 8 columns and of one row, a row pitch beyond the
+# columns, columns that end inside 16 bytes (stored row by row instead); tiles of 32 to 256 columns by one CTA or two, and
+# split k with as many stages as a rank has k blocks.
+@pytest.mark.parametrize("shape", [(129, 64, 136, 0), (72, 512, 4096, 8), (300, 512, 2504, 8), (257, 128, 2500, 12),
+                                   (500, 2048, 2048, 0), (1290, 192, 2561, 7), (1025, 2048, 4104, 24), (2049, 512, 4096, 0),
+                                   (130, 4096, 2048, 0), (80, 4096, 512, 16), (190, 704, 520, 8)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+def test_dense_output_edges(gemm, shape, out_dtype, beta):
+    rows, k, n, pad = shape
+    gen = torch.Generator().manual_seed(rows + n)
+    x = torch.randn((rows, k), generator=gen).to(torch.bfloat16)
+    w = torch.randn((n, k), generator=gen).to(torch.bfloat16)
+    full = torch.full((rows + 2, n + pad), 7.0, dtype=out_dtype, device="cuda")
+    gemm.gemm_bf16(x.cuda(), w.cuda(), full[:rows, :n], alpha=0.5, beta=beta)
+    got = full.cpu()
+    assert torch.all(got[rows:] == 7.0) and torch.all(got[:, n:] == 7.0)
+    # products of bf16 are exact in f32. The tensor core drops what lies below 2^-24 or so of an accumulator each time it adds
+    # one of k / 16 terms: k / 16 * 2^-24 of the sum of the magnitudes bounds that; a bf16 result is then rounded by 2^-9.
+    want = 0.5 * (x.double() @ w.double().T) + beta * 7.0
+    size = 0.5 * (x.double().abs() @ w.double().abs().T) + beta * 7.0
+    bound = size * (k / 16 + 4) * 2.0 ** -24
+    if out_dtype == torch.bfloat16:
+        bound += want.abs() * 2.0 ** -8
+    assert torch.all((got[:rows, :n].double() - want).abs() <= bound)
