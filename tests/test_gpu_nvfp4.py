@@ -273,6 +273,28 @@ def test_decode_batches_take_the_swapped_operand_kernel(ops, ctx, oracle, cfg):
     _check(to_np(out), ref)
 
 
+# panels whose rows do not divide the loaders' vectors (three and five blocks of 256 elements), tiles of one row to all,
+# rows beside multiples of four, an expert of several tiles
+@pytest.mark.parametrize("t,e,k,h,i,hot,rows", [(37, 16, 2, 768, 256, False, 32), (67, 16, 2, 1280, 768, True, 64),
+                                                (100, 32, 6, 1280, 256, False, 64), (5, 64, 5, 768, 256, False, 32)])
+def test_small_tile_panels(ops, ctx, oracle, t, e, k, h, i, hot, rows):
+    d = make_moe_inputs(71, t, h, e, i)
+    gu, dn, _ = _quantise_all(ops, ctx, d, False)
+    plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=t, hidden_size=h, intermediate_size=i, num_experts=e, top_k=k,
+                                              backend=ops.capi.MOE_BACKEND_NVFP4))
+    ws = torch.zeros(plan.layer_workspace_size(t, 0), dtype=torch.uint8, device="cuda")
+    ids = torch.empty((t, k), dtype=torch.int32, device="cuda")
+    w = torch.empty((t, k), dtype=torch.float32, device="cuda")
+    out = torch.empty((t, h), dtype=torch.bfloat16, device="cuda")
+    ops.moe_layer_execute(plan, to_dev(d["hidden"]), to_dev(d["router"]), gu, dn, out, ws, topk_ids=ids, topk_weights=w,
+                          router_bias=to_dev(_hot_bias(e)) if hot else None)
+    torch.cuda.synchronize()
+    assert ctx.read_device_error() == 0
+    assert tile_height(plan, ws, t) == rows
+    hp, hs = oracle.nvfp4_quantize_act(d["hidden"], 1.0)
+    _check(to_np(out), oracle.moe_nvfp4(hp, hs, to_np(ids), to_np(w), _triple(gu), _triple(dn)))
+
+
 # several feature blocks per CTA, so that both MMA issuers of the kernel work: a k of more blocks than the ring has stages
 # (2048 with 64-row tiles: eight over seven), of as many, and one of a single block
 @pytest.mark.parametrize("t,e,k,h,i,rows", [(100, 64, 8, 2048, 512, 64), (60, 64, 8, 2048, 512, 32),

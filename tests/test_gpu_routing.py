@@ -127,6 +127,23 @@ def test_route_permutation_is_bit_exact(ops, oracle, case):
         assert np.array_equal(g, r), name
 
 
+# more routes than one block sorts: two launches for 8 to 1024 experts and up to 256 chunks of 1024 routes, three beyond. The
+# ends of those ranges, whole chunks and one route more, experts held by another rank
+@pytest.mark.parametrize("t,k,e,local", [(2561, 1, 7, None), (2561, 1, 8, None), (3072, 1, 9, None), (3073, 1, 512, None),
+                                         (513, 5, 1023, None), (700, 6, 1024, None), (700, 6, 1025, None),
+                                         (900, 6, 64, (40, 8)), (900, 6, 64, (3, 57)), (900, 6, 64, (60, 4)),
+                                         (65536, 4, 16, None), (65537, 4, 16, None)])
+def test_sort_of_a_large_batch(ops, oracle, t, k, e, local):
+    rng = np.random.default_rng(t + e)
+    ids = rng.integers(0, e, size=(t, k), dtype=np.int32)
+    ids[: t // 3] = ids[0, 0]
+    w = rng.random((t, k), dtype=np.float32)
+    off, le = local or (0, e)
+    got = _route_tables(ops, ids, w, e, off, le)
+    for name, g, r in zip(("counts", "indptr", "route_rows", "row_tokens", "row_scales"), got, oracle.route_sort(ids, w, off, le)):
+        assert np.array_equal(g, r), name
+
+
 def test_silu_and_mul(ops, oracle, golden):
     case = golden["silu_and_mul"]
     gate = bf16(case["gate"]).reshape(case["tokens"], case["intermediate"])
