@@ -277,188 +277,188 @@ gemv_gate_up_kernel(const GemvParams p, const RouterParams r, const RouteTables 
     __syncthreads();
     uint32_t turn = 0;
     for (uint32_t unit = blockIdx.x - 1; unit < units; unit += gridDim.x - 1) {
-    const bool shared = p.shared && unit < per_token;
-    if (!shared && !routed) {
-        routed = true;
-        if (p.early)
-            chain_begin();
-        if constexpr (ITEMS > 0) {
-            if (warp < p.num_tokens) {
-                int id;
-                float weight;
-                topk_row<float, ITEMS>(r.logits + static_cast<size_t>(warp) * r.num_experts, r.bias, r.num_experts, p.top_k,
-                                       r.sigmoid_score, r.renormalize, r.scaling, s_cand[warp], &id, &weight);
-                if (lane < p.top_k)
-                    s_expert[warp * p.top_k + lane] = id - static_cast<int>(p.local_offset);
+        const bool shared = p.shared && unit < per_token;
+        if (!shared && !routed) {
+            routed = true;
+            if (p.early)
+                chain_begin();
+            if constexpr (ITEMS > 0) {
+                if (warp < p.num_tokens) {
+                    int id;
+                    float weight;
+                    topk_row<float, ITEMS>(r.logits + static_cast<size_t>(warp) * r.num_experts, r.bias, r.num_experts, p.top_k,
+                                           r.sigmoid_score, r.renormalize, r.scaling, s_cand[warp], &id, &weight);
+                    if (lane < p.top_k)
+                        s_expert[warp * p.top_k + lane] = id - static_cast<int>(p.local_offset);
+                }
+            } else {
+                for (uint32_t i = threadIdx.x; i < routes; i += kBlockSortThreads)
+                    s_expert[i] = p.ids[i] - static_cast<int>(p.local_offset);
             }
-        } else {
-            for (uint32_t i = threadIdx.x; i < routes; i += kBlockSortThreads)
-                s_expert[i] = p.ids[i] - static_cast<int>(p.local_offset);
+            __syncthreads();
+        }
+        const uint32_t fb = unit % blocks, token = unit / blocks % p.num_tokens;
+        const uint32_t slot = shared ? p.top_k : unit / per_token - p.shared;
+        const int expert = shared ? 0 : s_expert[token * p.top_k + slot];
+        if (expert < 0 || (!shared && expert >= static_cast<int>(p.experts))) // (uniform)
+            continue;
+        turn ^= 1; // (the last unit's sums are still being read)
+        uint8_t* s_x = s_dyn + token * x_bytes;
+        const float* s_scale = scales_of<FMT>(s_x, p.hidden_size);
+
+        const GemvWeights& w = shared ? p.shared_weights : p.routed;
+        const uint32_t g = lane / 4, t = lane % 4;
+        const uint32_t j64 = fb / 2, half = fb % 2; // NVFP4: features 16 half and 32 + 16 half onwards of a 64-feature block
+        const size_t group_row = static_cast<size_t>(expert) * 2 * p.inter;
+        if constexpr (FMT == GEMV_NVFP4) {
+            // a warp: the gate rows r and r + 32 and the up rows r + 64 and r + 96 of the block's scale tile, whose scales of 64
+            // elements are 16 bytes of it
+            const uint32_t chunks = p.hidden_size / 16, r = half * 16 + warp;
+            const size_t row_bytes = p.hidden_size / 2;
+            const uint8_t* src = w.gate_up + (group_row + j64 * 64 + r) * row_bytes;
+            const uint8_t* row[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q)
+                row[q] = src + (static_cast<size_t>(q & 1) * 32 + static_cast<size_t>(q >> 1) * p.inter) * row_bytes;
+            const uint8_t* sf = static_cast<const uint8_t*>(w.gate_up_scale) + expert * tiled_bytes(2 * p.inter, p.hidden_size)
+                + static_cast<uint64_t>(j64) * (p.hidden_size / 64) * 512 + r * 16;
+            float acc[4] = {};
+            constexpr uint32_t kUnroll = 2;
+            for (uint32_t c0 = lane; c0 < chunks; c0 += 32 * kUnroll) {
+                uint2 v[kUnroll][4];
+                uint4 sv[kUnroll];
+#pragma unroll
+                for (uint32_t u = 0; u < kUnroll; ++u) {
+                    const uint32_t c = c0 + 32 * u;
+                    if (c < chunks) {
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; ++q)
+                            v[u][q] = __ldg(reinterpret_cast<const uint2*>(row[q] + c * 8));
+                        sv[u] = load16(sf + static_cast<size_t>(c / 4) * 512);
+                    }
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < kUnroll; ++u) {
+                    const uint32_t c = c0 + 32 * u;
+                    if (c < chunks) {
+                        const uint4* xp = reinterpret_cast<const uint4*>(s_x + c * kGvXPitch);
+                        const uint4 x0 = xp[0], x1 = xp[1];
+                        const uint32_t x[8] = { x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w };
+                        const float xs = s_scale[c];
+                        const uint32_t sw[4] = { sv[u].x, sv[u].y, sv[u].z, sv[u].w };
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; ++q)
+                            acc[q] = fmaf(dot_nvfp4(v[u][q], x), xs * block_scale(sw[q]), acc[q]);
+                    }
+                }
+            }
+            // lanes 0 and 8: gate of the two features, lanes 16 and 24: up
+            const float sum = reduce4(acc);
+            if (lane % 8 == 0)
+                s_part[turn][0][(lane / 8 & 1) * 16 + warp][lane / 16] = sum;
+        } else if constexpr (FMT == GEMV_FP8) {
+            const uint32_t split = warp / 4, kbs = p.hidden_size / 128, rbs = p.inter / 128;
+            const uint32_t f = fb * kGvFeatures + warp % 4 * 8 + g;
+            const size_t row_bytes = p.hidden_size, up = static_cast<size_t>(p.inter) * row_bytes;
+            const uint8_t* src = w.gate_up + (group_row + f) * row_bytes + t * 16;
+            const float* ws0 = static_cast<const float*>(w.gate_up_scale) + (static_cast<size_t>(expert) * 2 * rbs + f / 128) * kbs;
+            const float* ws1 = ws0 + static_cast<size_t>(rbs) * kbs;
+            float acc[2] = {};
+#pragma unroll 1
+            for (uint32_t kb = split; kb < kbs; kb += G::kSplits) {
+                uint4 gate[2], upw[2];
+#pragma unroll
+                for (uint32_t q = 0; q < 2; ++q) {
+                    gate[q] = load16(src + kb * 128 + q * 64);
+                    upw[q] = load16(src + up + kb * 128 + q * 64);
+                }
+                const float s0 = __ldg(ws0 + kb), s1 = __ldg(ws1 + kb), xs = s_scale[kb];
+                uint32_t x[8] = {};
+                if (g == 0) {
+                    const uint4* xp = reinterpret_cast<const uint4*>(s_x) + kb * 8 + t;
+                    const uint4 x0 = xp[0], x1 = xp[4];
+                    x[0] = x0.x, x[1] = x0.y, x[2] = x0.z, x[3] = x0.w, x[4] = x1.x, x[5] = x1.y, x[6] = x1.z, x[7] = x1.w;
+                }
+                float c[4] = {};
+                dot_fp8(c, gate, upw, x);
+                acc[0] = fmaf(c[0], s0 * xs, acc[0]); // (column 0: lanes t = 0)
+                acc[1] = fmaf(c[2], s1 * xs, acc[1]);
+            }
+            if (t == 0) {
+                s_part[turn][split][warp % 4 * 8 + g][0] = acc[0];
+                s_part[turn][split][warp % 4 * 8 + g][1] = acc[1];
+            }
+        } else { // a warp: the gate and up rows of features `warp` and `warp` + 16
+            const uint32_t chunks = p.hidden_size / 8;
+            const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(w.gate_up) + (group_row + fb * kGvFeatures + warp) * p.hidden_size;
+            const __nv_bfloat16* row[4];
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q)
+                row[q] = src + (static_cast<size_t>(q & 1) * 16 + static_cast<size_t>(q >> 1) * p.inter) * p.hidden_size;
+            float acc[4] = {};
+            constexpr uint32_t kUnroll = 2;
+            for (uint32_t c0 = lane; c0 < chunks; c0 += 32 * kUnroll) {
+                uint4 v[kUnroll][4];
+#pragma unroll
+                for (uint32_t u = 0; u < kUnroll; ++u)
+                    if (c0 + 32 * u < chunks)
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; ++q)
+                            v[u][q] = load16(row[q] + (c0 + 32 * u) * 8);
+#pragma unroll
+                for (uint32_t u = 0; u < kUnroll; ++u) {
+                    if (c0 + 32 * u < chunks) {
+                        const float4* xp = reinterpret_cast<const float4*>(s_x + (c0 + 32 * u) * kGvXPitch);
+                        const float4 x0 = xp[0], x1 = xp[1];
+                        const float x[8] = { x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w };
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; ++q)
+                            acc[q] = dot_bf16(acc[q], v[u][q], x);
+                    }
+                }
+            }
+            // lanes 0 and 8: gate of the two features, lanes 16 and 24: up
+            const float sum = reduce4(acc);
+            if (lane % 8 == 0)
+                s_part[turn][0][(lane / 8 & 1) * 16 + warp][lane / 16] = sum;
         }
         __syncthreads();
-    }
-    const uint32_t fb = unit % blocks, token = unit / blocks % p.num_tokens;
-    const uint32_t slot = shared ? p.top_k : unit / per_token - p.shared;
-    const int expert = shared ? 0 : s_expert[token * p.top_k + slot];
-    if (expert < 0 || (!shared && expert >= static_cast<int>(p.experts))) // (uniform)
-        continue;
-    turn ^= 1; // (the last unit's sums are still being read)
-    uint8_t* s_x = s_dyn + token * x_bytes;
-    const float* s_scale = scales_of<FMT>(s_x, p.hidden_size);
 
-    const GemvWeights& w = shared ? p.shared_weights : p.routed;
-    const uint32_t g = lane / 4, t = lane % 4;
-    const uint32_t j64 = fb / 2, half = fb % 2; // NVFP4: features 16 half and 32 + 16 half onwards of a 64-feature block
-    const size_t group_row = static_cast<size_t>(expert) * 2 * p.inter;
-    if constexpr (FMT == GEMV_NVFP4) {
-        // a warp: the gate rows r and r + 32 and the up rows r + 64 and r + 96 of the block's scale tile, whose scales of 64
-        // elements are 16 bytes of it
-        const uint32_t chunks = p.hidden_size / 16, r = half * 16 + warp;
-        const size_t row_bytes = p.hidden_size / 2;
-        const uint8_t* src = w.gate_up + (group_row + j64 * 64 + r) * row_bytes;
-        const uint8_t* row[4];
+        if (warp == 0) { // a lane per feature: of an NVFP4 block, 16 neighbouring ones twice
+            const size_t act_row = static_cast<size_t>(token) * (p.top_k + p.shared) + slot;
+            float gv = s_part[turn][0][lane][0], uv = s_part[turn][0][lane][1];
 #pragma unroll
-        for (uint32_t q = 0; q < 4; ++q)
-            row[q] = src + (static_cast<size_t>(q & 1) * 32 + static_cast<size_t>(q >> 1) * p.inter) * row_bytes;
-        const uint8_t* sf = static_cast<const uint8_t*>(w.gate_up_scale) + expert * tiled_bytes(2 * p.inter, p.hidden_size)
-            + static_cast<uint64_t>(j64) * (p.hidden_size / 64) * 512 + r * 16;
-        float acc[4] = {};
-        constexpr uint32_t kUnroll = 2;
-        for (uint32_t c0 = lane; c0 < chunks; c0 += 32 * kUnroll) {
-            uint2 v[kUnroll][4];
-            uint4 sv[kUnroll];
-#pragma unroll
-            for (uint32_t u = 0; u < kUnroll; ++u) {
-                const uint32_t c = c0 + 32 * u;
-                if (c < chunks) {
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q)
-                        v[u][q] = __ldg(reinterpret_cast<const uint2*>(row[q] + c * 8));
-                    sv[u] = load16(sf + static_cast<size_t>(c / 4) * 512);
+            for (uint32_t s = 1; s < G::kSplits; ++s) {
+                gv += s_part[turn][s][lane][0];
+                uv += s_part[turn][s][lane][1];
+            }
+            if constexpr (FMT == GEMV_BF16) {
+                gv = __bfloat162float(__float2bfloat16(gv));
+                uv = __bfloat162float(__float2bfloat16(uv));
+                reinterpret_cast<__nv_bfloat16*>(p.act)[act_row * p.inter + fb * kGvFeatures + lane]
+                    = __float2bfloat16(gv * sigmoid_fast(gv) * uv);
+            } else if constexpr (FMT == GEMV_FP8) {
+                reinterpret_cast<float*>(p.act)[act_row * p.inter + fb * kGvFeatures + lane] = __fdividef(gv, 1.0f + __expf(-gv)) * uv;
+            } else {
+                float scale = p.act_global, scale_up = p.act_global;
+                if (w.gate_up_global != nullptr)
+                    scale *= w.gate_up_global[expert];
+                scale_up *= w.gate_up_global_up != nullptr ? w.gate_up_global_up[expert]
+                                                           : (w.gate_up_global != nullptr ? w.gate_up_global[expert] : 1.0f);
+                gv *= scale;
+                uv *= scale_up;
+                s_act[lane] = __fdividef(gv, 1.0f + __expf(-gv)) * uv;
+                __syncwarp();
+                if (lane < 2) { // the block's features are two 16-element blocks of the next product
+                    uint32_t lo, hi;
+                    const uint32_t blk = j64 * 4 + lane * 2 + half;
+                    const uint8_t code = quantize_block16(s_act + lane * 16, p.act2_global, &lo, &hi);
+                    *reinterpret_cast<uint2*>(p.act + act_row * (p.inter / 2) + blk * 8) = make_uint2(lo, hi);
+                    p.act_scale[act_row * (p.inter / 16) + blk] = code;
                 }
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < kUnroll; ++u) {
-                const uint32_t c = c0 + 32 * u;
-                if (c < chunks) {
-                    const uint4* xp = reinterpret_cast<const uint4*>(s_x + c * kGvXPitch);
-                    const uint4 x0 = xp[0], x1 = xp[1];
-                    const uint32_t x[8] = { x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w };
-                    const float xs = s_scale[c];
-                    const uint32_t sw[4] = { sv[u].x, sv[u].y, sv[u].z, sv[u].w };
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q)
-                        acc[q] = fmaf(dot_nvfp4(v[u][q], x), xs * block_scale(sw[q]), acc[q]);
-                }
+                __syncwarp();
             }
         }
-        // lanes 0 and 8: gate of the two features, lanes 16 and 24: up
-        const float sum = reduce4(acc);
-        if (lane % 8 == 0)
-            s_part[turn][0][(lane / 8 & 1) * 16 + warp][lane / 16] = sum;
-    } else if constexpr (FMT == GEMV_FP8) {
-        const uint32_t split = warp / 4, kbs = p.hidden_size / 128, rbs = p.inter / 128;
-        const uint32_t f = fb * kGvFeatures + warp % 4 * 8 + g;
-        const size_t row_bytes = p.hidden_size, up = static_cast<size_t>(p.inter) * row_bytes;
-        const uint8_t* src = w.gate_up + (group_row + f) * row_bytes + t * 16;
-        const float* ws0 = static_cast<const float*>(w.gate_up_scale) + (static_cast<size_t>(expert) * 2 * rbs + f / 128) * kbs;
-        const float* ws1 = ws0 + static_cast<size_t>(rbs) * kbs;
-        float acc[2] = {};
-#pragma unroll 1
-        for (uint32_t kb = split; kb < kbs; kb += G::kSplits) {
-            uint4 gate[2], upw[2];
-#pragma unroll
-            for (uint32_t q = 0; q < 2; ++q) {
-                gate[q] = load16(src + kb * 128 + q * 64);
-                upw[q] = load16(src + up + kb * 128 + q * 64);
-            }
-            const float s0 = __ldg(ws0 + kb), s1 = __ldg(ws1 + kb), xs = s_scale[kb];
-            uint32_t x[8] = {};
-            if (g == 0) {
-                const uint4* xp = reinterpret_cast<const uint4*>(s_x) + kb * 8 + t;
-                const uint4 x0 = xp[0], x1 = xp[4];
-                x[0] = x0.x, x[1] = x0.y, x[2] = x0.z, x[3] = x0.w, x[4] = x1.x, x[5] = x1.y, x[6] = x1.z, x[7] = x1.w;
-            }
-            float c[4] = {};
-            dot_fp8(c, gate, upw, x);
-            acc[0] = fmaf(c[0], s0 * xs, acc[0]); // (column 0: lanes t = 0)
-            acc[1] = fmaf(c[2], s1 * xs, acc[1]);
-        }
-        if (t == 0) {
-            s_part[turn][split][warp % 4 * 8 + g][0] = acc[0];
-            s_part[turn][split][warp % 4 * 8 + g][1] = acc[1];
-        }
-    } else { // a warp: the gate and up rows of features `warp` and `warp` + 16
-        const uint32_t chunks = p.hidden_size / 8;
-        const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(w.gate_up) + (group_row + fb * kGvFeatures + warp) * p.hidden_size;
-        const __nv_bfloat16* row[4];
-#pragma unroll
-        for (uint32_t q = 0; q < 4; ++q)
-            row[q] = src + (static_cast<size_t>(q & 1) * 16 + static_cast<size_t>(q >> 1) * p.inter) * p.hidden_size;
-        float acc[4] = {};
-        constexpr uint32_t kUnroll = 2;
-        for (uint32_t c0 = lane; c0 < chunks; c0 += 32 * kUnroll) {
-            uint4 v[kUnroll][4];
-#pragma unroll
-            for (uint32_t u = 0; u < kUnroll; ++u)
-                if (c0 + 32 * u < chunks)
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q)
-                        v[u][q] = load16(row[q] + (c0 + 32 * u) * 8);
-#pragma unroll
-            for (uint32_t u = 0; u < kUnroll; ++u) {
-                if (c0 + 32 * u < chunks) {
-                    const float4* xp = reinterpret_cast<const float4*>(s_x + (c0 + 32 * u) * kGvXPitch);
-                    const float4 x0 = xp[0], x1 = xp[1];
-                    const float x[8] = { x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w };
-#pragma unroll
-                    for (uint32_t q = 0; q < 4; ++q)
-                        acc[q] = dot_bf16(acc[q], v[u][q], x);
-                }
-            }
-        }
-        // lanes 0 and 8: gate of the two features, lanes 16 and 24: up
-        const float sum = reduce4(acc);
-        if (lane % 8 == 0)
-            s_part[turn][0][(lane / 8 & 1) * 16 + warp][lane / 16] = sum;
-    }
-    __syncthreads();
-
-    if (warp == 0) { // a lane per feature: of an NVFP4 block, 16 neighbouring ones twice
-        const size_t act_row = static_cast<size_t>(token) * (p.top_k + p.shared) + slot;
-        float gv = s_part[turn][0][lane][0], uv = s_part[turn][0][lane][1];
-#pragma unroll
-        for (uint32_t s = 1; s < G::kSplits; ++s) {
-            gv += s_part[turn][s][lane][0];
-            uv += s_part[turn][s][lane][1];
-        }
-        if constexpr (FMT == GEMV_BF16) {
-            gv = __bfloat162float(__float2bfloat16(gv));
-            uv = __bfloat162float(__float2bfloat16(uv));
-            reinterpret_cast<__nv_bfloat16*>(p.act)[act_row * p.inter + fb * kGvFeatures + lane]
-                = __float2bfloat16(gv * sigmoid_fast(gv) * uv);
-        } else if constexpr (FMT == GEMV_FP8) {
-            reinterpret_cast<float*>(p.act)[act_row * p.inter + fb * kGvFeatures + lane] = __fdividef(gv, 1.0f + __expf(-gv)) * uv;
-        } else {
-            float scale = p.act_global, scale_up = p.act_global;
-            if (w.gate_up_global != nullptr)
-                scale *= w.gate_up_global[expert];
-            scale_up *= w.gate_up_global_up != nullptr ? w.gate_up_global_up[expert]
-                                                       : (w.gate_up_global != nullptr ? w.gate_up_global[expert] : 1.0f);
-            gv *= scale;
-            uv *= scale_up;
-            s_act[lane] = __fdividef(gv, 1.0f + __expf(-gv)) * uv;
-            __syncwarp();
-            if (lane < 2) { // the block's features are two 16-element blocks of the next product
-                uint32_t lo, hi;
-                const uint32_t blk = j64 * 4 + lane * 2 + half;
-                const uint8_t code = quantize_block16(s_act + lane * 16, p.act2_global, &lo, &hi);
-                *reinterpret_cast<uint2*>(p.act + act_row * (p.inter / 2) + blk * 8) = make_uint2(lo, hi);
-                p.act_scale[act_row * (p.inter / 16) + blk] = code;
-            }
-            __syncwarp();
-        }
-    }
     }
     if (p.early && !routed)
         chain_begin();
@@ -673,7 +673,8 @@ cudaError_t launch_instance(const GemvParams& p, const RouterParams* router, con
     if (err != cudaSuccess)
         return err;
     stage_mark(stream, STAGE_DOWN_GEMM);
-    return launch_chained(slots <= kGvFewSlots ? gemv_down_kernel<FMT, kGvFewSlots> : gemv_down_kernel<FMT, kGvMaxSlots>, dim3(p.hidden_size / Gv<FMT>::kOut, p.num_tokens), slots * 32, 0, stream, p);
+    return launch_chained(slots <= kGvFewSlots ? gemv_down_kernel<FMT, kGvFewSlots> : gemv_down_kernel<FMT, kGvMaxSlots>,
+                          dim3(p.hidden_size / Gv<FMT>::kOut, p.num_tokens), slots * 32, 0, stream, p);
 }
 
 // The time grows with the weights that the slots multiply, again for every slot of one expert; the grouped GEMMs stream an

@@ -58,7 +58,7 @@ tensor_peak_kernel(int kind, uint32_t n, uint32_t iters, uint32_t* err, uint32_t
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32 && elect_one()) {
         const uint32_t nm = ((n >> 3) << 17) | ((kBM >> 4) << 24);
         const uint32_t idesc = kind == PROBE_BF16 ? ((1u << 4) | (1u << 7) | (1u << 10) | nm)
             : kind == PROBE_FP8                  ? ((1u << 4) | nm) // e4m3 x e4m3, f32 accumulate
@@ -89,7 +89,7 @@ tensor_peak_kernel(int kind, uint32_t n, uint32_t iters, uint32_t* err, uint32_t
         }
         tc_commit(done_bar);
         mbar_wait<true>(done_bar, 0, abort_flag, err, 0x53000001u);
-    } else if (threadIdx.x == 32 && cps_side != 0 && kind == PROBE_NVFP4) {
+    } else if (threadIdx.x / 32 == 1 && elect_one() && cps_side != 0 && kind == PROBE_NVFP4) {
         const uint64_t sdesc = scale_desc(smem_u32(sf_tile));
         const uint32_t side = tmem_base + 416; // columns no MMA of this probe reads
         for (uint32_t it = 0; it < iters; ++it)
@@ -150,7 +150,7 @@ tensor_peak_pair_kernel(int kind, uint32_t n, uint32_t iters, uint32_t* err)
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (cta_rank == 0 && threadIdx.x == 0) {
+    if (cta_rank == 0 && threadIdx.x < 32 && elect_one()) {
         const uint32_t nm = ((n >> 3) << 17) | ((256u >> 4) << 24);
         const uint32_t idesc = kind == PROBE_BF16 ? ((1u << 4) | (1u << 7) | (1u << 10) | nm)
             : kind == PROBE_FP8                  ? ((1u << 4) | nm)
