@@ -241,7 +241,7 @@ gemm_dense_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 mbar_arrive(&acc_empty[buf]);
         }
         if (lane == 0)
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); // the stores have left shared memory
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); // stores done before shared memory goes away
     }
 
     tc_fence_before();
@@ -446,7 +446,7 @@ gemm_dense_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 mbar_arrive_cluster(cluster_addr(&acc_empty[buf], 0));
         }
         if (lane == 0)
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); // the stores have left shared memory
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); // stores done before shared memory goes away
     }
 
     tc_fence_before();
@@ -522,6 +522,7 @@ bool gemm_dense_bf16_supported(const GemmProblem& g)
 //   a pair of CTAs, 256 x c       6.8 + rounds (1.5 + k blocks (0.15 + 0.00062 c)), a round not under the 3.5 c / 256 that
 //                                 its output takes
 //   split k (gemm_splitk.cu)      bf16 results only: f32 results have their own choice there
+// A sum over all of k in one accumulator is off by 2e-6 at k = 2048, a rank's share by less; rounding to bf16 by 2e-3.
 // Before, by the number of 128 x 256 tiles: 300 x 4096 x 4096 27.1 -> 18.0 us, 1200 x 4096 x 4096 46.3 -> 37.6,
 // 800 x 4096 x 2048 26.0 -> 18.0, 200 x 512 x 2048 6.9 -> 5.7, 2000 x 512 x 8192 26.9 -> 23.
 DenseChoice gemm_dense_choice(const GemmProblem& g)
