@@ -678,21 +678,24 @@ cudaError_t launch_instance(const GemvParams& p, const RouterParams* router, con
 }
 
 // The time grows with the weights that the slots multiply, again for every slot of one expert; the grouped GEMMs stream an
-// expert once, over five launches. Layer (hidden, experts top-k, intermediate; tokens: grouped / this, us):
+// expert once, over five launches, so a skewed router favours them. Layer (hidden, experts top-k, intermediate; tokens:
+// grouped / this, us; of a skewed router in brackets):
 //                              bf16                            nvfp4                          fp8
-//   2048, 8 top-2, 512         8: 32 / 19, 16: 34 / 34         8: 30 / 19, 16: 31 / 31        8: 28 / 19, 16: 28 / 29
-//   512, 16 top-4, 512         8: 23 / 16, 16: 25 / 23         8: 28 / 17, 16: 29 / 27        8: 21 / 17, 16: 22 / 25
-//   2048, 16 top-4, 768        4: 39 / 30, 8: 42 / 53          4: 31 / 20, 8: 34 / 34         4: 29 / 20, 8: 29 / 33
-//   1024, 64 top-6, 512        8: 33 / 29, 16: 47 / 59         8: 34 / 24, 16: 36 / 41        8: 26 / 24, 16: 33 / 42
-//   2048, 32 top-4, 512        4: 34 / 20, 8: 43 / 46          8: 35 / 26                     8: 30 / 27, 16: 34 / 47
-//   2048, 128 top-8, 768       4: 64 / 55, 5: 70 / 67                                         4: 47 / 43, 5: 50 / 51
-//   2048, 512 top-10, 512 + 1  4: 76 / 73, 5: 81 / 87          4: 48 / 43, 5: 50 / 52
+//   2048, 8 top-2, 512         8: 31 / 19, 16: 32 / 32         8: 24 / 19, 12: 24 / 25        8: 25 / 18, 16: 26 / 29
+//   512, 16 top-4, 512         8: 22 / 15, 16: 23 / 23         8: 22 / 16, 16: 23 / 27        8: 20 / 17, 16: 21 / 25
+//   2048, 16 top-4, 768        4: 35 / 29, 8: 39 / 51          4: 26 / 20, 8: 27 / 33         4: 25 / 20, 8: 26 / 32
+//   1024, 64 top-6, 512        8: 30 / 28, 10: 40 / 35         8: 26 / 24, 10: 28 / 29        8: 23 / 23, 10: 26 / 29
+//   2048, 32 top-4, 512        4: 31 / 19, 8: 41 / 45          6: 26 / 23, 8: 27 / 26         6: 26 / 21, 8: 27 / 27
+//   2048, 128 top-8, 768       3: 49 / 41 (37 / 33),                                          3: 33 / 29 (30 / 27),
+//                              4: 62 / 55 (39 / 43)                                           4: 43 / 43 (30 / 36)
+//   2048, 512 top-10, 512 + 1  4: 76 / 72 (58 / 56),           3: 36 / 34 (34 / 33),
+//                              5: 80 / 86 (59 / 66)            4: 39 / 42 (36 / 38)
 bool gemv_pays(int fmt, uint64_t routes, uint64_t slots, uint64_t experts, uint64_t hidden, uint64_t inter)
 {
     const uint64_t millions = slots * 3 * hidden * inter / 1000000;
     const uint64_t most = routes > 2 * experts ? 30 // every expert several times
-        : 2 * routes > experts                 ? (fmt == GEMV_NVFP4 ? 110 : 75)
-                                               : (fmt == GEMV_NVFP4 ? 140 : 155);
+        : 2 * routes > experts                 ? (fmt == GEMV_NVFP4 ? 90 : 75)
+                                               : (fmt == GEMV_NVFP4 ? 110 : fmt == GEMV_FP8 ? 115 : 140);
     return millions <= most;
 }
 
