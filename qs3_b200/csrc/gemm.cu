@@ -681,19 +681,38 @@ cudaError_t launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const TcPara
     return launch_chained(kernel, grid, kThreads, smem, stream, ma, mb, tp);
 }
 
+// Shared memory of the resident-A kernel: the panel with its scales, with `staging` the two 32-KB tiles through which bf16
+// output leaves, and a ring of the rest. Two k blocks per ring stage: one barrier round trip of the single issuing thread
+// costs about as much as four 128x128x64 MMAs, so stages carry eight of them.
+constexpr size_t kAsSmemBudget = 227 * 1024 - 1024 /* alignment slack */ - 512 /* barriers */;
+constexpr size_t astat_fixed(uint32_t k_blocks, bool staging)
+{
+    return static_cast<size_t>(k_blocks) * (kTileBytes + kSfBytes) + (staging ? 4 * kTileBytes : 0);
+}
+struct AstatRing {
+    uint32_t kbs, stages;
+};
+constexpr AstatRing astat_ring(uint32_t k_blocks, bool staging)
+{
+    const uint32_t kbs = k_blocks % 2 == 0 ? 2u : 1u;
+    const size_t left = kAsSmemBudget - astat_fixed(k_blocks, staging);
+    // 16 scale columns per k block in flight, 128 in all
+    return { kbs, std::min<uint32_t>(static_cast<uint32_t>(left / (kbs * kAsStageBytes)), kAsMaxStages / kbs) };
+}
+// Beside eight k blocks (k = 2048) the staging leaves no room for a ring: those tiles store their rows directly.
+constexpr bool astat_staging_fits(uint32_t k_blocks) { return astat_ring(k_blocks, true).stages > 0; }
+static_assert(astat_fixed(kAsMaxKBlocks, true) < kAsSmemBudget && astat_ring(kAsMaxKBlocks, false).stages >= 2
+              && astat_staging_fits(7) && astat_staging_fits(6) && !astat_staging_fits(8));
+
 template <bool GATED, int EPI>
 cudaError_t launch_astat(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mo, const TcParams& tp,
                          dim3 grid, uint32_t nt_per_split, cudaStream_t stream)
 {
-    constexpr size_t kSmemBudget = 227 * 1024 - 1024 /* alignment slack */ - 512 /* barriers */;
-    const size_t panel = static_cast<size_t>(tp.k_blocks) * (kTileBytes + kSfBytes);
-    // two k-blocks per ring stage: one barrier round trip of the single issuing thread
-    // costs about as much as four 128x128x64 MMAs, so stages carry eight of them
-    const uint32_t kbs = tp.k_blocks % 2 == 0 ? 2u : 1u;
-    const size_t staging = tp.tma_store ? 4 * kTileBytes : 0;
-    uint32_t stages = static_cast<uint32_t>((kSmemBudget - panel - staging) / (kbs * kAsStageBytes));
-    stages = std::min<uint32_t>(stages, kAsMaxStages / kbs); // 16 scale columns per k block in flight, 128 in all
-    const size_t smem = panel + staging + static_cast<size_t>(stages) * kbs * kAsStageBytes + 1024 + 512;
+    const AstatRing ring = astat_ring(tp.k_blocks, tp.tma_store != 0);
+    if (ring.stages == 0)
+        return cudaErrorInvalidConfiguration;
+    const uint32_t kbs = ring.kbs, stages = ring.stages;
+    const size_t smem = astat_fixed(tp.k_blocks, tp.tma_store != 0) + static_cast<size_t>(stages) * kbs * kAsStageBytes + 1024 + 512;
     auto kernel = gemm_tc_astat_kernel<GATED, EPI>;
     static bool configured[64] = {};
     int dev = 0;
@@ -1002,7 +1021,7 @@ cudaError_t launch_gemm(const GemmProblem& g, cudaStream_t stream, const char** 
                 // row-major matrix whose rows may all be written (no beta read-modify-write)
                 CUtensorMap mo = ma;
                 TcParams tpo = tp;
-                if (g.beta == 0.0f && aligned16(g.out) && (g.out_pitch_elems * 2) % 16 == 0
+                if (astat_staging_fits(tp.k_blocks) && g.beta == 0.0f && aligned16(g.out) && (g.out_pitch_elems * 2) % 16 == 0
                     && make_map(&mo, false, g.out, g.n, g.a_rows, g.out_pitch_elems * 2, kBM))
                     tpo.tma_store = 1;
                 return launch_astat<false, EPI_STORE_BF16>(ma, mb, mo, tpo, agrid, nt_per, stream);

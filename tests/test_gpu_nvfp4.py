@@ -422,3 +422,26 @@ def test_tile_height_chosen_in_the_declared_call(ops, ctx, oracle, hot, rows):
     assert ctx.read_device_error() == 0
     assert _chosen_height(ids, e) == rows == tile_height(plan, ws, t)
     _check(to_np(out), oracle.moe_nvfp4(hp, hs, ids, w, gu, dn))
+
+
+# k of the down projections up to the longest resident panel: six and seven blocks of 256 leave a ring of one stage beside the
+# staged output, eight none (rows stored directly); tiles with few rows and with many, a shared expert of another size
+@pytest.mark.parametrize("t,e,k,h,i,s", [(130, 2, 1, 256, 1536, 0), (130, 2, 1, 256, 1792, 2048), (300, 2, 2, 512, 2048, 0),
+                                         (3, 8, 1, 512, 256, 2048), (200, 4, 1, 256, 2048, 2048)])
+def test_longest_down_projections(ops, ctx, oracle, t, e, k, h, i, s):
+    d = make_moe_inputs(72, t, h, e, i, s)
+    gu, dn, sh = _quantise_all(ops, ctx, d, bool(s))
+    plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=t, hidden_size=h, intermediate_size=i, num_experts=e, top_k=k,
+                                              backend=ops.capi.MOE_BACKEND_NVFP4))
+    ws = torch.zeros(plan.layer_workspace_size(t, s), dtype=torch.uint8, device="cuda")
+    ids = torch.empty((t, k), dtype=torch.int32, device="cuda")
+    w = torch.empty((t, k), dtype=torch.float32, device="cuda")
+    out = torch.empty((t, h), dtype=torch.bfloat16, device="cuda")
+    ops.moe_layer_execute(plan, to_dev(d["hidden"]), to_dev(d["router"]), gu, dn, out, ws, topk_ids=ids, topk_weights=w,
+                          shared=ops.SharedExpert(sh[0], sh[1], to_dev(d["sh_gate"]), s) if s else None)
+    torch.cuda.synchronize()
+    assert ctx.read_device_error() == 0
+    hp, hs = oracle.nvfp4_quantize_act(d["hidden"], 1.0)
+    shared_ref = dict(gu=_triple(sh[0]), d=_triple(sh[1]), gate_w=d["sh_gate"]) if s else None
+    _check(to_np(out), oracle.moe_nvfp4(hp, hs, to_np(ids), to_np(w), _triple(gu), _triple(dn), shared=shared_ref,
+                                        hidden_bf16=d["hidden"]))
