@@ -709,6 +709,7 @@ bool gemv_supported(int fmt, uint32_t num_tokens, uint32_t top_k, uint32_t num_e
         && top_k + 1 <= kGvMaxSlots && num_tokens <= kGvWarps
         && (shared_inter == 0 || shared_inter == inter) && router_sort_supported(num_tokens, num_experts, top_k, experts)
         && (fmt == GEMV_BF16 || inter % 128 == 0)
+        && (fmt != GEMV_FP8 || (hidden <= 4096 && inter <= 4096)) // (as far as FP8 plans go: larger batches are refused beyond)
         && gemv_pays(fmt, num_tokens * top_k, num_tokens * (top_k + (shared_inter != 0)), experts, hidden, inter);
 }
 

@@ -160,3 +160,15 @@ def test_result_in_the_tokens_place(oracle):
     torch.cuda.synchronize()
     ref = oracle.moe_bf16(d["hidden"], to_np(ids), to_np(w), d["gate_up"], d["down"])
     _check(to_np(x), oracle.shared_expert_bf16(d["hidden"], d["sh_gate_up"], d["sh_down"], d["sh_gate"], ref))
+
+
+@pytest.mark.parametrize("h,i,refused", [(4096, 128, False), (4224, 128, True), (128, 4096, False), (128, 4224, True)])
+def test_fp8_refusals_do_not_depend_on_the_batch(oracle, h, i, refused):
+    from qs3_b200 import capi, ops
+    case = ("fp8", 1, h, i, 2, 1, False, None)
+    if not refused:
+        r = _run(*case)
+        return _check(r["out"], _reference(oracle, "fp8", r))
+    with pytest.raises(ops.Qs3Error) as error:
+        _run(*case)
+    assert error.value.status == capi.STATUS_UNSUPPORTED
