@@ -23,16 +23,19 @@ struct qsfi_context {
     size_t host_int_workspace_bytes;
     uint64_t scratch_generation;
     qsfi_error_info last_error;
-    // (after upstream's fields) Side stream of the whole-layer call, taken on first use: the token quantiser and the shared
-    // expert run there beside the router chain. Each context has its own, so that calls of several contexts on one plan
-    // do not meet in an event.
+    // (after upstream's fields) Side streams of the whole-layer call, one for each stream that the context was on lately, latest
+    // first: the token quantiser and the shared expert run there beside the router chain. Each context has its own, so that
+    // calls of several contexts on one plan do not meet in an event; each stream has its own, so that a call on one neither
+    // waits for what another stream has queued nor meets a capture that is open there.
     struct qs3_side_stream* side;
 };
 
 struct qs3_side_stream {
     int device;
+    cudaStream_t beside; // of the context
     cudaStream_t stream;
     cudaEvent_t fork, quant, shared; // fork / join with the context's stream
+    qs3_side_stream* next;
 };
 
 struct qsfi_moe_plan {
@@ -55,7 +58,7 @@ qsfi_status set_cuda_error(qsfi_context* ctx, cudaError_t err, const char* op);
 qsfi_status activate_context(qsfi_context* ctx);
 qsfi_status status_from_cuda(cudaError_t err);
 
-// The context's side stream, NULL when none can be had; given back with the context.
+// The side stream beside the context's present stream, NULL when none can be had; given back with the context.
 qs3_side_stream* side_stream(qsfi_context* ctx);
 
 // SMs of the current device.

@@ -6,7 +6,6 @@
 #include <atomic>
 #include <mutex>
 #include <new>
-#include <vector>
 
 namespace qs3 {
 
@@ -17,8 +16,10 @@ namespace {
 // Side streams of destroyed contexts, for the next ones: creating one and its events takes about 0.2 ms, which the first
 // layer call of every context paid.
 constexpr size_t kSideStreamsKept = 8;
+constexpr uint32_t kSideStreamsOfContext = 4;
 std::mutex side_mutex;
-std::vector<qs3_side_stream*>& side_free = *new std::vector<qs3_side_stream*>; // (contexts may outlive static objects)
+qs3_side_stream* side_free[kSideStreamsKept]; // (contexts may outlive static objects)
+size_t side_count = 0;
 
 void destroy_side(qs3_side_stream* s)
 {
@@ -30,20 +31,57 @@ void destroy_side(qs3_side_stream* s)
     delete s;
 }
 
+bool capturing(const qs3_side_stream* s)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s->stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone;
+}
+
+// One that is being captured is of no use to others.
 void give_back(qs3_side_stream* s)
 {
-    if (s == nullptr)
-        return;
-    // (what still runs on it only delays its next user; one that is being captured is of no use to others)
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+    if (!capturing(s)) {
         std::lock_guard<std::mutex> lock(side_mutex);
-        if (side_free.size() < kSideStreamsKept) {
-            side_free.push_back(s);
+        if (side_count < kSideStreamsKept) {
+            side_free[side_count++] = s;
             return;
         }
     }
     destroy_side(s);
+}
+
+// One of the kept streams, on which nothing is left to run: its work waits for the stream of the context that queued it,
+// which an unrelated context must not.
+qs3_side_stream* take_side(int device)
+{
+    std::lock_guard<std::mutex> lock(side_mutex);
+    for (size_t i = 0; i < side_count; ++i) {
+        qs3_side_stream* s = side_free[i];
+        if (s->device != device)
+            continue;
+        if (cudaStreamQuery(s->stream) == cudaSuccess) {
+            side_free[i] = side_free[--side_count];
+            return s;
+        }
+        cudaGetLastError(); // (not ready)
+    }
+    return nullptr;
+}
+
+qs3_side_stream* make_side(int device)
+{
+    qs3_side_stream* s = new (std::nothrow) qs3_side_stream {};
+    if (s == nullptr)
+        return nullptr;
+    s->device = device;
+    if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) == cudaSuccess
+        && cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess
+        && cudaEventCreateWithFlags(&s->quant, cudaEventDisableTiming) == cudaSuccess
+        && cudaEventCreateWithFlags(&s->shared, cudaEventDisableTiming) == cudaSuccess)
+        return s;
+    cudaGetLastError();
+    destroy_side(s);
+    return nullptr;
 }
 
 } // namespace
@@ -53,37 +91,37 @@ qs3_side_stream* side_stream(qsfi_context* ctx)
     int device = -1;
     if (cudaGetDevice(&device) != cudaSuccess)
         return nullptr;
-    if (ctx->side != nullptr) {
-        if (ctx->side->device == device)
-            return ctx->side;
-        give_back(ctx->side); // a context of no device of its own, used on another one
-        ctx->side = nullptr;
+    uint32_t count = 0;
+    for (qs3_side_stream** at = &ctx->side; *at != nullptr; at = &(*at)->next, ++count) {
+        qs3_side_stream* s = *at;
+        if (s->device == device && s->beside == ctx->stream) { // to the front
+            *at = s->next;
+            s->next = ctx->side;
+            return ctx->side = s;
+        }
     }
-    {
-        std::lock_guard<std::mutex> lock(side_mutex);
-        for (auto it = side_free.begin(); it != side_free.end(); ++it)
-            if ((*it)->device == device) {
-                ctx->side = *it;
-                side_free.erase(it);
-                return ctx->side;
-            }
+    if (count >= kSideStreamsOfContext) { // the one that was not wanted for longest, unless a capture still needs it
+        qs3_side_stream** drop = nullptr;
+        for (qs3_side_stream** at = &ctx->side; *at != nullptr; at = &(*at)->next)
+            if (!capturing(*at))
+                drop = at;
+        if (drop == nullptr)
+            return nullptr;
+        qs3_side_stream* s = *drop;
+        *drop = s->next;
+        give_back(s);
     }
-    qs3_side_stream* s = new (std::nothrow) qs3_side_stream {};
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed; // the first call on a stream may be one that is captured
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    qs3_side_stream* s = take_side(device);
+    if (s == nullptr)
+        s = make_side(device);
+    cudaThreadExchangeStreamCaptureMode(&mode);
     if (s == nullptr)
         return nullptr;
-    s->device = device;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed; // the first call of a context may be one that is captured
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    const bool made = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) == cudaSuccess
-        && cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess
-        && cudaEventCreateWithFlags(&s->quant, cudaEventDisableTiming) == cudaSuccess
-        && cudaEventCreateWithFlags(&s->shared, cudaEventDisableTiming) == cudaSuccess;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (made)
-        return ctx->side = s;
-    cudaGetLastError();
-    destroy_side(s);
-    return nullptr;
+    s->beside = ctx->stream;
+    s->next = ctx->side;
+    return ctx->side = s;
 }
 
 void clear_error(qsfi_error_info* err)
@@ -273,7 +311,11 @@ void qsfi_context_destroy(qsfi_context* ctx)
             cudaSetDevice(ctx->device_ordinal);
         cudaFree(ctx->float_workspace);
     }
-    give_back(ctx->side);
+    while (ctx->side != nullptr) {
+        qs3_side_stream* s = ctx->side;
+        ctx->side = s->next;
+        give_back(s);
+    }
     delete ctx;
 }
 
