@@ -745,7 +745,9 @@ qsfi_status qs3_moe_read_device_error(qsfi_context* ctx, uint32_t* code);
  * qs3_moe_layer_execute records a CUDA event on the context's stream at each stage
  * boundary; _end synchronises the stream and returns, per recorded stage, its id
  * (1 router-logits GEMM, 2 router top-k, 3 route sort, 4 gather/quantise, 5 gate_up
- * GEMM + SwiGLU, 6 down GEMM, 7 shared expert, 8 combine) and its duration in ms. */
+ * GEMM + SwiGLU, 6 down GEMM, 7 shared expert, 8 combine) and its duration in ms. What
+ * runs beside the main chain, or in one launch with another stage (the experts of a
+ * handful of tokens, FP8 tokens quantised beside the sort), runs by itself meanwhile. */
 uint64_t qs3_moe_launch_count(void);
 qsfi_status qs3_moe_profile_begin(qsfi_context* ctx);
 qsfi_status qs3_moe_profile_end(

@@ -1294,11 +1294,12 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
     const int gemv_fmt = nvfp4 ? GEMV_NVFP4 : fp8 ? GEMV_FP8 : GEMV_BF16;
     const size_t slot_rows = routes + (shared ? d->num_tokens : 0u);
     const size_t act_room = static_cast<size_t>(rt.max_pad_rows) * p.intermediate_size / (nvfp4 ? 2 : 1) * (nvfp4 || fp8 ? 1 : 2);
-    // (a result in the tokens' place would be written while other blocks still read them for the gate)
+    // (a result in the tokens' place would be written while other blocks still read them for the gate; and a profile has the
+    // stages apart)
     const char *xb = static_cast<const char*>(d->hidden.data), *ob = static_cast<const char*>(d->out.data);
     const ptrdiff_t token_bytes = static_cast<ptrdiff_t>(t * h * 2);
     const bool in_place = xb < ob + token_bytes && ob < xb + token_bytes;
-    const bool gemv = (!nvfp4 || !shared || merged) && !(shared && in_place)
+    const bool gemv = (!nvfp4 || !shared || merged) && !(shared && in_place) && !stage_recording()
         && gemv_supported(gemv_fmt, d->num_tokens, p.top_k, p.num_experts, p.local_num_experts, p.hidden_size,
                           p.intermediate_size, shared ? is : 0)
         && gemv_act_bytes(gemv_fmt, slot_rows, p.intermediate_size) <= act_room;
@@ -1354,7 +1355,7 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
     const bool small_tiles = nvfp4 && rt.tile_rows != static_cast<uint32_t>(kTileM);
     TokenQuant tq { hidden, d->num_tokens, p.hidden_size, d->act_global_scale == 0.0f ? 1.0f : d->act_global_scale,
                     fp8 ? x.f8_x : x.sh_xq, x.sh_xq_sf, fp8 ? x.f8_s : nullptr };
-    const TokenQuant* quant = fp8 || (small_tiles && !fork && !prequant) ? &tq : nullptr;
+    const TokenQuant* quant = (fp8 && !stage_recording()) || (small_tiles && !fork && !prequant) ? &tq : nullptr;
     cudaError_t err = cudaSuccess;
     if (gemv) { // 2. to 8. of a handful of tokens
         stage_mark(st, STAGE_GATE_UP_GEMM);
@@ -1427,8 +1428,12 @@ qsfi_status qs3_moe_layer_execute(qsfi_context* ctx, const qsfi_moe_plan* plan, 
     if (gemv) {
         y2 = nvfp4 ? wn.y2 : fp8 ? wf.y2 : wb.y2;
     } else if (fp8) {
-        // 4. the tokens, quantised beside the sort; 5./6. grouped GEMMs
+        // 4. the tokens, quantised beside the sort (a profile has them here); 5./6. grouped GEMMs
         stage_mark(st, STAGE_GATHER);
+        if (quant == nullptr)
+            err = launch_fp8_quantize_rows(hidden, d->num_tokens, p.hidden_size, x.f8_x, x.f8_s, st);
+        if (err != cudaSuccess)
+            return set_cuda_error(ctx, err, "FP8 token quantiser");
         status = run_routed_fp8(ctx, p, wf, d->num_tokens, x.f8_x, x.f8_s, static_cast<const uint8_t*>(d->gate_up_weight.data),
                                 static_cast<const float*>(d->gate_up_scale_tiled.data),
                                 static_cast<const uint8_t*>(d->down_weight.data),

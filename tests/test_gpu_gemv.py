@@ -172,3 +172,24 @@ def test_fp8_refusals_do_not_depend_on_the_batch(oracle, h, i, refused):
     with pytest.raises(ops.Qs3Error) as error:
         _run(*case)
     assert error.value.status == capi.STATUS_UNSUPPORTED
+
+
+@pytest.mark.parametrize("fmt,shared", [("nvfp4", True), ("fp8", False), ("bf16", True), ("bf16", False)])
+def test_profile_has_the_stages_apart(oracle, fmt, shared):
+    """A profiled call of a handful of tokens takes the stages one by one, with the same result."""
+    from qs3_b200 import ops
+    ctx = ops.Context()
+    case = (fmt, 2, 512, 256, 24, 4, shared, None)
+    ops.profile_begin(ctx)
+    r = _run(*case)
+    stages = ops.profile_end(ctx)
+    _check(r["out"], _reference(oracle, fmt, r))
+    names = [name for name, _ in stages]
+    # (a shared expert of the experts' size joins the NVFP4 GEMMs)
+    want = ["router_logits_gemm", "router_topk", "route_sort", "gather_quantize", "gate_up_gemm_swiglu", "down_gemm",
+            "shared_expert", "combine"]
+    assert names == [n for n in want if n != "shared_expert" or (shared and fmt == "bf16")]
+    # the sort is in the top-k's launch; bf16 rows of small tiles are read in place, NVFP4 tokens quantised beside the sort
+    empty = {"route_sort"} | ({"gather_quantize"} if fmt != "fp8" else set())
+    assert all(ms > 1e-3 for name, ms in stages if name not in empty)
+    assert r["launches"] > 3
