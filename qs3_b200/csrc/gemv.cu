@@ -677,26 +677,30 @@ cudaError_t launch_instance(const GemvParams& p, const RouterParams* router, con
                           dim3(p.hidden_size / Gv<FMT>::kOut, p.num_tokens), slots * 32, 0, stream, p);
 }
 
-// The time grows with the weights that the slots multiply, again for every slot of one expert; the grouped GEMMs stream an
-// expert once, over five launches, so a skewed router favours them. Layer (hidden, experts top-k, intermediate; tokens:
-// grouped / this, us; of a skewed router in brackets):
+// Where the products win. Their time grows with the weights that the slots multiply, again for every slot of one expert, with
+// the rows of a slot (more of them for the same weights where hidden is small), and with the tokens and experts that every
+// block routes; the grouped GEMMs stream an expert once, over five launches, and are quickest with a skewed router. The cost
+// is in millions of weights; the limits are where, over 125 shapes (hidden 256..4096, 4..512 experts top-1..16, intermediate
+// 128..1536, with and without a shared expert, even and skewed router, 1..16 tokens), the first calls come out slower
+// than they were before these products: of the 1698 taken three are, by 3 to 4 %. By the weights alone, up to 110, 115 and
+// 140 million, and fewer where the experts have several routes each, 78 of 1848 were, by 3 to 56 %
+// (layer of 12 tokens, 128 experts top-8, 256 x 1024, FP8: 23.6 us grouped, 36.7 this; 8 tokens, 512 experts top-10, 2048 x
+// 256, bf16: 37.9 and 54.9; 16 tokens, 128 experts top-4, 512 x 768, NVFP4: 25.7 and 34.0). Layer (hidden, experts top-k,
+// intermediate; tokens: grouped / this, us; of a skewed router in brackets):
 //                              bf16                            nvfp4                          fp8
-//   2048, 8 top-2, 512         8: 31 / 19, 16: 32 / 32         8: 24 / 19, 12: 24 / 25        8: 25 / 18, 16: 26 / 29
-//   512, 16 top-4, 512         8: 22 / 15, 16: 23 / 23         8: 22 / 16, 16: 23 / 27        8: 20 / 17, 16: 21 / 25
-//   2048, 16 top-4, 768        4: 35 / 29, 8: 39 / 51          4: 26 / 20, 8: 27 / 33         4: 25 / 20, 8: 26 / 32
-//   1024, 64 top-6, 512        8: 30 / 28, 10: 40 / 35         8: 26 / 24, 10: 28 / 29        8: 23 / 23, 10: 26 / 29
-//   2048, 32 top-4, 512        4: 31 / 19, 8: 41 / 45          6: 26 / 23, 8: 27 / 26         6: 26 / 21, 8: 27 / 27
-//   2048, 128 top-8, 768       3: 49 / 41 (37 / 33),                                          3: 33 / 29 (30 / 27),
-//                              4: 62 / 55 (39 / 43)                                           4: 43 / 43 (30 / 36)
-//   2048, 512 top-10, 512 + 1  4: 76 / 72 (58 / 56),           3: 36 / 34 (34 / 33),
-//                              5: 80 / 86 (59 / 66)            4: 39 / 42 (36 / 38)
-bool gemv_pays(int fmt, uint64_t routes, uint64_t slots, uint64_t experts, uint64_t hidden, uint64_t inter)
+//   2048, 128 top-8, 768       3: 48 / 42 (39 / 34),                                          3: 35 / 31 (28 / 28),
+//                              4: 59 / 54 (41 / 43)                                           4: 41 / 43 (29 / 37)
+//   2048, 512 top-10, 512 + 1  3: 54 / 55 (49 / 46),           2: 32 / 28 (31 / 27),
+//                              4: 72 / 71 (51 / 55)            3: 34 / 35 (31 / 33)
+struct GemvCost {
+    float rows, slot, token, experts, most; // of a thousand intermediate features of a slot, a slot, a token, a hundred experts
+};
+constexpr GemvCost kGvCost[] = { { 2, 2, 4, 0, 220 }, { 3, 1, 4, 10, 220 }, { 3, 0.5f, 6, 0, 180 } }; // by GemvFormat
+bool gemv_pays(int fmt, uint32_t tokens, uint32_t slots, uint32_t experts, uint32_t hidden, uint32_t inter)
 {
-    const uint64_t millions = slots * 3 * hidden * inter / 1000000;
-    const uint64_t most = routes > 2 * experts ? 30 // every expert several times
-        : 2 * routes > experts                 ? (fmt == GEMV_NVFP4 ? 90 : 75)
-                                               : (fmt == GEMV_NVFP4 ? 110 : fmt == GEMV_FP8 ? 115 : 140);
-    return millions <= most;
+    const GemvCost& c = kGvCost[fmt];
+    const float rows = 1e-3f * static_cast<float>(slots) * static_cast<float>(inter);
+    return rows * (3e-3f * static_cast<float>(hidden) + c.rows) + c.slot * slots + c.token * tokens + c.experts * 0.01f * experts <= c.most;
 }
 
 } // namespace
@@ -710,7 +714,7 @@ bool gemv_supported(int fmt, uint32_t num_tokens, uint32_t top_k, uint32_t num_e
         && (shared_inter == 0 || shared_inter == inter) && router_sort_supported(num_tokens, num_experts, top_k, experts)
         && (fmt == GEMV_BF16 || inter % 128 == 0)
         && (fmt != GEMV_FP8 || (hidden <= 4096 && inter <= 4096)) // (as far as FP8 plans go: larger batches are refused beyond)
-        && gemv_pays(fmt, num_tokens * top_k, num_tokens * (top_k + (shared_inter != 0)), experts, hidden, inter);
+        && gemv_pays(fmt, num_tokens, num_tokens * (top_k + (shared_inter != 0)), num_experts, hidden, inter);
 }
 
 cudaError_t launch_gemv(int fmt, const GemvParams& p, const RouterParams* router, const RouteTables& rt, cudaStream_t stream)
