@@ -522,13 +522,16 @@ bool gemm_dense_bf16_supported(const GemmProblem& g)
 //   a pair of CTAs, 256 x c       6.8 + rounds (1.5 + k blocks (0.15 + 0.00062 c)), a round not under the 3.5 c / 256 that
 //                                 its output takes
 //   split k (gemm_splitk.cu)      bf16 results only: f32 results have their own choice there
+// With beta the first two read and store the output row by row, 1.5 us more, split k along the rows, 0.01 times its rows a rank
+// (127 x 1024 x 512: split 5.8 us, one CTA per tile 8.5; 1500 x 512 x 128: 6.0 and 7.6; over 91 shapes the choice takes 1 %
+// longer than the quickest, without beta over 54 as well).
 // A sum over all of k in one accumulator is off by 2e-6 at k = 2048, a rank's share by less; rounding to bf16 by 2e-3.
 // Before, by the number of 128 x 256 tiles: 300 x 4096 x 4096 27.1 -> 18.0 us, 1200 x 4096 x 4096 46.3 -> 37.6,
 // 800 x 4096 x 2048 26.0 -> 18.0, 200 x 512 x 2048 6.9 -> 5.7, 2000 x 512 x 8192 26.9 -> 23.
 DenseChoice gemm_dense_choice(const GemmProblem& g)
 {
     const uint32_t sms = device_sm_count();
-    const float kb = static_cast<float>(g.k / 64);
+    const float kb = static_cast<float>(g.k / 64), by_rows = g.beta != 0.0f ? 1.5f : 0.0f;
     const auto rounds = [](uint64_t tiles, uint32_t at_once) { return static_cast<float>((tiles + at_once - 1) / at_once); };
     const uint64_t tiles_m = (g.a_rows + kBM - 1) / kBM, pair_m = (g.a_rows + 255) / 256;
     DenseChoice best { DENSE_ONE, kDnBN };
@@ -541,11 +544,11 @@ DenseChoice gemm_dense_choice(const GemmProblem& g)
     };
     for (uint32_t c = kDnBN; c >= 32; c -= 16) {
         const float r = rounds(tiles_m * ((g.n + c - 1) / c), sms);
-        offer(DENSE_ONE, c, 2.9f + 0.0125f * c + r * (1.0f + kb * (1.1f / dense_stages(c) + 0.0003f * c)));
+        offer(DENSE_ONE, c, 2.9f + by_rows + 0.0125f * c + r * (1.0f + kb * (1.1f / dense_stages(c) + 0.0003f * c)));
     }
     for (uint32_t c = 256; c >= 128; c -= 32) {
         const float r = rounds(pair_m * ((g.n + c - 1) / c), sms / 2);
-        offer(DENSE_PAIR, c, 6.8f + r * (1.5f + std::max(kb * (0.15f + 0.00062f * c), 3.5f * c / 256)));
+        offer(DENSE_PAIR, c, 6.8f + by_rows + r * (1.5f + std::max(kb * (0.15f + 0.00062f * c), 3.5f * c / 256)));
     }
     if (g.epilogue == EPI_STORE_BF16)
         for (uint32_t nt : { 64u, 96u, 128u })

@@ -458,7 +458,8 @@ float gemm_splitk_estimate(const GemmProblem& g, uint32_t nt)
         return 1e30f;
     const uint32_t splits = splitk_splits(g, nt), kbs = ((g.k + 63) / 64 + splits - 1) / splits;
     const uint32_t stages = splitk_stages(nt, splitk_tiles(g, nt), splits, 8);
-    return 4.6f + 0.028f * nt + kbs * (1.1f / stages + 0.0003f * nt + 0.01f);
+    const float output = g.beta != 0.0f ? 0.01f * nt / splits : 0.0f;
+    return 4.6f + output + 0.028f * nt + kbs * (1.1f / stages + 0.0003f * nt + 0.01f);
 }
 
 cudaError_t launch_gemm_splitk(const GemmProblem& g, uint32_t rows, cudaStream_t stream, const char** why)

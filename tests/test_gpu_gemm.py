@@ -231,3 +231,10 @@ def test_dense_output_edges(gemm, shape, out_dtype, beta):
     if out_dtype == torch.bfloat16:
         bound += want.abs() * 2.0 ** -8
     assert torch.all((got[:rows, :n].double() - want).abs() <= bound)
+
+
+# short problems whose output is read as well: split over k, where the other kernels would go through the output row by row
+@pytest.mark.parametrize("shape", [(127, 1024, 512, 0), (1500, 512, 128, 8), (257, 512, 250, 7)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_short_dense_problems_with_beta(gemm, shape, out_dtype):
+    test_dense_output_edges(gemm, shape, out_dtype, 0.75)
