@@ -326,7 +326,7 @@ cudaError_t launch_gemm(const GemmProblem& p, cudaStream_t stream, const char** 
 bool gemm_splitk_supported(const GemmProblem& p);
 // `rows` of A per tile, 0: this kernel's own choice.
 cudaError_t launch_gemm_splitk(const GemmProblem& p, uint32_t rows, cudaStream_t stream, const char** why_unsupported);
-float gemm_splitk_estimate(const GemmProblem& p, uint32_t rows); // microseconds, bf16 results
+float gemm_splitk_estimate(const GemmProblem& p, uint32_t rows, uint32_t sms); // microseconds, bf16 results
 // Persistent 128 x 256 kernel for dense bf16 problems with more than 64 rows (gemm_dense.cu).
 bool gemm_dense_bf16_supported(const GemmProblem& p);
 enum DenseKernel : uint32_t { DENSE_ONE, DENSE_PAIR, DENSE_SPLIT };

@@ -530,10 +530,11 @@ bool gemm_dense_bf16_supported(const GemmProblem& g)
 // 800 x 4096 x 2048 26.0 -> 18.0, 200 x 512 x 2048 6.9 -> 5.7, 2000 x 512 x 8192 26.9 -> 23.
 DenseChoice gemm_dense_choice(const GemmProblem& g)
 {
-    const uint32_t sms = device_sm_count();
+    // (32 bits hold the tiles: gemm_dense_bf16_supported; a call of a small problem takes as long on the host as on the device)
+    const uint32_t sms = device_sm_count(), m = static_cast<uint32_t>(g.a_rows);
     const float kb = static_cast<float>(g.k / 64), by_rows = g.beta != 0.0f ? 1.5f : 0.0f;
-    const auto rounds = [](uint64_t tiles, uint32_t at_once) { return static_cast<float>((tiles + at_once - 1) / at_once); };
-    const uint64_t tiles_m = (g.a_rows + kBM - 1) / kBM, pair_m = (g.a_rows + 255) / 256;
+    const auto rounds = [](uint32_t tiles, uint32_t at_once) { return static_cast<float>((tiles + at_once - 1) / at_once); };
+    const uint32_t tiles_m = (m + kBM - 1) / kBM, pair_m = (m + 255) / 256;
     DenseChoice best { DENSE_ONE, kDnBN };
     float least = 1e30f;
     const auto offer = [&](DenseKernel kernel, uint32_t width, float time) {
@@ -552,7 +553,7 @@ DenseChoice gemm_dense_choice(const GemmProblem& g)
     }
     if (g.epilogue == EPI_STORE_BF16)
         for (uint32_t nt : { 64u, 96u, 128u })
-            offer(DENSE_SPLIT, nt, gemm_splitk_estimate(g, nt));
+            offer(DENSE_SPLIT, nt, gemm_splitk_estimate(g, nt, sms));
     return best;
 }
 

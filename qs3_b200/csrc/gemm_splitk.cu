@@ -355,9 +355,9 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
 // eight 0.0136). Two share an SM when there are more tiles than SMs, and when clusters of four or eight would take most of the
 // SMs, since not every one finds its SMs free side by side then (33 x 4096 x 2048, 16 clusters of eight: 0.0133 ms with eight
 // stages, 0.0090 with four; 809 x 4096 x 512, 36 of four: 0.0159 against 0.0118 with fewer tiles).
-uint32_t splitk_stages(uint32_t nt, uint64_t tiles, uint32_t splits, uint32_t kb_per_split)
+uint32_t splitk_stages(uint32_t nt, uint64_t tiles, uint32_t splits, uint32_t kb_per_split, uint64_t sms)
 {
-    const uint64_t ctas = tiles * splits, sms = device_sm_count();
+    const uint64_t ctas = tiles * splits;
     const bool alone = ctas <= (splits < 4 ? sms : splits == 4 ? sms * 7 / 8 : sms * 3 / 4);
     return std::min({ alone ? kSkMaxStages : 4u, kSkRing / (kTileBytes + nt * 128), kb_per_split });
 }
@@ -367,7 +367,7 @@ cudaError_t launch_splitk_instance(const CUtensorMap& mb, const CUtensorMap& ma,
                                    cudaStream_t stream)
 {
     auto kernel = gemm_splitk_kernel<NT, F32, SUM>;
-    sp.stages = splitk_stages(NT, static_cast<uint64_t>(grid.y) * grid.z, grid.x, sp.kb_per_split);
+    sp.stages = splitk_stages(NT, static_cast<uint64_t>(grid.y) * grid.z, grid.x, sp.kb_per_split, device_sm_count());
     const size_t smem = 1024 + SkSmem<NT>::bytes(sp.stages) + 256, most = 1024 + SkSmem<NT>::bytes(SkSmem<NT>::kMostStages) + 256;
     static bool configured[64] = {}; // per instantiation and device
     int dev = 0;
@@ -414,12 +414,12 @@ SkSum splitk_sum(const GemmProblem& g, uint32_t nt)
 
 // As many splits as fit one CTA per SM, two k blocks each at least; none for compensated sums of a short k, which a
 // rounding per rank would leave further off (64 x 512 x 512: 6.4e-8, 5.8e-8 unsplit, on CUDA cores 6.2e-8).
-uint32_t splitk_splits(const GemmProblem& g, uint32_t nt)
+uint32_t splitk_splits(const GemmProblem& g, uint32_t nt, uint64_t sms)
 {
     const uint64_t tiles = splitk_tiles(g, nt);
     const uint32_t k_blocks = (g.k + 63) / 64;
     uint32_t splits = 1;
-    while (splits < kSkMaxSplits && 2 * splits * tiles <= device_sm_count() && 2 * (2 * splits) <= k_blocks
+    while (splits < kSkMaxSplits && 2 * splits * tiles <= sms && 2 * (2 * splits) <= k_blocks
            && (splitk_sum(g, nt) != SUM_COMPENSATED || k_blocks > 8))
         splits *= 2;
     return splits;
@@ -452,14 +452,14 @@ bool gemm_splitk_supported(const GemmProblem& g)
 }
 
 // 200 x 4096 x 2048, 64 rows a tile: 11.8 us both; 130 x 4096 x 2048, 96 rows: 11.1, measured 10.5.
-float gemm_splitk_estimate(const GemmProblem& g, uint32_t nt)
+float gemm_splitk_estimate(const GemmProblem& g, uint32_t nt, uint32_t sms)
 {
-    if (splitk_tiles(g, nt) > device_sm_count())
+    const uint64_t tiles = splitk_tiles(g, nt);
+    if (tiles > sms)
         return 1e30f;
-    const uint32_t splits = splitk_splits(g, nt), kbs = ((g.k + 63) / 64 + splits - 1) / splits;
-    const uint32_t stages = splitk_stages(nt, splitk_tiles(g, nt), splits, 8);
+    const uint32_t splits = splitk_splits(g, nt, sms), kbs = ((g.k + 63) / 64 + splits - 1) / splits;
     const float output = g.beta != 0.0f ? 0.01f * nt / splits : 0.0f;
-    return 4.6f + output + 0.028f * nt + kbs * (1.1f / stages + 0.0003f * nt + 0.01f);
+    return 4.6f + output + 0.028f * nt + kbs * (1.1f / splitk_stages(nt, tiles, splits, 8, sms) + 0.0003f * nt + 0.01f);
 }
 
 cudaError_t launch_gemm_splitk(const GemmProblem& g, uint32_t rows, cudaStream_t stream, const char** why)
@@ -476,7 +476,7 @@ cudaError_t launch_gemm_splitk(const GemmProblem& g, uint32_t rows, cudaStream_t
     sp.err = device_error_word();
     const uint32_t nt = rows != 0 ? rows : splitk_choice(g);
     const uint64_t tiles = splitk_tiles(g, nt);
-    const uint32_t splits = splitk_splits(g, nt);
+    const uint32_t splits = splitk_splits(g, nt, device_sm_count());
     sp.kb_per_split = (sp.k_blocks + splits - 1) / splits;
     CUtensorMap mb, ma;
     if (!make_operand_map(&mb, false, g.b, g.k, g.n, g.b_pitch_bytes, 128)
