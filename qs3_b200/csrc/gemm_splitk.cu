@@ -69,6 +69,10 @@ template <int NT> struct SkSmem {
 // How the products of a row are summed (see above).
 enum SkSum { SUM_CHAIN = 0, SUM_SHORT_CHAINS = 1, SUM_COMPENSATED = 2 };
 
+// Stages of the ring, 0: as many as splitk_stages() says. Of f32 results of more than 64 rows a constant: 130 x 2048 x 1536 6.7
+// us, with a number that only the launch knows 7.3, and 1021 x 7168 x 256 with eight 15.2 instead of 14.8.
+template <bool F32, int SUM> constexpr uint32_t kSkStages = F32 && SUM != SUM_COMPENSATED ? 4 : 0;
+
 // Tensor-memory buffers: short chains two accumulators per k block, in turn; else one accumulator for all of k.
 template <int NT, int SUM> struct SkTmem {
     static constexpr uint32_t kBufs = SUM == SUM_CHAIN ? 1 : NT <= 32 ? 4 : 2;
@@ -116,10 +120,12 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
     constexpr uint32_t kTmemCols = SkTmem<NT, SUM>::kCols, kBufs = SkTmem<NT, SUM>::kBufs;
     constexpr uint32_t kAdders = SkTmem<NT, SUM>::kAdders, kMine = SkTmem<NT, SUM>::kMine;
 
+    const uint32_t stages = kSkStages<F32, SUM> != 0 ? kSkStages<F32, SUM> : p.stages;
+
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
     float* part = reinterpret_cast<float*>(smem); // [NT][kSkPitch], after the ring
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + SkSmem<NT>::bytes(p.stages));
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + SkSmem<NT>::bytes(stages));
     uint64_t* empty_bar = full_bar + kSkMaxStages;
     uint64_t* acc_full = empty_bar + kSkMaxStages;
     uint64_t* acc_empty = acc_full + kBufs; // short chains
@@ -132,7 +138,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
     const uint32_t kb0 = min(rank * p.kb_per_split, p.k_blocks), kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
 
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < p.stages; ++s) {
+        for (uint32_t s = 0; s < stages; ++s) {
             mbar_init(&full_bar[s], 1);
             mbar_init(&empty_bar[s], 1);
         }
@@ -169,7 +175,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
                 const int c0 = static_cast<int>(kb0 + i) * 64;
                 tma_load_2d(sb, &map_b, &full_bar[s], c0, static_cast<int>(n0));
                 tma_load_2d(sb + kTileBytes, &map_a, &full_bar[s], c0, static_cast<int>(m0));
-                if (++s == p.stages) {
+                if (++s == stages) {
                     s = 0;
                     ph ^= 1;
                 }
@@ -203,7 +209,7 @@ gemm_splitk_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_const
                 tc_commit(&empty_bar[s]);
                 if (SUM != SUM_CHAIN)
                     tc_commit(&acc_full[b]);
-                if (++s == p.stages) {
+                if (++s == stages) {
                     s = 0;
                     ph ^= 1;
                 }
@@ -367,7 +373,9 @@ cudaError_t launch_splitk_instance(const CUtensorMap& mb, const CUtensorMap& ma,
                                    cudaStream_t stream)
 {
     auto kernel = gemm_splitk_kernel<NT, F32, SUM>;
-    sp.stages = splitk_stages(NT, static_cast<uint64_t>(grid.y) * grid.z, grid.x, sp.kb_per_split, device_sm_count());
+    sp.stages = kSkStages<F32, SUM> != 0
+        ? kSkStages<F32, SUM>
+        : splitk_stages(NT, static_cast<uint64_t>(grid.y) * grid.z, grid.x, sp.kb_per_split, device_sm_count());
     const size_t smem = 1024 + SkSmem<NT>::bytes(sp.stages) + 256, most = 1024 + SkSmem<NT>::bytes(SkSmem<NT>::kMostStages) + 256;
     static bool configured[64] = {}; // per instantiation and device
     int dev = 0;
