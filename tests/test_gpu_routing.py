@@ -201,3 +201,77 @@ def test_router_and_sort_of_a_small_batch(ops, oracle, t, e, k, local):
     tables = [to_np(x) for x in plan.routing_tables(ws, t)]
     for g, r in zip(tables, oracle.route_sort(to_np(ids), to_np(w), off, le)):
         assert np.array_equal(g, r)
+
+
+def _tile_tables(counts, choose):
+    """Host restatement of the padded segments and tiles that the NVFP4 GEMMs read: 128-row tiles and their pairs, or, where
+    the sort may choose and they come out cheaper, 64-row tiles."""
+    tiles = lambda h: (counts + h - 1) // h
+    small = choose and 5 * tiles(64).sum() < 7 * tiles(128).sum()
+    h = 64 if small else 128
+    pad = np.concatenate([[0], np.cumsum(tiles(h) * h)])
+    table = [(e, pad[e] + m * h, min(h, n - m * h)) for e, n in enumerate(counts) for m in range((n + h - 1) // h)]
+    pairs = [] if small else [(e, pad[e] + m * 256, min(256, n - m * 256)) for e, n in enumerate(counts) for m in range((n + 127) // 256)]
+    # (an expert's odd last tile; the singles fill the table from its end)
+    singles = [] if small else [(e, pad[e] + (n - 1) // 128 * 128, (n - 1) % 128 + 1)
+                                for e, n in enumerate(counts) if (n + 127) // 128 % 2]
+    return small, pad, table, pairs, singles
+
+
+# the two-launch sort at the ends of its range, for the tables of the NVFP4 GEMMs: whole chunks and one more or less, one
+# expert's tiles beside another block's, both tile heights where the sort chooses, none where it may not (few routes; experts
+# with more than 80 routes on average), experts held by another rank
+@pytest.mark.parametrize("t,k,e,local,skew", [
+    (2400, 10, 1023, None, False), (2400, 10, 1024, None, True), (2560, 10, 1024, None, False), (321, 8, 9, None, False),
+    (1024, 3, 8, None, False), (513, 6, 64, None, False), (513, 6, 64, None, True), (700, 6, 64, (5, 50), False),
+    (1025, 6, 257, None, False), (6000, 3, 200, (100, 100), False)])
+def test_tile_tables_of_a_large_batch(ops, oracle, t, k, e, local, skew):
+    off, le = local or (0, e)
+    rng = np.random.default_rng(t + e)
+    ids = rng.integers(0, e, size=(t, k), dtype=np.int32)
+    if skew: # to a sixteenth of the experts
+        ids = (off + ids % (le // 16)).astype(np.int32)
+    w = rng.random((t, k), dtype=np.float32)
+    h = i = 256
+    ctx = ops.Context()
+    plan = ops.MoePlan(ctx, ops.MoePlanConfig(max_num_tokens=t, hidden_size=h, intermediate_size=i, num_experts=e, top_k=k,
+                                              local_expert_offset=off, local_num_experts=le,
+                                              backend=ops.capi.MOE_BACKEND_NVFP4))
+    ws = torch.full((plan.workspace_size(t),), 0xff, dtype=torch.uint8, device="cuda")
+    zeros = lambda *shape: torch.zeros(shape, dtype=torch.uint8, device="cuda")
+    ops.moe_execute_nvfp4(plan, zeros(t, h // 2), zeros(t, h // 16), to_dev(ids), to_dev(w), zeros(le, 2 * i, h // 2),
+                          zeros(le, 2 * i, h // 16), zeros(le, h, i // 2), zeros(le, h, i // 16),
+                          torch.empty((t, h), dtype=torch.bfloat16, device="cuda"), ws)
+    torch.cuda.synchronize()
+    assert ctx.read_device_error() == 0
+    # the tables' places, in the order and alignment of the workspace
+    routes = t * k
+    assert routes > 2560 and routes > 22 * le    # two launches, tiles of 128 rows or a choice
+    up = lambda v, a: (v + a - 1) // a * a
+    seg, choose = min(routes, le), routes <= 80 * le
+    max_tiles = (up(routes, 128) + seg * 128) // 128
+    room = max(max_tiles, up(routes if choose else 80 * le, 64) // 64 + seg)
+    sizes = [le, le + 1, le + 1, routes, routes, routes, routes, room, room, room, 1, 1, max_tiles, max_tiles, max_tiles, 2]
+    at, tables = 0, []
+    for n in sizes:
+        at = up(at, 256)
+        tables.append(to_np(ws[at:at + 4 * n].view(torch.int32)))
+        at += 4 * n
+    counts, indptr, pad, rows, prows, tokens, _, tile_e, tile_r, tile_n, total, alt, pair_e, pair_r, pair_n, pair_counts = tables
+    want = oracle.route_sort(ids, w, off, le)
+    assert np.array_equal(counts, want[0]) and np.array_equal(indptr, want[1]) and np.array_equal(rows, want[2])
+    small, want_pad, table, pairs, singles = _tile_tables(want[0].astype(np.int64), choose)
+    assert small == (choose and not skew)          # the case means both heights to occur
+    assert np.array_equal(pad, want_pad)
+    local_ids = ids.ravel() - off
+    held = (local_ids >= 0) & (local_ids < le)
+    assert np.array_equal(prows[held], (rows - np.asarray(want[1])[local_ids * held] + want_pad[local_ids * held])[held])
+    assert np.all(prows[~held] == -1)
+    assert np.array_equal(np.stack([tile_e, tile_r, tile_n], 1)[:len(table)], np.array(table).reshape(-1, 3))
+    assert total[0] == (0 if small else len(table))
+    if choose:
+        assert alt[0] == (len(table) if small else 0)
+    assert pair_counts.tolist() == [len(pairs), len(singles)]
+    got = np.stack([pair_e, pair_r, pair_n], 1)
+    assert np.array_equal(got[:len(pairs)], np.array(pairs).reshape(-1, 3))
+    assert np.array_equal(got[::-1][:len(singles)], np.array(singles).reshape(-1, 3))
