@@ -15,8 +15,10 @@
 //   warps       0-15 promotion and epilogue (lane quadrant warp % 4, column quarter warp / 4), 16 producer, 17 MMA, 18-19
 //               note writers: they follow the tables and fetch the scales of the next unit
 //
-// Bound by operand delivery: a k block is 48 KB, which an SM takes in at 75 GB/s, 0.64 us, against 0.35 (690 cycles) for
-// its four MMAs. 4096 tokens x 128 experts top-8 (hidden 2048, intermediate 768): gate_up 0.800 -> 0.156 ms, down 0.238
+// Bound by the hand-over of the two buffers: products, commit, the promotion's wait and the way back take a buffer 1.3 us,
+// 0.65 a k block, of which the four MMAs are 0.35 (690 cycles). 4096 tokens, gate_up and down: 164 and 90 us; without the
+// loads (48 KB a k block) 157 and 82, without the promotion 148 and 86, without both still 136 and 68. With few rows an expert
+// the weights bound it: 1024 tokens 91 and 51, without the loads 72 and 38. 4096 tokens x 128 experts top-8 (hidden 2048, intermediate 768): gate_up 0.800 -> 0.156 ms, down 0.238
 // -> 0.087 ms against the decode kernel on 32-row tiles, which streamed every weight through shared memory once per 32
 // rows. With the scales and tables fetched between the units by the promotion warps, and whole token tiles moved for a
 // few rows: layer of 1024 tokens 0.200 -> 0.177 ms, 2048 0.257 -> 0.222 (4096: 0.377 -> 0.366). Eight promotion warps

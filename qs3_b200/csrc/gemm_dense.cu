@@ -514,8 +514,8 @@ bool gemm_dense_bf16_supported(const GemmProblem& g)
 }
 
 // What computes a dense problem of more than 64 rows: the kernel, and the columns (rows of A for the split one) of a tile, by
-// an estimate of its time in microseconds. Fitted to 72..3001 rows, k 512..4096, 512..8192 features, operands from HBM, which it
-// meets within a tenth; what it has to get right is the order. A CTA's operands come through a ring that holds 192 KB, a trip
+// an estimate of its time in microseconds. Fitted to 72..3001 rows, k 512..4096, 512..8192 features, operands from HBM; with
+// operands in L2 the times are 0.7 to 1.0 of it, for shorter k 0.65 to 1.35. What it has to get right is the order. A CTA's operands come through a ring that holds 192 KB, a trip
 // of 1.1 us, so a k block takes 1.1 us / stages however few SMs work: narrow tiles are quick by themselves, wide ones move
 // fewer bytes, and the rounds of the SMs decide between them.
 //   one CTA per tile of 128 x c   2.9 + c / 80 + rounds (1 + k blocks (1.1 / stages + 0.0003 c))
@@ -525,8 +525,9 @@ bool gemm_dense_bf16_supported(const GemmProblem& g)
 // With beta the first two read and store the output row by row, 1.5 us more, split k along the rows, 0.01 times its rows a rank
 // (127 x 1024 x 512: split 5.8 us, one CTA per tile 8.5; 1500 x 512 x 128: 6.0 and 7.6; over 91 shapes the choice takes 1 %
 // longer than the quickest, without beta over 54 as well).
-// A sum over all of k in one accumulator is off by 2e-6 at k = 2048, a rank's share by less; rounding to bf16 by 2e-3.
-// Before, by the number of 128 x 256 tiles: 300 x 4096 x 4096 27.1 -> 18.0 us, 1200 x 4096 x 4096 46.3 -> 37.6,
+// A sum over all of k in one accumulator is off by 2e-6 at k = 2048, a rank's share by less; rounding to bf16 by 2e-3, which
+// is all that 106 shapes show against 64 bits, whichever kernel computes them (within 3e-6 of that error).
+// Before, by the number of 128 x 256 tiles: 300 x 4096 x 4096 25.9 -> 16.8 us, 1200 x 4096 x 4096 46.3 -> 37.6,
 // 800 x 4096 x 2048 26.0 -> 18.0, 200 x 512 x 2048 6.9 -> 5.7, 2000 x 512 x 8192 26.9 -> 23.
 DenseChoice gemm_dense_choice(const GemmProblem& g)
 {

@@ -19,8 +19,8 @@
 // Two shapes (PairShape):
 //
 //   gated (gate_up + SwiGLU + NVFP4 re-quantisation): column tiles of 256 accumulator columns (128
-//     gate + 128 up features), 256 x 256 instructions, which reach a ~1.33x higher tensor-pipe ceiling
-//     than 128-column ones (6.6 vs 5.0 PFLOP/s measured with the issue-loop probe). A 256-column f32
+//     gate + 128 up features), 256 x 256 instructions, which reach a ~1.26x higher tensor-pipe ceiling
+//     than 128-column ones (6.6 vs 5.2 PFLOP/s measured with the issue-loop probe). A 256-column f32
 //     accumulator plus resident scales leaves no room in the 512 tensor-memory columns for a second
 //     one, so the epilogue warps first DRAIN the accumulator into registers (128 values per thread),
 //     hand it back to the MMA thread, and only then run SwiGLU + quantisation from registers while
@@ -77,8 +77,8 @@ constexpr uint32_t kPgTmemCols = 512;
 template <bool GATED> struct PairShape {
     static constexpr uint32_t kBN = GATED ? 256u : 128u;             // accumulator columns per column tile
     static constexpr uint32_t kAccs = GATED ? 1u : 2u;               // accumulators in tensor memory
-    // k blocks (256 elements) per ring stage. Every tcgen05 instruction and every barrier wait costs the one
-    // issuing thread 50-100 cycles; with 128-column instructions (147 cycles of tensor pipe each) a stage of
+    // k blocks (256 elements) per ring stage. Every commit and every barrier wait costs the one issuing thread 50-100
+    // cycles, every tcgen05 instruction 40 to 50 (100 in a branch on the lane's number, as it was then); with 128-column instructions (147 cycles of tensor pipe each) a stage of
     // four instructions plus its commits and waits takes that thread longer than the pipe needs, so plain
     // stages carry two k blocks (measured: down GEMM 0.150 -> 0.134 ms).
     static constexpr uint32_t kKbs = GATED ? 1u : 2u;
@@ -207,8 +207,8 @@ __device__ __forceinline__ void commit_pair(uint32_t bar_cluster_addr)
 }
 
 // One commit that arrives on the barrier at the same shared-memory offset in BOTH CTAs of the pair
-// (the multicast here is of the barrier arrival, not of a load): the issuing thread pays 50-100
-// cycles per tcgen05 instruction, so one commit instead of two per ring stage matters.
+// (the multicast here is of the barrier arrival, not of a load): the issuing thread pays about 60 cycles
+// per commit, so one instead of two per ring stage matters.
 __device__ __forceinline__ void commit_both(const void* local_bar)
 {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::
@@ -600,7 +600,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
     } else if (warp == 11) {
         // ------------------------------------------- second scale copier --
-        // tcgen05.cp costs its issuing thread 50-70 cycles apiece; the eight copies of a stage's B scales
+        // tcgen05.cp cost its issuing thread 50-70 cycles apiece (in a branch on the lane's number); the eight copies of a stage's B scales
         // (plus four of A scales in a unit's first column tile) from one thread take longer than the
         // stage's four MMAs, so the two 128-row halves of the B scales have a copier thread each.
         if (kPgBN == 256 && rank == 0 && elect_one()) {

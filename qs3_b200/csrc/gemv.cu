@@ -3,10 +3,10 @@
 // itself: with so few rows there is next to nothing to share, and what such a call waits for is the chain of dependent
 // launches and table loads.
 //
-//   gate_up  persistent, two blocks per SM. Block 0 routes all tokens and sorts the routes into the tables (nothing
-//            below waits for those); every other block stages and quantises the tokens before the predecessor ends, routes
-//            them itself, a warp per token, and takes units of 32 features of one slot, the shared expert's first, which
-//            do not wait
+//   gate_up  persistent, two blocks per SM. Block 0 routes all tokens, writes ids and weights and sorts the routes into the
+//            tables; every other block stages and quantises the tokens before the predecessor ends, routes them itself, a
+//            warp per token, and takes units of 32 features of one slot, the shared expert's first, which do not wait.
+//            (The down launch waits for all of them, block 0 among them, whose ids it reads; a combine reads its tables)
 //   down     blocks (features, tokens), a warp per slot, then the weighted sum over the slots in shared memory, in
 //            ascending order as the combine kernel adds them
 //
@@ -16,9 +16,10 @@
 //   bf16     a lane takes 16 bytes of four rows at a time, f32
 //
 // Bound by latency for one token (three launches; routing, expert, weights, table after table), then by the weights, which
-// arrive at 3 to 5 TB/s. Layer of one token over 512 experts top-10 + shared, NVFP4: 0.0366 -> 0.0225 ms; 128 experts top-8,
-// FP8: 0.0290 -> 0.0180, bf16 0.0337 -> 0.0181; 16 tokens over 8 experts, 256 x 128, bf16: 0.0193 -> 0.0105. Routing in every
-// block of a grid (features, tokens) instead: 4 tokens NVFP4 0.052 against 0.043. Decoding e2m1 by byte permutation into
+// arrive at 3 to 5 TB/s. Layer of one token over 512 experts top-10 + shared, NVFP4: 0.0368 -> 0.0229 ms a call, 0.0335 ->
+// 0.0213 replayed from a graph, as are the following; 128 experts top-8, FP8: 0.0279 -> 0.0201, bf16 0.0351 -> 0.0215; 16
+// tokens over 8 experts, 256 x 128, bf16: 0.0199 -> 0.0121 a call. Routing in every block of a grid (features, tokens)
+// instead: 4 tokens NVFP4 0.052 against 0.043. Decoding e2m1 by byte permutation into
 // e4m3 for mma.sync 0.0278, into f16 0.0265 against 0.0225 with the conversion instruction; e4m3 into f16 by shifts for
 // mma.sync m16n8k16: FP8 0.0231 against 0.0180.
 #include "nvfp4.cuh"

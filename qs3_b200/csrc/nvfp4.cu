@@ -16,9 +16,11 @@ namespace {
 // Weight quantisation in ONE launch: a cluster of kQwCluster blocks per expert finds the expert's amax
 // (pass 1, exchanged through distributed shared memory) and then quantises it (pass 2, whose reads come
 // from L2: about seventeen experts are in flight, 70 MB for 4-MB gate_up experts, against 126 MB of L2).
-// Bound by HBM: 2 bytes in, 0.63 bytes out per weight. Separate amax / finish / quantise kernels read the
+// 2 bytes in, 0.63 bytes out per weight; bound by its two passes taking turns: all clusters read HBM first, then L2 and
+// compute, and clusters of 16 leave SMs out (active for 83 % of the busiest one's cycles, some for none). Of the rest half the
+// issue slots are taken, 26 of 64 warps resident, HBM at 38 %. Separate amax / finish / quantise kernels read the
 // weights twice from HBM and sent every warp's amax to one address per expert; 64 experts of 1024 x 2048:
-// 0.453 -> 0.102 ms (3.5 TB/s), of which the arithmetic of pass 2 is about half.
+// 0.453 -> 0.108 ms (3.3 TB/s); half the arithmetic of pass 2 changed nothing.
 constexpr uint32_t kQwCluster = 16;
 constexpr uint32_t kQwThreads = 512;
 constexpr uint32_t kQwChunk = 512;   // k elements of one unit of pass 2: a 16-element block per lane

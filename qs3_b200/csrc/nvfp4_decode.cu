@@ -32,7 +32,8 @@
 //
 // Bound by HBM: hit experts * weight bytes. 128 tokens, 512 experts top-10 (471 hit): gate_up 0.112 -> 0.092 ms
 // (6.0 TB/s), down 0.055 -> 0.050; 1021 tokens: gate_up 0.150 -> 0.110, down 0.110 -> 0.058 ms against 128-row tiles. Since
-// then, by shorter panel loaders and issue from elected lanes: layer of 128 tokens 0.177 -> 0.162, of 1021 0.222 -> 0.206.
+// then, by shorter panel loaders and issue from elected lanes, replayed from a graph in turn on one board (others take up to 4 %
+// longer): layer of 128 tokens 0.177 -> 0.162, of 1021 0.222 -> 0.206.
 #include "common.cuh"
 #include "nvfp4.cuh"
 #include "tcgen05.cuh"

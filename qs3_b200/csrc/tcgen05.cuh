@@ -71,7 +71,7 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p)
 // commits branch on this, not on the lane's number: their operands live in uniform registers, and a branch of which the
 // compiler cannot tell that one thread takes it costs more of them (products of 128 x 64 x 16 with a commit every four: 110
 // cycles apiece in a branch on the lane's number, 64 here, of which the tensor core needs 49). NVFP4 layer, 8192 tokens of a
-// skewed router: 0.446 -> 0.416 ms; 64 tokens 0.138 -> 0.130; FP8 64 tokens 0.119 -> 0.116; bf16 33 tokens 0.179 -> 0.175.
+// skewed router, replayed from a graph in turn on one board (others take up to 7 % longer): 0.446 -> 0.416 ms; 64 tokens 0.138 -> 0.130; FP8 64 tokens 0.119 -> 0.116; bf16 33 tokens 0.179 -> 0.175.
 // Where lanes load parts of a tile each, a loop of one elected lane takes longer (2048 bf16 tokens 0.587 -> 0.970 ms).
 __device__ __forceinline__ bool elect_one()
 {
